@@ -138,6 +138,25 @@ def load() -> C.CDLL:
 lib = load()
 
 
+def load_native():
+    """The CPython module under the per-token launchers (csrc/python/native.cpp), bound to the library loaded above."""
+    import importlib.util
+
+    import torch  # noqa: F401  (its shared objects must be in the process first)
+
+    path = Path(__file__).resolve().parent / "lib" / "_native.so"
+    if not path.exists():
+        raise ImportError(f"{path} is missing: build it with `python -m miinfer_b200.build`")
+    spec = importlib.util.spec_from_file_location("_native", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES})
+    return module
+
+
+native = load_native()
+
+
 class B200KvError(RuntimeError):
     def __init__(self, status: int, where: str):
         self.status = status

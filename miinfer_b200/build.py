@@ -1,8 +1,9 @@
 """Builds the CUDA library (sm_100a) in-tree with nvcc.
 
 `python -m miinfer_b200.build` compiles miinfer_b200/csrc/*.cu into
-miinfer_b200/lib/libb200kv.so.  There is no JIT and no fallback: the Python
-mirror loads exactly this file and fails loudly when it is missing.
+miinfer_b200/lib/libb200kv.so, and csrc/python/native.cpp (the CPython module under the
+Python mirror's launchers) into miinfer_b200/lib/_native.so.  There is no JIT and no fallback: the Python
+mirror loads exactly these files and fails loudly when one is missing.
 """
 from __future__ import annotations
 
@@ -17,6 +18,8 @@ CSRC = ROOT / "csrc"
 LIB_DIR = ROOT / "lib"
 LIB_PATH = LIB_DIR / "libb200kv.so"
 INCLUDE = ROOT.parent / "include"
+NATIVE_SRC = CSRC / "python" / "native.cpp"
+NATIVE_PATH = LIB_DIR / "_native.so"     # the CPython module under the Python mirror's launchers
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -38,10 +41,22 @@ def sources() -> list[Path]:
 
 
 def needs_build() -> bool:
-    if not LIB_PATH.exists():
+    if not LIB_PATH.exists() or not NATIVE_PATH.exists():
         return True
-    newest = max(p.stat().st_mtime for p in list(CSRC.glob("*")) + [INCLUDE / "b200kv.h"])
-    return newest > LIB_PATH.stat().st_mtime
+    newest = max(p.stat().st_mtime for p in list(CSRC.glob("*")) + [NATIVE_SRC, INCLUDE / "b200kv.h"])
+    return newest > min(LIB_PATH.stat().st_mtime, NATIVE_PATH.stat().st_mtime)
+
+
+def native_command() -> list[str]:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f"-I{INCLUDE}", *[f"-isystem{p}" for p in [*include_paths(), sysconfig.get_paths()["include"], str(cuda)]], str(NATIVE_SRC),
+            "-o", str(NATIVE_PATH), *[f"-L{p}" for p in library_paths()], "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ltorch"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -60,8 +75,15 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             raise RuntimeError(f"nvcc failed for {src.name}:\n{res.stdout}\n{res.stderr}")
         return obj, res.stderr
 
+    def compile_native() -> None:
+        res = subprocess.run(native_command(), capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"g++ failed for {NATIVE_SRC.name}:\n{res.stdout}\n{res.stderr}")
+
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        native = pool.submit(compile_native)
         results = list(pool.map(compile_one, sources()))
+        native.result()
     log = "\n".join(f"== {obj.name}\n{err}" for obj, err in results)
     (obj_dir / "ptxas.log").write_text(log)
     if verbose:

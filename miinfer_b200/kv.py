@@ -15,7 +15,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import B200KvError, PoolCounters, ReuseOptions, ReuseStats, View, check, lib
+from ._lib import B200KvError, PoolCounters, ReuseOptions, ReuseStats, View, check, lib, native
 
 __all__ = [
     "KvCacheQuantMode", "RopeMode", "AttentionKvCacheView", "AttentionLayerKvCacheStorage",
@@ -207,11 +207,10 @@ def launch_kv_store_quant(view: View, key: torch.Tensor, value: torch.Tensor, k_
 
     key/value: [token][kv_heads*head_dim] fp16 or fp32; the cache planes and
     quant mode travel in `view`."""
-    if key.dtype != value.dtype:
-        raise ValueError("key and value must share a dtype")
-    check(lib.b200kv_append(C.byref(view), _ptr(key), _ptr(value), _dtype(key), _ptr(k_norm_weight), int(rope_mode),
-                            theta, epsilon, token_count, base_position, _ptr(prefill_state), _ptr(decode_state),
-                            _stream(stream)), "b200kv_append")
+    rc = native.append(view, key, value, k_norm_weight, rope_mode, theta, epsilon, token_count, base_position, prefill_state,
+                       decode_state, stream)
+    if rc:
+        check(rc, "b200kv_append")
 
 
 def launch_q_split_norm_rope(qfull: torch.Tensor, q_norm_weight: Optional[torch.Tensor], query: torch.Tensor,
@@ -221,9 +220,10 @@ def launch_q_split_norm_rope(qfull: torch.Tensor, q_norm_weight: Optional[torch.
                              stream: Optional[torch.cuda.Stream] = None) -> None:
     """launch_qwen35_decoupled_q_split_norm_rope_batch / launch_qwen35_fused_q_split_norm_rope_dynamic
     (qwen3_gpu_primitives.hpp:869-881, 934-938): qfull [token][heads][q | gate] -> query, gate [token][heads][d]."""
-    check(lib.b200kv_q_split_norm_rope(_ptr(qfull), _dtype(qfull), _ptr(q_norm_weight), _ptr(query), _dtype(query), _ptr(gate),
-                                       token_count, base_position, heads, head_dim, int(rope_mode), theta, epsilon,
-                                       _ptr(prefill_state), _ptr(decode_state), _stream(stream)), "b200kv_q_split_norm_rope")
+    rc = native.q_split_norm_rope(qfull, q_norm_weight, query, gate, token_count, base_position, heads, head_dim, rope_mode, theta,
+                                  epsilon, prefill_state, decode_state, stream)
+    if rc:
+        check(rc, "b200kv_q_split_norm_rope")
 
 
 def launch_decode_state_advance(state: torch.Tensor, token_output: torch.Tensor, stream: Optional[torch.cuda.Stream] = None) -> None:
@@ -240,10 +240,10 @@ def launch_decode_attention_quant(view: View, q: torch.Tensor, *, query_heads: i
                                   stream: Optional[torch.cuda.Stream] = None) -> None:
     """launch_qwen35_tiled_online_attention_quant_dynamic (qwen3_gpu_primitives.hpp:719-739).
     gated_output_q8: uint8 tensor of query_heads * head_dim / 32 Q8_1 blocks (36 bytes each), see `q8_1_blocks`."""
-    check(lib.b200kv_decode_attn(C.byref(view), _ptr(q), _dtype(q), _ptr(gate), _ptr(output), _ptr(gated_output), _ptr(gated_output_q8),
-                                 query_heads, scale, cache_length, _ptr(decode_state),
-                                 _ptr(workspace),
-                                 workspace.numel(), num_splits, _stream(stream)), "b200kv_decode_attn")
+    rc = native.decode_attn(view, q, gate, output, gated_output, gated_output_q8, query_heads, scale, cache_length, decode_state,
+                            workspace, num_splits, stream)
+    if rc:
+        check(rc, "b200kv_decode_attn")
 
 
 def launch_decode_step(view: View, key: torch.Tensor, value: torch.Tensor, q: torch.Tensor, *, query_heads: int, scale: float,
@@ -255,14 +255,10 @@ def launch_decode_step(view: View, key: torch.Tensor, value: torch.Tensor, q: to
                        stream: Optional[torch.cuda.Stream] = None) -> None:
     """Append one token and attend in one launch (b200kv_decode_step): the fused form of the store + decode-attention
     call pair of src/prefill_v2/attention_layer.cpp:599-632."""
-    if key.dtype != value.dtype:
-        raise ValueError("key and value must share a dtype")
-    check(lib.b200kv_decode_step(C.byref(view), _ptr(key), _ptr(value), _dtype(key), _ptr(k_norm_weight), int(rope_mode), theta,
-                                 epsilon, _ptr(q), _dtype(q), _ptr(gate), _ptr(output), _ptr(gated_output), _ptr(gated_output_q8),
-                                 query_heads, scale,
-                                 position, _ptr(decode_state), _ptr(workspace),
-                                 workspace.numel(), num_splits, _stream(stream)),
-          "b200kv_decode_step")
+    rc = native.decode_step(view, key, value, k_norm_weight, rope_mode, theta, epsilon, q, gate, output, gated_output, gated_output_q8,
+                            query_heads, scale, position, decode_state, workspace, num_splits, stream)
+    if rc:
+        check(rc, "b200kv_decode_step")
 
 
 def launch_decode_attention_batched(views, view_table: torch.Tensor, lengths: torch.Tensor, max_length: int,
@@ -273,14 +269,11 @@ def launch_decode_attention_batched(views, view_table: torch.Tensor, lengths: to
     """One decode step for many sessions in one launch (b200kv_decode_attn_batched).
 
     views: sequence of View, or None to reuse the table filled by an earlier call."""
-    sessions = int(lengths.numel())
-    arr = None
-    if views is not None:
-        arr = (View * sessions)(*views)
-    check(lib.b200kv_decode_attn_batched(arr, _ptr(view_table), _ptr(lengths), sessions, max_length, _ptr(q), _dtype(q),
-                                         _ptr(gate), _ptr(output), _ptr(gated_output), query_heads, scale,
-                                         _ptr(workspace), workspace.numel(), num_splits, _stream(stream)),
-          "b200kv_decode_attn_batched")
+    arr = None if views is None else (View * int(lengths.numel()))(*views)
+    rc = native.decode_attn_batched(arr, view_table, lengths, max_length, q, gate, output, gated_output, query_heads, scale, workspace,
+                                    num_splits, stream)
+    if rc:
+        check(rc, "b200kv_decode_attn_batched")
 
 
 def launch_decode_partials(view: View, q: torch.Tensor, *, query_heads: int, scale: float, range_begin: int,
@@ -430,10 +423,10 @@ def launch_suffix_attention_quant(view: View, q: torch.Tensor, gate: Optional[to
                                   stream: Optional[torch.cuda.Stream] = None) -> None:
     """launch_qwen35_splitk_suffix_attention_quant (qwen3_gpu_primitives.hpp:670-692).  `prepared_rows`: cache positions
     whose fp16 copy `prepare_suffix_attention` has already put into this workspace."""
-    check(lib.b200kv_prefill_attn_prepared(C.byref(view), _ptr(q), _dtype(q), _ptr(gate), _ptr(gated_output), token_count,
-                                           base_position, query_heads, scale, _ptr(prefill_state), _ptr(workspace),
-                                           0 if workspace is None else workspace.numel(), prepared_rows, _stream(stream)),
-          "b200kv_prefill_attn_prepared")
+    rc = native.suffix_attn(view, q, gate, gated_output, token_count, base_position, query_heads, scale, prefill_state, workspace,
+                            prepared_rows, stream)
+    if rc:
+        check(rc, "b200kv_prefill_attn_prepared")
 
 
 def plan_batched_decode(lengths, kv_heads: int, cta_slots: int = 0):
@@ -559,13 +552,14 @@ class SnapshotPool:
 
     def capture(self, tokens, storages=None, *, index_only_bytes: Optional[int] = None, stream: Optional[torch.cuda.Stream] = None) -> bool:
         """Keep the first len(tokens) positions of every layer (or, with index_only_bytes, only the bookkeeping)."""
+        if index_only_bytes is None:
+            rc, done = native.pool_capture(self._h.value, tokens, storages, stream)
+            if rc:
+                check(rc, "b200kv_pool_capture")
+            return bool(done)
         done = C.c_int()
-        if index_only_bytes is not None:
-            check(lib.b200kv_pool_capture_index_only(self._h, _tokens(tokens), len(tokens), index_only_bytes, C.byref(done)),
-                  "b200kv_pool_capture_index_only")
-        else:
-            check(lib.b200kv_pool_capture(self._h, _tokens(tokens), len(tokens), _views(storages), len(storages), _stream(stream), C.byref(done)),
-                  "b200kv_pool_capture")
+        check(lib.b200kv_pool_capture_index_only(self._h, _tokens(tokens), len(tokens), index_only_bytes, C.byref(done)),
+              "b200kv_pool_capture_index_only")
         return bool(done.value)
 
     def lookup(self, prompt, model_id: Optional[str] = None, quantization: Optional[str] = None):
@@ -578,10 +572,10 @@ class SnapshotPool:
 
     def restore(self, prompt, storages, stream: Optional[torch.cuda.Stream] = None) -> int:
         """Copy the longest stored proper prefix of `prompt` into the caches; returns its length (0 = none)."""
-        m = C.c_uint32()
-        check(lib.b200kv_pool_restore(self._h, _tokens(prompt), len(prompt), _views(storages), len(storages), _stream(stream), C.byref(m)),
-              "b200kv_pool_restore")
-        return m.value
+        rc, matched = native.pool_restore(self._h.value, prompt, storages, stream)
+        if rc:
+            check(rc, "b200kv_pool_restore")
+        return matched
 
     def stats(self) -> dict:
         c = PoolCounters()
