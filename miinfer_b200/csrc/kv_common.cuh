@@ -63,6 +63,11 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Checks the geometry and the pointers a view needs for its mode.
 int validate_view(const b200kv_view* view);
 
+// The first `tokens` rows of `layers` caches to (to_blob) or from compact snapshots in this device's memory, one launch for
+// all layers; snapshot l starts at blob + offsets[l].  The views are valid, of one geometry, and hold `tokens` rows.
+int snapshot_copy_device(const b200kv_view* views, uint32_t layers, uint64_t tokens, uint8_t* blob, const uint64_t* offsets, bool to_blob,
+                         cudaStream_t stream);
+
 // ---- device helpers ------------------------------------------------------------
 
 __device__ __forceinline__ float warp_max(float v) {

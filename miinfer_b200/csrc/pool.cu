@@ -9,8 +9,8 @@
 // the session directory second; :869-887: cache_prefix_after / cache_prefix_len, files only for prefixes of at
 // least 256 tokens and only if not there yet, write errors not fatal) with the telemetry fields of GenerateStats
 // (include/miinfer/prefill_v2/model.hpp:61-68).  A snapshot is kept in the compact raw layout of
-// AttentionLayerKvCacheStorage::download_raw, one device allocation per entry, filled and read back with
-// b200kv_snapshot_save / b200kv_snapshot_restore on device memory.
+// AttentionLayerKvCacheStorage::download_raw, one device allocation per entry, filled and read back by one
+// copy launch over all layers (snapshot.cu).
 #include "kv_common.cuh"
 
 #include <chrono>
@@ -175,6 +175,24 @@ bool same_shape(const b200kv_view& a, const b200kv_view& b) {
     return a.kv_heads == b.kv_heads && a.head_dim == b.head_dim && a.qblock == b.qblock && a.quant_mode == b.quant_mode;
 }
 
+// All layers between the caches and one payload (the layers' snapshots one behind the other).  Layers that share a geometry
+// -- normally all -- travel in one launch.
+int copy_layers(const b200kv_view* views, const std::vector<uint64_t>& per_layer, uint64_t tokens, void* payload, bool to_blob, void* stream) {
+    if (tokens == 0) return B200KV_OK;
+    std::vector<uint64_t> offsets(per_layer.size());
+    uint64_t off = 0;
+    for (size_t l = 0; l < per_layer.size(); off += per_layer[l++]) offsets[l] = off;
+    for (size_t l = 0; l < per_layer.size();) {
+        size_t end = l + 1;
+        while (end < per_layer.size() && same_shape(views[end], views[l])) ++end;
+        const int rc = snapshot_copy_device(views + l, static_cast<uint32_t>(end - l), tokens, static_cast<uint8_t*>(payload), offsets.data() + l,
+                                            to_blob, static_cast<cudaStream_t>(stream));
+        if (rc != B200KV_OK) return rc;
+        l = end;
+    }
+    return B200KV_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -239,12 +257,8 @@ int b200kv_pool_capture(b200kv_pool* pool, const uint32_t* tokens, uint32_t pref
         }
         dst.layer_bytes = per_layer;
         dst.geometry = layer_views[0];
-        uint64_t off = 0;
-        for (uint32_t l = 0; l < layers; ++l) {
-            rc = b200kv_snapshot_save(&layer_views[l], prefix_length, static_cast<uint8_t*>(dst.payload) + off, stream);
-            if (rc != B200KV_OK) return rc;
-            off += per_layer[l];
-        }
+        rc = copy_layers(layer_views, per_layer, prefix_length, dst.payload, true, stream);
+        if (rc != B200KV_OK) return rc;
         if (captured != nullptr) *captured = 1;
     } catch (const std::exception&) {
         return B200KV_ERR_CUDA;
@@ -305,12 +319,7 @@ int b200kv_pool_restore(b200kv_pool* pool, const uint32_t* prompt, uint32_t prom
         if (!same_shape(e.geometry, layer_views[l])) return B200KV_ERR_MISMATCH;
         if (n > layer_views[l].capacity) return B200KV_ERR_RANGE;
     }
-    uint64_t off = 0;
-    for (uint32_t l = 0; l < layers; ++l) {
-        rc = b200kv_snapshot_restore(&layer_views[l], n, static_cast<const uint8_t*>(e.payload) + off, stream);
-        if (rc != B200KV_OK) return rc;
-        off += e.layer_bytes[l];
-    }
+    if ((rc = copy_layers(layer_views, e.layer_bytes, n, e.payload, false, stream)) != B200KV_OK) return rc;
     ++pool->counters.hits;
     e.last_used = ++pool->clock;
     if (matched_length != nullptr) *matched_length = n;
