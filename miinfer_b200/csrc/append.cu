@@ -49,17 +49,6 @@ struct AppendParams {
 constexpr int kAppendWarps = 2;
 constexpr int kAppendCtasPerSm = 8;    // 128 registers per thread: a pass keeps 32 row values per lane (10, 12 and 16 CTAs spill and measured slower)
 
-__device__ __forceinline__ int quantize_s8(float v) {
-    // round to nearest even and saturate to [-128, 127] (NaN -> 0): __float2int_rn followed by the clamp, in one step
-    int q;
-    asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q) : "f"(v));
-    return q;
-}
-// max over the warp of non-negative floats (NaN counts as 0, as with fmaxf): one redux on the bit patterns
-__device__ __forceinline__ float warp_amax(float a) {
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(a, 0.0f))));
-}
-
 template <int D, bool IN_F16>
 __global__ void __launch_bounds__(kAppendWarps * 32, kAppendCtasPerSm)
 append_kernel(const __grid_constant__ AppendParams p, const bool vec) {

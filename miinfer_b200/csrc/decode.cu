@@ -20,95 +20,6 @@
 namespace b200kv {
 
 // ---------------------------------------------------------------------------
-// Generic stage 1: one warp per (query head, split, session); lane L owns the
-// D/32 consecutive dims starting at L*D/32.
-// ---------------------------------------------------------------------------
-template <int D, bool K_Q8, bool V_Q8>
-__global__ void __launch_bounds__(32) decode_generic_kernel(const __grid_constant__ DecodeParams p) {
-    constexpr int E = D / 32;
-    const uint32_t head = blockIdx.x, split = blockIdx.y, session = blockIdx.z;
-    const int lane = threadIdx.x;
-    const b200kv_view& view = session_view(p, session);
-    uint32_t begin, end;
-    resolve_range(p, session, view, &begin, &end);
-    const uint32_t per = (end - begin + p.num_splits - 1) / p.num_splits;
-    const uint32_t pos0 = begin + split * per;
-    const uint32_t pos1 = min(pos0 + per, end);
-    const uint32_t kv_head = head / (p.query_heads / view.kv_heads);
-    const uint32_t nblk = D / view.qblock;
-    const uint32_t blk = (nblk == 1) ? 0u : static_cast<uint32_t>(lane * E) / 32u;
-
-    float q[E];
-    const size_t q_base = (static_cast<size_t>(session) * p.query_heads + head) * D + lane * E;
-#pragma unroll
-    for (int i = 0; i < E; ++i)
-        q[i] = p.q_is_f16 ? __half2float(static_cast<const __half*>(p.q)[q_base + i])
-                          : static_cast<const float*>(p.q)[q_base + i];
-
-    float acc[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i) acc[i] = 0.0f;
-    float m = -INFINITY, l = 0.0f;
-
-    const size_t head_row0 = static_cast<size_t>(kv_head) * view.capacity;
-    for (uint32_t pos = pos0; pos < pos1; ++pos) {
-        const size_t row = head_row0 + pos;
-        float kf[E], vf[E];
-        float ks = 1.0f, vs = 1.0f;
-        if (K_Q8) {
-            const int8_t* src = view.key_q8 + row * D + lane * E;
-#pragma unroll
-            for (int w = 0; w < E / 4; ++w) {
-                const uint32_t raw = reinterpret_cast<const uint32_t*>(src)[w];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) kf[w * 4 + b] = static_cast<float>(static_cast<int8_t>(raw >> (8 * b)));
-            }
-            ks = __half2float(static_cast<const __half*>(view.key_scales)[row * nblk + blk]);
-        } else {
-            const __half* src = static_cast<const __half*>(view.key_f16) + row * D + lane * E;
-#pragma unroll
-            for (int i = 0; i < E; ++i) kf[i] = __half2float(src[i]);
-        }
-        float prod = 0.0f;
-#pragma unroll
-        for (int i = 0; i < E; ++i) prod = fmaf(q[i], kf[i], prod);
-        const float dot = warp_sum(prod * ks) * p.scale;
-
-        const float m_new = fmaxf(m, dot);
-        const float alpha = __expf(m - m_new);  // m == -inf on the first position: exp(-inf) = 0
-        const float weight = __expf(dot - m_new);
-        l = l * alpha + weight;
-        m = m_new;
-
-        if (V_Q8) {
-            const int8_t* src = view.value_q8 + row * D + lane * E;
-#pragma unroll
-            for (int w = 0; w < E / 4; ++w) {
-                const uint32_t raw = reinterpret_cast<const uint32_t*>(src)[w];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) vf[w * 4 + b] = static_cast<float>(static_cast<int8_t>(raw >> (8 * b)));
-            }
-            vs = __half2float(static_cast<const __half*>(view.value_scales)[row * nblk + blk]);
-        } else {
-            const __half* src = static_cast<const __half*>(view.value_f16) + row * D + lane * E;
-#pragma unroll
-            for (int i = 0; i < E; ++i) vf[i] = __half2float(src[i]);
-        }
-        const float ew = weight * vs;
-#pragma unroll
-        for (int i = 0; i < E; ++i) acc[i] = fmaf(acc[i], alpha, ew * vf[i]);
-    }
-
-    const size_t slot = (static_cast<size_t>(session) * p.num_splits + split) * p.query_heads + head;
-#pragma unroll
-    for (int i = 0; i < E; ++i) p.ws_acc[slot * D + lane * E + i] = acc[i];
-    if (lane == 0) {
-        p.ws_m[slot] = m;
-        p.ws_l[slot] = l;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Merge (stage 2): one block per (head, group), one thread per dim.  The (m, l)
 // of all parts are staged in shared memory first so the accumulation is a run
 // of independent loads.  A part with l <= 0 or m == -inf is empty and skipped
@@ -206,25 +117,10 @@ int launch_merge(const MergeParams& p, uint32_t groups, cudaStream_t stream) {
     return B200KV_OK;
 }
 
-static uint32_t pick_splits_generic(uint32_t query_heads, uint32_t sessions, uint32_t max_length) {
-    // one warp per (head, split, session): aim at ~16 warps per SM on 148 SMs
-    uint32_t want = (148u * 16u + query_heads * sessions - 1) / (query_heads * sessions);
-    uint32_t by_length = (max_length + 63) / 64;  // at least 64 positions per split
-    uint32_t s = want < by_length ? want : by_length;
-    const uint32_t cap = max_splits_per_session(sessions);
-    if (s > cap) s = cap;
-    return s ? s : 1;
-}
-
-template <int D>
-static void launch_generic(const DecodeParams& p, uint32_t mode, dim3 grid, cudaStream_t s) {
-    switch (mode) {
-        case B200KV_F16_F16: decode_generic_kernel<D, false, false><<<grid, 32, 0, s>>>(p); break;
-        case B200KV_Q8_F16: decode_generic_kernel<D, true, false><<<grid, 32, 0, s>>>(p); break;
-        case B200KV_F16_Q8: decode_generic_kernel<D, false, true><<<grid, 32, 0, s>>>(p); break;
-        default: decode_generic_kernel<D, true, true><<<grid, 32, 0, s>>>(p); break;
-    }
-}
+// max_length x kv heads up to which a single session takes the mma.sync kernel.  Measured (decode step, q8_0, us): 8 kv heads of
+// 128 dims: 6.5 against 8.2 at 1500 positions, 8.3 / 8.5 at 3000, 8.8 / 8.7 at 4096, 9.6 / 9.1 at 6000; 4 kv heads of 256 dims: 7.9 /
+// 12.7 at 1500, 9.7 / 10.3 at 4096, 11.4 / 11.4 at 7777, 14.0 / 13.1 at 12000 (one scale per row: 12.8 / 12.6 there).
+constexpr uint64_t kStreamRows128 = 32768, kStreamRows256 = 40000;
 
 // Runs stage 1 (streaming kernel if available, else generic) into the workspace.
 // Workspace layout: [tagged partials of the streaming kernel (zero between launches)] [m] [l] [acc].
@@ -232,21 +128,29 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
                       size_t workspace_bytes, uint32_t num_splits_arg, const MergeParams& merge, bool* merged,
                       cudaStream_t stream) {
     *merged = false;
-    const bool force_generic = (num_splits_arg & B200KV_SPLITS_FORCE_GENERIC) != 0;
+    const bool force_stream = (num_splits_arg & B200KV_SPLITS_FORCE_GENERIC) != 0;
     uint32_t num_splits = num_splits_arg & ~B200KV_SPLITS_FORCE_GENERIC;
     const uint32_t cap = max_splits_per_session(p.sessions);
-    bool use_fast = !force_generic && q8_fast_path_ok(geometry, p.query_heads);
-    // head_dim 256: a tcgen05 stage 1 for single-session launches (it leaves plain partials, like the generic kernel)
-    const bool use_wide = !force_generic && !use_fast && p.views == nullptr && p.lengths == nullptr && !p.causal && p.sessions == 1 &&
-                          p.new_key == nullptr && streaming_kernel_choice() != 1 && decode_tc5_wide_ok(geometry, p.query_heads);
+    const bool many = p.sessions > 1 || p.lengths != nullptr;
+    bool use_fast = !force_stream && q8_fast_path_ok(geometry, p.query_heads);
+    // head_dim 256: the tcgen05 kernel for single-session launches
+    bool use_wide = !force_stream && !use_fast && !many && streaming_kernel_choice() != 1 && decode_tc5_wide_ok(geometry, p.query_heads);
+    // Single sessions that are short for the device: the mma.sync kernel starts, splits and merges faster than the tcgen05
+    // kernels' pipelines fill, until its instruction issue shows.
+    if (num_splits == 0 && !many && streaming_kernel_choice() != 1) {
+        const uint64_t rows = static_cast<uint64_t>(max_length) * geometry.kv_heads;
+        if (rows <= (use_fast ? kStreamRows128 : kStreamRows256)) use_fast = use_wide = false;
+    }
     if (num_splits == 0) {
         uint32_t fast = use_fast ? pick_splits_q8(geometry, p.query_heads, p.sessions, max_length) : 0;
         if (fast == 0) use_fast = false;
-        num_splits = use_fast ? fast : (use_wide ? pick_splits_tc5_wide(geometry, max_length) : pick_splits_generic(p.query_heads, p.sessions, max_length));
+        num_splits = use_fast ? fast
+                   : use_wide ? pick_splits_tc5_wide(geometry, max_length)
+                              : pick_splits_stream(geometry.kv_heads, p.query_heads, geometry.head_dim, p.sessions, max_length);
     }
     if (num_splits > cap) num_splits = cap;
     const size_t slots = static_cast<size_t>(p.sessions) * num_splits * p.query_heads;
-    const size_t plain_bytes = slots * (geometry.head_dim + 2u) * sizeof(float);
+    const size_t plain_bytes = slots * partial_floats(geometry.head_dim) * sizeof(float);
     if (workspace == nullptr) return B200KV_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return B200KV_ERR_INVALID;
     const size_t plain_offset = workspace_plain_offset(workspace_bytes);
@@ -272,15 +176,17 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         if (rc != B200KV_ERR_UNSUPPORTED) return rc;
         p.ws_tagged = nullptr;
     }
-    if (use_wide) {
-        const int rc = launch_decode_tc5_wide(p, geometry, stream);
-        if (rc != B200KV_ERR_UNSUPPORTED) return rc;
-    }
-    dim3 grid(p.query_heads, num_splits, p.sessions);
-    if (geometry.head_dim == 128) launch_generic<128>(p, geometry.quant_mode, grid, stream);
-    else launch_generic<256>(p, geometry.quant_mode, grid, stream);
-    B200KV_CUDA_TRY(cudaGetLastError());
-    return B200KV_OK;
+    const bool fuse_merge = !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && plain_offset >= 2 * plain_bytes &&
+                            stream_merge_fits(geometry.kv_heads, num_splits, many);
+    if (merge.xchg.world > 1 && !fuse_merge) return B200KV_ERR_UNSUPPORTED;   // the exchange is part of the in-launch merge
+    p.ws_tagged = fuse_merge ? static_cast<uint64_t*>(workspace) : nullptr;
+    p.tag = next_launch_tag();
+    p.fuse = merge;
+    int rc = B200KV_ERR_UNSUPPORTED;
+    if (use_wide) rc = launch_decode_tc5_wide(p, geometry, stream);
+    if (rc == B200KV_ERR_UNSUPPORTED) rc = launch_decode_stream(p, geometry, max_length, stream);
+    if (rc == B200KV_OK) *merged = fuse_merge;
+    return rc;
 }
 
 // Stage 1 followed (unless the kernel merged by itself) by the merge kernel.
@@ -348,7 +254,7 @@ size_t b200kv_decode_workspace_bytes(uint32_t query_heads, uint32_t head_dim, ui
     if (sessions == 0) sessions = 1;
     const size_t slots = static_cast<size_t>(sessions) * max_splits_per_session(sessions) * query_heads;
     // plain partials behind, twice that for the tagged partials of the streaming kernels in front
-    return (slots * (head_dim + 2u) * sizeof(float) + 255) / 256 * 256 * 3;
+    return (slots * partial_floats(head_dim) * sizeof(float) + 255) / 256 * 256 * 3;
 }
 
 int b200kv_decode_attn(const b200kv_view* view, const void* q, int q_dtype, const float* gate,
@@ -400,14 +306,6 @@ int b200kv_decode_step(const b200kv_view* view, const void* key, const void* val
     if (!std::isfinite(theta) || !std::isfinite(epsilon) || (rope_mode != B200KV_ROPE_NONE && !(theta > 0.0f))) return B200KV_ERR_INVALID;
     if ((rc = check_heads(view, query_heads, scale)) != B200KV_OK) return rc;
     if (decode_state == nullptr && position >= view->capacity) return B200KV_ERR_RANGE;
-    const bool force_generic = (num_splits & B200KV_SPLITS_FORCE_GENERIC) != 0;
-    if (force_generic || !q8_fast_path_ok(*view, query_heads)) {
-        // no fused kernel for this cache: the two launches the fused one stands for
-        rc = b200kv_append(view, key, value, kv_dtype, k_norm_weight, rope_mode, theta, epsilon, 1, position, nullptr, decode_state, stream);
-        if (rc != B200KV_OK) return rc;
-        return b200kv_decode_attn(view, q, q_dtype, gate, output, gated_output, gated_output_q8, query_heads, scale, position + 1,
-                                  decode_state, workspace, workspace_bytes, num_splits, stream);
-    }
     if ((rc = ensure_device()) != B200KV_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     DecodeParams p{};

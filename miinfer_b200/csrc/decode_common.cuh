@@ -69,11 +69,6 @@ struct DecodeParams {
     const b200kv_decode_state* decode_state; // device, or null
     uint32_t cache_length;                   // used when neither of the above is given
     uint32_t range_begin;                    // first position scanned (sequence shard), normally 0
-    // Suffix/prefill use: "session" t is query token t of ONE cache and attends
-    // [0, causal_base + t + 1); prefill_state (device) overrides base and count.
-    int causal;
-    uint32_t causal_base;
-    const b200kv_prefill_state* prefill_state;
     uint32_t sessions;
     const void* q;                           // [sessions][query_heads][d]
     int q_is_f16;
@@ -96,7 +91,7 @@ struct DecodeParams {
     int rope_mode;
     float epsilon;
     float sectioned_step;
-    float inv_freq[64];                      // NeoX frequencies for d = 128
+    float inv_freq[128];                     // NeoX frequencies, head_dim / 2 of them
     uint32_t overlap_tail;                   // launch overlap: the last n positions of the range are read only after pdl_wait
     uint32_t head_fastest;                   // tcgen05 kernel: grid is (kv heads, splits, sessions) instead of (splits, kv heads, sessions)
     uint64_t* ws_tagged;
@@ -135,15 +130,7 @@ int streaming_kernel_choice();
 __device__ __forceinline__ void resolve_range(const DecodeParams& p, uint32_t session, const b200kv_view& view,
                                               uint32_t* begin, uint32_t* end) {
     uint32_t length = p.cache_length;
-    if (p.causal) {
-        uint32_t base = p.causal_base, count = p.sessions;
-        if (p.prefill_state != nullptr) {
-            base = p.prefill_state->base_position;
-            count = p.prefill_state->token_count;
-        }
-        // tokens past the device-side count, or whose causal range leaves the cache, scan nothing
-        length = (session < count && static_cast<uint64_t>(base) + session + 1u <= view.capacity) ? base + session + 1u : 0u;
-    } else if (p.lengths != nullptr) length = p.lengths[session];
+    if (p.lengths != nullptr) length = p.lengths[session];
     else if (p.decode_state != nullptr) length = p.decode_state->position + 1u;
     if (length > view.capacity) length = static_cast<uint32_t>(view.capacity);
     *end = length;
@@ -164,14 +151,20 @@ int launch_merge(const MergeParams& p, uint32_t groups, cudaStream_t stream);
 int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, void* workspace,
                       size_t workspace_bytes, uint32_t num_splits_arg, const MergeParams& merge, bool* merged,
                       cudaStream_t stream);
+// Floats of one (split, query head) partial: the accumulators and, per segment of 128 dims, (m, l) (decode_tail.cuh).
+inline size_t partial_floats(uint32_t head_dim) { return head_dim + 2u * ((head_dim + 127u) / 128u); }
 // Split of a caller's workspace of `bytes` bytes: tagged partials in front (two thirds), plain [m][l][acc] partials
 // behind.  The split depends only on the size.
 inline size_t workspace_plain_offset(size_t bytes) { return bytes / 3 * 2 / 256 * 256; }
 int run_decode(DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, void* workspace, size_t workspace_bytes,
                uint32_t num_splits_arg, MergeParams mp, uint32_t groups, cudaStream_t stream);
 
-// Fast path for int8 K and V (decode_q8.cu).  Returns B200KV_ERR_UNSUPPORTED when
-// the geometry has no specialised kernel, so the caller can use the generic one.
+// Every cache mode and shape (decode_stream.cu).
+uint32_t pick_splits_stream(uint32_t kv_heads, uint32_t query_heads, uint32_t head_dim, uint32_t sessions, uint32_t max_length);
+bool stream_merge_fits(uint32_t kv_heads, uint32_t num_splits, bool many);
+int launch_decode_stream(const DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream);
+// int8 K and V at head_dim 128 (decode_q8.cu).  Returns B200KV_ERR_UNSUPPORTED when
+// the geometry is not one it takes, so the caller can use the kernel above.
 int launch_decode_q8(const DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream);
 // The same launch on the tcgen05 kernel (decode_tc5.cu); B200KV_ERR_UNSUPPORTED where it does not apply.
 int launch_decode_tc5(const DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream);

@@ -186,7 +186,7 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     const uint64_t total_tiles = end > begin ? tile_end - tile_begin : 0;
     const uint32_t nworkers = num_splits * kWarps, gw = split * kWarps + warp;
     // A fused append is counted as extra units at the end of the range, so the warp that does it is handed fewer tiles.
-    const bool fuse = p.new_key != nullptr;
+    const bool fuse = tail::appends_row(p, begin, end);
     const uint64_t units = total_tiles + (fuse ? kAppendUnits : 0);
     const uint64_t u0 = units * gw / nworkers, u1 = units * (gw + 1) / nworkers;
     const uint32_t t0 = tile_begin + static_cast<uint32_t>(u0 < total_tiles ? u0 : total_tiles);
@@ -195,8 +195,8 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     const bool owner = fuse && ntiles > 0 && t1 == tile_end;   // this warp holds the tile of the appended token
     // With launch overlap the previous kernel may still be appending: rows at or above early_end wait for it.  The
     // row a fused append writes is never loaded early either.
-    uint32_t early_end = end > p.overlap_tail ? end - p.overlap_tail : 0;
-    if (fuse && early_end >= end) early_end = end - 1;
+    const uint32_t needed_end = fuse ? end - 1 : end;
+    const uint32_t early_end = needed_end > p.overlap_tail ? needed_end - p.overlap_tail : 0;
 
     uint8_t* k_ring = smem + warp * kStages * L::kKTile;
     uint8_t* v_ring = smem + L::kOffV + warp * kStages * L::kKTile;
@@ -242,8 +242,8 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     // is streaming, a dependent load waits behind tens of megabytes of queued tile traffic (microseconds).
     float new_k[4], new_v[4];
     if (owner) {
-        tail::load_new_row(p.new_key, p.new_is_f16, kv_head, lane, new_k);
-        tail::load_new_row(p.new_value, p.new_is_f16, kv_head, lane, new_v);
+        tail::load_new_row<kD>(p.new_key, p.new_is_f16, kv_head, lane, new_k);
+        tail::load_new_row<kD>(p.new_value, p.new_is_f16, kv_head, lane, new_v);
     }
     {
         // the tile that holds the row of a fused append is loaded only after that row has been stored (below)
@@ -290,7 +290,11 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     if (owner) {
         // After the barrier, so that only this warp (which was handed fewer tiles) pays for the append.  The new row
         // goes to the cache first; its tile is loaded (by TMA, an asynchronous-proxy read) only afterwards.
-        tail::fused_append_row<NBLK>(p, view, new_k, new_v, end - 1, head_row0 + end - 1, lane);
+        Rotation<kD> rot;
+        row_rotation<kD>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);
+        tail::RowScratch<kD>* no_copy = nullptr;
+        tail::store_new_key<kD>(p, view, new_k, rot, head_row0 + end - 1, lane, no_copy);
+        tail::store_new_value<kD>(view, new_v, head_row0 + end - 1, lane, no_copy);
         __threadfence();
         asm volatile("fence.proxy.async;" ::: "memory");
         __syncwarp();
@@ -514,12 +518,12 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
         }
         const uint32_t head = kv_head * G + h;
         const float m_nat = M * 0.6931471805599453f;   // natural-log units, as the merge expects
-        tail::emit_partial(p, session, split, num_splits, head, dim, at, m_nat, lt);
+        tail::emit_partial<1>(p, session, split, num_splits, head, dim, at, m_nat, lt);
     }
     if (failed) tail::report(p, B200KV_STATUS_COPY_TIMEOUT);
     if (p.ws_tagged == nullptr) return;   // a separate merge kernel follows
     // the CTA of split h merges query head h of this kv head once all splits' tagged partials have landed
-    tail::fused_merge(p, session, kv_head, split, num_splits, G, reinterpret_cast<float*>(smem + L::kOffMisc));
+    tail::fused_merge<1, 256>(p, session, kv_head, split, num_splits, G, reinterpret_cast<float*>(smem + L::kOffMisc));
 }
 
 // ---- host side -----------------------------------------------------------------------------------------

@@ -1,6 +1,9 @@
-// What the two streaming decode kernels (decode_q8.cu: warp-level mma; decode_tc5.cu: tcgen05) share after
-// their tile loops: the tagged-word partials, the merge of a kv head's splits inside the launch, the cross-GPU
-// exchange of a sequence shard, and the single-token append a decode step fuses in.
+// What the streaming decode kernels (decode_tc5.cu and decode_q8.cu for int8 at head_dim 128, decode_stream.cu for every
+// other mode and shape) share after their tile loops: the tagged-word partials, the merge of a kv head's splits inside
+// the launch, the cross-GPU exchange of a sequence shard, and the single-token append a decode step fuses in.
+//
+// Everything works on SEGMENTS of 128 dims: a head of 256 dims is two, each with its own copy of (m, l), so that the two
+// halves of a head are merged by two CTAs side by side.
 //
 // The merge is MIInfer's decode stage 2 (gfx906/kernels/qwen3_primitives.hip:2295-2352) with the empty-split rule
 // of its suffix twin (.hip:6681,6701); the optional Q8_1 re-quantisation of the output follows .hip:2354-2383.
@@ -46,48 +49,84 @@ __device__ __forceinline__ void report(const DecodeParams& p, uint32_t bit) {
 }
 
 // ---- fused single-token append -----------------------------------------------------------------------------
-// Kept out of line so the rarely-taken path does not widen the register allocation of the streaming loops.
-// Loads the new row of `kv_head` (lane L: elements L, L+32, L+64, L+96); head_dim 128.
-static __device__ __noinline__ void load_new_row(const void* src, int is_f16, uint32_t kv_head, int lane, float (&x)[4]) {
+// The CTA that owns the last position's tile appends the new row of its kv head: one warp per side (or one for both) fetches
+// the row as soon as the dependency wait is over, transforms and quantises it, stores it to the cache and leaves a copy in
+// shared memory, from which it is patched into the tile once that has landed.  The tile itself is fetched with all the
+// others -- its copy of the new row, whatever it holds, is overwritten -- so neither a fence nor a second trip to the
+// cache lies between the row and its use.  (Storing the row, fencing and only then fetching the tile cost 3 to 7 us
+// of a decode step at short contexts.)
+template <int BYTES>
+struct alignas(16) RowScratch {      // one side's new row: data in natural order, then its scales
+    uint8_t data[BYTES];
+    __half scales[8];
+};
+
+template <int D>
+__device__ __forceinline__ void load_new_row(const void* src, int is_f16, uint32_t kv_head, int lane, float (&x)[D / 32]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const size_t i = static_cast<size_t>(kv_head) * 128 + lane + 32 * j;
+    for (int j = 0; j < D / 32; ++j) {
+        const size_t i = static_cast<size_t>(kv_head) * D + lane + 32 * j;
         x[j] = is_f16 ? __half2float(static_cast<const __half*>(src)[i]) : static_cast<const float*>(src)[i];
     }
 }
 
-// Quantises the new K and V rows of a kv head (already in registers) and stores them (int8 + fp16 block scales) at
-// cache row `row_index`.  One warp; head_dim 128.
-template <int NBLK>
-static __device__ __noinline__ void fused_append_row(const DecodeParams& p, const b200kv_view& view, float (&k)[4], float (&v)[4],
-                                              uint32_t position, uint64_t row_index, int lane) {
-    constexpr int kD = 128;
-    transform_k_row<kD>(k, lane, position, p.k_norm_weight, p.epsilon, p.rope_mode, p.inv_freq, p.sectioned_step);
-    int8_t kq[4], vq[4];
-    float ksc[4], vsc[4];
-    quantize_row<4>(k, NBLK == 1, kq, ksc);
-    quantize_row<4>(v, NBLK == 1, vq, vsc);
+// One side's row (already transformed) in the cache's format, to cache row `row_index` and to `scratch` (may be null).  One warp.
+template <int D, int BYTES>
+__device__ __forceinline__ void store_new_row(const float (&x)[D / 32], bool q8, bool row_scale, int8_t* plane_q8, void* plane_f16, void* scales,
+                                              uint64_t row_index, int lane, RowScratch<BYTES>* scratch) {
+    constexpr int NJ = D / 32;
+    if (q8) {
+        int q[NJ];
+        const float scale = quantize_row<NJ>(x, row_scale, lane, q);
+        int8_t* dst = plane_q8 + row_index * D + lane;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        view.key_q8[row_index * kD + lane + 32 * j] = kq[j];
-        view.value_q8[row_index * kD + lane + 32 * j] = vq[j];
+        for (int j = 0; j < NJ; ++j) {
+            if (scratch != nullptr) scratch->data[lane + 32 * j] = static_cast<uint8_t>(q[j]);
+            dst[32 * j] = static_cast<int8_t>(q[j]);
+        }
+        if (lane < (row_scale ? 1 : NJ)) {
+            const __half h = __float2half_rn(scale);
+            if (scratch != nullptr) scratch->scales[lane] = h;
+            static_cast<__half*>(scales)[row_scale ? row_index : row_index * NJ + lane] = h;
+        }
+    } else {
+        __half* dst = static_cast<__half*>(plane_f16) + row_index * D + lane;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const __half h = __float2half_rn(x[j]);
+            if (BYTES == 2 * D && scratch != nullptr) reinterpret_cast<__half*>(scratch->data)[lane + 32 * j] = h;
+            dst[32 * j] = h;
+        }
     }
-    if (lane < NBLK) {
-        static_cast<__half*>(view.key_scales)[row_index * NBLK + lane] = __float2half_rn(ksc[NBLK == 1 ? 0 : lane]);
-        static_cast<__half*>(view.value_scales)[row_index * NBLK + lane] = __float2half_rn(vsc[NBLK == 1 ? 0 : lane]);
-    }
+}
+template <int D, int BYTES>
+__device__ __forceinline__ void store_new_key(const DecodeParams& p, const b200kv_view& view, float (&k)[D / 32], const Rotation<D>& rot,
+                                              uint64_t row_index, int lane, RowScratch<BYTES>* scratch) {
+    transform_k_row<D>(k, lane, p.k_norm_weight, p.epsilon, p.rope_mode, rot);
+    store_new_row<D, BYTES>(k, (view.quant_mode & 1u) != 0, view.qblock == D, view.key_q8, view.key_f16, view.key_scales, row_index, lane, scratch);
+}
+template <int D, int BYTES>
+__device__ __forceinline__ void store_new_value(const b200kv_view& view, const float (&v)[D / 32], uint64_t row_index, int lane, RowScratch<BYTES>* scratch) {
+    store_new_row<D, BYTES>(v, (view.quant_mode & 2u) != 0, view.qblock == D, view.value_q8, view.value_f16, view.value_scales, row_index, lane, scratch);
+}
+// Whether this launch appends a row: only inside the cache (a device-side position is not checked on the host).
+__device__ __forceinline__ bool appends_row(const DecodeParams& p, uint32_t begin, uint32_t end) {
+    return p.new_key != nullptr && end > begin && (p.decode_state != nullptr ? p.decode_state->position + 1u : p.cache_length) == end;
 }
 
 // ---- where a CTA's partial of one (query head, dim) goes -----------------------------------------------------
-// kD = 128.  `at` is the unnormalised accumulator relative to the maximum m_nat (natural-log units), `lt` the sum.
+// SEG = head_dim / 128.  `at` is the unnormalised accumulator relative to the maximum m_nat (natural-log units), `lt` the sum.
+constexpr int kSegDims = 128;
+constexpr int kSegWords = kSegDims + 2;   // tagged words of one segment's partial: accumulators, m, l
+
+template <int SEG>
 __device__ __forceinline__ void emit_partial(const DecodeParams& p, uint32_t session, uint32_t split, uint32_t num_splits,
                                              uint32_t head, int dim, float at, float m_nat, float lt) {
-    constexpr int kD = 128;
-    constexpr int kPartialWords = kD + 2;
+    constexpr int D = SEG * kSegDims;
     const size_t slot_idx = (static_cast<size_t>(session) * p.num_splits + split) * p.query_heads + head;
     if (p.ws_tagged != nullptr && num_splits == 1 && p.fuse.xchg.world <= 1) {
         // a single split has nothing to merge with: the result leaves from here (short contexts)
-        const size_t out_idx = (static_cast<size_t>(session) * p.query_heads + head) * kD + dim;
+        const size_t out_idx = (static_cast<size_t>(session) * p.query_heads + head) * D + dim;
         if (p.fuse.out_m != nullptr) {
             p.fuse.out_acc[out_idx] = at;
             if (dim == 0) {
@@ -104,11 +143,12 @@ __device__ __forceinline__ void emit_partial(const DecodeParams& p, uint32_t ses
             }
         }
     } else if (p.ws_tagged != nullptr) {
-        uint64_t* dst = p.ws_tagged + slot_idx * kPartialWords;
-        st_tagged(dst + dim, at, p.tag);
-        if (dim == 0) { st_tagged(dst + kD, m_nat, p.tag); st_tagged(dst + kD + 1, lt, p.tag); }
+        const int seg = SEG == 1 ? 0 : dim / kSegDims, in_seg = SEG == 1 ? dim : dim % kSegDims;
+        uint64_t* dst = p.ws_tagged + (slot_idx * SEG + seg) * kSegWords;
+        st_tagged(dst + in_seg, at, p.tag);
+        if (in_seg == 0) { st_tagged(dst + kSegDims, m_nat, p.tag); st_tagged(dst + kSegDims + 1, lt, p.tag); }
     } else {
-        p.ws_acc[slot_idx * kD + dim] = at;
+        p.ws_acc[slot_idx * D + dim] = at;
         if (dim == 0) { p.ws_m[slot_idx] = m_nat; p.ws_l[slot_idx] = lt; }
     }
 }
@@ -191,14 +231,13 @@ __device__ __forceinline__ void exchange_partials(const DecodeParams& p, uint32_
 // Normalise, gate and store the merged result of one head (64 threads, two dims each), with the optional Q8_1
 // re-quantisation of the gated output the reference's stage 2 offers for the projection that follows
 // (.hip:2354-2383: blocks of 32, d = amax/127, q = roundf(x/d) clamped to +-127, s = d * sum(q), both fp16).
-// Uses named barrier 1 (64 threads) only when the Q8_1 output is requested.
-__device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t session, uint32_t head, int pr, float2 tot, float gsum,
+template <int SEG>
+__device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t session, uint32_t head, int seg, int pr, float2 tot, float gsum,
                                              float m_merged) {
-    constexpr int kD = 128;
-    const size_t out_idx = (static_cast<size_t>(session) * f.query_heads + head) * kD + 2 * pr;
+    const size_t out_idx = ((static_cast<size_t>(session) * f.query_heads + head) * SEG + seg) * kSegDims + 2 * pr;
     if (f.out_m != nullptr) {   // sequence shard: one merged, unnormalised partial
         *reinterpret_cast<float2*>(f.out_acc + out_idx) = tot;
-        if (pr == 0) {
+        if (pr == 0 && seg == 0) {
             f.out_m[static_cast<size_t>(session) * f.query_heads + head] = m_merged;
             f.out_l[static_cast<size_t>(session) * f.query_heads + head] = gsum;
         }
@@ -225,8 +264,7 @@ __device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t sess
             int qs = q0 + q1;
 #pragma unroll
             for (int off = 8; off > 0; off >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, off);
-            const size_t block = ((static_cast<size_t>(session) * f.query_heads + head) * kD) / 32 + (pr >> 4);
-            b200kv_q8_1_block* dst = f.gated_output_q8 + block;
+            b200kv_q8_1_block* dst = f.gated_output_q8 + out_idx / 32;
             reinterpret_cast<char2*>(dst->qs)[pr & 15] = make_char2(static_cast<signed char>(q0), static_cast<signed char>(q1));
             if ((pr & 15) == 0) {
                 const __half dh = __float2half_rn(dq), sh = __float2half_rn(__fmul_rn(static_cast<float>(qs), dq));
@@ -237,36 +275,39 @@ __device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t sess
     }
 }
 
-// ---- fused merge: the CTA of split h merges query head h of its kv head (h, h + splits, ... if there are fewer
-// splits than heads).  It polls the tagged partials of all splits -- normally they are all there by the time it
+// ---- fused merge: the CTA of split u merges unit u = (query head of its kv head, segment); u, u + splits, ... if there are
+// fewer splits than units.  It polls the tagged partials of all splits -- normally they are all there by the time it
 // has finished its own share -- and every other CTA simply leaves.  (Electing instead the CTAs that arrive last, with
 // an atomic counter behind the partial stores, measured slower: the atomic's round trip and the merger reading its
-// own partial back through L2 cost more than the polls they save.)  Called by ALL 256 threads of the CTA after they
+// own partial back through L2 cost more than the polls they save.)  Called by ALL `THREADS` threads of the CTA after they
 // have issued their emit_partial stores (the CTAs that have nothing to merge return at once); uses named barriers
-// 1 (64 threads) and 2 (256 threads).  fold_area: (8 + 3 * 64 * 2) floats of shared memory nothing else uses any more.
+// 1 (64 threads) and 2 (all).  fold_area: (8 + 3 * 64 * 2) floats of shared memory nothing else uses any more.
+template <int SEG, int THREADS>
 __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t session, uint32_t kv_head, uint32_t split,
                                             uint32_t num_splits, int G, float* fold_area) {
-    constexpr int kD = 128;
-    constexpr int kPartialWords = kD + 2;
+    constexpr int kGroups = THREADS / 64;
+    static_assert(kGroups == 2 || kGroups == 4, "128 or 256 threads");
     if (merge_not_needed(p, num_splits)) return;
     const uint32_t S = num_splits;     // <= kMaxSplitsPerSession == 128; the partial arrays keep the launch-wide stride
     const uint32_t rank = split;
-    if (rank >= static_cast<uint32_t>(G)) return;
+    const uint32_t units = static_cast<uint32_t>(G) * SEG;
+    if (rank >= units) return;
     const uint32_t tag = p.tag;
-    float* fold_ml = fold_area;                                   // [3] x {max, sum} of split groups 1..3
-    float2* fold = reinterpret_cast<float2*>(fold_ml + 8);        // [3][64] partial sums of split groups 1..3
+    float* fold_ml = fold_area;                                   // {max, sum} of split groups 1 ..
+    float2* fold = reinterpret_cast<float2*>(fold_ml + 8);        // [64] partial sums of each of them
     constexpr int kBatch = 10;   // splits per thread and round: 4 groups x 10 = 40 splits in one trip to L2
-    // 256 threads = 4 split groups (sp % 4) x 64 pairs of dims.  A group merges its own splits on line (every thread
-    // of a group also reads the group's (m, l) words itself: no staging, no barrier), then the 4 groups are folded.
+    // Threads = split groups (sp % groups) x 64 pairs of dims.  A group merges its own splits on line (every thread
+    // of a group also reads the group's (m, l) words itself: no staging, no barrier), then the groups are folded.
     const int grp = threadIdx.x >> 6, pr = threadIdx.x & 63;
-    for (uint32_t h = rank; h < static_cast<uint32_t>(G); h += S) {
-        const uint32_t head = kv_head * G + h;
-        const size_t stride = static_cast<size_t>(p.query_heads) * kPartialWords;   // words between consecutive splits
-        uint64_t* base = p.ws_tagged + ((static_cast<size_t>(session) * p.num_splits) * p.query_heads + head) * kPartialWords;
+    for (uint32_t u0 = rank; u0 < units; u0 += S) {
+        const uint32_t head = kv_head * G + u0 / SEG;
+        const int seg = static_cast<int>(u0 % SEG);
+        const size_t stride = static_cast<size_t>(p.query_heads) * SEG * kSegWords;   // words between consecutive splits
+        uint64_t* base = p.ws_tagged + ((static_cast<size_t>(session) * p.num_splits * p.query_heads + head) * SEG + seg) * kSegWords;
         bool lost = false;
         float2 tot = make_float2(0.0f, 0.0f);
         float Mg = -INFINITY, lg = 0.0f;
-        for (uint32_t sp0 = 0; sp0 < S; sp0 += 4 * kBatch) {
+        for (uint32_t sp0 = 0; sp0 < S; sp0 += kGroups * kBatch) {
             // Poll in rounds: every round re-issues, back to back, the loads of all words of this thread that have
             // not shown their tag yet, so that once the last partial has landed one trip to L2 completes the set.
             float fa[kBatch], fb[kBatch], fm[kBatch], fl[kBatch];
@@ -275,7 +316,7 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
             for (int u = 0; u < kBatch; ++u) {
                 fa[u] = fb[u] = fl[u] = 0.0f;
                 fm[u] = -INFINITY;
-                if (sp0 + grp + 4 * u < S) pending |= 1u << u;
+                if (sp0 + grp + kGroups * u < S) pending |= 1u << u;
             }
             uint32_t ml_pending = pending;
             for (uint32_t polls = 0; (pending | ml_pending) != 0 && !lost; ++polls) {
@@ -284,10 +325,10 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
                 uint64_t wa[kBatch], wb[kBatch], wm[kBatch], wl[kBatch];
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
-                    uint64_t* src = base + (sp0 + grp + 4 * u) * stride;
+                    uint64_t* src = base + (sp0 + grp + kGroups * u) * stride;
                     wa[u] = wb[u] = wm[u] = wl[u] = 0;
                     if (pending & (1u << u)) ld_tagged2(src + 2 * pr, wa[u], wb[u]);
-                    if (ml_pending & (1u << u)) ld_tagged2(src + kD, wm[u], wl[u]);
+                    if (ml_pending & (1u << u)) ld_tagged2(src + kSegDims, wm[u], wl[u]);
                 }
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
@@ -321,21 +362,21 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
             // the group, so they are zeroed after the fold barrier below
 #pragma unroll
             for (int u = 0; u < kBatch; ++u)
-                if (sp0 + grp + 4 * u < S) zero2(base + (sp0 + grp + 4 * u) * stride + 2 * pr);
+                if (sp0 + grp + kGroups * u < S) zero2(base + (sp0 + grp + kGroups * u) * stride + 2 * pr);
         }
         if (lost) tot.x = tot.y = lg = __int_as_float(0x7fc00000);
-        // fold the 4 split groups through shared memory
+        // fold the split groups through shared memory
         if (grp > 0) {
             fold[(grp - 1) * 64 + pr] = tot;
             if (pr == 0) { fold_ml[2 * (grp - 1)] = Mg; fold_ml[2 * (grp - 1) + 1] = lg; }
         }
-        asm volatile("bar.sync 2, 256;" ::: "memory");
-        for (uint32_t sp = threadIdx.x; sp < S; sp += 256)   // every thread of every group is past its polls
-            zero2(base + sp * stride + kD);
+        asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");
+        for (uint32_t sp = threadIdx.x; sp < S; sp += THREADS)   // every thread of every group is past its polls
+            zero2(base + sp * stride + kSegDims);
         if (grp == 0) {
             float M = Mg;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < kGroups - 1; ++k) {
                 const float mk = fold_ml[2 * k], lk = fold_ml[2 * k + 1];
                 if (!(lk <= 0.0f) && mk != -INFINITY) M = fmaxf(M, mk);
             }
@@ -344,7 +385,7 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
                 tot.x *= a0; tot.y *= a0; lg *= a0;
             }
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < kGroups - 1; ++k) {
                 const float mk = fold_ml[2 * k], lk = fold_ml[2 * k + 1];
                 const float a = (!(lk <= 0.0f) && mk != -INFINITY) ? __expf(mk - M) : 0.0f;
                 const float2 o2 = fold[k * 64 + pr];
@@ -353,10 +394,12 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
             }
             float gsum = lg;
             const float m_merged = M;
-            if (p.fuse.xchg.world > 1) exchange_partials(p, head, pr, m_merged, tot, gsum, lost);
-            write_merged(p.fuse, session, head, pr, tot, gsum, m_merged);
+            if constexpr (SEG == 1) {   // the cross-GPU exchange is the 128-dim kernels'
+                if (p.fuse.xchg.world > 1) exchange_partials(p, head, pr, m_merged, tot, gsum, lost);
+            }
+            write_merged<SEG>(p.fuse, session, head, seg, pr, tot, gsum, m_merged);
         }
-        asm volatile("bar.sync 2, 256;" ::: "memory");   // the fold area is reused by the next head of this CTA
+        asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");   // the fold area is reused by the next head of this CTA
     }
 }
 

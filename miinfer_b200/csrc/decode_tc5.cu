@@ -73,9 +73,10 @@ struct Smem {
     static constexpr int kOffL = kOffXch + 2 * 4 * 8 * 4;             // [4 warps][4] row sums
     static constexpr int kOffQmul = kOffL + 64;                       // [4]
     static constexpr int kOffBar = kOffQmul + 16;
-    static constexpr int kNumBars = 2 * kStages + 9;                  // full[3] empty[3] s_full[2] s_empty[2] p_full[2] p_empty[2] row
+    static constexpr int kNumBars = 2 * kStages + 10;                 // full[3] empty[3] s_full[2] s_empty[2] p_full[2] p_empty[2] row landed
     static constexpr int kOffMisc = kOffBar + kNumBars * 8;           // tmem slot, fail flag
-    static constexpr int kTotal = kOffMisc + 16;
+    static constexpr int kOffRow = (kOffMisc + 8 + 15) / 16 * 16;     // the appended row's two sides
+    static constexpr int kTotal = kOffRow + 2 * static_cast<int>(sizeof(tail::RowScratch<kD>));
     static constexpr int kAlloc = kTotal + 1024;                      // slack to align the base to 1024
 };
 static_assert(Smem<4>::kAlloc <= 115712, "two CTAs per SM");
@@ -197,12 +198,12 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
     const uint32_t t0 = tile_begin + static_cast<uint32_t>(total_tiles * split / num_splits);
     const uint32_t t1 = tile_begin + static_cast<uint32_t>(total_tiles * (split + 1) / num_splits);
     const int ntiles = static_cast<int>(t1 - t0);
-    const bool fuse = p.new_key != nullptr;
+    const bool fuse = tail::appends_row(p, begin, end);
     const bool owner = fuse && ntiles > 0 && t1 == tile_end;   // this CTA holds the tile of the appended token
-    // With launch overlap the previous kernel may still be appending: rows at or above early_end wait for it.  The
-    // row a fused append writes is never loaded early either.
-    uint32_t early_end = end > p.overlap_tail ? end - p.overlap_tail : 0;
-    if (fuse && early_end >= end) early_end = end - 1;
+    // With launch overlap the previous kernel may still be appending: rows at or above early_end wait for it.  The row
+    // that this launch appends does not count: the copy of it that comes with its tile is overwritten in shared memory.
+    const uint32_t needed_end = fuse ? end - 1 : end;
+    const uint32_t early_end = needed_end > p.overlap_tail ? needed_end - p.overlap_tail : 0;
 
     const uint32_t bar0 = sbase + L::kOffBar;
     auto bar_full = [&](int s) { return bar0 + s * 8; };
@@ -211,7 +212,9 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
     auto bar_s_empty = [&](int b) { return bar0 + (2 * kStages + 2 + b) * 8; };
     auto bar_p_full = [&](int b) { return bar0 + (2 * kStages + 4 + b) * 8; };
     auto bar_p_empty = [&](int b) { return bar0 + (2 * kStages + 6 + b) * 8; };
-    const uint32_t bar_row = bar0 + (2 * kStages + 8) * 8;   // the appended row is in the cache
+    const uint32_t bar_row = bar0 + (2 * kStages + 8) * 8;       // the appended row is in its scratch
+    const uint32_t bar_landed = bar0 + (2 * kStages + 9) * 8;    // the tile it belongs to has landed (its "full" follows when the row is in it)
+    tail::RowScratch<kD>* new_row = reinterpret_cast<tail::RowScratch<kD>*>(smem + L::kOffRow);   // K, V
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
     uint32_t* fail_flag = tmem_slot + 1;
 
@@ -228,7 +231,7 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
         const int stage = i % kStages;
         const uint32_t pos0 = (t0 + i) * kTileM;
         const uint32_t sbytes = min(static_cast<uint32_t>(kTileM), capacity - pos0) * (NBLK * 2);
-        const uint32_t bar = bar_full(stage);
+        const uint32_t bar = owner && i == ntiles - 1 ? bar_landed : bar_full(stage);
         mbar_expect_tx(bar, 2 * L::kKTile + 2 * sbytes);
         tma_load_2d(sbase + L::kOffK + stage * L::kKTile, kmap, 0, row_base + static_cast<int>(pos0), bar);
         tma_load_2d(sbase + L::kOffV + stage * L::kKTile, vmap, 0, row_base + static_cast<int>(pos0), bar);
@@ -247,31 +250,32 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
                 mbar_init(bar_p_full(b), kConsumers); mbar_init(bar_p_empty(b), 1);
             }
             mbar_init(bar_row, 1);
+            mbar_init(bar_landed, 1);
             *fail_flag = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             // old cache rows do not depend on the preceding kernels: start streaming them before waiting for those
-            while (issued < kEarlyTiles && issued < ntiles && (t0 + issued + 1) * kTileM <= early_end) { issue(issued); ++issued; }
+            while (issued < kEarlyTiles && issued < ntiles && min((t0 + issued + 1) * kTileM, needed_end) <= early_end) { issue(issued); ++issued; }
         }
     } else if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    const bool appends = warp == kAppendWarp && owner;
+    Rotation<kD> rot{};
+    if (appends) row_rotation<kD>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();
     if (TL && tid == 0) tl[1] = global_ns();
     // The new row of a fused append is fetched now, while the memory system is still quiet (once the rings stream, a
     // dependent load waits behind megabytes of queued tile traffic); its own warp transforms and stores it after the
     // set-up barrier, while the other warps are already at work on the tiles before it.
     float new_k[4], new_v[4];
-    const bool appends = warp == kAppendWarp && owner;
     if (appends) {
-        tail::load_new_row(p.new_key, p.new_is_f16, kv_head, lane, new_k);
-        tail::load_new_row(p.new_value, p.new_is_f16, kv_head, lane, new_v);
+        tail::load_new_row<kD>(p.new_key, p.new_is_f16, kv_head, lane, new_k);
+        tail::load_new_row<kD>(p.new_value, p.new_is_f16, kv_head, lane, new_v);
     }
-    if (warp == kProducerWarp && lane == 0) {
-        const int limit = owner ? ntiles - 1 : ntiles;   // the tile that holds the appended row is loaded only after the row is stored
-        while (issued < kStages && issued < limit) { issue(issued); ++issued; }
-    }
+    if (warp == kProducerWarp && lane == 0)
+        while (issued < kStages && issued < ntiles) { issue(issued); ++issued; }
 
     // ---- Q: 15 bits per head as two int8 planes.  Rows of the B operand of S^T = K . Q^T:
     //      [hi h0 .. hi h3, lo h0 .. lo h3].  The operand has 16 rows (the smallest N next to
@@ -326,16 +330,36 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
             for (int i = issued; i < ntiles; ++i) {
                 // stage i % kStages is free once the P.V of tile i - kStages has completed
                 if (i >= kStages && !mbar_wait(bar_empty(i % kStages), static_cast<uint32_t>((i / kStages - 1) & 1))) { failed = true; break; }
-                if (owner && i == ntiles - 1 && !mbar_wait(bar_row, 0)) { failed = true; break; }
                 issue(i);
+            }
+        }
+        if (owner) {
+            // the last tile has landed and the new row is in its scratch: put the row into the tile, then let the tile's readers at it
+            const int stage = (ntiles - 1) % kStages;
+            bool ready = !failed;
+            if (lane == 0) ready = ready && mbar_wait(bar_landed, 0) && mbar_wait(bar_row, 0);
+            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0)) {
+                const uint32_t r = (end - 1) % kTileM;
+                if (lane < 16) {
+                    const int side = lane >> 3, c = lane & 7;
+                    uint8_t* tile = smem + (side == 0 ? L::kOffK : L::kOffV) + stage * L::kKTile;
+                    *reinterpret_cast<uint4*>(tile + r * kD + ((c ^ (r & 7)) << 4)) = *reinterpret_cast<const uint4*>(new_row[side].data + c * 16);
+                } else if (lane < 18) {
+                    const int side = lane - 16;
+                    uint8_t* dst = smem + L::kOffS + stage * 2 * L::kSTile + side * L::kSTile + r * (NBLK * 2);
+                    if constexpr (NBLK == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(new_row[side].scales);
+                    else *reinterpret_cast<__half*>(dst) = new_row[side].scales[0];
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read the tile through the async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full(stage));
             }
         }
     } else if (warp == kAppendWarp) {
         // =============================== fused append of the new token's row ===============================
         if (appends) {
-            tail::fused_append_row<NBLK>(p, view, new_k, new_v, end - 1, head_row0 + end - 1, lane);
-            __threadfence();
-            asm volatile("fence.proxy.async;" ::: "memory");   // the row goes to the cache first; its tile is read by TMA (async proxy) afterwards
+            tail::store_new_key<kD>(p, view, new_k, rot, head_row0 + end - 1, lane, new_row);
+            tail::store_new_value<kD>(view, new_v, head_row0 + end - 1, lane, new_row + 1);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_row);
         }
@@ -563,7 +587,7 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
             if (h >= G) break;
             float at = acc[h], mh = m_run[h] * 0.6931471805599453f, lh = lt[h];   // natural-log units, as the merge expects
             if (poisoned) { at = __int_as_float(0x7fc00000); mh = at; lh = at; }
-            tail::emit_partial(p, session, split, num_splits, kv_head * G + h, tid, at, mh, lh);
+            tail::emit_partial<1>(p, session, split, num_splits, kv_head * G + h, tid, at, mh, lh);
         }
         if (TL && tid == 0) tl[6] = global_ns();
     }
@@ -578,7 +602,7 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
     if (p.ws_tagged == nullptr) return;   // a separate merge kernel follows
     // the CTA of split h merges query head h of this kv head once all splits' tagged partials have landed (256 threads;
     // the merger's scratch takes the place of the P buffers, which every MMA has long consumed)
-    tail::fused_merge(p, session, kv_head, split, num_splits, G, reinterpret_cast<float*>(smem + L::kOffP));
+    tail::fused_merge<1, 256>(p, session, kv_head, split, num_splits, G, reinterpret_cast<float*>(smem + L::kOffP));
     if (TL && tid == 0) tl[7] = global_ns();
 }
 

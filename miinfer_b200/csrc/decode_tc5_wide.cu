@@ -15,10 +15,11 @@
 //  * with one CTA on an SM nothing else hides a tile's chain S MMA -> softmax -> P -> P.V MMA -> fold, so two groups of 128
 //    softmax threads take the even and the odd tiles (S, P and O are double-buffered: a buffer per group), each with its own
 //    running maxima, sums and accumulators, which are merged once at the end;
-//  * it is stage 1 only: the partials leave as plain (m, l, acc) and the merge kernel follows, and it neither appends
-//    nor exchanges (those stay with the 128-dim kernels); a launch that asks for them is declined.
+//  * the merge of the splits and the single-token append of a decode step run inside the launch, as there (decode_tail.cuh);
+//    the append is the P.V issuer warp's first job, which has nothing to do before the first tile's weights are there.
+//    (As launches of their own the merge cost 1.7 us at 32768 positions -- 21.1 against 19.4 us -- and the append 4 to 5 more.)
 //  * Every wait is bounded, as there.
-#include "decode_common.cuh"
+#include "decode_tail.cuh"
 
 #include <climits>
 #include <cstring>
@@ -56,12 +57,14 @@ struct Smem {
     static constexpr int kOffL = kOffXch + 2 * 2 * 4 * 16 * 4;         // [2 groups][4 warps][8] row sums
     static constexpr int kOffQmul = kOffL + 2 * 4 * 8 * 4;             // [8]
     static constexpr int kOffBar = kOffQmul + 32;
-    static constexpr int kNumBars = 2 * kKStages + 2 * kVStages + 8;   // k_full k_empty v_full v_empty s_full[2] s_empty[2] p_full[2] p_empty[2]
+    static constexpr int kNumBars = 2 * kKStages + 2 * kVStages + 11;  // k_full k_empty v_full v_empty s_full[2] s_empty[2] p_full[2] p_empty[2] row k_landed v_landed
     static constexpr int kOffMisc = kOffBar + kNumBars * 8;            // tmem slot, fail flag
-    static constexpr int kTotal = kOffMisc + 16;
+    static constexpr int kOffRow = (kOffMisc + 8 + 15) / 16 * 16;      // the appended row's two sides
+    static constexpr int kTotal = kOffRow + 2 * static_cast<int>(sizeof(tail::RowScratch<kD>));
     static constexpr int kAlloc = kTotal + 1024;                       // slack to align the base to 1024
 };
 static_assert(Smem<8>::kAlloc <= 232448, "one CTA per SM");
+static_assert(2 * Smem<8>::kPBuf >= (8 + 3 * 64 * 2) * 4, "the merger's scratch fits where P was");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
@@ -127,6 +130,14 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ int ordered(float f) { const int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); }
 __device__ __forceinline__ float unordered(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
 
+// The appended row's 256 bytes into row r of a K or V tile (two 128-byte-wide halves, 128-byte swizzle); lanes 0-15.
+__device__ __forceinline__ void patch_row(uint8_t* tile, const uint8_t* row, uint32_t r, int lane) {
+    if (lane < 16) {
+        const uint32_t c = lane & 7;
+        *reinterpret_cast<uint4*>(tile + (lane >> 3) * kHalfTile + r * 128 + ((c ^ (r & 7)) << 4)) = *reinterpret_cast<const uint4*>(row + lane * 16);
+    }
+}
+
 // NBLK scales per row (8 = q8_0 blocks of 32, 1 = one per row); G query heads per kv head (at most 8).
 template <int NBLK, int G, bool Q_F16>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -139,7 +150,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t split = blockIdx.x, kv_head = blockIdx.y, session = blockIdx.z;
+    const uint32_t kv_head = blockIdx.x, split = blockIdx.y, session = blockIdx.z;
     const b200kv_view& view = p.view;
     uint32_t begin, end;
     resolve_range(p, session, view, &begin, &end);
@@ -152,7 +163,11 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     const uint32_t t1 = tile_begin + static_cast<uint32_t>(total_tiles * (split + 1) / num_splits);
     const int ntiles = static_cast<int>(t1 - t0);
     // With launch overlap the previous kernel may still be appending: rows at or above early_end wait for it.
-    const uint32_t early_end = end > p.overlap_tail ? end - p.overlap_tail : 0;
+    // The row that this launch appends does not count: the copy of it that comes with its tile is overwritten in shared memory.
+    const bool fuse = tail::appends_row(p, begin, end);
+    const bool owner = fuse && ntiles > 0 && t1 == tile_end;
+    const uint32_t needed_end = fuse ? end - 1 : end;
+    const uint32_t early_end = needed_end > p.overlap_tail ? needed_end - p.overlap_tail : 0;
 
     const uint32_t bar0 = sbase + L::kOffBar;
     auto bar_k_full = [&](int s) { return bar0 + s * 8; };
@@ -164,6 +179,10 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     auto bar_s_empty = [&](int b) { return bar0 + (kB0 + 2 + b) * 8; };
     auto bar_p_full = [&](int b) { return bar0 + (kB0 + 4 + b) * 8; };
     auto bar_p_empty = [&](int b) { return bar0 + (kB0 + 6 + b) * 8; };
+    const uint32_t bar_row = bar0 + (kB0 + 8) * 8;                                              // the appended row is in its scratch
+    // the tile it belongs to has landed (its "full" barriers follow when the row is in it)
+    const uint32_t bar_k_landed = bar0 + (kB0 + 9) * 8, bar_v_landed = bar0 + (kB0 + 10) * 8;
+    tail::RowScratch<kD>* new_row = reinterpret_cast<tail::RowScratch<kD>*>(smem + L::kOffRow);   // K, V
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
     uint32_t* fail_flag = tmem_slot + 1;
 
@@ -177,7 +196,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     auto issue_k = [&](int i) {
         const int stage = i % kKStages;
         const uint32_t pos0 = (t0 + i) * kTileM;
-        const uint32_t bar = bar_k_full(stage);
+        const uint32_t bar = owner && i == ntiles - 1 ? bar_k_landed : bar_k_full(stage);
         mbar_expect_tx(bar, L::kKTile);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf)
@@ -187,7 +206,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
         const int stage = i % kVStages;
         const uint32_t pos0 = (t0 + i) * kTileM;
         const uint32_t sbytes = min(static_cast<uint32_t>(kTileM), capacity - pos0) * (NBLK * 2);
-        const uint32_t bar = bar_v_full(stage);
+        const uint32_t bar = owner && i == ntiles - 1 ? bar_v_landed : bar_v_full(stage);
         mbar_expect_tx(bar, L::kKTile + 2 * sbytes);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf)
@@ -200,7 +219,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     // ---- set-up ---------------------------------------------------------------------------------------------
     // tiles whose rows are old enough to be fetched before the dependency wait
     int early = 0;
-    while (early < ntiles && early < kVStages && (t0 + early + 1) * kTileM <= early_end) ++early;
+    while (early < ntiles && early < kVStages && min((t0 + early + 1) * kTileM, needed_end) <= early_end) ++early;
     const int k_early = min(early, kKStages), v_early = early;
     if (warp == kProducerWarp) {
         if (lane == 0) {
@@ -210,6 +229,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
                 mbar_init(bar_s_full(b), 1); mbar_init(bar_s_empty(b), kConsumers);
                 mbar_init(bar_p_full(b), kConsumers); mbar_init(bar_p_empty(b), 1);
             }
+            mbar_init(bar_row, 1); mbar_init(bar_k_landed, 1); mbar_init(bar_v_landed, 1);
             *fail_flag = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -220,7 +240,15 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    const bool appends = owner && warp == kPvWarp;
+    Rotation<kD> rot{};
+    if (appends) row_rotation<kD>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();
+    float new_k[kD / 32], new_v[kD / 32];
+    if (appends) {
+        tail::load_new_row<kD>(p.new_key, p.new_is_f16, kv_head, lane, new_k);
+        tail::load_new_row<kD>(p.new_value, p.new_is_f16, kv_head, lane, new_v);
+    }
     // the rest of the first ring fill, by the thread that set the barriers up
     if (warp == kProducerWarp && lane == 0)
         for (int i = 0; i < min(kVStages, ntiles); ++i) {
@@ -293,6 +321,17 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
                 issue_k(i);
             }
         }
+        if (owner) {   // the last tile's K has landed and the new row is in its scratch: put the row into the tile, then let its readers at it
+            const int stage = (ntiles - 1) % kKStages;
+            bool ready = !failed;
+            if (lane == 0) ready = ready && mbar_wait(bar_k_landed, 0) && mbar_wait(bar_row, 0);
+            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0)) {
+                patch_row(smem + L::kOffK + stage * L::kKTile, new_row[0].data, (end - 1) % kTileM, lane);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read the tile through the async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_k_full(stage));
+            }
+        }
     } else if (warp == kVProducerWarp) {
         // =============================== TMA producer, V and scale tiles ===============================
         if (lane == 0) {
@@ -300,6 +339,24 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
                 // V stage i % kVStages is free once the P.V of tile i - kVStages has completed
                 if (!mbar_wait(bar_v_empty(i % kVStages), static_cast<uint32_t>((i / kVStages - 1) & 1))) { failed = true; break; }
                 issue_v(i);
+            }
+        }
+        if (owner) {   // the same for V and the scales
+            const int stage = (ntiles - 1) % kVStages;
+            bool ready = !failed;
+            if (lane == 0) ready = ready && mbar_wait(bar_v_landed, 0) && mbar_wait(bar_row, 0);
+            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0)) {
+                const uint32_t r = (end - 1) % kTileM;
+                patch_row(smem + L::kOffV + stage * L::kKTile, new_row[1].data, r, lane);
+                if (lane >= 16 && lane < 18) {
+                    const int side = lane - 16;
+                    uint8_t* dst = smem + L::kOffS + stage * 2 * L::kSTile + side * L::kSTile + r * (NBLK * 2);
+                    if constexpr (NBLK == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(new_row[side].scales);
+                    else *reinterpret_cast<__half*>(dst) = new_row[side].scales[0];
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_v_full(stage));
             }
         }
     } else if (warp == kMmaWarp) {
@@ -321,7 +378,13 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
             }
         }
     } else if (warp == kPvWarp) {
-        // =============================== issuer of O^T = V^T . P ===============================
+        // =============================== the fused append, then the issuer of O^T = V^T . P ===============================
+        if (appends) {
+            tail::store_new_key<kD>(p, view, new_k, rot, head_row0 + end - 1, lane, new_row);
+            tail::store_new_value<kD>(view, new_v, head_row0 + end - 1, lane, new_row + 1);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_row);
+        }
         if (lane == 0) {
             constexpr uint32_t idesc_o = umma_idesc_i8(128, 64, 1, 0, 1, 1);    // V^T (signed, MN-major) x P planes (unsigned, MN-major)
             for (int i = 0; i < ntiles; ++i) {
@@ -563,10 +626,9 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
                 float lt = fmaf(l0, s0, l1 * s1);
                 float mh = M * 0.6931471805599453f;   // natural-log units, as the merge expects
                 if (poisoned) { a0 = a1 = mh = lt = __int_as_float(0x7fc00000); }
-                const size_t slot = (static_cast<size_t>(session) * p.num_splits + split) * p.query_heads + kv_head * G + h;
-                p.ws_acc[slot * kD + ltid] = a0;
-                p.ws_acc[slot * kD + 128 + ltid] = a1;
-                if (ltid == 0) { p.ws_m[slot] = mh; p.ws_l[slot] = lt; }
+                const uint32_t head = kv_head * G + h;
+                tail::emit_partial<2>(p, session, split, num_splits, head, ltid, a0, mh, lt);
+                tail::emit_partial<2>(p, session, split, num_splits, head, 128 + ltid, a1, mh, lt);
             }
         }
     }
@@ -578,6 +640,8 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
+    if (p.ws_tagged == nullptr || tid >= 256) return;   // a separate merge kernel follows, or this warp has no part in the merge
+    tail::fused_merge<2, 256>(p, session, kv_head, split, num_splits, G, reinterpret_cast<float*>(smem + L::kOffP));
 }
 
 // ---- host side -----------------------------------------------------------------------------------------
@@ -655,20 +719,19 @@ uint32_t pick_splits_tc5_wide(const b200kv_view& view, uint32_t max_length) {
     return s ? s : 1;
 }
 
-// Stage 1 of a single-session launch into the plain partial arrays (p.ws_m / ws_l / ws_acc, p.num_splits set by the
-// caller); B200KV_ERR_UNSUPPORTED when the launch is not one this kernel takes.
+// A single-session launch (p.num_splits and the workspace pointers set by the caller); B200KV_ERR_UNSUPPORTED when the
+// launch is not one this kernel takes.
 int launch_decode_tc5_wide(const DecodeParams& p_in, const b200kv_view& geometry, cudaStream_t stream) {
     if (!decode_tc5_wide_ok(geometry, p_in.query_heads)) return B200KV_ERR_UNSUPPORTED;
-    if (p_in.views != nullptr || p_in.lengths != nullptr || p_in.causal || p_in.sessions != 1 || p_in.new_key != nullptr)
+    if (p_in.views != nullptr || p_in.lengths != nullptr || p_in.sessions != 1)
         return B200KV_ERR_UNSUPPORTED;
     DecodeParams p = p_in;
     p.overlap_tail = launch_overlap_tail();
-    p.ws_tagged = nullptr;
     CUtensorMap kmap, vmap;
     if (!encode_wide_plane(&kmap, geometry.key_q8, geometry) || !encode_wide_plane(&vmap, geometry.value_q8, geometry)) return B200KV_ERR_UNSUPPORTED;
     const bool blocks = geometry.qblock == 32;
     const uint32_t g = p.query_heads / geometry.kv_heads;
-    dim3 grid(p.num_splits, geometry.kv_heads, 1);
+    const dim3 grid(geometry.kv_heads, p.num_splits, 1);   // kv head fastest, as in decode_tc5.cu
     if (blocks) {
         if (g == 4) return launch_q<8, 4>(p, kmap, vmap, grid, stream);
         if (g == 6) return launch_q<8, 6>(p, kmap, vmap, grid, stream);

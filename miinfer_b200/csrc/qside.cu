@@ -59,7 +59,9 @@ __global__ void __launch_bounds__(kQSideWarps * 32) q_split_norm_rope_kernel(con
         }
         if (p.gate != nullptr) p.gate[out_base + lane + 32 * j] = g;
     }
-    transform_k_row<D>(q, lane, base_position + token, p.q_norm_weight, p.epsilon, p.rope_mode, p.inv_freq, p.sectioned_step);
+    Rotation<D> rot;
+    row_rotation<D>(rot, lane, base_position + token, p.rope_mode, p.inv_freq, p.sectioned_step);
+    transform_k_row<D>(q, lane, p.q_norm_weight, p.epsilon, p.rope_mode, rot);
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
         if (OUT_F16) static_cast<__half*>(p.query)[out_base + lane + 32 * j] = __float2half_rn(q[j]);

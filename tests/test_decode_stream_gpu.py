@@ -1,0 +1,89 @@
+"""The decode kernel that serves every cache mode and shape (csrc/decode_stream.cu), at the edges of its tiles (16
+positions), warps, splits and alignments: batched launches, and decode steps with the append fused in."""
+import numpy as np
+import pytest
+import torch
+
+import kvoracle as ko
+from gpu_util import assert_planes_equal, to_dev, upload
+from miinfer_b200 import kv
+
+pytestmark = pytest.mark.gpu
+# fp32 sums of products exact to 2^-22 and ex2.approx (2^-22) weights: 1e-5 relative leaves room for a few thousand terms
+REL = 1.0e-5
+
+
+def _filled(rng, L, H, d, qb, mode, cap):
+    host = ko.HostCache(cap, H, d, qb, mode)
+    host.append(ko.normal_f16(rng, (L, H * d)).astype(np.float32), ko.normal_f16(rng, (L, H * d)).astype(np.float32), None, 0, rope_mode=0)
+    return host
+
+
+def _close(got, ref, what):
+    rel = np.linalg.norm(got.astype(np.float64) - ref) / np.linalg.norm(ref)
+    assert np.isfinite(got).all() and rel <= REL, (what, rel)
+
+
+# odd capacities: 2-byte aligned row scales, 8-byte aligned block scales
+@pytest.mark.parametrize("d,H,Hq,qb,mode", [(256, 4, 24, 32, 3), (256, 4, 24, 256, 3), (256, 2, 16, 256, 0), (256, 1, 3, 256, 1), (256, 2, 4, 32, 2),
+                                            (128, 8, 32, 128, 0), (128, 2, 14, 32, 3), (128, 3, 3, 128, 2), (128, 2, 10, 128, 3), (128, 2, 8, 32, 1)])
+def test_batched_lengths_at_tile_and_split_edges(cuda, d, H, Hq, qb, mode):
+    rng = np.random.default_rng(d + H + qb + mode)
+    lengths = [1, 15, 16, 17, 127, 129, 511, 700]
+    hosts = [_filled(rng, n, H, d, qb, mode, n + 1 + n % 3) for n in lengths]
+    q16 = ko.normal_f16(rng, (len(lengths), Hq, d), 2.0)
+    gate = rng.standard_normal((len(lengths), Hq, d)).astype(np.float32)
+    sts, table = [upload(h) for h in hosts], kv.view_table(len(lengths))
+    lens, ws = torch.tensor(lengths, dtype=torch.int32, device="cuda"), kv.decode_workspace(Hq, d, len(lengths))
+    for q in (to_dev(q16), to_dev(q16.astype(np.float32) * 1.37)):
+        for splits in (0, 5, 128):   # 128: more CTAs per session than fit on the device with some shapes, so the merge is a launch of its own
+            out, gated = (torch.full((len(lengths), Hq, d), float("nan"), device="cuda") for _ in range(2))
+            kv.launch_decode_attention_batched([s.view() for s in sts], table, lens, max(lengths), q, query_heads=Hq, scale=d ** -0.5,
+                                               output=out, gate=to_dev(gate), gated_output=gated, workspace=ws, num_splits=splits | kv.FORCE_GENERIC)
+            for i, h in enumerate(hosts):
+                ref, ref_g = h.decode_ref(q[i].float().cpu().numpy(), d ** -0.5, lengths[i], gate[i])
+                _close(out[i].cpu().numpy(), ref, (lengths[i], splits))
+                _close(gated[i].cpu().numpy(), ref_g, (lengths[i], splits, "gated"))
+
+
+@pytest.mark.parametrize("d,H,Hq,qb,mode,dtype", [(256, 4, 24, 256, 0, np.float16), (256, 4, 24, 32, 3, np.float32), (256, 4, 24, 256, 3, np.float32),
+                                                  (128, 8, 32, 32, 1, np.float16), (128, 8, 32, 128, 2, np.float32), (128, 8, 32, 32, 3, np.float16)])
+def test_fused_append_in_every_mode(cuda, d, H, Hq, qb, mode, dtype):
+    rng = np.random.default_rng(7 * d + qb + mode)
+    w = (1.0 + 0.1 * rng.standard_normal(d)).astype(np.float32)
+    for L0 in (0, 15, 127, 1150):        # the new row first in a tile, last in one, behind many tiles; alone in the cache
+        host = _filled(rng, max(L0, 1), H, d, qb, mode, 1211)
+        st, ws = upload(host), kv.decode_workspace(Hq, d)
+        for step in range(3):
+            kn, vn = (rng.standard_normal((1, H * d)).astype(dtype) for _ in range(2))
+            q = rng.standard_normal((Hq, d)).astype(dtype)
+            pos = L0 + step
+            host.append(kn.astype(np.float32), vn.astype(np.float32), w, pos, rope_mode=1 + step % 2)
+            out = torch.full((Hq, d), float("nan"), device="cuda")
+            kv.launch_decode_step(st.view(), to_dev(kn), to_dev(vn), to_dev(q), query_heads=Hq, scale=d ** -0.5, k_norm_weight=to_dev(w),
+                                  rope_mode=kv.RopeMode(1 + step % 2), output=out, workspace=ws, num_splits=kv.FORCE_GENERIC,
+                                  **({"position": pos} if step != 1 else {"decode_state": kv.make_decode_state(pos)}))
+            ref, _ = host.decode_ref(q.astype(np.float32), d ** -0.5, pos + 1)
+            _close(out.cpu().numpy(), ref, (L0, step))
+        assert_planes_equal(st, host, f"mode {mode} at {L0}")
+    # a device-side position beyond the capacity appends nothing
+    before = [t.clone() for t in st.planes()]
+    kv.launch_decode_step(st.view(), to_dev(kn), to_dev(vn), to_dev(q), query_heads=Hq, scale=d ** -0.5, rope_mode=kv.RopeMode.NONE, output=out,
+                          workspace=ws, decode_state=kv.make_decode_state(1211))
+    assert all(torch.equal(a, b) for a, b in zip(before, st.planes())) and torch.isfinite(out).all()
+
+
+def test_value_scales_that_grow_by_orders_of_magnitude(cuda):
+    """The multiplier of the weights is re-chosen, and the sums rescaled, when a later tile's value scales outgrow it."""
+    rng = np.random.default_rng(3)
+    for d, qb in ((256, 32), (256, 256), (128, 32)):
+        L, H, Hq = 700, 2, 8
+        host = ko.HostCache(L, H, d, qb, 3)
+        v = ko.normal_f16(rng, (L, H * d)).astype(np.float32) * np.logspace(-4, 3, L, dtype=np.float32)[:, None]
+        host.append(ko.normal_f16(rng, (L, H * d)).astype(np.float32), v.astype(np.float16).astype(np.float32), None, 0, rope_mode=0)
+        st, q16, out = upload(host), ko.normal_f16(rng, (Hq, d)), torch.empty(Hq, d, device="cuda")
+        ref, _ = host.decode_ref(q16.astype(np.float32), d ** -0.5, L)
+        for splits in (1, 3):
+            kv.launch_decode_attention_quant(st.view(), to_dev(q16), query_heads=Hq, scale=d ** -0.5, cache_length=L, output=out,
+                                             workspace=kv.decode_workspace(Hq, d), num_splits=splits | kv.FORCE_GENERIC)
+            _close(out.cpu().numpy(), ref, (d, qb, splits))
