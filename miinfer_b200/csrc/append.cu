@@ -5,22 +5,22 @@
 // Behaviour follows MIInfer's store kernel
 // (gfx906/kernels/qwen3_primitives.hip:7213-7326): same operation order, same
 // quantizer, positions optionally read from device-resident state.  The mapping
-// is new: the unit of work is one PASS of one token -- 16 K blocks and 16 V blocks of 32 dims, i.e. four kv heads
-// at head_dim 128, two at 256 -- and every warp of a grid sized to the device takes one contiguous run of units.
-//   - K rows: lane L holds elements L, L+32, L+64, ... so a q8_0 block is one register index across the warp (its
-//     maximum is one `redux.sync` on the bits of |x|), both RoPE pairings (i, i+d/2) and (i, i+32) pair two
-//     registers of the SAME lane, and the reference's shared-memory binary tree for the sum of squares (stride
-//     d/2 .. 1) becomes register adds followed by a shuffle-down tree that adds exactly the same pairs in the same
-//     order (bit-identical sum).  Elements are read and written one by one: every access of the warp is one
-//     contiguous run of 32 elements, so nothing is staged.
-//   - V rows, which are only quantised: lane L holds the 4 (8) consecutive elements 4L .. (8L ..), one vector load and
-//     one vector store per row; a block is 8 (4) neighbouring lanes and its maximum takes 3 (2) shuffles.
-//   - the sines and cosines depend on the token only and are computed when a warp's run reaches a new token;
-//   - the warp-uniform IEEE divisions are spread over the lanes: lane h takes head h's 1/rms, lanes 0-15 the K
-//     blocks' amax/127 and reciprocal, lanes 16-31 the V blocks'; the results come back by shuffle.
-// (Earlier layouts -- a warp per row pair with every division repeated by all lanes; all rows lane-strided through
-// shared-memory staging rows -- ran at 0.11 and 0.33 of the HBM rate on 8192-token chunks; this one at 0.37.  Fetching a
-// unit's rows one unit ahead of the arithmetic measured slower: 34 us against 21.5.)
+// is new: the unit of work is 1024 elements of K or of V of one token -- eight kv heads at head_dim 128, four at 256, 32
+// q8_0 blocks -- and every warp of a grid sized to the device takes one contiguous run of units.
+//   - The next unit's input is fetched into registers as it lies (16 of them for fp16) before the arithmetic of the current one.
+//   - D/8 lanes hold a row, lane l of them elements 4l .. 4l+3 and D/2 + 4l .. D/2 + 4l+3: NeoX pairs (i, i + d/2) lie in
+//     one lane, sectioned pairs (i, i + 32) eight lanes apart, and every store is four bytes of int8 per lane.
+//   - The reference's shared-memory binary tree for the sum of squares (stride d/2 .. 1) becomes one register add and a
+//     butterfly that adds exactly the same pairs (addition commutes: identical bits); each exchange halves the values a
+//     lane carries.
+//   - The 32 block maxima are reduced the same way, eight values over eight lanes in seven shuffles, and come out one
+//     block per lane -- so each IEEE division (scale, reciprocal, 1/rms) is taken once, by one lane.
+//   - The sines and cosines depend on the token only; they are computed while the unit's data is in flight.
+//   - Products run two to an instruction (f32x2), four int8 are packed by two cvt.pack.
+// Bound by instruction issue (half of all issue slots at 8192 tokens; the writes stay in L2): 8192 tokens x 8 heads of 128
+// dims, fp16 to q8_0, take 17.1 us.  A layout with lanes 32 elements apart, element-wise K accesses and one redux per block
+// took 21.8 us; this layout with its input in a cp.async ring 20.0 us alone, and its shared memory kept the next
+// layer's launch off SMs that still held attention CTAs (4 us a layer).
 // The row arithmetic is the same, operation for operation, as append_row.cuh's (used by the decode kernel's fused
 // single-token append and the query-side kernel): all three write identical bits.
 #include "append_row.cuh"
@@ -47,16 +47,92 @@ struct AppendParams {
 };
 
 constexpr int kAppendWarps = 2;
-constexpr int kAppendCtasPerSm = 8;    // 128 registers per thread: a pass keeps 32 row values per lane (10, 12 and 16 CTAs spill and measured slower)
+constexpr int kUnitElems = 1024;       // 32 q8_0 blocks: one scale per lane
+template <bool IN_F16>
+constexpr int kAppendCtasPerSm = IN_F16 ? 10 : 8;   // 20 warps of 96 registers: a unit, the next one's raw input and the rotation (fp32 input: 16 of 128)
+
+// Two fp32 products in one instruction (each rounds like its scalar form; .ftz as the scalar intrinsics under this build).
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pack(float lo, float hi) { Pair r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 unpack(Pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) { Pair r; asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// Sums of products are taken one at a time: an f32x2 add behind an f32x2 multiply came out contracted (measured: single
+// fp16 results one unit off the oracle's), the scalar intrinsics never are.
+__device__ __forceinline__ Pair add_products(Pair t, Pair u) {
+    const float2 a = unpack(t), b = unpack(u);
+    return pack(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+__device__ __forceinline__ Pair sub_products(Pair t, Pair u) {
+    const float2 a = unpack(t), b = unpack(u);
+    return pack(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
+}
+
+// Four consecutive input elements as they lie in memory, and as two pairs of floats.
+template <bool IN_F16> struct Raw4 { uint2 v; };
+template <> struct Raw4<false> { float4 v; };
+template <bool IN_F16>
+__device__ __forceinline__ Raw4<IN_F16> load4(const void* src, size_t element, bool vec) {
+    Raw4<IN_F16> r;
+    if constexpr (IN_F16) {
+        const __half* s = static_cast<const __half*>(src) + element;
+        if (vec) {
+            r.v = *reinterpret_cast<const uint2*>(s);
+        } else {
+            const uint16_t* u = reinterpret_cast<const uint16_t*>(s);
+            r.v = make_uint2(u[0] | (static_cast<uint32_t>(u[1]) << 16), u[2] | (static_cast<uint32_t>(u[3]) << 16));
+        }
+    } else {
+        const float* s = static_cast<const float*>(src) + element;
+        r.v = vec ? *reinterpret_cast<const float4*>(s) : make_float4(s[0], s[1], s[2], s[3]);
+    }
+    return r;
+}
+template <bool IN_F16>
+__device__ __forceinline__ void widen(const Raw4<IN_F16>& r, Pair (&x)[2]) {
+    if constexpr (IN_F16) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&r.v.y));
+        x[0] = pack(a.x, a.y); x[1] = pack(b.x, b.y);
+    } else {
+        x[0] = pack(r.v.x, r.v.y); x[1] = pack(r.v.z, r.v.w);
+    }
+}
+__device__ __forceinline__ float amax4(const Pair (&x)[2]) {
+    const float2 a = unpack(x[0]), b = unpack(x[1]);
+    return fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))), 0.0f);   // a NaN counts as 0, as in warp_amax
+}
+// round to nearest even, saturate to [-128, 127], NaN -> 0: quantize_s8 on four values, packed
+__device__ __forceinline__ uint32_t quantize4(const Pair (&x)[2], float inv) {
+    const Pair inv2 = pack(inv, inv);
+    const float2 a = unpack(mul2(x[0], inv2)), b = unpack(mul2(x[1], inv2));
+    uint32_t w;
+    asm("{ .reg .b32 t; cvt.pack.sat.s8.s32.b32 t, %4, %3, 0; cvt.pack.sat.s8.s32.b32 %0, %2, %1, t; }"
+        : "=r"(w) : "r"(__float2int_rn(a.x)), "r"(__float2int_rn(a.y)), "r"(__float2int_rn(b.x)), "r"(__float2int_rn(b.y)));
+    return w;
+}
+__device__ __forceinline__ uint2 half4(const Pair (&x)[2]) {
+    const float2 a = unpack(x[0]), b = unpack(x[1]);
+    const __half2 lo = __floats2half2_rn(a.x, a.y), hi = __floats2half2_rn(b.x, b.y);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
 
 template <int D, bool IN_F16>
-__global__ void __launch_bounds__(kAppendWarps * 32, kAppendCtasPerSm)
+__global__ void __launch_bounds__(kAppendWarps * 32, kAppendCtasPerSm<IN_F16>)
 append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
-    constexpr int NJ = D / 32;                  // q8_0 blocks per row = K registers per lane
-    constexpr int HB = 16 / NJ;                 // kv heads per pass: 16 K blocks + 16 V blocks, one scale per lane
-    constexpr int GS = 32 / NJ;                 // lanes that share one V block (each holds NJ consecutive elements of it)
-    __shared__ float freq_s[D / 2];
-    __shared__ float kmax_s[kAppendWarps][16];
+    constexpr int LPR = D / 8;                  // lanes per row
+    constexpr int RPS = 32 / LPR;               // rows per step
+    constexpr int HB = kUnitElems / D;          // kv heads per unit, four steps
+    constexpr int NB = D / 32;                  // q8_0 blocks per row
+    static_assert(HB == 4 * RPS);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int l = lane & (LPR - 1), sub = lane / LPR;          // lane of the row, row of the step
+    const int rope_mode = p.rope_mode;
+    // NeoX: the lane rotates pairs 4l .. 4l+3; the two rows of a step at head_dim 128 share them, so each of their lanes
+    // evaluates two and fetches the other two
+    constexpr int SC = 4 / RPS;
+    float freq[SC];
+    if (rope_mode == B200KV_ROPE_NEOX_FULL)
+#pragma unroll
+        for (int i = 0; i < SC; ++i) freq[i] = p.inv_freq[4 * l + SC * sub + i];
     // Let the next kernel of the stream become resident now (it orders itself against this one), then wait
     // for everything before us: K/V inputs and the device-side position come from preceding kernels.
     pdl_launch_dependents();
@@ -73,254 +149,204 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
         base_position = p.decode_state->position;
         token_count = min(token_count, 1u);
     }
-    if (p.rope_mode == B200KV_ROPE_NEOX_FULL)
-        for (int i = threadIdx.x; i < D / 2; i += kAppendWarps * 32) freq_s[i] = p.inv_freq[i];
-    __syncthreads();
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t H = p.view.kv_heads;
     const uint32_t mode = p.view.quant_mode;
     const bool k_q8 = (mode == B200KV_Q8_F16 || mode == B200KV_Q8_Q8);
     const bool v_q8 = (mode == B200KV_F16_Q8 || mode == B200KV_Q8_Q8);
     const bool row_scale = p.view.qblock == D;
     const bool have_norm = p.k_norm_weight != nullptr;
-    const int rope_mode = p.rope_mode;
 
-    float w[NJ];
-    if (have_norm) {
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) w[j] = p.k_norm_weight[lane + 32 * j];
-    }
-    float sn[NJ / 2], cs[NJ / 2];   // what depends on the token alone: the rotation of every pair this lane holds
-
-    // One pass: K and V of kv heads g0 .. g0 + hn - 1 of one token.
-    //   K rows: lane L holds elements L, L+32, ... (a block = one register index across the warp), fetched and stored
-    //           element by element -- every access of the warp is one contiguous run of 32 elements;
-    //   V rows: lane L holds the NJ consecutive elements NJ*L ..  (a block = GS neighbouring lanes), one vector load and
-    //           one vector store per row.
-    // FAST: a full pass (hn == HB) of an int8/int8 cache with q8_0 blocks -- every check below is decided at compile time.
-    auto pass = [&](auto fast_c, uint32_t token, uint32_t g0, uint64_t position, int hn) {
-        constexpr bool FAST = decltype(fast_c)::value;
-        if constexpr (FAST) hn = HB;
-        const bool kq = FAST || k_q8, vq = FAST || v_q8, rows = !FAST && row_scale;
-        const uint64_t row0 = g0 * capacity + position;   // cache row of the pass's first head; the next head is `capacity` rows on
-        const size_t in0 = (static_cast<size_t>(token) * H + g0) * D;
-        float kx[HB][NJ], vx[HB][NJ];
-#pragma unroll
-        for (int h = 0; h < HB; ++h) {
-            if (!FAST && h >= hn) break;
-            const size_t in_h = in0 + static_cast<size_t>(h) * D;
-            if (IN_F16) {
-                const __half* ksrc = static_cast<const __half*>(p.key) + in_h;
-                const __half* vsrc = static_cast<const __half*>(p.value) + in_h + NJ * lane;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) kx[h][j] = __half2float(ksrc[lane + 32 * j]);
-                if (vec) {
-                    if constexpr (NJ == 4) {
-                        const uint2 raw = *reinterpret_cast<const uint2*>(vsrc);
-                        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                        vx[h][0] = a.x; vx[h][1] = a.y; vx[h][2] = b.x; vx[h][3] = b.y;
-                    } else {
-                        const uint4 raw = *reinterpret_cast<const uint4*>(vsrc);
-                        const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u[i]));
-                            vx[h][2 * i] = a.x; vx[h][2 * i + 1] = a.y;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < NJ; ++j) vx[h][j] = __half2float(vsrc[j]);
-                }
-            } else {
-                const float* ksrc = static_cast<const float*>(p.key) + in_h;
-                const float* vsrc = static_cast<const float*>(p.value) + in_h + NJ * lane;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) kx[h][j] = ksrc[lane + 32 * j];
-                if (vec) {
-#pragma unroll
-                    for (int i = 0; i < NJ / 4; ++i) {
-                        const float4 a = *reinterpret_cast<const float4*>(vsrc + 4 * i);
-                        vx[h][4 * i] = a.x; vx[h][4 * i + 1] = a.y; vx[h][4 * i + 2] = a.z; vx[h][4 * i + 3] = a.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < NJ; ++j) vx[h][j] = vsrc[j];
-                }
-            }
-        }
-
-        // ---- K: RMSNorm * weight.  The reference's shared-memory tree (stride D/2 .. 1): register adds, then a shuffle-down
-        //      tree over the same pairs; lane h then takes head h's IEEE division and square root ----
-        if (have_norm) {
-            float ss_mine = 0.0f;
-#pragma unroll
-            for (int h = 0; h < HB; ++h) {
-                if (!FAST && h >= hn) break;
-                float sq[NJ];
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) sq[j] = __fmul_rn(kx[h][j], kx[h][j]);
-#pragma unroll
-                for (int half = NJ / 2; half >= 1; half >>= 1)
-#pragma unroll
-                    for (int j = 0; j < half; ++j) sq[j] = __fadd_rn(sq[j], sq[j + half]);
-                float ss = sq[0];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss = __fadd_rn(ss, __shfl_down_sync(0xffffffffu, ss, o));
-                ss = __shfl_sync(0xffffffffu, ss, 0);
-                if (lane == h) ss_mine = ss;
-            }
-            const float r_mine = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss_mine, static_cast<float>(D)), p.epsilon)));
-#pragma unroll
-            for (int h = 0; h < HB; ++h) {
-                if (!FAST && h >= hn) break;
-                const float r = __shfl_sync(0xffffffffu, r_mine, h);
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) kx[h][j] = __fmul_rn(__fmul_rn(kx[h][j], r), w[j]);
-            }
-        }
-        // ---- K: RoPE
-        if (rope_mode == B200KV_ROPE_NEOX_FULL) {
-#pragma unroll
-            for (int h = 0; h < HB; ++h) {
-                if (!FAST && h >= hn) break;
-#pragma unroll
-                for (int j = 0; j < NJ / 2; ++j) {
-                    const float x0 = kx[h][j], x1 = kx[h][j + NJ / 2];
-                    kx[h][j] = __fsub_rn(__fmul_rn(x0, cs[j]), __fmul_rn(x1, sn[j]));
-                    kx[h][j + NJ / 2] = __fadd_rn(__fmul_rn(x0, sn[j]), __fmul_rn(x1, cs[j]));
-                }
-            }
-        } else if (rope_mode == B200KV_ROPE_SECTIONED64) {
-#pragma unroll
-            for (int h = 0; h < HB; ++h) {
-                if (!FAST && h >= hn) break;
-                const float x0 = kx[h][0], x1 = kx[h][1];
-                kx[h][0] = __fsub_rn(__fmul_rn(x0, cs[0]), __fmul_rn(x1, sn[0]));
-                kx[h][1] = __fadd_rn(__fmul_rn(x0, sn[0]), __fmul_rn(x1, cs[0]));
-            }
-        }
-
-        // ---- block maxima.  K: one redux per block, the 16 results through shared memory to lanes 0-15 (lane = HB... NJ*h + j).
-        //      V: a block's GS lanes reduce among themselves; lane 16 + NJ*h + j fetches the result from the block's first lane.
-        //      With one scale per row (rows): lanes h and 16 + h. ----
-        float amax_mine = 0.0f;
-#pragma unroll
-        for (int h = 0; h < HB; ++h) {
-            if (!FAST && h >= hn) break;
-            if (rows) {
-                float a = 0.0f, b = 0.0f;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) { a = fmaxf(a, fabsf(kx[h][j])); b = fmaxf(b, fabsf(vx[h][j])); }
-                a = warp_amax(a); b = warp_amax(b);
-                if (lane == h) amax_mine = a;
-                if (lane == 16 + h) amax_mine = b;
-            } else {
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) kmax_s[warp][NJ * h + j] = warp_amax(fabsf(kx[h][j]));   // every lane holds the value: no predicate
-                float b = 0.0f;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) b = fmaxf(b, fabsf(vx[h][j]));
-#pragma unroll
-                for (int o = GS / 2; o > 0; o >>= 1) b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
-                const float got = __shfl_sync(0xffffffffu, b, (lane & (NJ - 1)) * GS);   // block j = lane % NJ of head h
-                if ((lane >> 4) == 1 && ((lane & 15) / NJ) == h) amax_mine = got;
-            }
-        }
-        if (!rows) {
-            __syncwarp();
-            if (lane < 16) amax_mine = kmax_s[warp][lane];
-            __syncwarp();   // the next pass overwrites the words
-        }
-        // ---- scales: amax / 127, its reciprocal, the fp16 scale to the cache -- one block per lane
-        const float scale_mine = (amax_mine > 0.0f) ? __fdiv_rn(amax_mine, 127.0f) : 1.0f;
-        const float inv_mine = (scale_mine > 0.0f) ? __fdiv_rn(1.0f, scale_mine) : 1.0f;
-        {
-            const int side = lane >> 4, idx = lane & 15;
-            const int h = rows ? idx : idx / NJ, j = rows ? 0 : idx % NJ;
-            const bool mine = rows ? idx < hn : h < hn;
-            if (mine && (side == 0 ? kq : vq)) {
-                __half* plane = static_cast<__half*>(side == 0 ? p.view.key_scales : p.view.value_scales);
-                const uint64_t r = row0 + static_cast<uint64_t>(h) * capacity;
-                plane[rows ? r : r * NJ + j] = __float2half_rn(scale_mine);
-            }
-        }
-        // ---- quantise and store
-#pragma unroll
-        for (int h = 0; h < HB; ++h) {
-            if (!FAST && h >= hn) break;
-            const uint64_t r = row0 + static_cast<uint64_t>(h) * capacity;
-            if (kq) {
-                int8_t* dst = p.view.key_q8 + r * D + lane;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) {
-                    const float inv = __shfl_sync(0xffffffffu, inv_mine, rows ? h : NJ * h + j);
-                    dst[32 * j] = static_cast<int8_t>(quantize_s8(__fmul_rn(kx[h][j], inv)));
-                }
-            } else {
-                __half* dst = static_cast<__half*>(p.view.key_f16) + r * D + lane;
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) dst[32 * j] = __float2half_rn(kx[h][j]);
-            }
-            if (vq) {
-                const float inv = __shfl_sync(0xffffffffu, inv_mine, 16 + (rows ? h : NJ * h + lane / GS));
-                uint32_t packed[NJ / 4];
-#pragma unroll
-                for (int i = 0; i < NJ / 4; ++i) {
-                    const uint32_t b0 = quantize_s8(__fmul_rn(vx[h][4 * i], inv)) & 0xff, b1 = quantize_s8(__fmul_rn(vx[h][4 * i + 1], inv)) & 0xff;
-                    const uint32_t b2 = quantize_s8(__fmul_rn(vx[h][4 * i + 2], inv)) & 0xff, b3 = quantize_s8(__fmul_rn(vx[h][4 * i + 3], inv)) & 0xff;
-                    packed[i] = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
-                }
-                int8_t* dst = p.view.value_q8 + r * D + NJ * lane;
-                if constexpr (NJ == 4) *reinterpret_cast<uint32_t*>(dst) = packed[0];
-                else *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
-            } else {
-                __half* dst = static_cast<__half*>(p.view.value_f16) + r * D + NJ * lane;
-#pragma unroll
-                for (int j = 0; j < NJ; j += 2) *reinterpret_cast<__half2*>(dst + j) = __floats2half2_rn(vx[h][j], vx[h][j + 1]);
-            }
-        }
-    };
-
-    // The unit of work is one pass of one token; every warp of the grid takes one contiguous run of units, so a
-    // large launch spreads evenly over the resident warps (and a warp meets few tokens), while a small one
-    // spreads the passes of a token over several warps.  (32-bit arithmetic: the host keeps units below 2^32.)
+    // Units in the order token, pass (HB heads), side (K, V).  (32-bit arithmetic: the host keeps units below 2^32.)
     const uint32_t passes = (H + HB - 1) / HB;
-    const uint32_t total_units = token_count * passes;
+    const uint32_t total_units = token_count * passes * 2;
     const uint32_t warps = gridDim.x * kAppendWarps;
     const uint32_t per_warp = (total_units + warps - 1) / warps;
     const uint32_t unit0 = min(total_units, (blockIdx.x * kAppendWarps + warp) * per_warp);
     const uint32_t unit1 = min(total_units, unit0 + per_warp);
-    uint32_t token = unit0 / passes;
-    uint32_t pass_index = unit0 - token * passes;
-    bool fresh = true;   // the rotation has to be computed for `token`
-    const bool fast_cache = k_q8 && v_q8 && !row_scale;
-    for (uint32_t unit = unit0; unit < unit1; ++unit) {
-        const uint64_t position = static_cast<uint64_t>(base_position) + token;
-        if (position < capacity) {   // never write outside the cache
-            if (fresh) {
-                fresh = false;
-                if (rope_mode == B200KV_ROPE_NEOX_FULL) {
+
+    struct Cursor { uint32_t token, pass, side; };
+    auto advance = [&](Cursor& c) {
+        if (++c.side == 2) {
+            c.side = 0;
+            if (++c.pass == passes) { c.pass = 0; ++c.token; }
+        }
+    };
+    auto inside = [&](const Cursor& c) { return static_cast<uint64_t>(base_position) + c.token < capacity; };   // never write outside the cache
+    auto heads = [&](const Cursor& c) { return static_cast<int>(min(static_cast<uint32_t>(HB), H - c.pass * HB)); };
+    Raw4<IN_F16> raw[4][2];   // per step: elements 4l .. and D/2 + 4l .. of the unit that comes next
+    auto fetch = [&](const Cursor& c) {
+        const void* src = c.side == 0 ? p.key : p.value;
+        const size_t e0 = (static_cast<size_t>(c.token) * H + c.pass * HB + sub) * D + 4 * l;
+        const int hn = heads(c);
 #pragma unroll
-                    for (int j = 0; j < NJ / 2; ++j)
-                        sincos_pinned(__fmul_rn(static_cast<float>(static_cast<uint32_t>(position)), freq_s[lane + 32 * j]), &sn[j], &cs[j]);
-                } else if (rope_mode == B200KV_ROPE_SECTIONED64) {
-                    float angle = static_cast<float>(static_cast<uint32_t>(position));
-                    for (int i = 0; i < lane; ++i) angle = __fmul_rn(angle, p.sectioned_step);
-                    sincos_pinned(angle, &sn[0], &cs[0]);
+        for (int s = 0; s < 4; ++s)
+            if (s * RPS + sub < hn) {
+                raw[s][0] = load4<IN_F16>(src, e0 + s * RPS * D, vec);
+                raw[s][1] = load4<IN_F16>(src, e0 + s * RPS * D + D / 2, vec);
+            } else {
+                raw[s][0] = raw[s][1] = Raw4<IN_F16>{};
+            }
+    };
+
+    Pair sn[2], cs[2];   // NeoX: pairs 4l + i; sectioned: pairs 4 (l % 8) + i
+    auto rotation = [&](uint32_t position) {
+        if (rope_mode == B200KV_ROPE_NEOX_FULL) {
+            float s[SC], c[SC];
+#pragma unroll
+            for (int i = 0; i < SC; ++i) sincos_pinned(__fmul_rn(static_cast<float>(position), freq[i]), &s[i], &c[i]);
+            if constexpr (RPS == 1) {
+                sn[0] = pack(s[0], s[1]); sn[1] = pack(s[2], s[3]);
+                cs[0] = pack(c[0], c[1]); cs[1] = pack(c[2], c[3]);
+            } else {
+                const Pair sm = pack(s[0], s[1]), cm = pack(c[0], c[1]);
+                const Pair so = __shfl_xor_sync(0xffffffffu, sm, 16), co = __shfl_xor_sync(0xffffffffu, cm, 16);
+                sn[0] = sub ? so : sm; sn[1] = sub ? sm : so;
+                cs[0] = sub ? co : cm; cs[1] = sub ? cm : co;
+            }
+        } else if (rope_mode == B200KV_ROPE_SECTIONED64) {
+            float angle = static_cast<float>(position), s, c;
+            for (int i = 0; i < lane; ++i) angle = __fmul_rn(angle, p.sectioned_step);
+            sincos_pinned(angle, &s, &c);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int src = 4 * (lane & 7) + 2 * i;
+                sn[i] = pack(__shfl_sync(0xffffffffu, s, src), __shfl_sync(0xffffffffu, s, src + 1));
+                cs[i] = pack(__shfl_sync(0xffffffffu, c, src), __shfl_sync(0xffffffffu, c, src + 1));
+            }
+        }
+    };
+
+    // FAST: a full unit (hn == HB) of a q8_0 side -- every check is decided at compile time.  Rows of a ragged unit that do
+    // not exist came in as zeros and are only not stored.
+    auto process = [&](auto fast_c, const Cursor& cur, Pair (&a)[4][2], Pair (&b)[4][2], uint64_t position, int hn) {
+        constexpr bool FAST = decltype(fast_c)::value;
+        if constexpr (FAST) hn = HB;
+        const bool is_k = cur.side == 0;
+        const bool quantised = FAST || (is_k ? k_q8 : v_q8), rows = !FAST && row_scale;
+        if (is_k) {
+            if (have_norm) {
+                float ss_mine = 0.0f;
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const bool up2 = lane & (LPR / 2), up1 = lane & (LPR / 4);
+                    const Pair q01 = add_products(mul2(a[s][0], a[s][0]), mul2(b[s][0], b[s][0])), q23 = add_products(mul2(a[s][1], a[s][1]), mul2(b[s][1], b[s][1]));   // stride D/2
+                    const float2 t = unpack(add_products(up2 ? q23 : q01, __shfl_xor_sync(0xffffffffu, up2 ? q01 : q23, LPR / 2)));                                // stride D/4
+                    float ss = __fadd_rn(up1 ? t.y : t.x, __shfl_xor_sync(0xffffffffu, up1 ? t.x : t.y, LPR / 4));                                        // stride D/8
+#pragma unroll
+                    for (int o = LPR / 8; o > 0; o >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));                                        // down to stride 4
+                    ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, LPR / 2));                                                                        // stride 2
+                    ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, LPR / 4));                                                                        // stride 1
+                    if ((lane & 3) == s) ss_mine = ss;
+                }
+                const float r_mine = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss_mine, static_cast<float>(D)), p.epsilon)));
+                Pair w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float* src = p.k_norm_weight + (i >> 1) * (D / 2) + 4 * l + 2 * (i & 1);
+                    w[i] = pack(src[0], src[1]);
+                }
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const float r = __shfl_sync(0xffffffffu, r_mine, (lane & ~3) | s);
+                    const Pair r2 = pack(r, r);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        a[s][i] = mul2(mul2(a[s][i], r2), w[i]);
+                        b[s][i] = mul2(mul2(b[s][i], r2), w[2 + i]);
+                    }
                 }
             }
-            const uint32_t g0 = pass_index * HB;
-            const int hn = static_cast<int>(min(static_cast<uint32_t>(HB), H - g0));
-            if (fast_cache && hn == HB) pass(std::true_type{}, token, g0, position, hn);
-            else pass(std::false_type{}, token, g0, position, hn);
+            if (rope_mode == B200KV_ROPE_NEOX_FULL) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const Pair x0 = a[s][i], x1 = b[s][i];
+                        a[s][i] = sub_products(mul2(x0, cs[i]), mul2(x1, sn[i]));
+                        b[s][i] = add_products(mul2(x0, sn[i]), mul2(x1, cs[i]));
+                    }
+            } else if (rope_mode == B200KV_ROPE_SECTIONED64) {
+                // elements 0-31 lie in lanes 0-7 of the row (x0 cos - x1 sin), 32-63 in lanes 8-15 (x0 sin + x1 cos)
+                const bool second = lane & 8;
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const Pair other = __shfl_xor_sync(0xffffffffu, a[s][i], 8);
+                        const Pair t = mul2(a[s][i], cs[i]), u = mul2(other, sn[i]);
+                        if (l < 16) a[s][i] = second ? add_products(u, t) : sub_products(t, u);
+                    }
+            }
         }
-        if (++pass_index == passes) {
-            pass_index = 0;
-            ++token;
-            fresh = true;
+        const uint64_t row0 = (static_cast<uint64_t>(cur.pass) * HB + sub) * capacity + position;   // this lane's cache row of step 0; the next step's is RPS * capacity on
+        if (!quantised) {
+            __half* dst = static_cast<__half*>(is_k ? p.view.key_f16 : p.view.value_f16) + row0 * D + 4 * l;
+#pragma unroll
+            for (int s = 0; s < 4; ++s, dst += RPS * capacity * D) {
+                if (s * RPS + sub >= hn) break;
+                *reinterpret_cast<uint2*>(dst) = half4(a[s]);
+                *reinterpret_cast<uint2*>(dst + D / 2) = half4(b[s]);
+            }
+            return;
         }
+        // ---- block maxima: values 2s (elements below D/2) and 2s + 1, over the eight lanes of a block; lane keeps value lane % 8.
+        float m[8];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) { m[2 * s] = amax4(a[s]); m[2 * s + 1] = amax4(b[s]); }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < o; ++i) m[i] = fmaxf(up ? m[i + o] : m[i], __shfl_xor_sync(0xffffffffu, up ? m[i] : m[i + o], o));
+        }
+        float amax = m[0];
+        if (rows) {
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+#pragma unroll
+            for (int o = 8; o < LPR; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        }
+        // ---- scales: amax / 127, its reciprocal, the fp16 scale to the cache -- one block per lane
+        const float scale = (amax > 0.0f) ? __fdiv_rn(amax, 127.0f) : 1.0f;
+        const float inv_mine = (scale > 0.0f) ? __fdiv_rn(1.0f, scale) : 1.0f;
+        {
+            const int s = (lane & 7) >> 1, block = (lane & 1) * (NB / 2) + (l >> 3);
+            __half* plane = static_cast<__half*>(is_k ? p.view.key_scales : p.view.value_scales);
+            const uint64_t r = row0 + s * RPS * capacity;
+            if (s * RPS + sub < hn && (!rows || block == 0)) plane[rows ? r : r * NB + block] = __float2half_rn(scale);
+        }
+        int8_t* dst = (is_k ? p.view.key_q8 : p.view.value_q8) + row0 * D + 4 * l;
+#pragma unroll
+        for (int s = 0; s < 4; ++s, dst += RPS * capacity * D) {
+            const float inv_a = __shfl_sync(0xffffffffu, inv_mine, (lane & 24) | (2 * s)), inv_b = __shfl_sync(0xffffffffu, inv_mine, (lane & 24) | (2 * s + 1));
+            const uint32_t wa = quantize4(a[s], inv_a), wb = quantize4(b[s], inv_b);
+            if (FAST || s * RPS + sub < hn) {
+                *reinterpret_cast<uint32_t*>(dst) = wa;
+                *reinterpret_cast<uint32_t*>(dst + D / 2) = wb;
+            }
+        }
+    };
+
+    Cursor cur{unit0 / (2 * passes), (unit0 / 2) % passes, unit0 & 1};
+    if (unit0 < unit1 && inside(cur)) fetch(cur);
+    uint32_t rotated_token = 0xffffffffu;
+    for (uint32_t unit = unit0; unit < unit1; ++unit) {
+        const uint64_t position = static_cast<uint64_t>(base_position) + cur.token;
+        if (cur.side == 0 && cur.token != rotated_token) {
+            rotated_token = cur.token;
+            rotation(static_cast<uint32_t>(position));
+        }
+        Pair a[4][2], b[4][2];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) { widen<IN_F16>(raw[s][0], a[s]); widen<IN_F16>(raw[s][1], b[s]); }
+        Cursor next = cur;
+        advance(next);
+        if (unit + 1 < unit1 && inside(next)) fetch(next);   // under this unit's arithmetic
+        if (inside(cur)) {
+            const int hn = heads(cur);
+            if (!row_scale && hn == HB && (cur.side == 0 ? k_q8 : v_q8)) process(std::true_type{}, cur, a, b, position, hn);
+            else process(std::false_type{}, cur, a, b, position, hn);
+        }
+        cur = next;
     }
 }
 
@@ -353,6 +379,7 @@ extern "C" int b200kv_append(const b200kv_view* view, const void* key, const voi
     p.k_norm_weight = k_norm_weight;
     p.prefill_state = prefill_state;
     p.decode_state = decode_state;
+    token_count = std::min(token_count, 0x7fffffffu);   // a device-side count is at most this: capacities are
     p.token_count = token_count;
     p.base_position = base_position;
     p.rope_mode = rope_mode;
@@ -360,17 +387,18 @@ extern "C" int b200kv_append(const b200kv_view* view, const void* key, const voi
     rope_constants(rope_mode, theta, view->head_dim, p.inv_freq, &p.sectioned_step);
 
     const uint32_t d = view->head_dim;
-    const uint32_t heads_per_pass = 512 / d;   // 16 K blocks and 16 V blocks of 32 dims per pass
-    const uint64_t units = static_cast<uint64_t>(token_count) * ((view->kv_heads + heads_per_pass - 1) / heads_per_pass);
+    const uint32_t heads_per_unit = kUnitElems / d;
+    const uint64_t units = 2ull * token_count * ((view->kv_heads + heads_per_unit - 1) / heads_per_unit);
     if (units >= (1ull << 32)) return B200KV_ERR_RANGE;
     int device = 0, sms = 0;
     B200KV_CUDA_TRY(cudaGetDevice(&device));
     B200KV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const uint64_t resident = static_cast<uint64_t>(sms) * kAppendCtasPerSm;
+    const bool f16 = (dtype == B200KV_F16);
+    const uint64_t resident = static_cast<uint64_t>(sms) * (f16 ? kAppendCtasPerSm<true> : kAppendCtasPerSm<false>);
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((units + kAppendWarps - 1) / kAppendWarps, resident));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool f16 = (dtype == B200KV_F16);
-    const bool vec = (reinterpret_cast<uintptr_t>(value) & 15u) == 0;   // vector loads of the V rows need an aligned input
+    // vector loads need aligned inputs (a lane's four elements start at a multiple of four of them)
+    const bool vec = ((reinterpret_cast<uintptr_t>(key) | reinterpret_cast<uintptr_t>(value)) & 15u) == 0;
     const dim3 block(kAppendWarps * 32);
     cudaError_t err;
     auto launch = [&](auto kernel) { return launch_kernel(kernel, grid, block, 0, s, true, p, vec); };
