@@ -46,6 +46,7 @@ constexpr int kThreads = kSoftmaxThreads + 128;
 constexpr int kKPairs = 2;                         // K ring: stages of two tiles each (one S MMA covers a pair)
 constexpr uint32_t kSpin = 1u << 20;
 constexpr float kRescaleThreshold = 8.0f;        // log2 units
+constexpr uint32_t kMaxKvSplits = 8;
 
 struct Tc5Params {
     CUtensorMap kmap, vmap;      // fp16 [kv_heads * rows][d], box 64 x 64, 128-byte swizzle
@@ -59,7 +60,7 @@ struct Tc5Params {
     uint64_t capacity;           // cache capacity (causal ranges past it give zero rows)
     uint32_t scratch_rows;       // rows per kv head in the fp16 scratch
     float scale_log2;
-    // KV split: blockIdx.z walks tiles [ntiles*z/S, ntiles*(z+1)/S) of its rows and leaves an unnormalised partial
+    // KV split: split z walks tiles [ntiles*z/S, ntiles*(z+1)/S) of its rows and leaves an unnormalised partial
     // (O, reference maximum, sum) for prefill_merge_kernel.  kv_splits == 1: the kernel writes the output itself.
     uint32_t kv_splits;
     uint32_t rows_padded;        // query rows per kv head, rounded up to the row tile
@@ -187,7 +188,7 @@ struct Layout {
     static constexpr int kOffP = kOffV + 2 * kTileBytes;   // 2 x [row][128 B] fp16 P tiles
     static constexpr int kPBytes = kBM * 128;
     static constexpr int kOffBar = kOffP + 2 * kPBytes;
-    static constexpr int kNumBars = 20;   // 16 used
+    static constexpr int kNumBars = 20;   // 17 used
     static constexpr int kOffRef = kOffBar + kNumBars * 8 + 16;   // [128 rows] {reference maximum, sequence}: handed from tile to tile
     static constexpr int kOffSum = kOffK;                         // [2 groups][128 rows] partial row sums: the K ring is idle in the epilogue
     static constexpr int kTotal = kOffRef + kBM * 8;
@@ -204,11 +205,14 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bar0 = sbase + L::kOffBar;
     auto bar = [&](int i) { return bar0 + i * 8; };
-    enum { K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = 9, P_FULL = 11, P_EMPTY = 13, O_DONE = 15 };
+    enum { K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = 9, P_FULL = 11, P_EMPTY = 13, O_DONE = 15, Q_FULL = 16 };
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffBar + L::kNumBars * 8);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t kv_head = blockIdx.y;
+    // Row tiles from the last (the longest causal range) to the first, kv heads and KV splits of a row tile next to each
+    // other: the CTAs dispatched last are the short ones, and a fresh chunk's last wave is nearly even.
+    const uint32_t split_u = blockIdx.x % p.kv_splits, tile_head = blockIdx.x / p.kv_splits;
+    const uint32_t kv_head = tile_head % p.kv_heads;
     const uint32_t G = p.query_heads / p.kv_heads;
     uint32_t base = p.base_position, count = p.token_count;
     if (p.prefill_state != nullptr) {
@@ -217,11 +221,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
         count = min(count, p.prefill_state->token_count);
     }
     const uint32_t total_rows = p.token_count * G;
-    const uint32_t row0 = blockIdx.x * kBM;
+    const uint32_t row0 = ((total_rows + kBM - 1) / kBM - 1 - tile_head / p.kv_heads) * kBM;
     // The next kernel of the stream (the merge of the KV splits) may become resident once every CTA has got here; it
     // orders itself against this one.  This kernel's own dependency wait comes after its set-up.
     pdl_launch_dependents();
-    if (row0 >= total_rows) return;
 
     // longest causal range among this CTA's rows (rows are token-major; see prefill_mma.cu)
     uint32_t kv_end = 0;
@@ -235,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     }
     if (kv_end > p.scratch_rows) kv_end = p.scratch_rows;   // never read past what the pre-pass wrote
     const int ntiles_all = static_cast<int>((kv_end + kBN - 1) / kBN);
-    const int split = static_cast<int>(blockIdx.z), nsplit = static_cast<int>(p.kv_splits);
+    const int split = static_cast<int>(split_u), nsplit = static_cast<int>(p.kv_splits);
     const int tile0 = static_cast<int>(static_cast<long long>(ntiles_all) * split / nsplit);
     const int ntiles = static_cast<int>(static_cast<long long>(ntiles_all) * (split + 1) / nsplit) - tile0;   // tiles of this CTA
 
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     // ---- set-up: barriers, TMEM, Q tile -----------------------------------------------------------------
     if (tid == 0) {
         for (int i = 0; i < L::kNumBars; ++i)
-            mbar_init(bar(i), (i == S_EMPTY || i == S_EMPTY + 1 || i == P_FULL || i == P_FULL + 1) ? kBM : 1);
+            mbar_init(bar(i), (i == S_EMPTY || i == S_EMPTY + 1 || i == P_FULL || i == P_FULL + 1) ? kBM : i == Q_FULL ? kSoftmaxThreads : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < kBM * 2; i += kThreads) reinterpret_cast<uint32_t*>(smem + L::kOffRef)[i] = 0;
@@ -274,42 +277,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();   // Q, the fp16 scratch and the device-side state come from preceding kernels
-    // Q: the CTA's rows as fp16 pairs in TMEM (row = lane, dims 2c and 2c+1 in column c), the A operand of every S MMA:
-    // read from there it costs no shared-memory bandwidth, which at N = 64 would bound the MMA.  Each of a row's two
-    // softmax threads stores half of the row.
-    if (warp < kSoftmaxThreads / 32) {
-        const int r = tid & (kBM - 1), half = tid >> 7;
-        const uint32_t gr = row0 + r;
-        const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const bool live = gr < total_rows;
-        const uint32_t token = live ? gr / G : 0, head = kv_head * G + (live ? gr % G : 0);
-        const size_t off = (static_cast<size_t>(token) * p.query_heads + head) * D + half * (D / 2);
-#pragma unroll 1
-        for (int c0 = 0; c0 < D / 4; c0 += 32) {   // 32 columns = 64 dims per store
-            uint32_t w[32];
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (live) {
-                    const size_t e = off + (c0 + i) * 2;
-                    if (p.q_is_f16) {
-                        v = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + e);
-                    } else {
-                        const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + e);
-                        const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + e + 4);
-                        v = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
-                    }
-                }
-                w[i] = v.x; w[i + 1] = v.y; w[i + 2] = v.z; w[i + 3] = v.w;
-            }
-            tmem_st32_bits(tmem_base + lane_addr + L::kColQ + half * (D / 4) + c0, w);
-        }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
     bool failed = false;
 
     if (warp == kTmaWarp) {
@@ -348,7 +315,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
         // pair costs what a single tile would.
         if (lane == 0) {
             constexpr uint32_t idesc_pair = umma_idesc(kBM, 2 * kBN, 0, 0), idesc_one = umma_idesc(kBM, kBN, 0, 0);
-            for (int i = 0; 2 * i < ntiles; ++i) {
+            const bool have_q = mbar_wait(bar(Q_FULL), 0);
+            for (int i = 0; have_q && 2 * i < ntiles; ++i) {
                 const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
                 if (!mbar_wait(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
                 // both groups have read the previous pair's scores (only the last pair can be a single tile)
@@ -385,6 +353,57 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
             }
         }
     } else {
+        // =============================== Q rows ===============================
+        // Q: the CTA's rows as fp16 pairs in TMEM (row = lane, dims 2c and 2c+1 in column c), the A operand of every S MMA:
+        // read from there it costs no shared-memory bandwidth.  Each of a row's two softmax threads stores half of the
+        // row.  A warp reads its 32 rows four at a time, 128 (fp32: 256) contiguous bytes each, and turns them through
+        // its own 4 KB of the P tiles (a load per thread and row touched 32 lines an instruction); the first K
+        // and V tiles are on their way meanwhile.
+        uint8_t* const turn = smem + L::kOffP + warp * 4096;   // [32 rows][8 chunks of 16 B], chunk c of row r at c ^ (r & 7)
+        const int turn_row = lane >> 3, turn_chunk = lane & 7;
+        const uint32_t warp_row0 = row0 + (warp & 3) * 32;
+        {
+            const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+            const int half = warp >> 2;
+#pragma unroll 1
+            for (int c0 = 0; c0 < D / 4; c0 += 32) {   // 32 columns = 64 dims per store
+                uint4 v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t row = warp_row0 + 4 * i + turn_row;
+                    v[i] = make_uint4(0, 0, 0, 0);
+                    if (row < total_rows) {
+                        const size_t e = (static_cast<size_t>(row / G) * p.query_heads + kv_head * G + row % G) * D + half * (D / 2) + c0 * 2 + turn_chunk * 8;
+                        if (p.q_is_f16) {
+                            v[i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + e);
+                        } else {
+                            const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + e);
+                            const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + e + 4);
+                            v[i] = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int row = 4 * i + turn_row;
+                    *reinterpret_cast<uint4*>(turn + row * 128 + ((turn_chunk ^ (row & 7)) << 4)) = v[i];
+                }
+                __syncwarp();
+                uint32_t w[32];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 q4 = *reinterpret_cast<const uint4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4));
+                    w[4 * c] = q4.x; w[4 * c + 1] = q4.y; w[4 * c + 2] = q4.z; w[4 * c + 3] = q4.w;
+                }
+                __syncwarp();
+                tmem_st32_bits(tmem_base + lane_base + L::kColQ + half * (D / 4) + c0, w);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            mbar_arrive(bar(Q_FULL));
+            // P tiles are written by every warp of a group: nobody may write one while a neighbour still turns rows in it
+            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
+        }
         // =============================== softmax rows ===============================
         // Two groups of 128 threads, one thread per query row in each: warps 0-3 take the even tiles, warps 4-7 the odd
         // ones (a warp reaches the 32 TMEM lanes of its number modulo 4), so two tiles are in flight: while one group
@@ -508,44 +527,60 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
             if (l_sum != l_sum) failed = true;   // either thread of the row gave up
             const float m_ref = m_final;
             const int hsel = grp;
-            // tcgen05.ld is warp-collective: every lane takes part, rows past the launch only skip the store
-            const bool live = gr < total_rows;
-            const uint32_t token = live ? gr / G : 0, head = kv_head * G + (live ? gr % G : 0);
-            const size_t off = (static_cast<size_t>(token) * p.query_heads + head) * D;
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
             const bool have_o = ntiles > 0 && !__any_sync(0xffffffffu, failed);
             const bool partial = nsplit > 1;
-            const size_t prow_idx = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0 + r;
-            if (partial && live && hsel == 0)   // a poisoned or empty partial is recognised by its sum
-                p.part_ml[prow_idx] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
+            const size_t part_row0 = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0;
+            if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum
+                p.part_ml[part_row0 + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
+            // Rows leave 32 columns at a time through the same 4 KB per warp: read back four rows an instruction, 128
+            // contiguous bytes each, so that the gate is fetched and the result stored in whole lines.
+            size_t out_off[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t row = warp_row0 + 4 * i + turn_row;
+                out_off[i] = partial ? (part_row0 + (row - row0)) * D : (static_cast<size_t>(row / G) * p.query_heads + kv_head * G + row % G) * D;
+            }
+            float* const dst = partial ? p.part_o : p.out;
+            const float factor = partial ? 1.0f : inv;
+            const bool gated = !partial && p.gate != nullptr;
 #pragma unroll 1
             for (int c0 = hsel * (D / 2); c0 < (hsel + 1) * (D / 2); c0 += 32) {
+                float4 g[8];
+                if (gated) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (warp_row0 + 4 * i + turn_row < total_rows) g[i] = *reinterpret_cast<const float4*>(p.gate + out_off[i] + c0 + 4 * turn_chunk);
+                }
                 float o[32];
+                // tcgen05.ld is warp-collective: every lane takes part, rows past the launch only skip the store
                 if (have_o) {
                     tmem_ld32(tmem_base + lane_addr + L::kColO + c0, o);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = failed ? __int_as_float(0x7fc00000) : 0.0f;
-                }
-                if (!live) continue;
-                if (partial) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(p.part_o + prow_idx * D + c0 + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-                    continue;
+                    for (int i = 0; i < 32; ++i) o[i] = 0.0f;
                 }
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    float4 v = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
-                    if (failed) v = make_float4(o[i], o[i], o[i], o[i]);
-                    else if (len == 0) v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (p.gate != nullptr) {
-                        const float4 g = *reinterpret_cast<const float4*>(p.gate + off + c0 + i);
-                        v.x *= 1.0f / (1.0f + __expf(-g.x)); v.y *= 1.0f / (1.0f + __expf(-g.y));
-                        v.z *= 1.0f / (1.0f + __expf(-g.z)); v.w *= 1.0f / (1.0f + __expf(-g.w));
+                for (int i = 0; i < 32; ++i) {
+                    o[i] = (len == 0 && !partial) ? 0.0f : o[i] * factor;
+                    if (failed) o[i] = __int_as_float(0x7fc00000);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<float4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int row = 4 * i + turn_row;
+                    float4 v = *reinterpret_cast<const float4*>(turn + row * 128 + ((turn_chunk ^ (row & 7)) << 4));
+                    if (warp_row0 + row >= total_rows) continue;
+                    if (gated) {
+                        v.x *= 1.0f / (1.0f + __expf(-g[i].x)); v.y *= 1.0f / (1.0f + __expf(-g[i].y));
+                        v.z *= 1.0f / (1.0f + __expf(-g[i].z)); v.w *= 1.0f / (1.0f + __expf(-g[i].w));
                     }
-                    *reinterpret_cast<float4*>(p.out + off + c0 + i) = v;
+                    *reinterpret_cast<float4*>(dst + out_off[i] + c0 + 4 * turn_chunk) = v;
                 }
+                __syncwarp();
             }
         }
     }
@@ -577,20 +612,31 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const __grid_constan
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<size_t>(p.total_rows) * VPR) return;
     const uint32_t gr = static_cast<uint32_t>(idx / VPR), c = static_cast<uint32_t>(idx % VPR) * 4;
-    float m[8], l[8], M = -INFINITY;   // kv_splits <= 8
-    for (uint32_t s = 0; s < p.kv_splits; ++s) {
-        const float2 ml = p.part_ml[(static_cast<size_t>(s) * p.kv_heads + kv_head) * p.rows_padded + gr];
-        m[s] = ml.x; l[s] = ml.y;
-        if (!(ml.y <= 0.0f) && ml.x != -INFINITY) M = fmaxf(M, ml.x);   // keeps NaN partials in play
+    // every load of the row's splits is issued before the first is used; an empty split's O was never written and counts for nothing
+    float2 ml[kMaxKvSplits];
+    float4 o[kMaxKvSplits];
+#pragma unroll
+    for (uint32_t s = 0; s < kMaxKvSplits; ++s) {
+        ml[s] = make_float2(-INFINITY, 0.0f);
+        o[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (s < p.kv_splits) {
+            const size_t row = (static_cast<size_t>(s) * p.kv_heads + kv_head) * p.rows_padded + gr;
+            ml[s] = p.part_ml[row];
+            o[s] = *reinterpret_cast<const float4*>(p.part_o + row * D + c);
+        }
     }
+    float M = -INFINITY;
+#pragma unroll
+    for (uint32_t s = 0; s < kMaxKvSplits; ++s)
+        if (!(ml[s].y <= 0.0f) && ml[s].x != -INFINITY) M = fmaxf(M, ml[s].x);   // keeps NaN partials in play
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float lsum = 0.0f;
-    for (uint32_t s = 0; s < p.kv_splits; ++s) {
-        if (l[s] <= 0.0f || m[s] == -INFINITY) continue;   // empty split: its O was never written
-        const float w = exp2f(m[s] - M);
-        const float4 o = *reinterpret_cast<const float4*>(p.part_o + ((static_cast<size_t>(s) * p.kv_heads + kv_head) * p.rows_padded + gr) * D + c);
-        acc.x = fmaf(o.x, w, acc.x); acc.y = fmaf(o.y, w, acc.y); acc.z = fmaf(o.z, w, acc.z); acc.w = fmaf(o.w, w, acc.w);
-        lsum = fmaf(l[s], w, lsum);
+#pragma unroll
+    for (uint32_t s = 0; s < kMaxKvSplits; ++s) {
+        if (ml[s].y <= 0.0f || ml[s].x == -INFINITY) continue;
+        const float w = exp2f(ml[s].x - M);
+        acc.x = fmaf(o[s].x, w, acc.x); acc.y = fmaf(o[s].y, w, acc.y); acc.z = fmaf(o[s].z, w, acc.z); acc.w = fmaf(o[s].w, w, acc.w);
+        lsum = fmaf(ml[s].y, w, lsum);
     }
     const float inv = lsum > 0.0f ? 1.0f / lsum : (lsum == lsum ? 0.0f : lsum);
     float4 v = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
@@ -716,7 +762,7 @@ int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half*
     }
     const uint32_t G = p.query_heads / p.kv_heads;
     const uint32_t row_tiles = (p.token_count * G + kBM - 1) / kBM;
-    B200KV_CUDA_TRY(launch_kernel(prefill_tc5_kernel<D>, dim3(row_tiles, p.kv_heads, p.kv_splits), dim3(kThreads), L::kAlloc, stream, true, p));
+    B200KV_CUDA_TRY(launch_kernel(prefill_tc5_kernel<D>, dim3(row_tiles * p.kv_heads * p.kv_splits), dim3(kThreads), L::kAlloc, stream, true, p));
     if (p.kv_splits > 1) {
         PrefillMergeParams mp{};
         mp.part_o = p.part_o;
@@ -740,8 +786,6 @@ size_t prefill_tc5_workspace_bytes(uint32_t rows, uint32_t kv_heads, uint32_t he
     const size_t r = (static_cast<size_t>(rows) + kBN - 1) / kBN * kBN;
     return 2 * r * kv_heads * head_dim * sizeof(__half) + 1024;   // K and V planes, 1 KB to align the base
 }
-
-constexpr uint32_t kMaxKvSplits = 8;
 
 // Extra workspace that lets a launch split the KV range of every row tile over several CTAs (partials of `splits` splits).
 size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint32_t kv_heads, uint32_t head_dim, uint32_t splits) {
