@@ -23,6 +23,10 @@
 //         memory), write P as fp16 into one of two swizzled A-operand tiles, and at the end scale O by 1/sum,
 //         apply the sigmoid gate (.hip:6714-6723) and store.
 //     TMEM: S (pair) | Q | O = 128 + d/2 + d columns.  Shared memory: 2 x 2 K tiles + 2 V tiles + 2 P tiles.
+//     At head_dim 128 a CTA takes TWO row tiles where there are enough of them (512 softmax threads; S and O of both fill
+//     TMEM, so Q is an A operand in shared memory): a single tile's loop waits for its softmax (about 1 us a pair of KV tiles against
+//     0.5 us of MMAs), two share every K and V tile and one's MMAs run under the other's softmax.  2048 fresh
+//     tokens, 32/8 heads: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA.
 // Every mbarrier wait is bounded; a wait that runs out poisons the output rows with NaN, and the CTA still frees
 // its TMEM and exits.
 #include "decode_common.cuh"
@@ -35,14 +39,8 @@ namespace b200kv {
 
 namespace {
 
-constexpr int kBM = 128;          // query rows per CTA
+constexpr int kBM = 128;          // query rows per row tile; a CTA takes one or two (RT)
 constexpr int kBN = 64;           // positions per KV tile
-constexpr int kSoftmaxThreads = 256;              // two groups of one thread per query row: even tiles, odd tiles
-constexpr int kTmaWarp = kSoftmaxThreads / 32;     // TMA producer of the K tiles
-constexpr int kSWarp = kTmaWarp + 1;               // S = Q.K^T issuer / TMEM owner
-constexpr int kPvWarp = kTmaWarp + 2;              // O += P.V issuer
-constexpr int kTmaVWarp = kTmaWarp + 3;            // TMA producer of the V tiles (a K load never waits for a V stage)
-constexpr int kThreads = kSoftmaxThreads + 128;
 constexpr int kKPairs = 2;                         // K ring: stages of two tiles each (one S MMA covers a pair)
 constexpr uint32_t kSpin = 1u << 20;
 constexpr float kRescaleThreshold = 8.0f;        // log2 units
@@ -178,35 +176,56 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
-template <int D>
+template <int D, int RT>
 struct Layout {
+    // warps: two softmax groups per row tile (one thread per query row: even tiles, odd tiles), then one warp per role
+    static constexpr int kSoftmaxThreads = RT * 256;
+    static constexpr int kTmaWarp = kSoftmaxThreads / 32;  // TMA producer of the K tiles
+    static constexpr int kSWarp = kTmaWarp + 1;            // S = Q.K^T issuer / TMEM owner
+    static constexpr int kPvWarp = kTmaWarp + 2;           // O += P.V issuer
+    static constexpr int kTmaVWarp = kTmaWarp + 3;         // TMA producer of the V tiles (a K load never waits for a V stage)
+    static constexpr int kThreads = kSoftmaxThreads + 128;
+    static constexpr int kRows = RT * kBM;
+    static constexpr bool kQInTmem = RT == 1;              // two row tiles' S and O fill TMEM: their Q stays in shared memory
     static constexpr int kSlabs = D / 64;                  // 128-byte (64 x fp16) slabs along d
     static constexpr int kTileBytes = kSlabs * kBN * 128;  // one K or V tile: [slab][row][128 B]
     static constexpr int kPairBytes = 2 * kTileBytes;      // two K tiles as one B operand: [slab][128 rows][128 B]
     static constexpr int kOffK = 0;
     static constexpr int kOffV = kOffK + kKPairs * kPairBytes;
-    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // 2 x [row][128 B] fp16 P tiles
+    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // [row tile][2][row][128 B] fp16 P tiles
     static constexpr int kPBytes = kBM * 128;
-    static constexpr int kOffBar = kOffP + 2 * kPBytes;
-    static constexpr int kNumBars = 20;   // 17 used
-    static constexpr int kOffRef = kOffBar + kNumBars * 8 + 16;   // [128 rows] {reference maximum, sequence}: handed from tile to tile
-    static constexpr int kOffSum = kOffK;                         // [2 groups][128 rows] partial row sums: the K ring is idle in the epilogue
-    static constexpr int kTotal = kOffRef + kBM * 8;
+    static constexpr int kOffQ = kOffP + RT * 2 * kPBytes; // [row tile][slab][row][128 B]
+    static constexpr int kQBytes = kSlabs * kBM * 128;
+    static constexpr int kOffBar = kOffQ + (kQInTmem ? 0 : RT * kQBytes);
+    // mbarriers; the ones after V_EMPTY are per row tile, S_EMPTY and the P pairs per row tile and softmax group
+    static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = S_FULL + RT, P_FULL = S_EMPTY + 2 * RT,
+                         P_EMPTY = P_FULL + 2 * RT, O_DONE = P_EMPTY + 2 * RT, Q_FULL = O_DONE + RT, kNumBars = Q_FULL + 1;
+    static constexpr int kOffSlot = kOffBar + (kNumBars * 8 + 15) / 16 * 16;
+    static constexpr int kOffRef = kOffSlot + 16;                 // [rows] {reference maximum, sequence}: handed from tile to tile
+    // [2 groups][128 rows] partial row sums of a row tile in its epilogue, where its own score MMAs are through: over the K
+    // ring, or over the row tile's Q where the other row tile may still need K
+    static constexpr int kOffSum = kQInTmem ? kOffK : kOffQ, kSumStride = kQBytes;
+    static constexpr int kTotal = kOffRef + kRows * 8;
     static constexpr int kAlloc = kTotal;   // the dynamic shared memory is declared 1024-byte aligned; the kernel checks it
+    static_assert(kAlloc <= 232448, "227 KB per CTA");
     static constexpr uint32_t kTmemCols = 512;
-    static constexpr uint32_t kColS = 0, kColQ = 128, kColO = 256;   // S: 2 x 64, Q: D/2 (fp16 pairs), O: D
+    static constexpr uint32_t kColS = 0, kColQ = 128, kColO = 256;   // S: RT x 2 x 64, Q (RT == 1): D/2 (fp16 pairs), O: RT x D
+    static_assert(RT == 1 ? kColQ + D / 2 <= kColO && kColO + D <= 512 : 2 * 128 <= kColO && kColO + 2 * D <= 512, "TMEM columns");
 };
 
-template <int D>
-__global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_constant__ Tc5Params p) {
-    using L = Layout<D>;
+template <int D, int RT>
+__global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel(const __grid_constant__ Tc5Params p) {
+    using L = Layout<D, RT>;
+    constexpr int kThreads = L::kThreads, kSoftmaxThreads = L::kSoftmaxThreads;
+    constexpr int kTmaWarp = L::kTmaWarp, kSWarp = L::kSWarp, kPvWarp = L::kPvWarp, kTmaVWarp = L::kTmaVWarp;
+    constexpr int K_FULL = L::K_FULL, K_EMPTY = L::K_EMPTY, V_FULL = L::V_FULL, V_EMPTY = L::V_EMPTY, S_FULL = L::S_FULL, S_EMPTY = L::S_EMPTY,
+                  P_FULL = L::P_FULL, P_EMPTY = L::P_EMPTY, O_DONE = L::O_DONE, Q_FULL = L::Q_FULL;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw;
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bar0 = sbase + L::kOffBar;
     auto bar = [&](int i) { return bar0 + i * 8; };
-    enum { K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = 9, P_FULL = 11, P_EMPTY = 13, O_DONE = 15, Q_FULL = 16 };
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffBar + L::kNumBars * 8);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffSlot);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Row tiles from the last (the longest causal range) to the first, kv heads and KV splits of a row tile next to each
@@ -221,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
         count = min(count, p.prefill_state->token_count);
     }
     const uint32_t total_rows = p.token_count * G;
-    const uint32_t row0 = ((total_rows + kBM - 1) / kBM - 1 - tile_head / p.kv_heads) * kBM;
+    const uint32_t row0 = ((total_rows + L::kRows - 1) / L::kRows - 1 - tile_head / p.kv_heads) * L::kRows;
     // The next kernel of the stream (the merge of the KV splits) may become resident once every CTA has got here; it
     // orders itself against this one.  This kernel's own dependency wait comes after its set-up.
     pdl_launch_dependents();
@@ -229,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     // longest causal range among this CTA's rows (rows are token-major; see prefill_mma.cu)
     uint32_t kv_end = 0;
     if (count > 0 && p.capacity > base) {
-        const uint32_t t_first = row0 / G, t_last = (min(row0 + kBM, total_rows) - 1) / G;
+        const uint32_t t_first = row0 / G, t_last = (min(row0 + L::kRows, total_rows) - 1) / G;
         const uint64_t t_cap = p.capacity - base - 1;
         uint64_t t_max = t_last;
         if (t_max > count - 1) t_max = count - 1;
@@ -248,11 +267,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     if ((sbase & 1023u) != 0) {
         pdl_wait();
         const float nan = __int_as_float(0x7fc00000);
-        for (uint32_t r = tid; r < static_cast<uint32_t>(kBM); r += kThreads)
+        for (uint32_t r = tid; r < static_cast<uint32_t>(L::kRows); r += kThreads)
             if (nsplit > 1 && row0 + r < total_rows)
                 p.part_ml[(static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0 + r] = make_float2(0.0f, nan);
         if (nsplit == 1)
-            for (uint32_t i = tid; i < static_cast<uint32_t>(kBM) * (D / 4); i += kThreads) {
+            for (uint32_t i = tid; i < static_cast<uint32_t>(L::kRows) * (D / 4); i += kThreads) {
                 const uint32_t gr = row0 + i / (D / 4);
                 if (gr >= total_rows) continue;
                 const size_t off = (static_cast<size_t>(gr / G) * p.query_heads + kv_head * G + gr % G) * D + (i % (D / 4)) * 4;
@@ -264,10 +283,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     // ---- set-up: barriers, TMEM, Q tile -----------------------------------------------------------------
     if (tid == 0) {
         for (int i = 0; i < L::kNumBars; ++i)
-            mbar_init(bar(i), (i == S_EMPTY || i == S_EMPTY + 1 || i == P_FULL || i == P_FULL + 1) ? kBM : i == Q_FULL ? kSoftmaxThreads : 1);
+            mbar_init(bar(i), i >= S_EMPTY && i < P_EMPTY ? kBM : i == Q_FULL ? kSoftmaxThreads : 1);   // S_EMPTY and P_FULL: a group's threads
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = tid; i < kBM * 2; i += kThreads) reinterpret_cast<uint32_t*>(smem + L::kOffRef)[i] = 0;
+    for (int i = tid; i < L::kRows * 2; i += kThreads) reinterpret_cast<uint32_t*>(smem + L::kOffRef)[i] = 0;
     if (warp == kSWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -278,6 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();   // Q, the fp16 scratch and the device-side state come from preceding kernels
     bool failed = false;
+    const int live_tiles = min(RT, static_cast<int>((total_rows - row0 + kBM - 1) / kBM));   // row tiles that hold rows
 
     if (warp == kTmaWarp) {
         // =============================== TMA producer, K tiles ===============================
@@ -319,15 +339,27 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
             for (int i = 0; have_q && 2 * i < ntiles; ++i) {
                 const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
                 if (!mbar_wait(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
-                // both groups have read the previous pair's scores (only the last pair can be a single tile)
-                if (!mbar_wait(bar(S_EMPTY), static_cast<uint32_t>(i & 1) ^ 1) || !mbar_wait(bar(S_EMPTY + 1), static_cast<uint32_t>(i & 1) ^ 1)) break;
-                tc_fence_after();
+                bool ok = true;
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t b = sbase + L::kOffK + ps * L::kPairBytes + (kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32;
-                    umma_f16_a_tmem(tmem_base + L::kColS, tmem_base + L::kColQ + kk * 8, umma_desc(b, 16, 1024), n == 2 ? idesc_pair : idesc_one, kk > 0);
+                for (int rt = 0; rt < RT; ++rt) {
+                    if (RT > 1 && rt >= live_tiles) break;
+                    // both groups have read the previous pair's scores (only the last pair can be a single tile)
+                    ok = mbar_wait(bar(S_EMPTY + 2 * rt), static_cast<uint32_t>(i & 1) ^ 1) && mbar_wait(bar(S_EMPTY + 2 * rt + 1), static_cast<uint32_t>(i & 1) ^ 1);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t b = sbase + L::kOffK + ps * L::kPairBytes + (kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32;
+                        const uint32_t idesc = n == 2 ? idesc_pair : idesc_one;
+                        if constexpr (L::kQInTmem)
+                            umma_f16_a_tmem(tmem_base + L::kColS, tmem_base + L::kColQ + kk * 8, umma_desc(b, 16, 1024), idesc, kk > 0);
+                        else
+                            umma_f16(tmem_base + L::kColS + rt * 2 * kBN, umma_desc(sbase + L::kOffQ + rt * L::kQBytes + (kk >> 2) * (kBM * 128) + (kk & 3) * 32, 16, 1024),
+                                     umma_desc(b, 16, 1024), idesc, kk > 0);
+                    }
+                    umma_commit(bar(S_FULL + rt));    // scores ready for both softmax groups
                 }
-                umma_commit(bar(S_FULL));         // scores ready for both softmax groups
+                if (!ok) break;
                 umma_commit(bar(K_EMPTY + ps));   // K stage may be refilled
             }
         }
@@ -339,17 +371,24 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
                 const int st = j & 1;
                 const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);
                 if (!mbar_wait(bar(V_FULL + st), ph)) break;
-                if (!mbar_wait(bar(P_FULL + st), ph)) break;
-                tc_fence_after();
+                bool ok = true;
 #pragma unroll
-                for (int kk = 0; kk < kBN / 16; ++kk) {
-                    const uint32_t b = sbase + L::kOffV + st * L::kTileBytes + kk * (16 * 128);      // V: MN-major, 16 positions per step
-                    const uint32_t a = sbase + L::kOffP + st * L::kPBytes + kk * 32;               // P: K-major, one 128-byte slab
-                    umma_f16(tmem_base + L::kColO, umma_desc(a, 16, 1024), umma_desc(b, kBN * 128, 1024), idesc_o, (j > 0 || kk > 0));
+                for (int rt = 0; rt < RT; ++rt) {
+                    if (RT > 1 && rt >= live_tiles) break;
+                    ok = mbar_wait(bar(P_FULL + 2 * rt + st), ph);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int kk = 0; kk < kBN / 16; ++kk) {
+                        const uint32_t b = sbase + L::kOffV + st * L::kTileBytes + kk * (16 * 128);      // V: MN-major, 16 positions per step
+                        const uint32_t a = sbase + L::kOffP + (2 * rt + st) * L::kPBytes + kk * 32;     // P: K-major, one 128-byte slab
+                        umma_f16(tmem_base + L::kColO + rt * D, umma_desc(a, 16, 1024), umma_desc(b, kBN * 128, 1024), idesc_o, (j > 0 || kk > 0));
+                    }
+                    umma_commit(bar(P_EMPTY + 2 * rt + st));   // P buffer free, O holds tiles 0..j
+                    if (j == ntiles - 1) umma_commit(bar(O_DONE + rt));   // O complete: the epilogue's signal for both groups
                 }
-                umma_commit(bar(P_EMPTY + st));   // P buffer free, O holds tiles 0..j
+                if (!ok) break;
                 umma_commit(bar(V_EMPTY + st));
-                if (j == ntiles - 1) umma_commit(bar(O_DONE));   // O complete: the epilogue's signal for both groups
             }
         }
     } else {
@@ -361,10 +400,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
         // and V tiles are on their way meanwhile.
         uint8_t* const turn = smem + L::kOffP + warp * 4096;   // [32 rows][8 chunks of 16 B], chunk c of row r at c ^ (r & 7)
         const int turn_row = lane >> 3, turn_chunk = lane & 7;
-        const uint32_t warp_row0 = row0 + (warp & 3) * 32;
+        const int rt = RT == 1 ? 0 : warp >> 3;                // row tile
+        const uint32_t tile_row0 = row0 + rt * kBM, warp_row0 = tile_row0 + (warp & 3) * 32;
         {
             const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-            const int half = warp >> 2;
+            const int half = (warp >> 2) & 1;
 #pragma unroll 1
             for (int c0 = 0; c0 < D / 4; c0 += 32) {   // 32 columns = 64 dims per store
                 uint4 v[8];
@@ -383,6 +423,15 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
                         }
                     }
                 }
+                if constexpr (!L::kQInTmem) {   // the swizzled A operand itself: slab `half * D/128 + c0/32` of the row tile
+                    uint8_t* slab = smem + L::kOffQ + rt * L::kQBytes + (half * (D / 128) + c0 / 32) * (kBM * 128) + (warp & 3) * (32 * 128);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int row = 4 * i + turn_row;
+                        *reinterpret_cast<uint4*>(slab + row * 128 + ((turn_chunk ^ (row & 7)) << 4)) = v[i];
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int row = 4 * i + turn_row;
@@ -398,8 +447,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
                 __syncwarp();
                 tmem_st32_bits(tmem_base + lane_base + L::kColQ + half * (D / 4) + c0, w);
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            tc_fence_before();
+            if constexpr (L::kQInTmem) {
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+            } else {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
             mbar_arrive(bar(Q_FULL));
             // P tiles are written by every warp of a group: nobody may write one while a neighbour still turns rows in it
             asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
@@ -410,16 +463,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
         // works through its exponentials the other one's S arrives and its P.V runs.  A row's reference maximum is handed
         // from tile to tile through an 8-byte {value, sequence} word in shared memory; each thread keeps the partial row
         // sum of its own tiles, relative to the reference it last saw.
-        const int r = tid & (kBM - 1), grp = tid >> 7;       // row of this thread == its TMEM lane; tile parity
+        const int r = tid & (kBM - 1), grp = (tid >> 7) & 1;   // row of this thread in its row tile == its TMEM lane; tile parity
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t gr = row0 + r;
+        const uint32_t gr = tile_row0 + r;
+        const int nt = RT == 1 || rt < live_tiles ? ntiles : 0;
         uint32_t len = 0;
         if (gr < total_rows) {
             const uint32_t token = gr / G;
             const uint64_t l64 = static_cast<uint64_t>(base) + token + 1u;
             len = (token < count && l64 <= p.capacity) ? static_cast<uint32_t>(l64) : 0u;
         }
-        volatile unsigned long long* ref = reinterpret_cast<volatile unsigned long long*>(smem + L::kOffRef) + r;
+        volatile unsigned long long* ref = reinterpret_cast<volatile unsigned long long*>(smem + L::kOffRef) + rt * kBM + r;
         auto ref_after = [&](uint32_t seq, float* value) -> bool {   // the reference as tile seq-1 left it
             for (uint32_t spin = 0; spin < kSpin; ++spin) {
                 const unsigned long long w = *ref;
@@ -435,21 +489,22 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
             }
         };
         const int st = grp;
-        for (int j = grp; j < ntiles; j += 2) {
+        const uint32_t s_col = L::kColS + (2 * rt + grp) * kBN, o_col = L::kColO + rt * D;
+        for (int j = grp; j < nt; j += 2) {
             const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);   // parity of the tile's pair
-            if (!mbar_wait(bar(S_FULL), ph)) { failed = true; break; }
+            if (!mbar_wait(bar(S_FULL + rt), ph)) { failed = true; break; }
             tc_fence_after();
             float s[kBN];
             {
                 uint32_t lo[32], hi[32];
-                tmem_ld32_nowait(tmem_base + lane_addr + L::kColS + st * kBN, lo);
-                tmem_ld32_nowait(tmem_base + lane_addr + L::kColS + st * kBN + 32, hi);
+                tmem_ld32_nowait(tmem_base + lane_addr + s_col, lo);
+                tmem_ld32_nowait(tmem_base + lane_addr + s_col + 32, hi);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) { s[i] = __uint_as_float(lo[i]); s[32 + i] = __uint_as_float(hi[i]); }
             }
             tc_fence_before();
-            mbar_arrive(bar(S_EMPTY + st));   // this row of S is in registers
+            mbar_arrive(bar(S_EMPTY + 2 * rt + st));   // this row of S is in registers
             const uint32_t pos0 = static_cast<uint32_t>(tile0 + j) * kBN;
             // Raw scores stay unscaled; the softmax scale is folded into the exponent: p = 2^(s*c - m*c).
             // Only the tiles that straddle this row's causal length need the mask.
@@ -488,51 +543,53 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
             }
             l_sum += sum;
             // this group's P buffer is free once the P.V of its previous tile has completed
-            if (!mbar_wait(bar(P_EMPTY + st), ph ^ 1)) { failed = true; break; }
+            if (!mbar_wait(bar(P_EMPTY + 2 * rt + st), ph ^ 1)) { failed = true; break; }
             tc_fence_after();
             if (__any_sync(0xffffffffu, alpha != 1.0f) && j > 0) {
                 // rare: the reference moved.  O holds tiles 0..j-1 once the previous tile's P.V (the other group's) has
                 // completed; then this warp rescales its 32 rows of O in TMEM before its own P is released.
-                if (!mbar_wait(bar(P_EMPTY + (st ^ 1)), static_cast<uint32_t>(((j - 1) >> 1) & 1))) { failed = true; break; }
+                if (!mbar_wait(bar(P_EMPTY + 2 * rt + (st ^ 1)), static_cast<uint32_t>(((j - 1) >> 1) & 1))) { failed = true; break; }
                 tc_fence_after();
 #pragma unroll 1
                 for (int c0 = 0; c0 < D; c0 += 32) {
                     float o[32];
-                    tmem_ld32(tmem_base + lane_addr + L::kColO + c0, o);
+                    tmem_ld32(tmem_base + lane_addr + o_col + c0, o);
 #pragma unroll
                     for (int i = 0; i < 32; ++i) o[i] *= alpha;
-                    tmem_st32(tmem_base + lane_addr + L::kColO + c0, o);
+                    tmem_st32(tmem_base + lane_addr + o_col + c0, o);
                 }
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // the rescale's stores, if any
-            uint8_t* prow = smem + L::kOffP + st * L::kPBytes + r * 128;
+            uint8_t* prow = smem + L::kOffP + (2 * rt + st) * L::kPBytes + r * 128;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
                 *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_fence_before();
-            mbar_arrive(bar(P_FULL + st));
+            mbar_arrive(bar(P_FULL + 2 * rt + st));
         }
         // ---- epilogue: O / sum, gate, store; each thread of a row's pair half of the columns ----
-        if (!failed && ntiles > 0 && !mbar_wait(bar(O_DONE), 0)) failed = true;
+        if (!failed && nt > 0 && !mbar_wait(bar(O_DONE + rt), 0)) failed = true;
         tc_fence_after();
         {
             float m_final = -INFINITY;
-            if (!failed && ntiles > 0 && !ref_after(static_cast<uint32_t>(ntiles), &m_final)) failed = true;
+            if (!failed && nt > 0 && !ref_after(static_cast<uint32_t>(nt), &m_final)) failed = true;
             rebase(m_final);
-            float* sums = reinterpret_cast<float*>(smem + L::kOffSum);
+            float* sums = reinterpret_cast<float*>(smem + L::kOffSum + rt * L::kSumStride);
             sums[grp * kBM + r] = failed ? __int_as_float(0x7fc00000) : l_sum;
-            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
+            // the row tile's threads (a branch over two constant barriers duplicates what follows: 4 % slower with two row tiles)
+            if constexpr (RT == 1) asm volatile("bar.sync 2, 256;" ::: "memory");
+            else asm volatile("bar.sync %0, 256;" ::"r"(2 + rt) : "memory");
             l_sum = sums[r] + sums[kBM + r];
             if (l_sum != l_sum) failed = true;   // either thread of the row gave up
             const float m_ref = m_final;
             const int hsel = grp;
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
-            const bool have_o = ntiles > 0 && !__any_sync(0xffffffffu, failed);
+            const bool have_o = nt > 0 && !__any_sync(0xffffffffu, failed);
             const bool partial = nsplit > 1;
             const size_t part_row0 = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0;
             if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum
-                p.part_ml[part_row0 + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
+                p.part_ml[part_row0 + rt * kBM + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
             // Rows leave 32 columns at a time through the same 4 KB per warp: read back four rows an instruction, 128
             // contiguous bytes each, so that the gate is fetched and the result stored in whole lines.
             size_t out_off[8];
@@ -555,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc5_kernel(const __grid_c
                 float o[32];
                 // tcgen05.ld is warp-collective: every lane takes part, rows past the launch only skip the store
                 if (have_o) {
-                    tmem_ld32(tmem_base + lane_addr + L::kColO + c0, o);
+                    tmem_ld32(tmem_base + lane_addr + o_col + c0, o);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) o[i] = 0.0f;
@@ -748,12 +805,12 @@ int launch_dequant(const b200kv_view& view, __half* k_scratch, __half* v_scratch
     return B200KV_OK;
 }
 
-template <int D>
+template <int D, int RT>
 int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half* v_scratch, uint32_t rows, uint32_t prepared_rows,
                cudaStream_t stream) {
-    using L = Layout<D>;
+    using L = Layout<D, RT>;
     static std::atomic<uint64_t> done{0};   // one per kernel instantiation: devices that have opted in
-    const cudaError_t attr_err = opt_in_dynamic_smem(reinterpret_cast<const void*>(prefill_tc5_kernel<D>), L::kAlloc, done);
+    const cudaError_t attr_err = opt_in_dynamic_smem(reinterpret_cast<const void*>(prefill_tc5_kernel<D, RT>), L::kAlloc, done);
     if (attr_err != cudaSuccess) { set_last_cuda_error(attr_err, "cudaFuncSetAttribute(prefill_tc5)"); return B200KV_ERR_CUDA; }
     if (rows > 0) {
         const int rc = launch_dequant<D>(view, k_scratch, v_scratch, rows, p.scratch_rows, prepared_rows < rows ? prepared_rows : rows,
@@ -761,8 +818,8 @@ int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half*
         if (rc != B200KV_OK) return rc;
     }
     const uint32_t G = p.query_heads / p.kv_heads;
-    const uint32_t row_tiles = (p.token_count * G + kBM - 1) / kBM;
-    B200KV_CUDA_TRY(launch_kernel(prefill_tc5_kernel<D>, dim3(row_tiles * p.kv_heads * p.kv_splits), dim3(kThreads), L::kAlloc, stream, true, p));
+    const uint32_t row_tiles = (p.token_count * G + L::kRows - 1) / L::kRows;
+    B200KV_CUDA_TRY(launch_kernel(prefill_tc5_kernel<D, RT>, dim3(row_tiles * p.kv_heads * p.kv_splits), dim3(L::kThreads), L::kAlloc, stream, true, p));
     if (p.kv_splits > 1) {
         PrefillMergeParams mp{};
         mp.part_o = p.part_o;
@@ -839,26 +896,30 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     p.capacity = view.capacity;
     p.scratch_rows = scratch_rows;
     p.scale_log2 = scale * 1.4426950408889634f;
+    // head_dim 128: two row tiles per CTA where that still leaves every SM a CTA.  Both take the same K and V tiles, and one tile's
+    // MMAs run under the other one's softmax.  Fewer rows spread better as single tiles.
+    const uint32_t row_tiles_128 = static_cast<uint32_t>((static_cast<uint64_t>(token_count) * (query_heads / view.kv_heads) + kBM - 1) / kBM);
+    const uint32_t tiles_per_cta = view.head_dim == 128 && (row_tiles_128 + 1) / 2 * static_cast<uint64_t>(view.kv_heads) >= 148 ? 2u : 1u;
     // KV split when the row tiles alone leave SMs idle and the caller's workspace has room for the partials
     p.kv_splits = 1;
     {
         const uint32_t G = query_heads / view.kv_heads;
-        const uint32_t row_tiles = (token_count * G + kBM - 1) / kBM;
+        const uint32_t row_tiles = (token_count * G + tiles_per_cta * kBM - 1) / (tiles_per_cta * kBM);
         const uint32_t min_tiles = static_cast<uint32_t>((static_cast<uint64_t>(prefill_state ? 0 : base_position) + kBN - 1) / kBN);
         uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, min_tiles);
         const size_t scratch = prefill_tc5_workspace_bytes(static_cast<uint32_t>(rows), view.kv_heads, view.head_dim);
         while (want > 1 && workspace_bytes < scratch + 1024 + prefill_tc5_split_bytes(token_count, query_heads, view.kv_heads, view.head_dim, want)) --want;
         if (want > 1) {
             p.kv_splits = want;
-            p.rows_padded = row_tiles * kBM;
+            p.rows_padded = row_tiles_128 * kBM;   // what the workspace is sized for; rows past the chunk's are never stored
             uint8_t* part = reinterpret_cast<uint8_t*>(v_scratch + static_cast<size_t>(view.kv_heads) * scratch_rows * view.head_dim);
             part = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(part) + 1023) & ~static_cast<uintptr_t>(1023));
             p.part_o = reinterpret_cast<float*>(part);
             p.part_ml = reinterpret_cast<float2*>(p.part_o + static_cast<size_t>(want) * view.kv_heads * p.rows_padded * view.head_dim);
         }
     }
-    return view.head_dim == 128 ? launch_tc5<128>(view, p, k_scratch, v_scratch, static_cast<uint32_t>(rows), prepared_rows, stream)
-                                : launch_tc5<256>(view, p, k_scratch, v_scratch, static_cast<uint32_t>(rows), prepared_rows, stream);
+    const auto launch = view.head_dim == 256 ? launch_tc5<256, 1> : tiles_per_cta == 2 ? launch_tc5<128, 2> : launch_tc5<128, 1>;
+    return launch(view, p, k_scratch, v_scratch, static_cast<uint32_t>(rows), prepared_rows, stream);
 }
 
 // The pre-pass alone, for positions [0, prepared_rows), into the scratch laid out for a chunk that sees `rows` positions
