@@ -169,8 +169,8 @@ B200KV_API int b200kv_workspace_reset(void* workspace, size_t workspace_bytes, v
  * whose grid does not fit the buffer are not traced. */
 B200KV_API int b200kv_set_timeline_buffer(uint64_t* device_words, uint32_t capacity_words);
 /* Which streaming kernel serves int8 caches (process-wide; for A/B measurement and tests): 0 = the tcgen05 kernels
- * where they apply (default), 1 = none of them: the warp-level mma kernel at head_dim 128, the generic kernel at
- * head_dim 256.  No counterpart in the reference. */
+ * where they apply (default), 1 = none of them: the warp-level mma kernel at head_dim 128, the streaming kernel for
+ * all modes at head_dim 256.  No counterpart in the reference. */
 B200KV_API int b200kv_set_decode_kernel(int choice);
 
 /* ---- cache storage ---------------------------------------------------------
@@ -331,9 +331,9 @@ B200KV_API int b200kv_exchange_destroy(void* buffer);
 /* Which stage-1 kernel b200kv_decode_attn picks for this view: 1 = the streaming
  * int8 kernels (int8 K and V, head_dim 128, 1/2/4 query heads per kv head,
  * capacity a multiple of 8; merge, append and cross-GPU exchange fused in),
- * 2 = the tcgen05 stage 1 for head_dim 256 (int8 K and V, 4/6/8 query heads per
- * kv head, capacity a multiple of 8; single-session launches, the merge kernel
- * follows), 0 = the generic kernel (every other mode and shape).
+ * 2 = the tcgen05 kernel for head_dim 256 (int8 K and V, 4/6/8 query heads per
+ * kv head, capacity a multiple of 8; single-session launches, merge and append
+ * fused in), 0 = the streaming kernel for all modes (every other mode and shape).
  * No counterpart in the reference. */
 B200KV_API int b200kv_decode_kernel_kind(const b200kv_view* view, uint32_t query_heads);
 
@@ -427,9 +427,9 @@ B200KV_API size_t b200kv_prefill_workspace_bytes(uint32_t token_count, uint32_t 
  * separate workspaces.  Cache rows below `rows` must hold finite values (freshly created caches are zero). */
 B200KV_API size_t b200kv_prefill_scratch_bytes(uint64_t rows, uint32_t kv_heads, uint32_t head_dim);
 /* Optional extra room behind that scratch (workspace_bytes >= scratch + this): when a chunk has too few query rows
- * to give every SM a row tile (512 tokens x 6 heads per kv head = 96 tiles on 148 SMs), the tcgen05 kernel then also
- * splits the KV range of each tile over up to 8 CTAs, which leave unnormalised partials here for a merge kernel.
- * 50 MB for 512 tokens x 24 heads x d=256.  Without it the launch runs unsplit. */
+ * to give every SM a row tile (37 tokens x 6 heads per kv head = 8 tiles on 148 SMs), the tcgen05 kernel may also
+ * split the KV range of each tile over up to 8 CTAs (16 for the smallest chunks), which leave unnormalised partials
+ * here for a merge kernel.  101 MB for 512 tokens x 24 heads x d=256.  Without it the launch runs unsplit. */
 B200KV_API size_t b200kv_prefill_split_bytes(uint32_t token_count, uint32_t query_heads, uint32_t kv_heads, uint32_t head_dim);
 
 /* Replaces launch_qwen35_splitk_suffix_attention_quant

@@ -38,7 +38,9 @@ size_t b200kv_prefill_scratch_bytes(uint64_t rows, uint32_t kv_heads, uint32_t h
 }
 
 size_t b200kv_prefill_split_bytes(uint32_t token_count, uint32_t query_heads, uint32_t kv_heads, uint32_t head_dim) {
-    return prefill_tc5_split_bytes(token_count, query_heads, kv_heads, head_dim, 8) + 2048;   // up to 8 splits, alignment slack
+    // small launches may be split further (a launch takes no more splits than its workspace holds); alignment slack
+    const uint64_t row_tiles = kv_heads == 0 ? 0 : (static_cast<uint64_t>(token_count) * (query_heads / kv_heads) + 127) / 128 * kv_heads;
+    return prefill_tc5_split_bytes(token_count, query_heads, kv_heads, head_dim, row_tiles <= 18 ? 16 : 8) + 2048;
 }
 
 int b200kv_prefill_prepare(const b200kv_view* view, uint32_t prepared_rows, uint64_t rows, void* workspace, size_t workspace_bytes,

@@ -44,7 +44,7 @@ constexpr int kBN = 64;           // positions per KV tile
 constexpr int kKPairs = 2;                         // K ring: stages of two tiles each (one S MMA covers a pair)
 constexpr uint32_t kSpin = 1u << 20;
 constexpr float kRescaleThreshold = 8.0f;        // log2 units
-constexpr uint32_t kMaxKvSplits = 8;
+constexpr uint32_t kMaxKvSplits = 16;
 
 struct Tc5Params {
     CUtensorMap kmap, vmap;      // fp16 [kv_heads * rows][d], box 64 x 64, 128-byte swizzle
@@ -660,7 +660,7 @@ struct PrefillMergeParams {
     uint32_t kv_splits, kv_heads, query_heads, rows_padded, total_rows;   // total_rows = token_count * G per kv head
 };
 
-template <int D>
+template <int D, uint32_t MAX_SPLITS>   // kv_splits <= MAX_SPLITS
 __global__ void __launch_bounds__(256) prefill_merge_kernel(const __grid_constant__ PrefillMergeParams p) {
     constexpr int VPR = D / 4;   // float4 per row
     pdl_launch_dependents();
@@ -670,10 +670,10 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const __grid_constan
     if (idx >= static_cast<size_t>(p.total_rows) * VPR) return;
     const uint32_t gr = static_cast<uint32_t>(idx / VPR), c = static_cast<uint32_t>(idx % VPR) * 4;
     // every load of the row's splits is issued before the first is used; an empty split's O was never written and counts for nothing
-    float2 ml[kMaxKvSplits];
-    float4 o[kMaxKvSplits];
+    float2 ml[MAX_SPLITS];
+    float4 o[MAX_SPLITS];
 #pragma unroll
-    for (uint32_t s = 0; s < kMaxKvSplits; ++s) {
+    for (uint32_t s = 0; s < MAX_SPLITS; ++s) {
         ml[s] = make_float2(-INFINITY, 0.0f);
         o[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (s < p.kv_splits) {
@@ -684,12 +684,12 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const __grid_constan
     }
     float M = -INFINITY;
 #pragma unroll
-    for (uint32_t s = 0; s < kMaxKvSplits; ++s)
+    for (uint32_t s = 0; s < MAX_SPLITS; ++s)
         if (!(ml[s].y <= 0.0f) && ml[s].x != -INFINITY) M = fmaxf(M, ml[s].x);   // keeps NaN partials in play
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float lsum = 0.0f;
 #pragma unroll
-    for (uint32_t s = 0; s < kMaxKvSplits; ++s) {
+    for (uint32_t s = 0; s < MAX_SPLITS; ++s) {
         if (ml[s].y <= 0.0f || ml[s].x == -INFINITY) continue;
         const float w = exp2f(ml[s].x - M);
         acc.x = fmaf(o[s].x, w, acc.x); acc.y = fmaf(o[s].y, w, acc.y); acc.z = fmaf(o[s].z, w, acc.z); acc.w = fmaf(o[s].w, w, acc.w);
@@ -832,7 +832,8 @@ int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half*
         mp.rows_padded = p.rows_padded;
         mp.total_rows = p.token_count * G;
         const size_t work = static_cast<size_t>(mp.total_rows) * (D / 4);
-        B200KV_CUDA_TRY(launch_kernel(prefill_merge_kernel<D>, dim3(static_cast<unsigned>((work + 255) / 256), p.kv_heads), dim3(256), 0, stream, true, mp));
+        const auto merge = p.kv_splits <= 4 ? prefill_merge_kernel<D, 4> : prefill_merge_kernel<D, kMaxKvSplits>;
+        B200KV_CUDA_TRY(launch_kernel(merge, dim3(static_cast<unsigned>((work + 255) / 256), p.kv_heads), dim3(256), 0, stream, true, mp));
     }
     return B200KV_OK;
 }
@@ -851,15 +852,21 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
     return static_cast<size_t>(splits) * kv_heads * rows_padded * (head_dim + 2) * sizeof(float);
 }
 
-// How many KV splits fill the SMs best: one CTA per SM, `units` row-tile CTAs per split.
-static uint32_t pick_kv_splits(uint32_t units, uint32_t min_tiles) {
-    const uint32_t sms = 148;
+// How many KV splits: the number with the least estimated time, for `units` row-tile CTAs of up to `tiles` KV tiles.  A wave of
+// 148 CTAs costs its tiles and about 8 us of set-up, Q, epilogue and launch; a split launch also its merge, 3 us and
+// the partials' way out and back.  Measured per layer, all kernels (head_dim 256 / 24 heads, q8_0):
+//   20 tokens over 16000 (4 units):   5 splits 77 us, 8: 66, 16: 58     37 over 3001 (8):  5: 38, 8: 35, 12: 34, 16: 34
+//   128 over 8192 (24):   5: 54, 6: 52, 8 (a second wave): 69           300 over 8192 (60): 1: 124, 2: 92, 4: 102
+//   512 over 8192 (96):   1: 127, 2: 158, 3 (what filling the last wave best asks for): 138
+static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t head_dim) {
+    const double tile_us = head_dim == 256 ? 0.73 : 0.52, wave_us = 8.0, merge_us = 3.0, partial_us = head_dim == 256 ? 0.11 : 0.055;
     uint32_t best = 1;
-    double best_eff = static_cast<double>(units) / ((units + sms - 1) / sms * sms);
-    for (uint32_t s = 2; s <= kMaxKvSplits; ++s) {
-        if (min_tiles < 8 * s) break;   // every split should still walk a few tiles
-        const double eff = static_cast<double>(units) * s / ((units * s + sms - 1) / sms * sms);
-        if (eff > best_eff * 1.15) { best = s; best_eff = eff; }   // a split costs a partial round trip: only for a clear gain
+    double best_us = 0.0;
+    for (uint32_t s = 1; s <= kMaxKvSplits; ++s) {
+        if (s > 1 && tiles < 3 * s) break;   // every split walks a few tiles
+        const uint64_t ctas = static_cast<uint64_t>(units) * s, waves = (ctas + 147) / 148;
+        const double us = static_cast<double>(waves) * (tiles * tile_us / s + wave_us) + (s > 1 ? merge_us + partial_us * static_cast<double>(ctas) : 0.0);
+        if (s == 1 || us < best_us) { best = s; best_us = us; }
     }
     return best;
 }
@@ -905,8 +912,9 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     {
         const uint32_t G = query_heads / view.kv_heads;
         const uint32_t row_tiles = (token_count * G + tiles_per_cta * kBM - 1) / (tiles_per_cta * kBM);
-        const uint32_t min_tiles = static_cast<uint32_t>((static_cast<uint64_t>(prefill_state ? 0 : base_position) + kBN - 1) / kBN);
-        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, min_tiles);
+        // a device-side state leaves the range unknown here (no split); so does a range that is mostly the chunk's own triangle
+        const bool prefix = prefill_state == nullptr && base_position >= token_count;
+        uint32_t want = prefix ? pick_kv_splits(row_tiles * view.kv_heads, static_cast<uint32_t>((rows + kBN - 1) / kBN), view.head_dim) : 1;
         const size_t scratch = prefill_tc5_workspace_bytes(static_cast<uint32_t>(rows), view.kv_heads, view.head_dim);
         while (want > 1 && workspace_bytes < scratch + 1024 + prefill_tc5_split_bytes(token_count, query_heads, view.kv_heads, view.head_dim, want)) --want;
         if (want > 1) {

@@ -21,7 +21,8 @@ def expected(st, q, gate, P, T, Hq, scale):
 # one row per token and kv head (G = 1) with 148 kv heads: two row tiles per CTA from the second token tile on;
 # 2 x 4 heads: the same launch below the line; 40 heads x G = 2: the line itself (ceil(tiles / 2) x 40 >= 148 from 7 tiles on)
 @pytest.mark.parametrize("H,G,P,T", [(148, 1, 0, 1), (148, 1, 70, 128), (148, 1, 0, 129), (148, 1, 65, 255), (148, 1, 3, 257), (148, 1, 600, 130),
-                                     (148, 2, 64, 193), (8, 4, 100, 33), (40, 2, 130, 384), (40, 2, 130, 385), (37, 1, 1100, 513)])
+                                     (148, 2, 64, 193), (8, 4, 100, 33), (40, 2, 130, 384), (40, 2, 130, 385), (37, 1, 1100, 513),
+                                     (2, 4, 3001, 33), (1, 1, 4000, 5)])   # few rows over a long prefix: up to 16 splits
 @pytest.mark.parametrize("act", [torch.float16, torch.float32])
 def test_row_tiles(cuda, H, G, P, T, act):
     g = torch.Generator(device="cuda")
