@@ -36,6 +36,14 @@ namespace b200kv {
 namespace {
 
 constexpr int kTile = 16;                     // positions per tile
+// The tensor core truncates (towards zero) where an fp32 instruction rounds, so a chain of MMAs into one accumulator leaves a bias of
+// half a unit per link.  Scores are therefore chains of kChain MMAs added up by fp32 instructions, and where a warp may have more than
+// kLongTiles tiles the O accumulators are emptied into fp32 sums every kHold of them (HOLD; those launches are bound by HBM, in the
+// others the extra code costs 2 to 7 %).  Relative error against float64, fp16 cache: 24 / 4 heads of 256, 6001 positions 2.1e-7 (one
+// chain of 16 per score: 5.5e-7; fp32 dot products lane by lane: 2.3e-7); 32 / 8 heads of 128, 131072 positions, 57 tiles a warp: 4e-7
+// (never emptied: 1.1e-6; lane by lane: 7.9e-7).
+template <int KF> constexpr int kChain = KF == 1 ? 4 : 2;
+constexpr int kLongTiles = 24, kHold = 16;
 enum Fmt { F16 = 0, ROW = 1, BLOCK = 2 };     // a side's storage: fp16, int8 with one scale per row, int8 with a scale per 32 dims
 
 template <int D, int FMT>
@@ -111,7 +119,7 @@ __device__ __forceinline__ float quad_max(float v) {
     return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
 }
 
-template <int D, int KF, int VF, int WARPS>
+template <int D, int KF, int VF, int WARPS, bool HOLD>
 __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(const __grid_constant__ DecodeParams p) {
     using P = Plan<D, KF, VF, WARPS>;
     using KU = Unit<D, KF>;
@@ -294,15 +302,44 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
             if (lane == 0) *reinterpret_cast<__half*>(at + kTile * U::kRow + skew + r * 2) = row.scales[0];
         }
     };
+    // Sums of earlier tiles and how far they have been rescaled since.  `local` is 0, but not to the compiler: the array stays out
+    // of the registers.
+    float held[HOLD ? 2 * NT : 1], held_by = 1.0f;
+    uint32_t local = 0;
+    if constexpr (HOLD) asm volatile("mov.u32 %0, 0;" : "=r"(local));
+    auto unhold = [&]() {
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                o[i][j] = fmaf(held[local + 2 * i + j], held_by, o[i][j] + o[i][j + 2]);
+                o[i][j + 2] = 0.0f;
+            }
+    };
+    auto hold = [&](bool first) {
+        if (!first) unhold();
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                held[local + 2 * i + j] = o[i][j] + o[i][j + 2];
+                o[i][j] = o[i][j + 2] = 0.0f;
+            }
+        held_by = 1.0f;
+    };
     auto rescale = [&](float f) {
 #pragma unroll
         for (int i = 0; i < NT; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) o[i][j] *= f;
+        if constexpr (HOLD) held_by *= f;
     };
 
     for (int t = 0; t < my_tiles; ++t) {
         const uint32_t pos = tile_pos(t);
+        if constexpr (HOLD) {
+            if (t % kHold == 0 && t != 0) hold(t == kHold);
+        }
         if (t == patch_tile) {                    // the appended row's tile: both units have to be there
             cp_wait<0>();
             asm volatile("bar.sync 3, 96;" ::: "memory");   // ... and both sides of the row
@@ -348,30 +385,36 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
                     }
                 }
             } else {
-                float acc[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+                float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint4 qa = *reinterpret_cast<const uint4*>(smem + (ks * 32 + lane) * 16);
-                    const uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w};
-                    uint32_t r[4];
-                    if constexpr (KF == F16) {
-                        ldsm4(row_at + (((2 * ks + lchunk) ^ flip) << 4), r);
-                        mma(acc[0], a, r[0], r[2]);
-                        mma(acc[1], a, r[1], r[3]);
-                    } else if ((ks & 1) == 0) {   // one ldmatrix serves two k steps of int8
-                        const uint4 qb = *reinterpret_cast<const uint4*>(smem + ((ks + 1) * 32 + lane) * 16);
-                        const uint32_t a2[4] = {qb.x, qb.y, qb.z, qb.w};
-                        ldsm4(row_at + (((ks + lchunk) ^ flip) << 4), r);
+                for (int k0 = 0; k0 < D / 16; k0 += kChain<KF>) {
+                    float acc[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) r[i] ^= 0x80808080u;
-                        mma(acc[0], a, i8x2<0x4140>(r[0]), i8x2<0x4342>(r[0]));
-                        mma(acc[1], a, i8x2<0x4140>(r[1]), i8x2<0x4342>(r[1]));
-                        mma(acc[0], a2, i8x2<0x4140>(r[2]), i8x2<0x4342>(r[2]));
-                        mma(acc[1], a2, i8x2<0x4140>(r[3]), i8x2<0x4342>(r[3]));
+                    for (int ks = k0; ks < k0 + kChain<KF>; ++ks) {
+                        const uint4 qa = *reinterpret_cast<const uint4*>(smem + (ks * 32 + lane) * 16);
+                        const uint32_t a[4] = {qa.x, qa.y, qa.z, qa.w};
+                        uint32_t r[4];
+                        if constexpr (KF == F16) {
+                            ldsm4(row_at + (((2 * ks + lchunk) ^ flip) << 4), r);
+                            mma(acc[0], a, r[0], r[2]);
+                            mma(acc[1], a, r[1], r[3]);
+                        } else if ((ks & 1) == 0) {   // one ldmatrix serves two k steps of int8
+                            const uint4 qb = *reinterpret_cast<const uint4*>(smem + ((ks + 1) * 32 + lane) * 16);
+                            const uint32_t a2[4] = {qb.x, qb.y, qb.z, qb.w};
+                            ldsm4(row_at + (((ks + lchunk) ^ flip) << 4), r);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) r[i] ^= 0x80808080u;
+                            mma(acc[0], a, i8x2<0x4140>(r[0]), i8x2<0x4342>(r[0]));
+                            mma(acc[1], a, i8x2<0x4140>(r[1]), i8x2<0x4342>(r[1]));
+                            mma(acc[0], a2, i8x2<0x4140>(r[2]), i8x2<0x4342>(r[2]));
+                            mma(acc[1], a2, i8x2<0x4140>(r[3]), i8x2<0x4342>(r[3]));
+                        }
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { hi[i] += acc[i >> 1][i & 1]; lo[i] += acc[i >> 1][(i & 1) + 2]; }
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[i] = acc[i >> 1][i & 1] + acc[i >> 1][(i & 1) + 2];
+                for (int i = 0; i < 4; ++i) s[i] = hi[i] + lo[i];
                 if constexpr (KF == ROW) {
                     const uint8_t* src = scale_at + (reinterpret_cast<uintptr_t>(k_scales + static_cast<uint64_t>(pos) * 2) & 2u);
 #pragma unroll
@@ -495,6 +538,9 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
 
     // ---- the warps' states, through the ring's memory, into one partial of the CTA --------------------------------
     cp_wait<0>();
+    if constexpr (HOLD) {
+        if (my_tiles > kHold) unhold();
+    }
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
     if (c4 == 0) *reinterpret_cast<float2*>(ml_s + (warp * 8 + (lane >> 2)) * 2) = make_float2(m_ref, l_run);
@@ -542,24 +588,30 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     tail::fused_merge<SEG, WARPS * 32>(p, session, kv_head, split, num_splits, G, reinterpret_cast<float*>(smem));
 }
 
-template <int D, int KF, int VF, int WARPS>
-int launch_one(const DecodeParams& p, dim3 grid, cudaStream_t stream) {
+template <int D, int KF, int VF, int WARPS, bool HOLD>
+int launch_kernel_of(const DecodeParams& p, dim3 grid, cudaStream_t stream) {
     using P = Plan<D, KF, VF, WARPS>;
     static std::atomic<uint64_t> done{0};   // one per kernel instantiation: devices that have opted in
-    const cudaError_t attr_err = opt_in_dynamic_smem(reinterpret_cast<const void*>(decode_stream_kernel<D, KF, VF, WARPS>), P::kAlloc, done);
+    const cudaError_t attr_err = opt_in_dynamic_smem(reinterpret_cast<const void*>(decode_stream_kernel<D, KF, VF, WARPS, HOLD>), P::kAlloc, done);
     if (attr_err != cudaSuccess) { set_last_cuda_error(attr_err, "cudaFuncSetAttribute(decode_stream)"); return B200KV_ERR_CUDA; }
-    B200KV_CUDA_TRY(launch_kernel(decode_stream_kernel<D, KF, VF, WARPS>, grid, dim3(P::kThreads), P::kAlloc, stream, true, p));
+    B200KV_CUDA_TRY(launch_kernel(decode_stream_kernel<D, KF, VF, WARPS, HOLD>, grid, dim3(P::kThreads), P::kAlloc, stream, true, p));
     return B200KV_OK;
+}
+
+template <int D, int KF, int VF, int WARPS>
+int launch_one(const DecodeParams& p, bool hold, dim3 grid, cudaStream_t s) {
+    return hold ? launch_kernel_of<D, KF, VF, WARPS, true>(p, grid, s) : launch_kernel_of<D, KF, VF, WARPS, false>(p, grid, s);
 }
 
 template <int D, int WARPS>
 int launch_mode(const DecodeParams& p, const b200kv_view& g, dim3 grid, cudaStream_t s) {
     const bool blocks = g.qblock == 32;
+    const bool hold = p.split_positions / kTile > static_cast<uint32_t>(kLongTiles * WARPS);   // positions a split may have, over its warps
     switch (g.quant_mode) {
-        case B200KV_F16_F16: return launch_one<D, F16, F16, WARPS>(p, grid, s);
-        case B200KV_Q8_F16: return blocks ? launch_one<D, BLOCK, F16, WARPS>(p, grid, s) : launch_one<D, ROW, F16, WARPS>(p, grid, s);
-        case B200KV_F16_Q8: return blocks ? launch_one<D, F16, BLOCK, WARPS>(p, grid, s) : launch_one<D, F16, ROW, WARPS>(p, grid, s);
-        default: return blocks ? launch_one<D, BLOCK, BLOCK, WARPS>(p, grid, s) : launch_one<D, ROW, ROW, WARPS>(p, grid, s);
+        case B200KV_F16_F16: return launch_one<D, F16, F16, WARPS>(p, hold, grid, s);
+        case B200KV_Q8_F16: return blocks ? launch_one<D, BLOCK, F16, WARPS>(p, hold, grid, s) : launch_one<D, ROW, F16, WARPS>(p, hold, grid, s);
+        case B200KV_F16_Q8: return blocks ? launch_one<D, F16, BLOCK, WARPS>(p, hold, grid, s) : launch_one<D, F16, ROW, WARPS>(p, hold, grid, s);
+        default: return blocks ? launch_one<D, BLOCK, BLOCK, WARPS>(p, hold, grid, s) : launch_one<D, ROW, ROW, WARPS>(p, hold, grid, s);
     }
 }
 

@@ -87,3 +87,26 @@ def test_value_scales_that_grow_by_orders_of_magnitude(cuda):
             kv.launch_decode_attention_quant(st.view(), to_dev(q16), query_heads=Hq, scale=d ** -0.5, cache_length=L, output=out,
                                              workspace=kv.decode_workspace(Hq, d), num_splits=splits | kv.FORCE_GENERIC)
             _close(out.cpu().numpy(), ref, (d, qb, splits))
+
+
+# Against float64 over the cache's own fp16 values; the relative 2-norm error has to stay that of fp32 arithmetic.  Per score a sum of d
+# products (rounding about 2^-24 per level of the sum), an exponential of 2^-22 and weights kept to 2^-22: measured 1.5e-7 to 2.4e-7 here,
+# and 4.4e-7 where one warp adds up 64 tiles or more (the last two cases); the bounds leave room for another draw of the inputs.  A chain
+# of MMAs per score, truncated by the tensor core at every link, came to 3.8e-7 .. 6.2e-7, and one per output over all tiles to 1.4e-6 and 3.3e-6.
+@pytest.mark.parametrize("d,H,Hq,L,splits,bound", [(256, 4, 24, 128, 0, 3.2e-7), (256, 4, 24, 1000, 0, 3.2e-7), (256, 4, 24, 6001, 0, 3.2e-7),
+                                                   (128, 8, 32, 1000, 0, 2.9e-7), (128, 1, 4, 65536, 8, 6.0e-7), (256, 1, 6, 20011, 1, 6.0e-7)])
+@pytest.mark.parametrize("act", [torch.float16, torch.float32])
+def test_error_of_fp16_caches_is_that_of_fp32_sums(cuda, d, H, Hq, L, splits, bound, act):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(L + d)
+    st = kv.AttentionLayerKvCacheStorage(L, kv.KvCacheQuantMode.kFp16Fp16, kv_heads=H, head_dim=d, qblock=d)
+    st.key_cache.copy_(torch.randn(H, L, d, generator=g, device="cuda"))
+    st.value_cache.copy_(torch.randn(H, L, d, generator=g, device="cuda"))
+    q = torch.randn(Hq, d, generator=g, device="cuda").to(act)
+    out = torch.empty(Hq, d, device="cuda")
+    kv.launch_decode_attention_quant(st.view(), q, query_heads=Hq, scale=d ** -0.5, cache_length=L, output=out,
+                                     workspace=kv.decode_workspace(Hq, d), num_splits=splits)
+    s = torch.einsum("hgd,hld->hgl", q.double().view(H, Hq // H, d), st.key_cache.double().view(H, L, d)) * d ** -0.5
+    ref = torch.einsum("hgl,hld->hgd", s.softmax(-1), st.value_cache.double().view(H, L, d)).reshape(Hq, d)
+    rel = ((out.double() - ref).norm() / ref.norm()).item()
+    assert rel <= bound, rel
