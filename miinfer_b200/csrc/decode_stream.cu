@@ -140,7 +140,14 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     if (p.lengths != nullptr) {   // as many splits as this session's own length warrants; the surplus CTAs leave at once
         const uint32_t want = (end - begin + p.split_positions - 1) / p.split_positions;
         num_splits = min(num_splits, max(want, 1u));
-        if (split >= num_splits) return;
+        if (split >= num_splits) {
+            if (p.ws_tagged == nullptr) {   // the separate merge kernel reads every split of the launch: an empty partial
+                pdl_wait();
+                for (int idx = tid; idx < G * D; idx += P::kThreads)
+                    tail::emit_partial<SEG>(p, session, split, num_splits, kv_head * G + idx / D, idx % D, 0.0f, -INFINITY, 0.0f);
+            }
+            return;
+        }
     }
     // this CTA's positions: whole tiles counted from `begin`
     const uint64_t tiles = (end - begin + kTile - 1) / kTile;

@@ -110,3 +110,21 @@ def test_error_of_fp16_caches_is_that_of_fp32_sums(cuda, d, H, Hq, L, splits, bo
     ref = torch.einsum("hgl,hld->hgd", s.softmax(-1), st.value_cache.double().view(H, L, d)).reshape(Hq, d)
     rel = ((out.double() - ref).norm() / ref.norm()).item()
     assert rel <= bound, rel
+
+
+@pytest.mark.parametrize("poison", [float("nan"), 3.0])
+def test_separate_merge_reads_only_what_its_launch_wrote(cuda, poison):
+    """More splits than fit on the device with their merge: the merge kernel follows, and reads all splits of all sessions.  What an
+    earlier launch with longer sessions, or anybody else, left in the workspace's plain third must not count."""
+    rng = np.random.default_rng(5)
+    d, H, Hq = 128, 4, 8
+    ws = kv.decode_workspace(Hq, d, 3)
+    ws[ws.numel() // 3 * 2 // 256 * 256:].view(torch.float32).fill_(poison)
+    for lengths, splits in (([900, 300, 7], 128), ([40, 17, 600], 100), ([1, 500, 16], 128)):
+        hosts = [_filled(rng, n, H, d, d, 0, n) for n in lengths]
+        sts, q = [upload(h) for h in hosts], ko.normal_f16(rng, (3, Hq, d))
+        out = torch.full((3, Hq, d), float("nan"), device="cuda")
+        kv.launch_decode_attention_batched([s.view() for s in sts], kv.view_table(3), torch.tensor(lengths, dtype=torch.int32, device="cuda"), max(lengths),
+                                           to_dev(q), query_heads=Hq, scale=d ** -0.5, output=out, workspace=ws, num_splits=splits)
+        for i, h in enumerate(hosts):
+            _close(out[i].cpu().numpy(), h.decode_ref(q[i].astype(np.float32), d ** -0.5, lengths[i])[0], (lengths, splits, i))
