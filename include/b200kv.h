@@ -252,6 +252,7 @@ B200KV_API size_t b200kv_decode_workspace_bytes(uint32_t query_heads, uint32_t h
  * gated_output (= output * sigmoid(gate), gate fp32 [query_heads][head_dim]) are
  * fp32 [query_heads][head_dim]; at least one must be non-NULL; gate may be NULL
  * (then gated_output == output).  num_splits 0 = choose for the device.
+ * q, gate and the outputs may start at any element; q aligned to 16 bytes and the others to 8 keep every kernel open.
  * gated_output_q8 (may be NULL): the gated output re-quantised to Q8_1 blocks of 32 for the projection that
  * follows, [query_heads * head_dim / 32] blocks, as the reference's stage 2 does (.hip:2354-2383: d = amax/127,
  * q = roundf(x/d) clamped to +-127, s = d * sum(q), d and s stored as fp16).  Unlike the reference it is also

@@ -132,9 +132,16 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     uint32_t num_splits = num_splits_arg & ~B200KV_SPLITS_FORCE_GENERIC;
     const uint32_t cap = max_splits_per_session(p.sessions);
     const bool many = p.sessions > 1 || p.lengths != nullptr;
-    bool use_fast = !force_stream && q8_fast_path_ok(geometry, p.query_heads);
+    // Q, gate and outputs may start at any element.  The kernels below fetch Q in 16-byte pieces, decode_stream.cu takes it as it lies.
+    auto aligned = [](const void* ptr, size_t bytes) { return reinterpret_cast<uintptr_t>(ptr) % bytes == 0; };   // null counts as aligned
+    p.q_pairs = aligned(p.q, p.q_is_f16 ? 4 : 8);
+    const bool q_vectors = aligned(p.q, 16);
+    // the in-launch merge takes gate and outputs two floats at a time; the merge kernel behind the launch one by one
+    const bool pairs = aligned(merge.gate, 8) && aligned(merge.output, 8) && aligned(merge.gated_output, 8) && aligned(merge.out_acc, 8);
+    if (merge.xchg.world > 1 && !pairs) return B200KV_ERR_INVALID;   // the exchange is part of the in-launch merge
+    bool use_fast = !force_stream && q_vectors && (pairs || !many) && q8_fast_path_ok(geometry, p.query_heads);
     // head_dim 256: the tcgen05 kernel for single-session launches
-    bool use_wide = !force_stream && !use_fast && !many && streaming_kernel_choice() != 1 && decode_tc5_wide_ok(geometry, p.query_heads);
+    bool use_wide = !force_stream && !use_fast && !many && q_vectors && streaming_kernel_choice() != 1 && decode_tc5_wide_ok(geometry, p.query_heads);
     // Single sessions that are short for the device: the mma.sync kernel starts, splits and merges faster than the tcgen05
     // kernels' pipelines fill, until its instruction issue shows.
     if (num_splits == 0 && !many && streaming_kernel_choice() != 1) {
@@ -156,6 +163,7 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     const size_t plain_offset = workspace_plain_offset(workspace_bytes);
     if (workspace_bytes - plain_offset < plain_bytes) return B200KV_ERR_WORKSPACE;
     p.num_splits = num_splits;
+    p.fuse = merge;
     p.ws_m = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + plain_offset);
     p.ws_l = p.ws_m + slots;
     p.ws_acc = p.ws_l + slots;
@@ -165,10 +173,9 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         if (plain_offset < 2 * plain_bytes) return B200KV_ERR_WORKSPACE;
         // The in-launch merge; a lone split that has to produce Q8_1 blocks goes through the merge kernel instead
         // (a block of 32 outputs is quantised by 16 cooperating threads, which the single-split shortcut has not).
-        const bool fuse_merge = !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1);
+        const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1);
         p.ws_tagged = fuse_merge ? static_cast<uint64_t*>(workspace) : nullptr;
         p.tag = next_launch_tag();
-        p.fuse = merge;
         int rc = B200KV_ERR_UNSUPPORTED;
         if (streaming_kernel_choice() != 1) rc = launch_decode_tc5(p, geometry, max_length, stream);
         if (rc == B200KV_ERR_UNSUPPORTED) rc = launch_decode_q8(p, geometry, max_length, stream);
@@ -176,12 +183,11 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         if (rc != B200KV_ERR_UNSUPPORTED) return rc;
         p.ws_tagged = nullptr;
     }
-    const bool fuse_merge = !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && plain_offset >= 2 * plain_bytes &&
+    const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && plain_offset >= 2 * plain_bytes &&
                             stream_merge_fits(geometry.kv_heads, num_splits, many);
     if (merge.xchg.world > 1 && !fuse_merge) return B200KV_ERR_UNSUPPORTED;   // the exchange is part of the in-launch merge
     p.ws_tagged = fuse_merge ? static_cast<uint64_t*>(workspace) : nullptr;
     p.tag = next_launch_tag();
-    p.fuse = merge;
     int rc = B200KV_ERR_UNSUPPORTED;
     if (use_wide) rc = launch_decode_tc5_wide(p, geometry, stream);
     if (rc == B200KV_ERR_UNSUPPORTED) rc = launch_decode_stream(p, geometry, max_length, stream);

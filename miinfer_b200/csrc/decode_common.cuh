@@ -72,6 +72,7 @@ struct DecodeParams {
     uint32_t sessions;
     const void* q;                           // [sessions][query_heads][d]
     int q_is_f16;
+    int q_pairs;                             // q is aligned to two elements (decode_stream.cu; the other kernels are launched only with 16 bytes)
     uint32_t query_heads;
     float scale;
     uint32_t num_splits;                     // per session (batched: of the longest session)

@@ -231,18 +231,27 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         float amax = 0.0f;
         if (h < G) {
             const size_t base = (static_cast<size_t>(session) * p.query_heads + kv_head * G + h) * D;
+            if (p.q_pairs && p.q_is_f16) {        // all loads of a head in flight together
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                const size_t at = base + (i * 32 + lane) * 2;
-                if (p.q_is_f16) {
-                    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(static_cast<const __half*>(p.q) + at));
-                    q[2 * i] = v.x; q[2 * i + 1] = v.y;
-                } else {
-                    const float2 v = *reinterpret_cast<const float2*>(static_cast<const float*>(p.q) + at);
+                for (int i = 0; i < NP; ++i) {
+                    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(static_cast<const __half*>(p.q) + base + (i * 32 + lane) * 2));
                     q[2 * i] = v.x; q[2 * i + 1] = v.y;
                 }
-                amax = fmaxf(amax, fmaxf(fabsf(q[2 * i]), fabsf(q[2 * i + 1])));
+            } else if (p.q_pairs) {
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    const float2 v = *reinterpret_cast<const float2*>(static_cast<const float*>(p.q) + base + (i * 32 + lane) * 2);
+                    q[2 * i] = v.x; q[2 * i + 1] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 2 * NP; ++i) {
+                    const size_t at = base + ((i >> 1) * 32 + lane) * 2 + (i & 1);
+                    q[i] = p.q_is_f16 ? __half2float(static_cast<const __half*>(p.q)[at]) : static_cast<const float*>(p.q)[at];
+                }
             }
+#pragma unroll
+            for (int i = 0; i < 2 * NP; ++i) amax = fmaxf(amax, fabsf(q[i]));
             amax = warp_max(amax);
         } else {
 #pragma unroll

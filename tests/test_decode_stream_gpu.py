@@ -128,3 +128,40 @@ def test_separate_merge_reads_only_what_its_launch_wrote(cuda, poison):
                                            to_dev(q), query_heads=Hq, scale=d ** -0.5, output=out, workspace=ws, num_splits=splits)
         for i, h in enumerate(hosts):
             _close(out[i].cpu().numpy(), h.decode_ref(q[i].astype(np.float32), d ** -0.5, lengths[i])[0], (lengths, splits, i))
+
+
+# the kernels that a 16-byte aligned call of these shapes takes: the streaming one, the two of int8 at head_dim 256 and 128, and a batch
+@pytest.mark.parametrize("d,H,Hq,qb,mode,splits", [(256, 4, 24, 256, 0, 0), (128, 2, 6, 32, 1, 0), (256, 4, 24, 32, 3, 9), (128, 8, 32, 32, 3, 9), (128, 8, 32, 32, 3, 1)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_tensors_that_start_at_any_element(cuda, d, H, Hq, qb, mode, splits, dtype):
+    rng = np.random.default_rng(d + mode)
+    L, scale = 1000, d ** -0.5
+    host = _filled(rng, L, H, d, qb, mode, L)
+    st, ws = upload(host), kv.decode_workspace(Hq, d, 2)
+    q16, gate = ko.normal_f16(rng, (2, Hq, d)), rng.standard_normal((2, Hq, d)).astype(np.float32)
+    at = lambda t, off, n: torch.cat([torch.zeros(off, device="cuda", dtype=t.dtype), t.flatten()[:n]])[off:].view(-1, Hq, d)
+    table, lengths = kv.view_table(2), torch.tensor([L, 333], dtype=torch.int32, device="cuda")
+    refs = [host.decode_ref(q16[i].astype(np.float32), scale, n, gate[i]) for i, n in enumerate((L, 333))]
+    for qoff, goff, ooff in ((1, 0, 0), (3, 1, 1), (0, 1, 0), (0, 0, 1), (4, 2, 2)):
+        n = Hq * d
+        q, g = to_dev(q16).to(dtype), to_dev(gate)
+        out, gated = (torch.full((2 * n + 4,), float("nan"), device="cuda") for _ in range(2))
+        one = lambda t: t[ooff:ooff + n].view(Hq, d)
+        kv.launch_decode_attention_quant(st.view(), at(q, qoff, n)[0], query_heads=Hq, scale=scale, cache_length=L, output=one(out), gate=at(g, goff, n)[0],
+                                         gated_output=one(gated), workspace=ws, num_splits=splits)
+        tol = 1e-5 if mode != 3 or qoff * q.element_size() % 16 else 3e-4   # an unaligned query goes to the streaming kernel, others are taken as 15-bit
+        for got, ref in ((one(out), refs[0][0]), (one(gated), refs[0][1])):
+            err = np.linalg.norm(got.cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref)
+            assert err <= tol, (qoff, goff, ooff, err)
+        two = lambda t: t[ooff:ooff + 2 * n].view(2, Hq, d)
+        kv.launch_decode_attention_batched([st.view(), st.view()], table, lengths, L, at(q, qoff, 2 * n), query_heads=Hq, scale=scale, output=two(out),
+                                           gate=at(g, goff, 2 * n), gated_output=two(gated), workspace=ws, num_splits=splits)
+        for i in range(2):
+            for got, ref in ((two(out)[i], refs[i][0]), (two(gated)[i], refs[i][1])):
+                err = np.linalg.norm(got.cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref)
+                assert err <= 3e-4, (qoff, goff, ooff, i, err)
+        m, l = (torch.empty(Hq, device="cuda") for _ in range(2))
+        kv.launch_decode_partials(st.view(), at(q, qoff, n)[0], query_heads=Hq, scale=scale, range_begin=0, range_end=L, part_m=m, part_l=l,
+                                  part_acc=one(out), workspace=ws, num_splits=splits)
+        got = (one(out) / l[:, None]).cpu().numpy()
+        assert np.linalg.norm(got.astype(np.float64) - refs[0][0]) / np.linalg.norm(refs[0][0]) <= 3e-4, (qoff, ooff, "partials")
