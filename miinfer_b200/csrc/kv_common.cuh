@@ -63,9 +63,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Checks the geometry and the pointers a view needs for its mode.
 int validate_view(const b200kv_view* view);
 
-// The first `tokens` rows of `layers` caches to (to_blob) or from compact snapshots in this device's memory, one launch for
-// all layers; snapshot l starts at blob + offsets[l].  The views are valid, of one geometry, and hold `tokens` rows.
-int snapshot_copy_device(const b200kv_view* views, uint32_t layers, uint64_t tokens, uint8_t* blob, const uint64_t* offsets, bool to_blob,
+// The first `tokens` rows of `layers` caches to (to_blob) or from compact snapshots that lie one behind the other at `blob`, snapshot l
+// of layer_bytes[l] bytes.  The views are valid and hold `tokens` rows.  One launch for all layers of a geometry where everything is
+// memory of the current device, strided copies otherwise.
+int snapshot_copy_layers(const b200kv_view* views, uint32_t layers, uint64_t tokens, uint8_t* blob, const uint64_t* layer_bytes, bool to_blob,
                          cudaStream_t stream);
 
 // ---- device helpers ------------------------------------------------------------

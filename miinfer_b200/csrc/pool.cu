@@ -175,24 +175,6 @@ bool same_shape(const b200kv_view& a, const b200kv_view& b) {
     return a.kv_heads == b.kv_heads && a.head_dim == b.head_dim && a.qblock == b.qblock && a.quant_mode == b.quant_mode;
 }
 
-// All layers between the caches and one payload (the layers' snapshots one behind the other).  Layers that share a geometry
-// -- normally all -- travel in one launch.
-int copy_layers(const b200kv_view* views, const std::vector<uint64_t>& per_layer, uint64_t tokens, void* payload, bool to_blob, void* stream) {
-    if (tokens == 0) return B200KV_OK;
-    std::vector<uint64_t> offsets(per_layer.size());
-    uint64_t off = 0;
-    for (size_t l = 0; l < per_layer.size(); off += per_layer[l++]) offsets[l] = off;
-    for (size_t l = 0; l < per_layer.size();) {
-        size_t end = l + 1;
-        while (end < per_layer.size() && same_shape(views[end], views[l])) ++end;
-        const int rc = snapshot_copy_device(views + l, static_cast<uint32_t>(end - l), tokens, static_cast<uint8_t*>(payload), offsets.data() + l,
-                                            to_blob, static_cast<cudaStream_t>(stream));
-        if (rc != B200KV_OK) return rc;
-        l = end;
-    }
-    return B200KV_OK;
-}
-
 }  // namespace
 
 extern "C" {
@@ -257,7 +239,7 @@ int b200kv_pool_capture(b200kv_pool* pool, const uint32_t* tokens, uint32_t pref
         }
         dst.layer_bytes = per_layer;
         dst.geometry = layer_views[0];
-        rc = copy_layers(layer_views, per_layer, prefix_length, dst.payload, true, stream);
+        rc = snapshot_copy_layers(layer_views, layers, prefix_length, static_cast<uint8_t*>(dst.payload), per_layer.data(), true, static_cast<cudaStream_t>(stream));
         if (rc != B200KV_OK) return rc;
         if (captured != nullptr) *captured = 1;
     } catch (const std::exception&) {
@@ -319,7 +301,8 @@ int b200kv_pool_restore(b200kv_pool* pool, const uint32_t* prompt, uint32_t prom
         if (!same_shape(e.geometry, layer_views[l])) return B200KV_ERR_MISMATCH;
         if (n > layer_views[l].capacity) return B200KV_ERR_RANGE;
     }
-    if ((rc = copy_layers(layer_views, e.layer_bytes, n, e.payload, false, stream)) != B200KV_OK) return rc;
+    rc = snapshot_copy_layers(layer_views, layers, n, static_cast<uint8_t*>(e.payload), e.layer_bytes.data(), false, static_cast<cudaStream_t>(stream));
+    if (rc != B200KV_OK) return rc;
     ++pool->counters.hits;
     e.last_used = ++pool->clock;
     if (matched_length != nullptr) *matched_length = n;

@@ -149,18 +149,21 @@ static int launch_copy(CopyParams& p, cudaStream_t stream) {
     return B200KV_OK;
 }
 
-// The first `tokens` rows of `layers` caches (one geometry; capacities may differ) to or from compact blobs in this
-// device's memory; blob l starts at blob + offsets[l].
-int snapshot_copy_device(const b200kv_view* views, uint32_t layers, uint64_t tokens, uint8_t* blob, const uint64_t* offsets, bool to_blob,
-                         cudaStream_t stream) {
-    for (uint32_t l0 = 0; l0 < layers; l0 += kCopyLayers) {
+static bool same_shape(const b200kv_view& a, const b200kv_view& b) {
+    return a.kv_heads == b.kv_heads && a.head_dim == b.head_dim && a.qblock == b.qblock && a.quant_mode == b.quant_mode;
+}
+
+// One launch per run of up to kCopyLayers layers of one geometry (capacities may differ); everything in this device's memory.
+static int copy_layers_here(const b200kv_view* views, uint32_t layers, uint64_t tokens, uint8_t* blob, const uint64_t* layer_bytes, bool to_blob,
+                            cudaStream_t stream) {
+    for (uint32_t l0 = 0; l0 < layers;) {
         CopyParams p{};
-        p.layers = layers - l0 < static_cast<uint32_t>(kCopyLayers) ? layers - l0 : kCopyLayers;
+        while (l0 + p.layers < layers && p.layers < static_cast<uint32_t>(kCopyLayers) && same_shape(views[l0 + p.layers], views[l0])) ++p.layers;
         p.heads = views[l0].kv_heads;
         p.tokens = tokens;
         const PlaneList shape = planes_of(views[l0]);
         p.planes = shape.count;
-        // where a plane's first head starts in the blob, and the distance between its heads (one side's record)
+        // where a plane's first head starts in a snapshot, and the distance between its heads (one side's record)
         uint64_t start[4], side_start = 0;
         const uint32_t k_planes = is_k_q8(views[l0].quant_mode) ? 2u : 1u;
         for (uint32_t side = 0, i = 0; side < 2; ++side) {
@@ -181,13 +184,15 @@ int snapshot_copy_device(const b200kv_view* views, uint32_t layers, uint64_t tok
             CopyLayer& y = p.layer[l];
             y.src_rows = y.dst_rows = views[l0 + l].capacity;
             for (uint32_t i = 0; i < p.planes; ++i) {
-                uint8_t* in_blob = blob + offsets[l0 + l] + start[i];
+                uint8_t* in_blob = blob + start[i];
                 y.src[i] = to_blob ? cache.base[i] : in_blob;
                 y.dst[i] = to_blob ? in_blob : cache.base[i];
             }
+            blob += layer_bytes[l0 + l];
         }
         const int rc = launch_copy(p, stream);
         if (rc != B200KV_OK) return rc;
+        l0 += p.layers;
     }
     return B200KV_OK;
 }
@@ -209,15 +214,29 @@ static int copy_cache_to_cache(const b200kv_view& dst, const b200kv_view& src, u
     return launch_copy(p, stream);
 }
 
-// Whether `p` is ordinary memory of the current device (what the copy kernel may touch; anything else takes the copy engine).
-static bool on_this_device(const void* p) {
-    cudaPointerAttributes a{};
+// Whether the copy kernel may touch all of it: ordinary memory of the current device (anything else takes the copy engine, which
+// also reaches host memory and other devices).
+static bool all_on_this_device(const b200kv_view* views, uint32_t layers, const void* blob) {
     int device = -1;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+    if (cudaGetDevice(&device) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == device && (reinterpret_cast<uintptr_t>(p) & 1u) == 0;
+    auto here = [device](const void* p) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        return a.type == cudaMemoryTypeDevice && a.device == device;
+    };
+    if ((reinterpret_cast<uintptr_t>(blob) & 1u) != 0 || !here(blob)) return false;
+    for (uint32_t l = 0; l < layers; ++l) {
+        const PlaneList planes = planes_of(views[l]);
+        for (uint32_t i = 0; i < planes.count; ++i)
+            if (!here(planes.base[i])) return false;
+    }
+    return true;
 }
 
 // One side (K or V) between the cache and the blob; to_blob selects direction.
@@ -239,22 +258,28 @@ static int copy_side(const b200kv_view& v, const SidePlanes& side, uint64_t toke
     return B200KV_OK;
 }
 
+int snapshot_copy_layers(const b200kv_view* views, uint32_t layers, uint64_t tokens, uint8_t* blob, const uint64_t* layer_bytes, bool to_blob,
+                         cudaStream_t stream) {
+    if (tokens == 0) return B200KV_OK;
+    if (all_on_this_device(views, layers, blob)) return copy_layers_here(views, layers, tokens, blob, layer_bytes, to_blob, stream);
+    for (uint32_t l = 0; l < layers; blob += layer_bytes[l++]) {
+        const SidePlanes ks = k_side(views[l]), vs = v_side(views[l]);
+        int rc = copy_side(views[l], ks, tokens, blob, to_blob, stream);
+        if (rc != B200KV_OK) return rc;
+        rc = copy_side(views[l], vs, tokens, blob + side_record_bytes(views[l], ks.q8, tokens) * views[l].kv_heads, to_blob, stream);
+        if (rc != B200KV_OK) return rc;
+    }
+    return B200KV_OK;
+}
+
 static int snapshot_copy(const b200kv_view* view, uint64_t tokens, void* blob, bool to_blob, void* stream) {
     int rc = validate_view(view);
     if (rc != B200KV_OK) return rc;
     if (tokens > view->capacity) return B200KV_ERR_RANGE;  // the reference throws here (kv_cache.cpp:228-230)
     if (tokens == 0 || blob == nullptr) return B200KV_OK;  // the reference returns silently (kv_cache.cpp:231)
     if ((rc = ensure_device()) != B200KV_OK) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    uint8_t* bytes = static_cast<uint8_t*>(blob);
-    if (on_this_device(blob)) {
-        const uint64_t offset = 0;
-        return snapshot_copy_device(view, 1, tokens, bytes, &offset, to_blob, s);
-    }
-    const SidePlanes ks = k_side(*view), vs = v_side(*view);
-    if ((rc = copy_side(*view, ks, tokens, bytes, to_blob, s)) != B200KV_OK) return rc;
-    const size_t k_bytes = side_record_bytes(*view, ks.q8, tokens) * view->kv_heads;
-    return copy_side(*view, vs, tokens, bytes + k_bytes, to_blob, s);
+    const uint64_t bytes = 0;   // of no use with one layer
+    return snapshot_copy_layers(view, 1, tokens, static_cast<uint8_t*>(blob), &bytes, to_blob, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace b200kv

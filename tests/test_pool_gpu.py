@@ -97,3 +97,59 @@ def test_reuse_policy_around_real_caches_resident_pool_and_disk(cuda, tmp_path):
         for name in ("key_q8", "value_q8", "key_scales", "value_scales"):
             getattr(restored, name)[:, :P] = getattr(h, name)[:, :P]
         assert_planes_equal(st, restored, "restored from the session directory")
+
+
+def _captured_node_types(call):
+    """Types of the nodes that `call(stream)` captures (0 = kernel, 1 = memcpy); nothing runs."""
+    import ctypes as C
+
+    rt = C.CDLL("libcudart.so.12")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        call(torch.cuda.current_stream().cuda_stream)
+    raw, n = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t()
+    assert rt.cudaGraphGetNodes(raw, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert rt.cudaGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    kind = C.c_int()
+    return [kind.value for node in nodes if rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0]
+
+
+def test_planes_that_are_not_this_devices_memory_take_the_copy_engine(cuda):
+    """The copy kernel may only touch the current device's own memory.  Another device's planes cannot be had with one GPU, but planes in
+    pinned host memory take the same decision: in a pool capture and restore, and in a snapshot whose blob is in device memory."""
+    import ctypes as C
+
+    from miinfer_b200._lib import View, check, lib
+
+    rng = np.random.default_rng(8)
+    P = 96
+    hosts, sts = _session(rng, P)
+    tokens = (C.c_uint32 * (P + 1))(*range(P + 1))
+    pool = kv.SnapshotPool(granularity=1)
+    assert pool.capture(list(tokens)[:P], sts)
+
+    host_planes = [[torch.zeros(p.shape, dtype=p.dtype).pin_memory() for p in st.planes()] for st in sts]
+    views = (View * LAYERS)(*[st.view() for st in sts])
+    for l, (k, ks, v, vs) in enumerate((h[0], h[1], h[2], h[3]) for h in host_planes):
+        views[l].key_q8, views[l].key_scales, views[l].value_q8, views[l].value_scales = k.data_ptr(), ks.data_ptr(), v.data_ptr(), vs.data_ptr()
+    n, done = C.c_uint32(), C.c_int()
+    restore = lambda s: check(lib.b200kv_pool_restore(pool._h, tokens, P + 1, views, LAYERS, s, C.byref(n)), "restore")
+    capture = lambda s: check(lib.b200kv_pool_capture(pool._h, tokens, P, views, LAYERS, s, C.byref(done)), "capture")
+    blob = torch.zeros(int(lib.b200kv_snapshot_bytes(C.byref(views[0]), P)), dtype=torch.uint8, device="cuda")
+    save = lambda s: check(lib.b200kv_snapshot_save(C.byref(views[0]), P, blob.data_ptr(), s), "save")
+    for call, copies in ((restore, 4 * LAYERS), (capture, 4 * LAYERS), (save, 4)):
+        assert _captured_node_types(call) == [1] * copies
+    own = (View * LAYERS)(*[st.view() for st in sts])
+    assert _captured_node_types(lambda s: check(lib.b200kv_pool_restore(pool._h, tokens, P + 1, own, LAYERS, s, C.byref(n)), "restore")) == [0]
+
+    restore(None)
+    save(None)
+    torch.cuda.synchronize()
+    for st, planes in zip(sts, host_planes):
+        for a, b in zip(st.planes(), planes):
+            assert torch.equal(a[:, :P].cpu(), b[:, :P])
+    back = kv.AttentionLayerKvCacheStorage(P, kv.KvCacheQuantMode.kQ8Q8, kv_heads=H, head_dim=D, qblock=32)
+    back.upload_raw(blob, P)
+    for a, b in zip(sts[0].planes(), back.planes()):
+        assert torch.equal(a[:, :P], b[:, :P])
