@@ -144,7 +144,10 @@ B200KV_API int b200kv_device_check(int device);
  * produce -- Q, gate, the workspace, outputs, and the last `tail_positions`
  * rows of the scanned cache range -- is only touched after that kernel has
  * completed (griddepcontrol.wait).  Set tail_positions >= the number of rows
- * the preceding kernel can append (1 in a decode loop).  Device-side state
+ * the last appending launch before a decode launch can append (1 in a decode loop):
+ * launches that append let the next kernel in only when everything before them has
+ * completed, so no more than one of them is unfinished when rows are read early.
+ * Device-side state
  * (decode_state, lengths) is read early, so it must not be written by a kernel
  * that itself triggers dependents early; kernels of this library never do, and
  * an ordinary kernel between two launches acts as a full barrier.  0 turns the

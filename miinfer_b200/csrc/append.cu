@@ -44,6 +44,10 @@ struct AppendParams {
     float epsilon;
     float sectioned_step;    // powf(theta, -2/64)
     float inv_freq[128];     // NeoX: powf(theta, -2i/d), i < d/2
+    // Dependents come in behind this kernel's wait (kv_common.cuh), or at once where its CTAs take every slot of the device: no CTA of
+    // a decode kernel, several times the size of one of these, can then start before one of these has gone, and none goes
+    // before the wait.  (12 launches of 8192 tokens: 205 us so, 216 behind the wait.)
+    int fills_device;
 };
 
 constexpr int kAppendWarps = 2;
@@ -133,10 +137,8 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
     if (rope_mode == B200KV_ROPE_NEOX_FULL)
 #pragma unroll
         for (int i = 0; i < SC; ++i) freq[i] = p.inv_freq[4 * l + SC * sub + i];
-    // Let the next kernel of the stream become resident now (it orders itself against this one), then wait
-    // for everything before us: K/V inputs and the device-side position come from preceding kernels.
-    pdl_launch_dependents();
-    pdl_wait();
+    if (p.fills_device) pdl_launch_dependents();   // the next kernel may become resident; it orders itself against this one
+    pdl_wait();                // K/V inputs and the device-side position come from preceding kernels
 
     uint32_t base_position = p.base_position;
     uint32_t token_count = p.token_count;
@@ -328,6 +330,7 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
 
     Cursor cur{unit0 / (2 * passes), (unit0 / 2) % passes, unit0 & 1};
     if (unit0 < unit1 && inside(cur)) fetch(cur);
+    if (!p.fills_device) pdl_launch_dependents();
     uint32_t rotated_token = 0xffffffffu;
     for (uint32_t unit = unit0; unit < unit1; ++unit) {
         const uint64_t position = static_cast<uint64_t>(base_position) + cur.token;
@@ -401,9 +404,19 @@ extern "C" int b200kv_append(const b200kv_view* view, const void* key, const voi
     const bool vec = ((reinterpret_cast<uintptr_t>(key) | reinterpret_cast<uintptr_t>(value)) & 15u) == 0;
     const dim3 block(kAppendWarps * 32);
     cudaError_t err;
-    auto launch = [&](auto kernel) { return launch_kernel(kernel, grid, block, 0, s, true, p, vec); };
-    if (d == 128) err = f16 ? launch(append_kernel<128, true>) : launch(append_kernel<128, false>);
-    else err = f16 ? launch(append_kernel<256, true>) : launch(append_kernel<256, false>);
+    auto launch = [&](auto kernel, std::atomic<int>& slots) {   // slots: CTAs of the kernel that fit on an SM
+        int n = slots.load(std::memory_order_relaxed);
+        if (n == 0) {
+            const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kAppendWarps * 32, 0);
+            if (e != cudaSuccess) return e;
+            slots.store(n, std::memory_order_relaxed);
+        }
+        p.fills_device = grid >= static_cast<uint64_t>(sms) * n;
+        return launch_kernel(kernel, grid, block, 0, s, true, p, vec);
+    };
+    static std::atomic<int> slots[4] = {};
+    if (d == 128) err = f16 ? launch(append_kernel<128, true>, slots[0]) : launch(append_kernel<128, false>, slots[1]);
+    else err = f16 ? launch(append_kernel<256, true>, slots[2]) : launch(append_kernel<256, false>, slots[3]);
     B200KV_CUDA_TRY(err);
     return B200KV_OK;
 }

@@ -163,7 +163,7 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1024-aligned, still a shared-space pointer
 
-    pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
+    if (p.new_key == nullptr) pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;   // mma fragment coordinates
@@ -251,6 +251,7 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
         if (lane == 0)
             while (issued < kStages && issued < limit) { issue(issued, issued); ++issued; }
     }
+    if (p.new_key != nullptr) pdl_launch_dependents();   // an appending launch: see pdl_launch_dependents
 
     // ---- quantise Q to 15 bits (two int8 planes), one warp per head; heads the group does not have are zero ----
     if (warp < 4) {

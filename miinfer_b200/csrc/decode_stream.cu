@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     constexpr int SEG = D / 128;
     constexpr float kLazy = 4.0f;                     // log2 of how far the weights may outgrow the reference
     extern __shared__ __align__(128) uint8_t smem[];
-    pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
+    if (p.new_key == nullptr) pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // kv head fastest for one session, splits fastest for many (as in decode_tc5.cu)
@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     float new_x[D / 32];
     if (makes_key || makes_value) tail::load_new_row<D>(makes_key ? p.new_key : p.new_value, p.new_is_f16, kv_head, lane, new_x);
     while (next_unit < P::kUnits - 1) issue();
+    if (p.new_key != nullptr) pdl_launch_dependents();   // an appending launch: see pdl_launch_dependents
 
     // ---- Q: scaled by a power of two per head (largest element to [2^13, 2^14)), split into two fp16 terms, as A fragments ----
     for (int h = warp; h < 8; h += WARPS) {

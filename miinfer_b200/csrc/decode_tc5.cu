@@ -165,7 +165,7 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1024-aligned, still a shared-space pointer
     const uint32_t sbase = smem_u32(smem);
 
-    pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
+    if (p.new_key == nullptr) pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // single-session launches put the kv head fastest (measured 0.4 us per launch better than split fastest at 32K: the CTAs that are dispatched last, into
@@ -276,6 +276,7 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
     }
     if (warp == kProducerWarp && lane == 0)
         while (issued < kStages && issued < ntiles) { issue(issued); ++issued; }
+    if (p.new_key != nullptr) pdl_launch_dependents();   // an appending launch: see pdl_launch_dependents
 
     // ---- Q: 15 bits per head as two int8 planes.  Rows of the B operand of S^T = K . Q^T:
     //      [hi h0 .. hi h3, lo h0 .. lo h3].  The operand has 16 rows (the smallest N next to

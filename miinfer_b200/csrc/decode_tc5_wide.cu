@@ -147,7 +147,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // 1024-aligned, still a shared-space pointer
     const uint32_t sbase = smem_u32(smem);
 
-    pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
+    if (p.new_key == nullptr) pdl_launch_dependents();   // the next kernel of the stream may become resident as SMs free up; it orders itself
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t kv_head = blockIdx.x, split = blockIdx.y, session = blockIdx.z;
@@ -255,6 +255,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
             if (i >= k_early && i < kKStages) issue_k(i);
             if (i >= v_early) issue_v(i);
         }
+    if (p.new_key != nullptr) pdl_launch_dependents();   // an appending launch: see pdl_launch_dependents
 
     // ---- Q: 15 bits per head as two int8 planes (q = 128 hi + lo).  Rows of the B operand of S^T = K . Q^T: hi planes of
     //      heads 0-7 in rows 0-7, lo planes in rows 8-15 (rows of heads past G are zero); one 16 x 128-byte tile per half

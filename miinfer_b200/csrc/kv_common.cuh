@@ -57,6 +57,9 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
 // device's context): `done_mask` is the kernel's own bit set of the device ordinals already done.
 cudaError_t opt_in_dynamic_smem(const void* kernel, int bytes, std::atomic<uint64_t>& done_mask);
 
+// A decode kernel reads cache rows before its wait, all but the last `launch_overlap_tail()` of those that preceding kernels may still be
+// writing: the rows of ONE launch.  So a kernel that writes cache rows lets its dependents in only behind its own wait: whoever starts
+// early then knows that every writer but the last has finished, whatever lies in between.  The other kernels do so at once.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

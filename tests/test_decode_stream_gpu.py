@@ -165,3 +165,34 @@ def test_tensors_that_start_at_any_element(cuda, d, H, Hq, qb, mode, splits, dty
                                   part_acc=one(out), workspace=ws, num_splits=splits)
         got = (one(out) / l[:, None]).cpu().numpy()
         assert np.linalg.norm(got.astype(np.float64) - refs[0][0]) / np.linalg.norm(refs[0][0]) <= 3e-4, (qoff, ooff, "partials")
+
+
+@pytest.mark.parametrize("d,H,Hq,qb,mode", [(256, 4, 24, 256, 0), (128, 8, 32, 32, 3), (256, 4, 24, 32, 3), (128, 2, 4, 128, 1)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_steps_on_one_cache_back_to_back_with_launch_overlap(cuda, d, H, Hq, qb, mode, fused):
+    """Few CTAs per launch, so that several launches are resident at once: a step may read rows early only if they are older than the row
+    of the appending launch before it, which is the only one that may be unfinished.  Same bits as without overlap."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d + mode)
+    L0, steps = 30, 100
+    k, v = (torch.randn(L0 + steps, H * d, generator=g, device="cuda").half() for _ in range(2))
+    q = torch.randn(steps, Hq, d, generator=g, device="cuda").half()
+    results = []
+    try:
+        for overlap in (0, 1):
+            kv.set_launch_overlap(overlap)
+            st, ws, out = kv.AttentionLayerKvCacheStorage(L0 + steps, kv.KvCacheQuantMode(mode), kv_heads=H, head_dim=d, qblock=qb), kv.decode_workspace(Hq, d), torch.empty(steps, Hq, d, device="cuda")
+            kv.launch_kv_store_quant(st.view(), k[:L0], v[:L0], None, L0, 0, rope_mode=kv.RopeMode.NONE)
+            torch.cuda.synchronize()
+            for i in range(steps):
+                pos, common = L0 + i, dict(query_heads=Hq, scale=d ** -0.5, output=out[i], workspace=ws)
+                if fused:
+                    kv.launch_decode_step(st.view(), k[pos:pos + 1], v[pos:pos + 1], q[i], position=pos, rope_mode=kv.RopeMode.NONE, **common)
+                else:
+                    kv.launch_kv_store_quant(st.view(), k[pos:pos + 1], v[pos:pos + 1], None, 1, pos, rope_mode=kv.RopeMode.NONE)
+                    kv.launch_decode_attention_quant(st.view(), q[i], cache_length=pos + 1, **common)
+            torch.cuda.synchronize()
+            results.append([out, *st.planes()])
+    finally:
+        kv.set_launch_overlap(0)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
