@@ -339,7 +339,8 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
             const int stage = (ntiles - 1) % kStages;
             bool ready = !failed;
             if (lane == 0) ready = ready && mbar_wait(bar_landed, 0) && mbar_wait(bar_row, 0);
-            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0)) {
+            // every lane waits for itself (the waits are over): it reads what another warp and the copy have written
+            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0) && mbar_wait(bar_landed, 0) && mbar_wait(bar_row, 0)) {
                 const uint32_t r = (end - 1) % kTileM;
                 if (lane < 16) {
                     const int side = lane >> 3, c = lane & 7;

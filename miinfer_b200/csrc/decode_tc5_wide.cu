@@ -326,7 +326,8 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
             const int stage = (ntiles - 1) % kKStages;
             bool ready = !failed;
             if (lane == 0) ready = ready && mbar_wait(bar_k_landed, 0) && mbar_wait(bar_row, 0);
-            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0)) {
+            // every lane waits for itself (the waits are over): it reads what another warp and the copy have written
+            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0) && mbar_wait(bar_k_landed, 0) && mbar_wait(bar_row, 0)) {
                 patch_row(smem + L::kOffK + stage * L::kKTile, new_row[0].data, (end - 1) % kTileM, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read the tile through the async proxy
                 __syncwarp();
@@ -346,7 +347,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
             const int stage = (ntiles - 1) % kVStages;
             bool ready = !failed;
             if (lane == 0) ready = ready && mbar_wait(bar_v_landed, 0) && mbar_wait(bar_row, 0);
-            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0)) {
+            if (__shfl_sync(0xffffffffu, static_cast<int>(ready), 0) && mbar_wait(bar_v_landed, 0) && mbar_wait(bar_row, 0)) {
                 const uint32_t r = (end - 1) % kTileM;
                 patch_row(smem + L::kOffV + stage * L::kKTile, new_row[1].data, r, lane);
                 if (lane >= 16 && lane < 18) {

@@ -445,3 +445,41 @@ def test_decode_steps_head_dim_256_back_to_back_with_launch_overlap(cuda):
     assert torch.isfinite(results[1][0]).all()
     for a, b in zip(results[0], results[1]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("d,H,Hq,qb", [(128, 8, 32, 32), (128, 2, 4, 128), (256, 4, 24, 32), (256, 2, 16, 256)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_append_inside_the_tcgen05_kernels_at_tile_edges(cuda, d, H, Hq, qb, splits):
+    """The new row is put into its tile of 128 positions after that has landed: first, inner and last row of a tile, alone in the cache, on
+    the kernels themselves (a split count of the caller's keeps short sessions from going to the streaming kernel), under overlap."""
+    rng = np.random.default_rng(d + qb + splits)
+    cap, w = 1104, (1.0 + 0.1 * rng.standard_normal(d)).astype(np.float32)
+    rows = [ko.normal_f16(rng, (cap, H * d)).astype(np.float32) for _ in range(2)]
+    positions = (0, 1, 127, 128, 200, 255, 256, 1023, 1024)
+    host, ws = ko.HostCache(cap, H, d, qb, 3), kv.decode_workspace(Hq, d)
+    st = upload(host)
+    assert kv.decode_kernel_kind(st.view(), Hq) == (1 if d == 128 else 2)
+    kv.set_launch_overlap(1)
+    try:
+        filled_to = 0
+        for i, pos in enumerate(positions):
+            if pos > filled_to:
+                n, at = pos - filled_to, slice(filled_to, pos)
+                host.append(rows[0][at], rows[1][at], w, filled_to, rope_mode=1)
+                kv.launch_kv_store_quant(st.view(), to_dev(rows[0][at]), to_dev(rows[1][at]), to_dev(w), n, filled_to, rope_mode=kv.RopeMode.NEOX_FULL)
+                torch.cuda.synchronize()   # more rows than the overlap's guard
+            dtype = np.float16 if i % 2 else np.float32
+            kn, vn = (rng.standard_normal((1, H * d)).astype(dtype) for _ in range(2))
+            q16, out = ko.normal_f16(rng, (Hq, d)), torch.full((Hq, d), float("nan"), device="cuda")
+            host.append(kn.astype(np.float32), vn.astype(np.float32), w, pos, rope_mode=1)
+            kv.launch_decode_step(st.view(), to_dev(kn), to_dev(vn), to_dev(q16), query_heads=Hq, scale=d ** -0.5, k_norm_weight=to_dev(w),
+                                  rope_mode=kv.RopeMode.NEOX_FULL, output=out, workspace=ws, num_splits=splits,
+                                  **({"position": pos} if i % 3 else {"decode_state": kv.make_decode_state(pos)}))
+            filled_to = pos + 1
+            ref, _ = host.decode_ref(q16.astype(np.float32), d ** -0.5, pos + 1)
+            got = out.cpu().numpy()
+            assert np.linalg.norm(got.astype(np.float64) - ref) <= 2e-4 * np.linalg.norm(ref), pos   # 15-bit queries, 16-bit weights
+    finally:
+        kv.set_launch_overlap(0)
+    from gpu_util import assert_planes_equal
+    assert_planes_equal(st, host, "rows appended inside the kernels")
