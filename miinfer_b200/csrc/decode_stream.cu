@@ -113,6 +113,8 @@ __device__ __forceinline__ void split_p(const float (&p)[4], uint32_t (&a)[4]) {
         a[2 * i + 1] = pack2(p[2 * i] - h.x, p[2 * i + 1] - h.y);
     }
 }
+// The sum of a value's two terms.  Where the first is infinite or NaN it is the result: the second is 0 x infinity, or what was left of infinity.
+__device__ __forceinline__ float terms(float hi, float lo) { return fabsf(hi) < INFINITY ? hi + lo : hi; }
 __device__ __forceinline__ float exp2i(int e) { return __int_as_float((e + 127) << 23); }   // 2^e for normal results
 __device__ __forceinline__ float quad_max(float v) {
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         for (int i = 0; i < NT; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                o[i][j] = fmaf(held[local + 2 * i + j], held_by, o[i][j] + o[i][j + 2]);
+                o[i][j] = fmaf(held[local + 2 * i + j], held_by, terms(o[i][j], o[i][j + 2]));
                 o[i][j + 2] = 0.0f;
             }
     };
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         for (int i = 0; i < NT; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                held[local + 2 * i + j] = o[i][j] + o[i][j + 2];
+                held[local + 2 * i + j] = terms(o[i][j], o[i][j + 2]);
                 o[i][j] = o[i][j + 2] = 0.0f;
             }
         held_by = 1.0f;
@@ -431,7 +433,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
                     for (int i = 0; i < 4; ++i) { hi[i] += acc[i >> 1][i & 1]; lo[i] += acc[i >> 1][(i & 1) + 2]; }
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[i] = hi[i] + lo[i];
+                for (int i = 0; i < 4; ++i) s[i] = terms(hi[i], lo[i]);
                 if constexpr (KF == ROW) {
                     const uint8_t* src = scale_at + (reinterpret_cast<uintptr_t>(k_scales + static_cast<uint64_t>(pos) * 2) & 2u);
 #pragma unroll
@@ -469,7 +471,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
             const uint8_t* scale_at = smem + (unit - smem_u32(smem)) + kTile * VU::kRow;
             const uint32_t row_at = unit + lrow * VU::kRow;
             const int flip = lrow & 7;
-            auto fit_multiplier = [&](float largest) {   // `largest` |value scale| of the tile, the same in every lane
+            auto fit_multiplier = [&](float largest) {   // `largest` finite |value scale| of the tile, the same in every lane
                 if (largest > vs_cap) {
                     // room for 2^kLazy x a cap one binade above what was seen: product x multiplier <= 2^15
                     const int e = max(-100, min(100, static_cast<int>(__float_as_uint(largest) >> 23) - 127 + 2));
@@ -493,7 +495,20 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
                     for (int w = 0; w < NB / 2; ++w) big = __hmax2(big, __habs2(*reinterpret_cast<const __half2*>(&vs[i][w])));
-                fit_multiplier(quad_max(fmaxf(__low2float(big), __high2float(big))));
+                float largest = quad_max(fmaxf(__low2float(big), __high2float(big)));
+                if (__any_sync(0xffffffffu, largest == INFINITY)) {   // an infinite scale is its own block's affair
+                    float finite = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int w = 0; w < NB / 2; ++w) {
+                            const float2 sc = unpack2(vs[i][w]);
+                            if (fabsf(sc.x) < INFINITY) finite = fmaxf(finite, fabsf(sc.x));
+                            if (fabsf(sc.y) < INFINITY) finite = fmaxf(finite, fabsf(sc.y));
+                        }
+                    largest = quad_max(finite);
+                }
+                fit_multiplier(largest);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) pw[i] *= exp2i(p_exp);
 #pragma unroll
@@ -522,7 +537,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
                     for (int i = 0; i < 4; ++i) {
                         vs[i] = __half2float(*reinterpret_cast<const __half*>(src + (2 * c4 + (i & 1) + (i >> 1) * 8) * 2));
                         if (pos + 2 * c4 + (i & 1) + (i >> 1) * 8 >= end) vs[i] = 0.0f;   // a word may carry a scale past the end
-                        big = fmaxf(big, fabsf(vs[i]));
+                        if (fabsf(vs[i]) < INFINITY) big = fmaxf(big, fabsf(vs[i]));
                     }
                     fit_multiplier(quad_max(big));
 #pragma unroll
@@ -567,8 +582,8 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         __syncwarp();                             // every lane is past its last ldmatrix
 #pragma unroll
         for (int i = 0; i < NT; i += 2) {
-            const float e0 = (o[i][0] + o[i][2]) * inv, e1 = (o[i][1] + o[i][3]) * inv;
-            const float f0 = (o[i + 1][0] + o[i + 1][2]) * inv, f1 = (o[i + 1][1] + o[i + 1][3]) * inv;
+            const float e0 = terms(o[i][0], o[i][2]) * inv, e1 = terms(o[i][1], o[i][3]) * inv;
+            const float f0 = terms(o[i + 1][0], o[i + 1][2]) * inv, f1 = terms(o[i + 1][1], o[i + 1][3]) * inv;
             if constexpr (VF == F16) {            // n tile i: dims 8i + 2c, + 1
                 *reinterpret_cast<float2*>(mine + 8 * i + 2 * c4) = make_float2(e0, e1);
                 *reinterpret_cast<float2*>(mine + 8 * (i + 1) + 2 * c4) = make_float2(f0, f1);

@@ -196,3 +196,38 @@ def test_steps_on_one_cache_back_to_back_with_launch_overlap(cuda, d, H, Hq, qb,
     finally:
         kv.set_launch_overlap(0)
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("d,qb,mode", [(256, 32, 0), (128, 32, 0), (256, 32, 2), (256, 256, 2), (128, 32, 2)])
+@pytest.mark.parametrize("splits", [0, 1])
+def test_infinities_stay_where_they_are(cuda, d, qb, mode, splits):
+    """fp16 K, V in fp16 or int8: an infinite value (or value scale) makes its own dims infinite for the heads that see it and nothing else; a
+    score of minus infinity takes its position out; one of plus infinity, or a NaN key, makes the head NaN.  As plain arithmetic does."""
+    rng = np.random.default_rng(d + qb)
+    L, H, Hq = 70, 2, 8
+    k, v, q = rng.standard_normal((H, L, d)), rng.standard_normal((H, L, d)), rng.standard_normal((Hq, d))
+    k[0, 5, 3] = -np.inf                                     # kv head 0: query heads 0 and 1 ignore position 5, 2 and 3 become NaN
+    q[:2, 3], q[2:4, 3] = np.abs(q[:2, 3]), -np.abs(q[2:4, 3])
+    st = kv.AttentionLayerKvCacheStorage(L, kv.KvCacheQuantMode(mode), kv_heads=H, head_dim=d, qblock=qb if mode else d)
+    st.key_cache.copy_(torch.from_numpy(k))
+    if mode == 0:
+        st.value_cache.copy_(torch.from_numpy(v))
+        st.value_cache[0, 40, 7], st.value_cache[1, 66, d - 1] = float("inf"), -float("inf")
+        vd = st.value_cache.double()
+    else:
+        st.value_cache_q8.copy_(torch.from_numpy(np.clip(np.rint(v * 40), -127, 127)))
+        st.value_cache_q8[st.value_cache_q8 == 0] = 1
+        st.value_scales.fill_(1 / 40)
+        st.value_scales[0, 40, 0], st.value_scales[1, 66, -1] = float("inf"), float("inf")
+        vd = (st.value_cache_q8.double().view(H, L, d // st.qblock, -1) * st.value_scales.double().unsqueeze(-1)).view(H, L, d)
+    q16 = torch.from_numpy(q).half().cuda()
+    out = torch.empty(Hq, d, device="cuda")
+    kv.launch_decode_attention_quant(st.view(), q16, query_heads=Hq, scale=d ** -0.5, cache_length=L, output=out,
+                                     workspace=kv.decode_workspace(Hq, d), num_splits=splits | kv.FORCE_GENERIC)
+    kd = st.key_cache.double()
+    ref = torch.cat([((q16.double().view(H, Hq // H, d)[h, :, None, :] * kd[h]).sum(-1) * d ** -0.5).softmax(-1)[..., None].mul(vd[h]).sum(1) for h in range(H)])
+    got = out.double()
+    assert torch.equal(got.isnan(), ref.isnan()) and bool(ref.isnan().any())
+    assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got[got.isinf()], ref[ref.isinf()]) and bool(ref.isinf().any())
+    ok = ref.isfinite()
+    assert bool((got[ok] - ref[ok]).norm() <= REL * ref[ok].norm())   # none are finite where every dim shares one infinite scale
