@@ -148,7 +148,8 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         const uint64_t rows = static_cast<uint64_t>(max_length) * geometry.kv_heads;
         if (rows <= (use_fast ? kStreamRows128 : kStreamRows256)) use_fast = use_wide = false;
     }
-    if (num_splits == 0) {
+    const bool chosen = num_splits == 0;
+    if (chosen) {
         uint32_t fast = use_fast ? pick_splits_q8(geometry, p.query_heads, p.sessions, max_length) : 0;
         if (fast == 0) use_fast = false;
         num_splits = use_fast ? fast
@@ -156,12 +157,16 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
                               : pick_splits_stream(geometry.kv_heads, p.query_heads, geometry.head_dim, p.sessions, max_length);
     }
     if (num_splits > cap) num_splits = cap;
-    const size_t slots = static_cast<size_t>(p.sessions) * num_splits * p.query_heads;
-    const size_t plain_bytes = slots * partial_floats(geometry.head_dim) * sizeof(float);
     if (workspace == nullptr) return B200KV_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return B200KV_ERR_INVALID;
     const size_t plain_offset = workspace_plain_offset(workspace_bytes);
-    if (workspace_bytes - plain_offset < plain_bytes) return B200KV_ERR_WORKSPACE;
+    // plain partials: (m, l) and the accumulators of every slot; a launch that chooses its splits itself takes no more than there is room for
+    auto plain_floats = [&](uint32_t splits) { return static_cast<size_t>(p.sessions) * splits * p.query_heads * (geometry.head_dim + 2u); };
+    if (chosen && !use_fast && !use_wide)
+        while (num_splits > 1 && workspace_bytes - plain_offset < plain_floats(num_splits) * sizeof(float)) --num_splits;
+    if (workspace_bytes - plain_offset < plain_floats(num_splits) * sizeof(float)) return B200KV_ERR_WORKSPACE;
+    const size_t slots = static_cast<size_t>(p.sessions) * num_splits * p.query_heads;
+    const bool tagged_fit = plain_offset >= slots * partial_floats(geometry.head_dim) * sizeof(uint64_t);
     p.num_splits = num_splits;
     p.fuse = merge;
     p.ws_m = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + plain_offset);
@@ -170,7 +175,7 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     p.status = current_status_word();
     p.timeline = current_timeline_buffer(num_splits * geometry.kv_heads);
     if (use_fast) {
-        if (plain_offset < 2 * plain_bytes) return B200KV_ERR_WORKSPACE;
+        if (!tagged_fit) return B200KV_ERR_WORKSPACE;
         // The in-launch merge; a lone split that has to produce Q8_1 blocks goes through the merge kernel instead
         // (a block of 32 outputs is quantised by 16 cooperating threads, which the single-split shortcut has not).
         const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1);
@@ -183,7 +188,7 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         if (rc != B200KV_ERR_UNSUPPORTED) return rc;
         p.ws_tagged = nullptr;
     }
-    const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && plain_offset >= 2 * plain_bytes &&
+    const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && tagged_fit &&
                             stream_merge_fits(geometry.kv_heads, num_splits, many);
     if (merge.xchg.world > 1 && !fuse_merge) return B200KV_ERR_UNSUPPORTED;   // the exchange is part of the in-launch merge
     p.ws_tagged = fuse_merge ? static_cast<uint64_t*>(workspace) : nullptr;

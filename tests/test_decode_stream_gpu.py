@@ -231,3 +231,25 @@ def test_infinities_stay_where_they_are(cuda, d, qb, mode, splits):
     assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got[got.isinf()], ref[ref.isinf()]) and bool(ref.isinf().any())
     ok = ref.isfinite()
     assert bool((got[ok] - ref[ok]).norm() <= REL * ref[ok].norm())   # none are finite where every dim shares one infinite scale
+
+
+@pytest.mark.parametrize("d,H,Hq,qb,mode", [(256, 4, 24, 256, 0), (256, 4, 24, 32, 3), (128, 8, 32, 128, 0)])
+def test_workspaces_that_hold_the_plain_partials_are_enough(cuda, d, H, Hq, qb, mode):
+    """head_dim + 2 floats per split and head in the last third; the in-launch merge needs a little more in front of it at head_dim 256, and a
+    launch that is short of it runs its merge behind.  A launch that chooses its splits fits them to what is there."""
+    rng = np.random.default_rng(d + mode)
+    host = _filled(rng, 1500, H, d, qb, mode, 1501)          # odd: no kernel with a workspace rule of its own
+    st, q = upload(host), ko.normal_f16(rng, (Hq, d))
+    ref, _ = host.decode_ref(q.astype(np.float32), d ** -0.5, 1500)
+    room = lambda n: n - n // 3 * 2 // 256 * 256
+    for splits, fits in ((5, 5), (0, 1), (0, 3)):
+        need = fits * Hq * (d + 2) * 4
+        size = next(n for n in range(need, 4 * need) if room(n) >= need)
+        out = torch.empty(Hq, d, device="cuda")
+        go = lambda ws: kv.launch_decode_attention_quant(st.view(), to_dev(q), query_heads=Hq, scale=d ** -0.5, cache_length=1500, output=out,
+                                                         workspace=ws, num_splits=splits)
+        go(torch.zeros(size, dtype=torch.uint8, device="cuda"))
+        _close(out.cpu().numpy(), ref, (splits, fits))
+        short = next(n for n in range(size, 0, -1) if room(n) < Hq * (d + 2) * 4 * max(splits, 1))
+        with pytest.raises(kv.B200KvError):
+            go(torch.zeros(short, dtype=torch.uint8, device="cuda"))
