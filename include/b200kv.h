@@ -38,9 +38,18 @@ extern "C" {
 #define B200KV_API
 #endif
 
-/* OR into `num_splits` to run the generic stage-1 kernel even where a
+/* OR into `num_splits` to run the streaming kernel for all modes even where a
  * specialised one exists (testing and A/B measurement). */
 #define B200KV_SPLITS_FORCE_GENERIC 0x80000000u
+/* OR into `num_splits` (up to 65535) to have the splits merged by a kernel of its own behind the launch, with no CTA that
+ * waits for another.  Without it a launch merges inside: some of its CTAs poll for the partials of all the others, so
+ * all of them have to get onto the device.  One launch always does, and so do launches of equal priority on any
+ * streams, whose CTAs are dispatched one launch after the other.  Ask for the separate merge where decode launches of
+ * SEVERAL stream priorities, or of contexts that share the SMs otherwise (MPS, green contexts), may be on the device
+ * at the same time: there each can hold SMs the other's missing splits need, and ends in NaN and
+ * B200KV_STATUS_SPLIT_TIMEOUT after its bounded wait.  Not for b200kv_decode_attn_sharded, whose exchange is part of
+ * the merge inside (B200KV_ERR_INVALID). */
+#define B200KV_SPLITS_SEPARATE_MERGE 0x40000000u
 
 typedef enum b200kv_status {
     B200KV_OK = 0,

@@ -130,6 +130,8 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     *merged = false;
     const bool force_stream = (num_splits_arg & B200KV_SPLITS_FORCE_GENERIC) != 0;
     uint32_t num_splits = num_splits_arg & ~B200KV_SPLITS_FORCE_GENERIC;
+    const bool separate_merge = (num_splits & 0x7fff0000u) == B200KV_SPLITS_SEPARATE_MERGE;   // a larger number is only that
+    if (separate_merge) num_splits &= 0xffffu;
     const uint32_t cap = max_splits_per_session(p.sessions);
     const bool many = p.sessions > 1 || p.lengths != nullptr;
     // Q, gate and outputs may start at any element.  The kernels below fetch Q in 16-byte pieces, decode_stream.cu takes it as it lies.
@@ -137,16 +139,18 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     p.q_pairs = aligned(p.q, p.q_is_f16 ? 4 : 8);
     const bool q_vectors = aligned(p.q, 16);
     // the in-launch merge takes gate and outputs two floats at a time; the merge kernel behind the launch one by one
-    const bool pairs = aligned(merge.gate, 8) && aligned(merge.output, 8) && aligned(merge.gated_output, 8) && aligned(merge.out_acc, 8);
-    if (merge.xchg.world > 1 && !pairs) return B200KV_ERR_INVALID;   // the exchange is part of the in-launch merge
-    bool use_fast = !force_stream && q_vectors && (pairs || !many) && q8_fast_path_ok(geometry, p.query_heads);
+    const bool merge_inside = !separate_merge && aligned(merge.gate, 8) && aligned(merge.output, 8) && aligned(merge.gated_output, 8) && aligned(merge.out_acc, 8);
+    if (merge.xchg.world > 1 && !merge_inside) return B200KV_ERR_INVALID;   // the exchange is part of the in-launch merge
+    bool use_fast = !force_stream && q_vectors && (merge_inside || !many) && q8_fast_path_ok(geometry, p.query_heads);
     // head_dim 256: the tcgen05 kernel for single-session launches
     bool use_wide = !force_stream && !use_fast && !many && q_vectors && streaming_kernel_choice() != 1 && decode_tc5_wide_ok(geometry, p.query_heads);
     // Single sessions that are short for the device: the mma.sync kernel starts, splits and merges faster than the tcgen05
     // kernels' pipelines fill, until its instruction issue shows.
     if (num_splits == 0 && !many && streaming_kernel_choice() != 1) {
         const uint64_t rows = static_cast<uint64_t>(max_length) * geometry.kv_heads;
-        if (rows <= (use_fast ? kStreamRows128 : kStreamRows256)) use_fast = use_wide = false;
+        // (a sharded launch has its exchange inside the merge: only where that fits)
+        if (rows <= (use_fast ? kStreamRows128 : kStreamRows256) && (merge.xchg.world <= 1 || stream_merge_fits(geometry.kv_heads, 1, false, device_sms())))
+            use_fast = use_wide = false;
     }
     const bool chosen = num_splits == 0;
     if (chosen) {
@@ -178,7 +182,7 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         if (!tagged_fit) return B200KV_ERR_WORKSPACE;
         // The in-launch merge; a lone split that has to produce Q8_1 blocks goes through the merge kernel instead
         // (a block of 32 outputs is quantised by 16 cooperating threads, which the single-split shortcut has not).
-        const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1);
+        const bool fuse_merge = merge_inside && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1);
         p.ws_tagged = fuse_merge ? static_cast<uint64_t*>(workspace) : nullptr;
         p.tag = next_launch_tag();
         int rc = B200KV_ERR_UNSUPPORTED;
@@ -188,8 +192,8 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
         if (rc != B200KV_ERR_UNSUPPORTED) return rc;
         p.ws_tagged = nullptr;
     }
-    const bool fuse_merge = pairs && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && tagged_fit &&
-                            stream_merge_fits(geometry.kv_heads, num_splits, many);
+    const bool fuse_merge = merge_inside && !(num_splits == 1 && merge.gated_output_q8 != nullptr && merge.xchg.world <= 1) && tagged_fit &&
+                            stream_merge_fits(geometry.kv_heads, num_splits, many, device_sms());
     if (merge.xchg.world > 1 && !fuse_merge) return B200KV_ERR_UNSUPPORTED;   // the exchange is part of the in-launch merge
     p.ws_tagged = fuse_merge ? static_cast<uint64_t*>(workspace) : nullptr;
     p.tag = next_launch_tag();

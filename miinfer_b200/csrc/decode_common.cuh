@@ -162,7 +162,7 @@ int run_decode(DecodeParams& p, const b200kv_view& geometry, uint32_t max_length
 
 // Every cache mode and shape (decode_stream.cu).
 uint32_t pick_splits_stream(uint32_t kv_heads, uint32_t query_heads, uint32_t head_dim, uint32_t sessions, uint32_t max_length);
-bool stream_merge_fits(uint32_t kv_heads, uint32_t num_splits, bool many);
+bool stream_merge_fits(uint32_t kv_heads, uint32_t num_splits, bool many, uint32_t sms);
 int launch_decode_stream(const DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream);
 // int8 K and V at head_dim 128 (decode_q8.cu).  Returns B200KV_ERR_UNSUPPORTED when
 // the geometry is not one it takes, so the caller can use the kernel above.

@@ -676,8 +676,8 @@ uint32_t pick_splits_stream(uint32_t kv_heads, uint32_t query_heads, uint32_t he
 
 // Whether the merge may run inside the launch: the CTAs of a session wait for one another, so all of a session's CTAs have to
 // fit on the device together (CTAs are dispatched in block order, a session's side by side).
-bool stream_merge_fits(uint32_t kv_heads, uint32_t num_splits, bool many) {
-    return static_cast<uint64_t>(kv_heads) * num_splits <= (many ? 296u : 148u);
+bool stream_merge_fits(uint32_t kv_heads, uint32_t num_splits, bool many, uint32_t sms) {
+    return static_cast<uint64_t>(kv_heads) * num_splits <= (many ? 2u : 1u) * sms;
 }
 
 int launch_decode_stream(const DecodeParams& p_in, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream) {

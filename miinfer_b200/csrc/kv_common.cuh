@@ -16,6 +16,7 @@ namespace b200kv {
 
 void set_last_cuda_error(cudaError_t err, const char* where);
 int ensure_device();  // B200KV_OK if the current device is sm_100; cached per device
+uint32_t device_sms();   // SMs of the current device (of the slice it is); behind ensure_device, cached per thread
 
 #define B200KV_CUDA_TRY(expr)                                        \
     do {                                                             \

@@ -116,6 +116,9 @@ void set_last_cuda_error(cudaError_t err, const char* where) {
     (void)cudaGetLastError();  // clear the sticky-less error so later calls report their own
 }
 
+static thread_local uint32_t g_device_sms = 0;
+uint32_t device_sms() { return g_device_sms; }
+
 int ensure_device() {
     static thread_local int checked_device = -1;
     int device = -1;
@@ -124,9 +127,12 @@ int ensure_device() {
         return B200KV_ERR_DEVICE;
     }
     if (device == checked_device) return B200KV_OK;
-    int rc = b200kv_device_check(device);
-    if (rc == B200KV_OK) checked_device = device;
-    return rc;
+    int rc = b200kv_device_check(device), sms = 0;
+    if (rc != B200KV_OK) return rc;
+    B200KV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    g_device_sms = static_cast<uint32_t>(sms);
+    checked_device = device;
+    return B200KV_OK;
 }
 
 int validate_view(const b200kv_view* v) {

@@ -23,10 +23,11 @@ __all__ = [
     "launch_decode_partials", "launch_merge_partials", "launch_merge_partials_packed", "packed_partial", "partial_views", "launch_suffix_attention_quant", "prepare_suffix_attention", "plan_batched_decode",
     "Exchange", "launch_decode_attention_sharded", "decode_workspace", "prefill_workspace", "view_table", "make_decode_state", "make_prefill_state",
     "SnapshotPool", "ReusableContext", "DistMerge", "launch_q_split_norm_rope", "launch_decode_state_advance", "q8_1_blocks", "exchange_words", "set_status_word", "workspace_reset", "set_decode_kernel",
-    "token_sequence_hash", "save_session", "load_session", "find_matching_session", "decode_kernel_kind", "set_launch_overlap", "B200KvError", "FORCE_GENERIC",
+    "token_sequence_hash", "save_session", "load_session", "find_matching_session", "decode_kernel_kind", "set_launch_overlap", "B200KvError", "FORCE_GENERIC", "SEPARATE_MERGE",
 ]
 
 FORCE_GENERIC = 0x80000000
+SEPARATE_MERGE = 0x40000000      # for launches beside others of another stream priority: see B200KV_SPLITS_SEPARATE_MERGE
 
 
 class KvCacheQuantMode(enum.IntEnum):

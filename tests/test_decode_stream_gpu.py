@@ -253,3 +253,29 @@ def test_workspaces_that_hold_the_plain_partials_are_enough(cuda, d, H, Hq, qb, 
         short = next(n for n in range(size, 0, -1) if room(n) < Hq * (d + 2) * 4 * max(splits, 1))
         with pytest.raises(kv.B200KvError):
             go(torch.zeros(short, dtype=torch.uint8, device="cuda"))
+
+
+@pytest.mark.parametrize("d,H,Hq,qb,mode", [(256, 4, 24, 32, 3), (128, 8, 32, 32, 3), (128, 2, 8, 128, 0)])
+def test_the_separate_merge_can_be_asked_for(cuda, d, H, Hq, qb, mode):
+    """Stage 1 and the merge kernel: two launches, and no word of the workspace's tagged part is touched (it may even hold garbage)."""
+    rng = np.random.default_rng(d)
+    L, lengths = 1500, [1500, 40]
+    host = _filled(rng, L, H, d, qb, mode, 1504)
+    st, ws = upload(host), kv.decode_workspace(Hq, d, 2)
+    tagged = ws[:ws.numel() // 3 * 2 // 256 * 256]
+    tagged.fill_(171)
+    q, out = ko.normal_f16(rng, (2, Hq, d)), torch.empty(2, Hq, d, device="cuda")
+    table, lens = kv.view_table(2), torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    for splits in (0, 3, 65535):
+        for i, n in enumerate(lengths):
+            kv.launch_decode_attention_quant(st.view(), to_dev(q[i]), query_heads=Hq, scale=d ** -0.5, cache_length=n, output=out[i], workspace=ws,
+                                             num_splits=splits | kv.SEPARATE_MERGE)
+        one = out.clone()
+        kv.launch_decode_attention_batched([st.view(), st.view()], table, lens, L, to_dev(q), query_heads=Hq, scale=d ** -0.5, output=out, workspace=ws,
+                                           num_splits=splits | kv.SEPARATE_MERGE)
+        for got in (one, out):
+            for i, n in enumerate(lengths):
+                ref, _ = host.decode_ref(q[i].astype(np.float32), d ** -0.5, n)
+                err = np.linalg.norm(got[i].cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref)
+                assert err <= 2e-4, (splits, n, err)
+    assert bool((tagged == 171).all())
