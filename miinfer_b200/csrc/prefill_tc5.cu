@@ -858,12 +858,11 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
 //   20 tokens over 16000 (4 units):   5 splits 77 us, 8: 66, 16: 58     37 over 3001 (8):  5: 38, 8: 35, 12: 34, 16: 34
 //   128 over 8192 (24):   5: 54, 6: 52, 8 (a second wave): 69           300 over 8192 (60): 1: 124, 2: 92, 4: 102
 //   512 over 8192 (96):   1: 127, 2: 158, 3 (what filling the last wave best asks for): 138
-static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t head_dim) {
+static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t most, uint32_t head_dim) {
     const double tile_us = head_dim == 256 ? 0.73 : 0.52, wave_us = 8.0, merge_us = 3.0, partial_us = head_dim == 256 ? 0.11 : 0.055;
     uint32_t best = 1;
     double best_us = 0.0;
-    for (uint32_t s = 1; s <= kMaxKvSplits; ++s) {
-        if (s > 1 && tiles < 3 * s) break;   // every split walks a few tiles
+    for (uint32_t s = 1; s <= kMaxKvSplits && s <= (most > 1 ? most : 1); ++s) {
         const uint64_t ctas = static_cast<uint64_t>(units) * s, waves = (ctas + 147) / 148;
         const double us = static_cast<double>(waves) * (tiles * tile_us / s + wave_us) + (s > 1 ? merge_us + partial_us * static_cast<double>(ctas) : 0.0);
         if (s == 1 || us < best_us) { best = s; best_us = us; }
@@ -912,9 +911,11 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     {
         const uint32_t G = query_heads / view.kv_heads;
         const uint32_t row_tiles = (token_count * G + tiles_per_cta * kBM - 1) / (tiles_per_cta * kBM);
-        // a device-side state leaves the range unknown here (no split); so does a range that is mostly the chunk's own triangle
-        const bool prefix = prefill_state == nullptr && base_position >= token_count;
-        uint32_t want = prefix ? pick_kv_splits(row_tiles * view.kv_heads, static_cast<uint32_t>((rows + kBN - 1) / kBN), view.head_dim) : 1;
+        // A device-side state leaves the range unknown here (no split).  Every split walks a few tiles: three of the longest range, or,
+        // where the chunk's own triangle is longer than its prefix, eight of the prefix, which is all that its first rows see.
+        const uint32_t tiles = static_cast<uint32_t>((rows + kBN - 1) / kBN), prefix_tiles = (base_position + kBN - 1) / kBN;
+        const uint32_t most = prefill_state != nullptr ? 1 : base_position >= token_count ? tiles / 3 : prefix_tiles / 8;
+        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, most, view.head_dim);
         const size_t scratch = prefill_tc5_workspace_bytes(static_cast<uint32_t>(rows), view.kv_heads, view.head_dim);
         while (want > 1 && workspace_bytes < scratch + 1024 + prefill_tc5_split_bytes(token_count, query_heads, view.kv_heads, view.head_dim, want)) --want;
         if (want > 1) {

@@ -68,3 +68,19 @@ def assert_attention_close(got: np.ndarray, ref: np.ndarray, what: str, tol_abs:
     assert max_abs <= tol_abs, f"{what}: max-abs error {max_abs:.3e} > {tol_abs}"
     assert rel_l2 <= tol_rel, f"{what}: relative L2 error {rel_l2:.3e} > {tol_rel}"
     return max_abs, rel_l2
+
+
+def captured_node_types(call):
+    """Types of the nodes that `call(stream)` captures (0 = kernel, 1 = memcpy); nothing runs."""
+    import ctypes as C
+
+    rt = C.CDLL("libcudart.so.12")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        call(torch.cuda.current_stream().cuda_stream)
+    raw, n = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t()
+    assert rt.cudaGraphGetNodes(raw, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert rt.cudaGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    kind = C.c_int()
+    return [kind.value for node in nodes if rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0]

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import kvoracle as ko
-from gpu_util import assert_planes_equal, to_dev, upload
+from gpu_util import assert_planes_equal, captured_node_types, to_dev, upload
 from miinfer_b200 import kv
 
 pytestmark = pytest.mark.gpu
@@ -99,22 +99,6 @@ def test_reuse_policy_around_real_caches_resident_pool_and_disk(cuda, tmp_path):
         assert_planes_equal(st, restored, "restored from the session directory")
 
 
-def _captured_node_types(call):
-    """Types of the nodes that `call(stream)` captures (0 = kernel, 1 = memcpy); nothing runs."""
-    import ctypes as C
-
-    rt = C.CDLL("libcudart.so.12")
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
-        call(torch.cuda.current_stream().cuda_stream)
-    raw, n = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t()
-    assert rt.cudaGraphGetNodes(raw, None, C.byref(n)) == 0
-    nodes = (C.c_void_p * n.value)()
-    assert rt.cudaGraphGetNodes(raw, nodes, C.byref(n)) == 0
-    kind = C.c_int()
-    return [kind.value for node in nodes if rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0]
-
-
 def test_planes_that_are_not_this_devices_memory_take_the_copy_engine(cuda):
     """The copy kernel may only touch the current device's own memory.  Another device's planes cannot be had with one GPU, but planes in
     pinned host memory take the same decision: in a pool capture and restore, and in a snapshot whose blob is in device memory."""
@@ -139,9 +123,9 @@ def test_planes_that_are_not_this_devices_memory_take_the_copy_engine(cuda):
     blob = torch.zeros(int(lib.b200kv_snapshot_bytes(C.byref(views[0]), P)), dtype=torch.uint8, device="cuda")
     save = lambda s: check(lib.b200kv_snapshot_save(C.byref(views[0]), P, blob.data_ptr(), s), "save")
     for call, copies in ((restore, 4 * LAYERS), (capture, 4 * LAYERS), (save, 4)):
-        assert _captured_node_types(call) == [1] * copies
+        assert captured_node_types(call) == [1] * copies
     own = (View * LAYERS)(*[st.view() for st in sts])
-    assert _captured_node_types(lambda s: check(lib.b200kv_pool_restore(pool._h, tokens, P + 1, own, LAYERS, s, C.byref(n)), "restore")) == [0]
+    assert captured_node_types(lambda s: check(lib.b200kv_pool_restore(pool._h, tokens, P + 1, own, LAYERS, s, C.byref(n)), "restore")) == [0]
 
     restore(None)
     save(None)

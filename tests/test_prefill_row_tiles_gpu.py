@@ -3,6 +3,7 @@ edges of the row tiles, against the same attention in float64 over the dequantis
 import pytest
 import torch
 
+from gpu_util import captured_node_types
 from miinfer_b200 import kv
 
 pytestmark = pytest.mark.gpu
@@ -43,3 +44,21 @@ def test_row_tiles(cuda, H, G, P, T, act):
     # of the result's norm; 1e-3 is the gate the other tests of this kernel use
     assert torch.isfinite(out).all() and (guard[T * Hq * d:] == 7.0).all()
     assert ((out.double() - ref).norm() / ref.norm()).item() <= 1e-3
+
+
+# whether the KV range is split (a merge kernel follows) goes by the prefix, with no step where the chunk grows longer than it
+@pytest.mark.parametrize("P,T,kernels", [(0, 2048, 2), (100, 2048, 2), (2047, 2048, 3), (2048, 2048, 3), (2049, 2048, 3), (1100, 1300, 3)])
+def test_kv_split_of_a_chunk_about_as_long_as_its_prefix(cuda, P, T, kernels):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(P)
+    d, H, Hq = 128, 1, 4
+    st = kv.AttentionLayerKvCacheStorage(P + T, kv.KvCacheQuantMode.kQ8Q8, kv_heads=H, head_dim=d, qblock=32)
+    k, v = (torch.randn(P + T, H * d, generator=g, device="cuda").half() for _ in range(2))
+    kv.launch_kv_store_quant(st.view(), k, v, None, P + T, 0, rope_mode=kv.RopeMode.NONE)
+    q, out = torch.randn(T, Hq, d, generator=g, device="cuda").half(), torch.empty(T, Hq, d, device="cuda")
+    ws = kv.prefill_workspace(P + T, H, d, token_count=T, query_heads=Hq)
+    go = lambda _: kv.launch_suffix_attention_quant(st.view(), q, None, out, ws, T, P, query_heads=Hq, scale=d ** -0.5)
+    go(None)
+    ref = expected(st, q, None, P, T, Hq, d ** -0.5)
+    assert ((out.double() - ref).norm() / ref.norm()).item() <= 1e-3   # fp16 operands, as above
+    assert captured_node_types(go) == [0] * kernels
