@@ -150,7 +150,7 @@ def load_native():
     spec = importlib.util.spec_from_file_location("_native", path)
     module = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(module)
-    module.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES})
+    module.bind({"View": View, **{name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES}})
     return module
 
 

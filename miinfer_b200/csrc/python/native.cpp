@@ -30,6 +30,7 @@ struct Api {
     decltype(&b200kv_pool_capture) pool_capture;
     decltype(&b200kv_pool_restore) pool_restore;
 } g_api;
+PyObject* g_view_type;   // the ctypes structure of a cache view
 
 // One call's arguments, read left to right; the first failure sticks and leaves a Python exception set.
 class Args {
@@ -83,8 +84,27 @@ public:
         if (v == -1.0 && PyErr_Occurred()) ok_ = false;
         return static_cast<float>(v);
     }
-    // A ctypes structure (or array of them), or None: its memory, through the buffer protocol.
-    const b200kv_view* view(uint32_t count = 1, bool optional = false) {
+    int rope() {   // an enum member, or anything else that int() takes
+        if (!ok_) return 0;
+        PyObject* v = PyNumber_Long(args_[i_++]);
+        if (v == nullptr) { ok_ = false; return 0; }
+        const uint32_t r = checked(static_cast<uint32_t>(PyLong_AsUnsignedLongMask(v)));
+        Py_DECREF(v);
+        return static_cast<int>(r);
+    }
+    // A cache view (the ctypes structure and nothing else): its memory, through the buffer protocol.
+    const b200kv_view* view() {
+        if (!ok_) return nullptr;
+        const int is_view = PyObject_IsInstance(args_[i_], g_view_type);
+        if (is_view <= 0) {
+            if (is_view == 0) PyErr_Format(PyExc_TypeError, "expected a cache view, got %s", Py_TYPE(args_[i_])->tp_name);
+            ok_ = false;
+            return nullptr;
+        }
+        return views(1, false);
+    }
+    // An array of them (the caller has built it), or None.
+    const b200kv_view* views(uint32_t count, bool optional) {
         if (!ok_) return nullptr;
         PyObject* o = args_[i_++];
         if (optional && o == Py_None) return nullptr;
@@ -152,7 +172,7 @@ PyObject* py_append(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const void* value = a.tensor(nullptr, &vd);
     if (a.ok() && kd != vd) a.fail(PyExc_ValueError, "key and value must share a dtype");
     const float* w = a.tensor_as<const float>();
-    const int rope = static_cast<int>(a.u32());
+    const int rope = a.rope();
     const float theta = a.f32(), eps = a.f32();
     const uint32_t count = a.u32(), base = a.u32();
     const auto* ps = a.tensor_as<const b200kv_prefill_state>();
@@ -169,7 +189,7 @@ PyObject* py_q_split_norm_rope(PyObject*, PyObject* const* args, Py_ssize_t n) {
     void* query = a.tensor(nullptr, &od);
     float* gate = a.tensor_as<float>();
     const uint32_t count = a.u32(), base = a.u32(), heads = a.u32(), dim = a.u32();
-    const int rope = static_cast<int>(a.u32());
+    const int rope = a.rope();
     const float theta = a.f32(), eps = a.f32();
     const auto* ps = a.tensor_as<const b200kv_prefill_state>();
     const auto* ds = a.tensor_as<const b200kv_decode_state>();
@@ -208,7 +228,7 @@ PyObject* py_decode_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const void* value = a.tensor(nullptr, &vd);
     if (a.ok() && kd != vd) a.fail(PyExc_ValueError, "key and value must share a dtype");
     const float* w = a.tensor_as<const float>();
-    const int rope = static_cast<int>(a.u32());
+    const int rope = a.rope();
     const float theta = a.f32(), eps = a.f32();
     const void* q = a.tensor(nullptr, &qd);
     const float* gate = a.tensor_as<const float>();
@@ -246,7 +266,7 @@ PyObject* py_decode_attn_batched(PyObject*, PyObject* const* args, Py_ssize_t n)
     const uint32_t splits = a.u32();
     void* s = a.stream();
     Args v(&views_arg, 1, 1);
-    const b200kv_view* views = a.ok() ? v.view(static_cast<uint32_t>(sessions), true) : nullptr;
+    const b200kv_view* views = a.ok() ? v.views(static_cast<uint32_t>(sessions), true) : nullptr;
     if (a.ok() && !v.ok()) return nullptr;
     return call(a, [&] {
         return g_api.decode_attn_batched(views, table, lengths, static_cast<uint32_t>(sessions), max_length, q, qd, gate, out, gated, heads, scale,
@@ -275,8 +295,11 @@ PyObject* py_suffix_attn(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // ---- the snapshot pool: token ids and storage objects in, one library call ------------------------------------
 
+// Anything with a length that can be iterated over, as a list or tuple.
+PyObject* items_of(PyObject* o, const char* text) { return PyObject_Size(o) < 0 ? nullptr : PySequence_Fast(o, text); }
+
 bool read_tokens(PyObject* seq, std::vector<uint32_t>& out) {
-    PyObject* fast = PySequence_Fast(seq, "a sequence of token ids is required");
+    PyObject* fast = items_of(seq, "a sequence of token ids is required");
     if (fast == nullptr) return false;
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
     PyObject** items = PySequence_Fast_ITEMS(fast);
@@ -295,7 +318,7 @@ bool read_tokens(PyObject* seq, std::vector<uint32_t>& out) {
     return true;
 }
 
-enum Name { KEY, VALUE, KEY_Q8, KEY_SCALES, VALUE_Q8, VALUE_SCALES, CAPACITY, KV_HEADS, HEAD_DIM, QBLOCK, QUANT_MODE, NAMES };
+enum Name { KEY, VALUE, KEY_Q8, KEY_SCALES, VALUE_Q8, VALUE_SCALES, CAPACITY, KV_HEADS, HEAD_DIM, QBLOCK, QUANT_MODE, VIEW, NAMES };
 PyObject* g_names[NAMES];
 
 bool plane(PyObject* o, Name name, void** out) {
@@ -321,30 +344,46 @@ bool number(PyObject* o, Name name, uint64_t* out) {
     return !(*out == ~0ull && PyErr_Occurred());
 }
 
-// The views of a sequence of AttentionLayerKvCacheStorage objects, from their attributes as they are now.
+PyObject* g_storage_view;   // AttentionLayerKvCacheStorage.view
+
+// The views of a sequence of cache storages: what their view() returns.  Where that is AttentionLayerKvCacheStorage's own, its
+// result is read from the attributes it would take it from (a view() in Python costs 3 us a layer).
+bool read_view(PyObject* o, b200kv_view& v) {
+    PyObject* method = PyObject_GetAttr(o, g_names[VIEW]);
+    if (method == nullptr) return false;
+    const bool own = PyMethod_Check(method) && PyMethod_GET_FUNCTION(method) == g_storage_view && PyMethod_GET_SELF(method) == o;
+    PyObject* result = own ? nullptr : PyObject_CallNoArgs(method);
+    Py_DECREF(method);
+    if (!own) {
+        if (result == nullptr) return false;
+        Args a(&result, 1, 1);
+        const b200kv_view* view = a.view();
+        if (view != nullptr) v = *view;
+        Py_DECREF(result);
+        return a.ok();
+    }
+    void *kq, *vq;
+    uint64_t cap, heads, dim, qb, mode;
+    if (!(plane(o, KEY, &v.key_f16) && plane(o, VALUE, &v.value_f16) && plane(o, KEY_Q8, &kq) && plane(o, KEY_SCALES, &v.key_scales) &&
+          plane(o, VALUE_Q8, &vq) && plane(o, VALUE_SCALES, &v.value_scales) && number(o, CAPACITY, &cap) && number(o, KV_HEADS, &heads) &&
+          number(o, HEAD_DIM, &dim) && number(o, QBLOCK, &qb) && number(o, QUANT_MODE, &mode)))
+        return false;
+    v.key_q8 = static_cast<int8_t*>(kq);
+    v.value_q8 = static_cast<int8_t*>(vq);
+    v.capacity = cap;
+    v.kv_heads = static_cast<uint32_t>(heads);
+    v.head_dim = static_cast<uint32_t>(dim);
+    v.qblock = static_cast<uint32_t>(qb);
+    v.quant_mode = static_cast<uint32_t>(mode);
+    return true;
+}
 bool read_views(PyObject* storages, std::vector<b200kv_view>& out) {
-    PyObject* fast = PySequence_Fast(storages, "a sequence of cache storages is required");
+    PyObject* fast = items_of(storages, "a sequence of cache storages is required");
     if (fast == nullptr) return false;
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
     out.resize(static_cast<size_t>(n));
     bool ok = true;
-    for (Py_ssize_t i = 0; i < n && ok; ++i) {
-        PyObject* o = PySequence_Fast_GET_ITEM(fast, i);
-        b200kv_view& v = out[i];
-        void *kq, *vq;
-        uint64_t cap, heads, dim, qb, mode;
-        ok = plane(o, KEY, &v.key_f16) && plane(o, VALUE, &v.value_f16) && plane(o, KEY_Q8, &kq) && plane(o, KEY_SCALES, &v.key_scales) &&
-             plane(o, VALUE_Q8, &vq) && plane(o, VALUE_SCALES, &v.value_scales) && number(o, CAPACITY, &cap) && number(o, KV_HEADS, &heads) &&
-             number(o, HEAD_DIM, &dim) && number(o, QBLOCK, &qb) && number(o, QUANT_MODE, &mode);
-        if (!ok) break;
-        v.key_q8 = static_cast<int8_t*>(kq);
-        v.value_q8 = static_cast<int8_t*>(vq);
-        v.capacity = cap;
-        v.kv_heads = static_cast<uint32_t>(heads);
-        v.head_dim = static_cast<uint32_t>(dim);
-        v.qblock = static_cast<uint32_t>(qb);
-        v.quant_mode = static_cast<uint32_t>(mode);
-    }
+    for (Py_ssize_t i = 0; i < n && ok; ++i) ok = read_view(PySequence_Fast_GET_ITEM(fast, i), out[i]);
     Py_DECREF(fast);
     return ok;
 }
@@ -375,7 +414,11 @@ PyObject* py_pool(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return Py_BuildValue("iI", rc, CAPTURE ? static_cast<unsigned>(captured) : matched);
 }
 
-PyObject* py_bind(PyObject*, PyObject* arg) {   // {name: address}
+PyObject* py_bind(PyObject*, PyObject* arg) {   // {name: address}, and "View": the structure
+    PyObject* view = PyDict_GetItemString(arg, "View");
+    if (view == nullptr || !PyType_Check(view)) return PyErr_Format(PyExc_KeyError, "View");
+    Py_INCREF(view);
+    Py_XSETREF(g_view_type, view);
     struct { const char* name; void** slot; } table[] = {
         {"b200kv_append", reinterpret_cast<void**>(&g_api.append)},
         {"b200kv_q_split_norm_rope", reinterpret_cast<void**>(&g_api.q_split_norm_rope)},
@@ -395,6 +438,12 @@ PyObject* py_bind(PyObject*, PyObject* arg) {   // {name: address}
     Py_RETURN_NONE;
 }
 
+PyObject* py_bind_storage(PyObject*, PyObject* view) {   // AttentionLayerKvCacheStorage.view
+    Py_INCREF(view);
+    Py_XSETREF(g_storage_view, view);
+    Py_RETURN_NONE;
+}
+
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {   // no C++ exception reaches the interpreter
     try {
@@ -406,6 +455,7 @@ PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {   // no
 }
 #define ENTRY(name, f) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<f>)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {{"bind", py_bind, METH_O, nullptr},
+                           {"bind_storage", py_bind_storage, METH_O, nullptr},
                            ENTRY("append", py_append),
                            ENTRY("q_split_norm_rope", py_q_split_norm_rope),
                            ENTRY("decode_attn", py_decode_attn),
@@ -421,7 +471,7 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods
 
 PyMODINIT_FUNC PyInit__native(void) {
     const char* names[NAMES] = {"key_cache", "value_cache", "key_cache_q8", "key_scales", "value_cache_q8", "value_scales",
-                                "capacity", "kv_heads", "head_dim", "qblock", "quant_mode"};
+                                "capacity", "kv_heads", "head_dim", "qblock", "quant_mode", "view"};
     for (int i = 0; i < NAMES; ++i) {
         g_names[i] = PyUnicode_InternFromString(names[i]);
         if (g_names[i] == nullptr) return nullptr;

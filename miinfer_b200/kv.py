@@ -165,6 +165,9 @@ class AttentionLayerKvCacheStorage:
         check(lib.b200kv_snapshot_clone(C.byref(d), C.byref(s), tokens, _stream(stream)), "b200kv_snapshot_clone")
 
 
+native.bind_storage(AttentionLayerKvCacheStorage.view)
+
+
 def make_decode_state(position: int, device=None) -> torch.Tensor:
     """A DeviceDecodeState (qwen3_gpu_primitives.hpp:30-37) as a 16-word uint32 tensor."""
     t = torch.zeros(16, dtype=torch.int32, device=device or "cuda")
