@@ -20,6 +20,7 @@ LIB_PATH = LIB_DIR / "libb200kv.so"
 INCLUDE = ROOT.parent / "include"
 NATIVE_SRC = CSRC / "python" / "native.cpp"
 NATIVE_PATH = LIB_DIR / "_native.so"     # the CPython module under the Python mirror's launchers
+NATIVE_STAMP = LIB_DIR / "_native.stamp"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -40,8 +41,17 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp"))
 
 
+def native_stamp() -> str:
+    """What the CPython module is bound to besides its source: it does not load, or not safely, under another."""
+    import torch
+
+    return f"python {sys.version}\ntorch {torch.__version__} cxx11abi {torch._C._GLIBCXX_USE_CXX11_ABI}\n"
+
+
 def needs_build() -> bool:
     if not LIB_PATH.exists() or not NATIVE_PATH.exists():
+        return True
+    if not NATIVE_STAMP.exists() or NATIVE_STAMP.read_text() != native_stamp():
         return True
     newest = max(p.stat().st_mtime for p in list(CSRC.glob("*")) + [NATIVE_SRC, INCLUDE / "b200kv.h"])
     return newest > min(LIB_PATH.stat().st_mtime, NATIVE_PATH.stat().st_mtime)
@@ -79,6 +89,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(native_command(), capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"g++ failed for {NATIVE_SRC.name}:\n{res.stdout}\n{res.stderr}")
+        NATIVE_STAMP.write_text(native_stamp())
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
         native = pool.submit(compile_native)

@@ -66,3 +66,15 @@ def test_pool_arguments():
     if not torch.cuda.is_available():   # through every argument, as far as the library
         with pytest.raises(kv.B200KvError, match="no sm_100 device"):
             pool.capture([1, 2], [Wrapped(good)], stream=NullStream())
+
+
+def test_another_python_or_torch_rebuilds_the_module(monkeypatch, tmp_path):
+    from miinfer_b200 import build
+
+    stamp = tmp_path / "_native.stamp"
+    monkeypatch.setattr(build, "NATIVE_STAMP", stamp)
+    assert build.needs_build()
+    stamp.write_text(build.native_stamp())
+    assert not build.needs_build()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.needs_build()
