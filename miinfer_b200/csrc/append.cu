@@ -382,7 +382,10 @@ extern "C" int b200kv_append(const b200kv_view* view, const void* key, const voi
     p.k_norm_weight = k_norm_weight;
     p.prefill_state = prefill_state;
     p.decode_state = decode_state;
-    token_count = std::min(token_count, 0x7fffffffu);   // a device-side count is at most this: capacities are
+    // A bound above any cache's capacity, where the count is on the device: as many tokens as the kernel's 32-bit unit numbers hold (with
+    // more than eight heads of 128 dims that is 2^30, a cache of terabytes).
+    const uint64_t passes = (static_cast<uint64_t>(view->kv_heads) + kUnitElems / view->head_dim - 1) / (kUnitElems / view->head_dim);
+    if (prefill_state != nullptr || decode_state != nullptr) token_count = static_cast<uint32_t>(std::min<uint64_t>(token_count, 0xffffffffu / (2 * passes)));
     p.token_count = token_count;
     p.base_position = base_position;
     p.rope_mode = rope_mode;
@@ -390,8 +393,7 @@ extern "C" int b200kv_append(const b200kv_view* view, const void* key, const voi
     rope_constants(rope_mode, theta, view->head_dim, p.inv_freq, &p.sectioned_step);
 
     const uint32_t d = view->head_dim;
-    const uint32_t heads_per_unit = kUnitElems / d;
-    const uint64_t units = 2ull * token_count * ((view->kv_heads + heads_per_unit - 1) / heads_per_unit);
+    const uint64_t units = 2 * token_count * passes;
     if (units >= (1ull << 32)) return B200KV_ERR_RANGE;
     int device = 0, sms = 0;
     B200KV_CUDA_TRY(cudaGetDevice(&device));

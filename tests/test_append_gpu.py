@@ -126,3 +126,17 @@ def test_append_unaligned_inputs_bit_exact(cuda):
     kv.launch_kv_store_quant(st.view(), kd, vd, None, T, 3, rope_mode=kv.RopeMode.NEOX_FULL)
     torch.cuda.synchronize()
     assert_planes_equal(st, host, "unaligned inputs")
+
+
+def test_append_count_on_the_device_under_a_bound_of_any_size(cuda):
+    # the launch bound is far above any cache, the count comes from the state
+    rng = np.random.default_rng(13)
+    H, d = 12, 128
+    k, v = ko.normal_f16(rng, (3, H * d)), ko.normal_f16(rng, (3, H * d))
+    host = ko.HostCache(8, H, d, 32, 3)
+    host.append(k.astype(np.float32), v.astype(np.float32), None, 2, rope_mode=1)
+    st = device_storage_like(host)
+    for bound in (3, 1200000000, 0xffffffff):
+        kv.launch_kv_store_quant(st.view(), to_dev(k), to_dev(v), None, bound, 0, rope_mode=1.0, prefill_state=kv.make_prefill_state(2, 3))
+        assert_planes_equal(st, host, f"bound {bound}")   # (a rope mode is whatever int() takes)
+        st.reset()
