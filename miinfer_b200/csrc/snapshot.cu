@@ -11,6 +11,8 @@
 // capacity, destination pitch = the per-head record).
 #include "kv_common.cuh"
 
+#include <cuda.h>   // types and enums only; the entry point is fetched at run time
+
 namespace b200kv {
 
 // ---- device-to-device copies of strided spans -----------------------------------------------------------------
@@ -215,26 +217,67 @@ static int copy_cache_to_cache(const b200kv_view& dst, const b200kv_view& src, u
 }
 
 // Whether the copy kernel may touch all of it: ordinary memory of the current device (anything else takes the copy engine, which
-// also reaches host memory and other devices).
+// also reaches host memory and other devices).  The driver is asked once per mapping, which is one physical allocation and so
+// lies on one device: a caching allocator's planes share a few (16 layers x 4 planes of a short prefix: asking for every plane took
+// 12 us a capture and restore, more than the copies).
+namespace {
+using PointerQuery = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+PointerQuery pointer_query() {
+    static PointerQuery fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &sym, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<PointerQuery>(sym);
+        (void)cudaGetLastError();
+        return static_cast<PointerQuery>(nullptr);
+    }();
+    return fn;
+}
+
+class DeviceMemory {
+public:
+    explicit DeviceMemory(int device) : device_(device), query_(pointer_query()) {}
+    bool holds(const void* p) {
+        const uint64_t at = reinterpret_cast<uintptr_t>(p);
+        for (uint32_t i = 0; i < kept_; ++i)
+            if (at - base_[i] < size_[i]) return true;
+        if (query_ == nullptr) return false;
+        uint32_t type = 0, managed = 0;
+        int device = -1;
+        uint64_t base = 0, size = 0;
+        CUpointer_attribute names[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                        CU_POINTER_ATTRIBUTE_MAPPING_BASE_ADDR, CU_POINTER_ATTRIBUTE_MAPPING_SIZE};
+        void* values[5] = {&type, &managed, &device, &base, &size};
+        if (query_(5, names, values, at) != CUDA_SUCCESS || type != CU_MEMORYTYPE_DEVICE || managed != 0 || device != device_) return false;
+        if (at - base < size) {
+            const uint32_t slot = kept_ < kRanges ? kept_++ : next_++ % kRanges;
+            base_[slot] = base;
+            size_[slot] = size;
+        }
+        return true;
+    }
+
+private:
+    static constexpr uint32_t kRanges = 16;
+    uint64_t base_[kRanges], size_[kRanges];
+    uint32_t kept_ = 0, next_ = 0;
+    int device_;
+    PointerQuery query_;
+};
+}  // namespace
+
 static bool all_on_this_device(const b200kv_view* views, uint32_t layers, const void* blob) {
     int device = -1;
     if (cudaGetDevice(&device) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
-    auto here = [device](const void* p) {
-        cudaPointerAttributes a{};
-        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
-        }
-        return a.type == cudaMemoryTypeDevice && a.device == device;
-    };
-    if ((reinterpret_cast<uintptr_t>(blob) & 1u) != 0 || !here(blob)) return false;
+    DeviceMemory here(device);
+    if ((reinterpret_cast<uintptr_t>(blob) & 1u) != 0 || !here.holds(blob)) return false;
     for (uint32_t l = 0; l < layers; ++l) {
         const PlaneList planes = planes_of(views[l]);
         for (uint32_t i = 0; i < planes.count; ++i)
-            if (!here(planes.base[i])) return false;
+            if (!here.holds(planes.base[i])) return false;
     }
     return true;
 }
