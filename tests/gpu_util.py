@@ -70,17 +70,43 @@ def assert_attention_close(got: np.ndarray, ref: np.ndarray, what: str, tol_abs:
     return max_abs, rel_l2
 
 
-def captured_node_types(call):
-    """Types of the nodes that `call(stream)` captures (0 = kernel, 1 = memcpy); nothing runs."""
+def _captured_nodes(call):
+    """The CUDA driver and the handles of the nodes that `call(stream)` captures; nothing runs."""
     import ctypes as C
 
-    rt = C.CDLL("libcudart.so.12")
+    cu = C.CDLL("libcuda.so.1")
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph, capture_error_mode="relaxed"):
         call(torch.cuda.current_stream().cuda_stream)
     raw, n = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t()
-    assert rt.cudaGraphGetNodes(raw, None, C.byref(n)) == 0
+    assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
     nodes = (C.c_void_p * n.value)()
-    assert rt.cudaGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    return graph, cu, [C.c_void_p(node) for node in nodes]
+
+
+def captured_node_types(call):
+    """Types of the nodes that `call(stream)` captures (0 = kernel, 1 = memcpy); nothing runs."""
+    import ctypes as C
+
+    graph, cu, nodes = _captured_nodes(call)
     kind = C.c_int()
-    return [kind.value for node in nodes if rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0]
+    return [kind.value for node in nodes if cu.cuGraphNodeGetType(node, C.byref(kind)) == 0]
+
+
+def captured_kernels(call):
+    """Mangled names of the kernels that `call(stream)` captures; nothing runs."""
+    import ctypes as C
+
+    class KernelNode(C.Structure):   # CUDA_KERNEL_NODE_PARAMS_v2
+        _fields_ = [("func", C.c_void_p), ("dims", C.c_uint * 7), ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+    graph, cu, nodes = _captured_nodes(call)
+    names = []
+    for node in nodes:
+        k, name = KernelNode(), C.c_char_p()
+        assert cu.cuGraphKernelNodeGetParams_v2(node, C.byref(k)) == 0
+        rc = cu.cuFuncGetName(C.byref(name), C.c_void_p(k.func)) if k.func else cu.cuKernelGetName(C.byref(name), C.c_void_p(k.kern))
+        assert rc == 0
+        names.append(name.value.decode())
+    return names

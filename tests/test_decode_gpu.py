@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import kvoracle as ko
-from gpu_util import assert_attention_close, to_dev, upload
+from gpu_util import assert_attention_close, captured_kernels, to_dev, upload
 from miinfer_b200 import kv
 
 pytestmark = pytest.mark.gpu
@@ -49,7 +49,7 @@ SHAPES = [
 
 
 @pytest.mark.parametrize("d,H,Hq,qb,mode,L", SHAPES)
-@pytest.mark.parametrize("path", ["auto", "mma", "generic"])
+@pytest.mark.parametrize("path", ["auto", "tcgen05", "mma", "generic"])
 def test_decode_matches_two_pass_reference(cuda, d, H, Hq, qb, mode, L, path):
     rng = np.random.default_rng(d + L + mode)
     host = filled(rng, L, H, d, qb, mode, cap=(L + 5 + 7) // 8 * 8)
@@ -61,7 +61,8 @@ def test_decode_matches_two_pass_reference(cuda, d, H, Hq, qb, mode, L, path):
     q16 = ko.normal_f16(rng, (Hq, d))
     gate = rng.standard_normal((Hq, d)).astype(np.float32)
     ref, ref_g = host.decode_ref(q16.astype(np.float32), d ** -0.5, L, gate)
-    flag = kv.FORCE_GENERIC if path == "generic" else 0
+    # short sessions go to the streaming kernel for all modes unless the caller gives a split count
+    flag = kv.FORCE_GENERIC if path == "generic" else 0 if path == "auto" else 5
     kv.set_decode_kernel(1 if path == "mma" else 0)     # which streaming kernel serves the int8 caches
     try:
         for q_dev in (to_dev(q16), to_dev(q16.astype(np.float32))):       # fp16 and fp32 queries
@@ -101,12 +102,12 @@ def test_decode_split_count_invariance_and_determinism(cuda):
             outs.append(out)
     # invariance up to rounding, not bit equality (the tcgen05 kernel carries the weights as 16-bit fixed point per tile)
     assert max(np.max(np.abs(o - outs[0])) for o in outs) <= 5e-5
-    for choice in (0, 1):
+    for choice, splits in ((0, 0), (0, 16), (1, 0)):   # streaming, tcgen05 and mma.sync kernel
         kv.set_decode_kernel(choice)
         try:
-            a, _ = gpu_decode(st, q, 32, 128 ** -0.5, 3000)
+            a, _ = gpu_decode(st, q, 32, 128 ** -0.5, 3000, num_splits=splits)
             for _ in range(8):
-                b, _ = gpu_decode(st, q, 32, 128 ** -0.5, 3000)
+                b, _ = gpu_decode(st, q, 32, 128 ** -0.5, 3000, num_splits=splits)
                 assert np.array_equal(a, b)   # replay is bit-identical
         finally:
             kv.set_decode_kernel(0)
@@ -125,7 +126,7 @@ def test_decode_peaked_softmax_and_large_magnitudes(cuda):
     host.append(kf, vf, None, 0, rope_mode=0)
     st = upload(host)
     ref, _ = host.decode_ref(q16.astype(np.float32), d ** -0.5, L)
-    for flag in (0, kv.FORCE_GENERIC):
+    for flag in (0, 16, kv.FORCE_GENERIC):   # streaming kernel, tcgen05 kernel, streaming kernel
         out, _ = gpu_decode(st, to_dev(q16), Hq, d ** -0.5, L, num_splits=flag)
         assert np.max(np.abs(out - ref)) <= TOL * max(1.0, np.abs(ref).max() / 4)
 
@@ -138,7 +139,7 @@ def test_decode_length_from_device_state_and_quirk_free_length(cuda):
     q = to_dev(ko.normal_f16(rng, (32, 128)))
     ref, _ = host.decode_ref(q.float().cpu().numpy(), 128 ** -0.5, 600)
     state = kv.make_decode_state(599)
-    for flag in (0, kv.FORCE_GENERIC):
+    for flag in (0, 5, kv.FORCE_GENERIC):
         out, _ = gpu_decode(st, q, 32, 128 ** -0.5, 0, decode_state=state, num_splits=flag)
         assert np.max(np.abs(out - ref)) <= TOL
     # attending one slot too many (the reference's non-graph path quirk) or too few is visible
@@ -300,10 +301,11 @@ def test_decode_loop_with_launch_overlap_matches_serial(cuda):
         assert torch.equal(out, ref_out), (overlap, use_graph, (out - ref_out).abs().max())
 
 
+@pytest.mark.parametrize("splits", [0, 4])   # the streaming kernel, the tcgen05 kernel
 @pytest.mark.parametrize("qb,norm,rope,dtype", [(32, False, 1, np.float16), (128, True, 2, np.float32), (32, True, 1, np.float32)])
-def test_fused_decode_step_appends_bit_exact_and_attends(cuda, qb, norm, rope, dtype):
+def test_fused_decode_step_appends_bit_exact_and_attends(cuda, qb, norm, rope, dtype, splits):
     """b200kv_decode_step == append + decode attention: cache rows bit-equal to the oracle, output within tolerance,
-    at positions that fall first, in the middle and last in a 32-position tile, eagerly and from device state."""
+    at positions that fall first, in the middle and last in a tile (of 16 and of 128), eagerly and from device state."""
     rng = np.random.default_rng(91)
     H, Hq, d, L0, cap = 8, 32, 128, 700, 1024
     k0 = ko.normal_f16(rng, (L0, H * d)).astype(np.float32); v0 = ko.normal_f16(rng, (L0, H * d)).astype(np.float32)
@@ -323,17 +325,17 @@ def test_fused_decode_step_appends_bit_exact_and_attends(cuda, qb, norm, rope, d
         if step % 2:
             state[1] = position
             kv.launch_decode_step(st.view(), to_dev(kn), to_dev(vn), to_dev(q16), query_heads=Hq, scale=d ** -0.5, decode_state=state,
-                                  k_norm_weight=wd, rope_mode=kv.RopeMode(rope), output=out, workspace=ws)
+                                  k_norm_weight=wd, rope_mode=kv.RopeMode(rope), output=out, workspace=ws, num_splits=splits)
         else:
             kv.launch_decode_step(st.view(), to_dev(kn), to_dev(vn), to_dev(q16), query_heads=Hq, scale=d ** -0.5, position=position,
-                                  k_norm_weight=wd, rope_mode=kv.RopeMode(rope), output=out, workspace=ws)
+                                  k_norm_weight=wd, rope_mode=kv.RopeMode(rope), output=out, workspace=ws, num_splits=splits)
         torch.cuda.synchronize()
-        if step in (0, 1, 27, 28, 29, 60, 69):     # 700 % 32 == 28: steps 27/28/29 straddle a tile boundary
+        if step in (0, 1, 3, 4, 5, 67, 68, 69):     # 704 begins a tile of 16, 768 one of 128
             ref, _ = host.decode_ref(q16.astype(np.float32), d ** -0.5, position + 1)
             assert np.max(np.abs(out.cpu().numpy() - ref)) <= TOL, position
     from gpu_util import assert_planes_equal
     assert_planes_equal(st, host, "after 70 fused decode steps")
-    # the fallback (generic kernel) gives the same planes and outputs
+    # the streaming kernel gives the same planes and outputs
     st2 = upload(host)
     kn, vn, q16 = ko.normal_f16(rng, (1, H * d)), ko.normal_f16(rng, (1, H * d)), ko.normal_f16(rng, (Hq, d))
     host.append(kn.astype(np.float32), vn.astype(np.float32), w, L0 + 70, rope_mode=rope)
@@ -382,7 +384,7 @@ def test_fused_decode_step_long_context_many_tiles_per_pair(cuda):
     assert np.max(np.abs(out.cpu().numpy() - ref)) <= TOL
 
 
-# (H, Hq, qblock, L): head_dim 256 on the tcgen05 stage-1 kernel
+# (H, Hq, qblock, L): head_dim 256 on the tcgen05 kernel (with splits 0: short sessions on the streaming kernel)
 WIDE = [
     (4, 24, 32, 8200),      # the reference's geometry, q8_0 blocks, many tiles per CTA
     (4, 24, 256, 4099),     # ... with its one-scale-per-row format
@@ -417,10 +419,11 @@ def test_decode_head_dim_256_tcgen05_stage1(cuda, H, Hq, qb, L):
     assert np.array_equal(a, b)
 
 
-def test_decode_steps_head_dim_256_back_to_back_with_launch_overlap(cuda):
-    """At head_dim 256 a decode step is the store kernel, the tcgen05 stage 1 and the merge kernel.  With launch overlap on,
-    each becomes resident while its predecessor still runs (stage 1 even fetches the old cache rows) and orders itself by
-    its own dependency wait: eight steps launched back to back must give, bit for bit, what the serialised launches give."""
+@pytest.mark.parametrize("splits", [0, 37])   # the streaming kernel (short sessions), the tcgen05 kernel
+def test_decode_steps_head_dim_256_back_to_back_with_launch_overlap(cuda, splits):
+    """At head_dim 256 a decode step is one launch that appends, attends and merges.  With launch overlap on, each becomes
+    resident while its predecessor still runs, fetches cache rows older than the predecessor's, and orders itself by its
+    own dependency wait: eight steps launched back to back must give, bit for bit, what the serialised launches give."""
     d, H, Hq, L0, steps = 256, 4, 24, 4000, 8
     rng = np.random.default_rng(256)
     host = filled(rng, L0, H, d, 32, 3, cap=L0 + 64)
@@ -437,7 +440,7 @@ def test_decode_steps_head_dim_256_back_to_back_with_launch_overlap(cuda):
         try:
             for i in range(steps):   # host-side positions: no kernel in between that would serialise the chain
                 kv.launch_decode_step(st.view(), kn[i], vn[i], qs[i], query_heads=Hq, scale=d ** -0.5, position=L0 + i,
-                                      k_norm_weight=w, rope_mode=kv.RopeMode.SECTIONED64, output=outs[i], workspace=ws)
+                                      k_norm_weight=w, rope_mode=kv.RopeMode.SECTIONED64, output=outs[i], workspace=ws, num_splits=splits)
             torch.cuda.synchronize()
         finally:
             kv.set_launch_overlap(0)
@@ -483,3 +486,33 @@ def test_append_inside_the_tcgen05_kernels_at_tile_edges(cuda, d, H, Hq, qb, spl
         kv.set_launch_overlap(0)
     from gpu_util import assert_planes_equal
     assert_planes_equal(st, host, "rows appended inside the kernels")
+
+
+# (d, H, Hq, qblock, mode, capacity, length, num_splits) -> the kernels of a launch
+ROUTES = [
+    ((128, 8, 32, 32, 3, 5000, 4096, 0), ["decode_stream"]),           # short sessions, up to 32768 rows of 128 dims
+    ((128, 8, 32, 32, 3, 5000, 4097, 0), ["decode_tc5_kernel"]),
+    ((128, 8, 32, 32, 3, 5000, 300, 4), ["decode_tc5_kernel"]),        # a count of the caller's keeps the specialised kernel
+    ((128, 8, 32, 32, 3, 5001, 4999, 0), ["decode_stream"]),           # an odd capacity has no TMA view
+    ((128, 2, 10, 32, 3, 5000, 4999, 8), ["decode_stream"]),           # neither has a group of five
+    ((256, 4, 24, 32, 3, 12000, 10000, 0), ["decode_stream"]),         # up to 40000 rows of 256 dims
+    ((256, 4, 24, 32, 3, 12000, 10001, 0), ["decode_tc5_wide"]),
+    ((256, 4, 24, 256, 3, 12000, 300, 3), ["decode_tc5_wide"]),
+    ((256, 4, 24, 256, 0, 12000, 11999, 0), ["decode_stream"]),        # fp16 and mixed caches
+    ((128, 8, 32, 128, 1, 5000, 4999, 0), ["decode_stream"]),
+    ((128, 8, 32, 32, 3, 5000, 4999, kv.FORCE_GENERIC), ["decode_stream"]),
+    ((128, 8, 32, 32, 3, 5000, 4999, kv.SEPARATE_MERGE), ["decode_tc5_kernel", "merge_kernel"]),
+    ((256, 4, 24, 32, 3, 12000, 11999, kv.SEPARATE_MERGE), ["decode_tc5_wide", "merge_kernel"]),
+    ((256, 4, 24, 256, 0, 12000, 11999, kv.SEPARATE_MERGE), ["decode_stream", "merge_kernel"]),
+    ((256, 4, 24, 256, 0, 12000, 11999, 64), ["decode_stream", "merge_kernel"]),   # 4 x 64 CTAs do not fit on 148 SMs together
+]
+
+
+@pytest.mark.parametrize("shape,kernels", ROUTES)
+def test_which_kernels_a_launch_takes(cuda, shape, kernels):
+    d, H, Hq, qb, mode, cap, length, splits = shape
+    st = kv.AttentionLayerKvCacheStorage(cap, kv.KvCacheQuantMode(mode), kv_heads=H, head_dim=d, qblock=qb)
+    q, out, ws = torch.zeros(Hq, d, device="cuda").half(), torch.empty(Hq, d, device="cuda"), kv.decode_workspace(Hq, d)
+    names = captured_kernels(lambda _: kv.launch_decode_attention_quant(st.view(), q, query_heads=Hq, scale=1.0, cache_length=length, output=out,
+                                                                        workspace=ws, num_splits=splits))
+    assert len(names) == len(kernels) and all(k in n for k, n in zip(kernels, names)), names

@@ -157,9 +157,9 @@ def test_sequence_sharded_decode_with_8_ranks_7_of_them_simulated(cuda):
 
 @pytest.mark.parametrize("length", [32768, 131072])
 def test_decode_attention_head_dim_256_at_benchmark_context(cuda, length):
-    """The reference's own geometry (24 query heads over 4 kv heads, head_dim 256, q8_0 blocks) on the tcgen05 stage-1
-    kernel for head_dim 256, at the contexts the benchmark set names; also through the fused-step entry point, which for
-    this geometry is the store kernel followed by the attention."""
+    """The reference's own geometry (24 query heads over 4 kv heads, head_dim 256, q8_0 blocks) on the tcgen05 kernel for
+    head_dim 256, at the contexts the benchmark set names; also through the fused-step entry point, which appends inside
+    the same launch."""
     Hk, Hq, d = 4, 24, 256
     rng = np.random.default_rng(length + d)
     host = ko.HostCache(length + 64, Hk, d, 32, 3)

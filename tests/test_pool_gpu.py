@@ -137,3 +137,26 @@ def test_planes_that_are_not_this_devices_memory_take_the_copy_engine(cuda):
     back.upload_raw(blob, P)
     for a, b in zip(sts[0].planes(), back.planes()):
         assert torch.equal(a[:, :P], b[:, :P])
+
+
+@pytest.mark.parametrize("layers,mode,qb,d", [(50, 3, 32, 128), (97, 0, 256, 256), (3, 2, 256, 256)])
+def test_pool_over_more_layers_than_one_launch_takes_and_uneven_capacities(cuda, layers, mode, qb, d):
+    """A copy launch takes up to 48 layers; capacities may differ between the layers and between the caches captured and restored."""
+    heads, P = 3, 37
+    new = lambda extra: [kv.AttentionLayerKvCacheStorage(P + extra(l), kv.KvCacheQuantMode(mode), kv_heads=heads, head_dim=d, qblock=qb) for l in range(layers)]
+    src, dst = new(lambda l: l % 5), new(lambda l: (7 * l) % 11)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(layers)
+    for st in src:
+        for p in st.planes():
+            p.copy_(torch.randint(-120, 120, p.shape, generator=g, device="cuda"))
+    pool, tokens = kv.SnapshotPool(granularity=1), list(range(P))
+    assert pool.capture(tokens, src) and pool.restore(tokens + [1], dst) == P
+    for a, b in zip(src, dst):
+        for x, y in zip(a.planes(), b.planes()):
+            assert torch.equal(x[:, :P], y[:, :P]) and not bool(y[:, P:].any())
+    # layers of several geometries: captured in one launch per run of equal ones; restored only into caches of the first one's
+    mixed = src[:2] + [kv.AttentionLayerKvCacheStorage(P, kv.KvCacheQuantMode.kQ8Q8, kv_heads=2, head_dim=128, qblock=32)] + src[2:]
+    assert pool.capture(tokens[:20], mixed)
+    with pytest.raises(kv.B200KvError):
+        pool.restore(tokens[:20] + [999], mixed)

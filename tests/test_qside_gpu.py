@@ -61,6 +61,7 @@ def test_query_and_key_at_one_position_are_rotated_by_the_same_bits(cuda):
 
 @pytest.mark.parametrize("d,H,Hq,L,splits,path", [
     (128, 8, 32, 3000, 0, "auto"), (128, 8, 32, 3000, 0, "mma"), (128, 8, 32, 200, 1, "auto"), (128, 8, 32, 200, 1, "mma"),
+    (128, 8, 32, 3000, 16, "auto"), (256, 4, 24, 700, 3, "auto"),
     (256, 4, 24, 700, 0, "generic"), (128, 8, 32, 700, 0, "generic")])
 def test_decode_output_requantised_to_q8_1_blocks(cuda, d, H, Hq, L, splits, path):
     """gated_output_q8 is the Q8_1 form of the gated output the same launch writes: bit-equal to the oracle's

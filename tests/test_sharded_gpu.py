@@ -30,16 +30,21 @@ def _setup(n, seed):
     return kv, host, upload(host), q16, to_dev(q16)
 
 
-def _reference(kv, st, q, n, ws):
+def _reference(kv, st, q, n, ws, splits):
     out = torch.empty(HQ, D, device="cuda")
-    kv.launch_decode_attention_quant(st.view(), q, query_heads=HQ, scale=D ** -0.5, cache_length=n, output=out, workspace=ws)
+    kv.launch_decode_attention_quant(st.view(), q, query_heads=HQ, scale=D ** -0.5, cache_length=n, output=out, workspace=ws, num_splits=splits)
     return out
 
 
-def test_world_of_one_equals_plain_decode(cuda):
+# splits 0: the streaming kernel, which serves shards this short; a count of the caller's: the tcgen05 kernel
+both_kernels = pytest.mark.parametrize("splits", [0, 16])
+
+
+@both_kernels
+def test_world_of_one_equals_plain_decode(cuda, splits):
     kv, host, st, q16, q = _setup(3000, 11)
     ws = kv.decode_workspace(HQ, D)
-    ref = _reference(kv, st, q, 3000, ws)
+    ref = _reference(kv, st, q, 3000, ws, splits)
     from miinfer_b200._lib import lib
     words = lib.b200kv_exchange_bytes(HQ, D, 1) // 8
     buf = torch.zeros(words, dtype=torch.int64, device="cuda")
@@ -47,23 +52,24 @@ def test_world_of_one_equals_plain_decode(cuda):
     for phase in (0, 1, 0):
         out = torch.full((HQ, D), float("nan"), device="cuda")
         kv.launch_decode_attention_sharded(st.view(), q, ex, query_heads=HQ, scale=D ** -0.5, range_begin=0, range_end=3000,
-                                           phase=phase, output=out, workspace=ws)
+                                           phase=phase, output=out, workspace=ws, num_splits=splits)
         torch.cuda.synchronize()
         # world == 1 takes no exchange step at all: the buffer stays untouched
         assert float((out - ref).abs().max()) <= 1e-6
     assert int(buf.abs().sum()) == 0
 
 
+@both_kernels
 @pytest.mark.parametrize("n,cut,phase", [(4096, 2048, 0), (5000, 1777, 1), (2500, 2500, 0), (4096, 1024, 36)])
-def test_two_ranks_with_the_peer_partial_already_delivered(cuda, n, cut, phase):
+def test_two_ranks_with_the_peer_partial_already_delivered(cuda, n, cut, phase, splits):
     kv, host, st, q16, q = _setup(n, 23 + phase)
     ws = kv.decode_workspace(HQ, D)
-    ref = _reference(kv, st, q, n, ws)
+    ref = _reference(kv, st, q, n, ws, splits)
     # rank 1's shard [cut, n) reduced to one partial per head, the way its kernel would
     mine = kv.packed_partial(HQ, D, 1)
     pm, pl, pa = kv.partial_views(mine[0], HQ, D)
     kv.launch_decode_partials(st.view(), q, query_heads=HQ, scale=D ** -0.5, range_begin=cut, range_end=n,
-                              part_m=pm, part_l=pl, part_acc=pa, workspace=ws)
+                              part_m=pm, part_l=pl, part_acc=pa, workspace=ws, num_splits=splits)
     torch.cuda.synchronize()
     words_per_rank = HQ * (D + 2)
     own = torch.zeros(2 * 2 * words_per_rank, dtype=torch.int64, device="cuda")     # [phase][src rank][head][d + 2]
@@ -78,7 +84,7 @@ def test_two_ranks_with_the_peer_partial_already_delivered(cuda, n, cut, phase):
     gate = torch.randn(HQ, D, device="cuda")
     gated = torch.empty(HQ, D, device="cuda")
     kv.launch_decode_attention_sharded(st.view(), q, ex, query_heads=HQ, scale=D ** -0.5, range_begin=0, range_end=cut,
-                                       phase=phase, output=out, gate=gate, gated_output=gated, workspace=ws)
+                                       phase=phase, output=out, gate=gate, gated_output=gated, workspace=ws, num_splits=splits)
     torch.cuda.synchronize()
     assert float((out - ref).abs().max()) <= 2e-5          # same partials, merged in a different order
     assert float((gated - ref * torch.sigmoid(gate)).abs().max()) <= 2e-5
@@ -93,8 +99,9 @@ def test_two_ranks_with_the_peer_partial_already_delivered(cuda, n, cut, phase):
     assert int(other.abs().sum()) == 0
 
 
+@both_kernels
 @pytest.mark.parametrize("stale", [False, True])
-def test_a_peer_that_never_delivers_poisons_the_output_and_sets_the_status_word(cuda, stale):
+def test_a_peer_that_never_delivers_poisons_the_output_and_sets_the_status_word(cuda, stale, splits):
     """The wait for a peer is bounded: with nothing in the peer's slot -- or only the words of an EARLIER call,
     as a rank that arrives after its peers gave up would leave them -- the kernel gives up, writes NaN and
     reports the timeout in the registered status word.  After clearing, the next call works again."""
@@ -111,19 +118,19 @@ def test_a_peer_that_never_delivers_poisons_the_output_and_sets_the_status_word(
     kv.set_status_word(status)
     try:
         kv.launch_decode_attention_sharded(st.view(), q, ex, query_heads=HQ, scale=D ** -0.5, range_begin=0, range_end=1024,
-                                           phase=6, output=out, workspace=ws)
+                                           phase=6, output=out, workspace=ws, num_splits=splits)
         torch.cuda.synchronize()
         assert bool(torch.isnan(out).all())
         assert int(status.item()) & kv.STATUS_PEER_TIMEOUT
         # recovery as documented: zero the status word, clear the workspace and the exchange buffers, go on
         status.zero_(); own.zero_(); peer.zero_()
         kv.workspace_reset(ws)
-        want = _reference(kv, st, q, 1024, ws)
+        want = _reference(kv, st, q, 1024, ws, splits)
         pm = torch.full((HQ,), float("-inf"), device="cuda"); pl = torch.zeros(HQ, device="cuda"); pa = torch.zeros(HQ, D, device="cuda")
         slot = own[(1 * 2 + 1) * words_per_rank:(1 * 2 + 2) * words_per_rank].view(HQ, D + 2)   # call 7 -> slot 1; the peer's shard is empty
         slot[:, :D] = _tagged(pa, 7); slot[:, D] = _tagged(pm, 7); slot[:, D + 1] = _tagged(pl, 7)
         kv.launch_decode_attention_sharded(st.view(), q, ex, query_heads=HQ, scale=D ** -0.5, range_begin=0, range_end=1024,
-                                           phase=7, output=out, workspace=ws)
+                                           phase=7, output=out, workspace=ws, num_splits=splits)
         torch.cuda.synchronize()
         assert int(status.item()) == 0
         assert float((out - want).abs().max()) <= 2e-5

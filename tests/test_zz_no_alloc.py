@@ -25,7 +25,7 @@ def test_static_scratch_entry_point_matches_workspace_entry_point(cuda):
     from gpu_util import assert_attention_close, upload
 
     rng = np.random.default_rng(99)
-    # (length, capacity, cache mode, kv heads, query heads, head_dim, split count): streaming kernel twice, then the generic one
+    # (length, capacity, cache mode, kv heads, query heads, head_dim, split count): the streaming kernel for all modes, the tcgen05 kernel, and the former again
     cases = ((3000, 3072, 3, 8, 32, 128, 0), (777, 1024, 3, 8, 32, 128, 5), (300, 304, 1, 4, 8, 256, 0))
     free_before = None
     for call, (length, capacity, mode, H, Hq, d, splits) in enumerate(cases):
