@@ -71,6 +71,28 @@ def _fill(kv, torch, st, tokens, seed, chunk=8192):
         kv.launch_kv_store_quant(st.view(), k, v, None, n, base, rope_mode=kv.RopeMode.NONE)
 
 
+def _kernels(torch, call) -> int:
+    """Kernels that `call()` launches, counted in a stream capture of it that never runs."""
+    import ctypes as C
+
+    cu = C.CDLL("libcuda.so.1")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        call()
+    raw, n, kind = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(), C.c_int()
+    if cu.cuGraphGetNodes(raw, None, C.byref(n)) != 0:
+        raise RuntimeError("cuGraphGetNodes")
+    nodes = (C.c_void_p * n.value)()
+    if cu.cuGraphGetNodes(raw, nodes, C.byref(n)) != 0:
+        raise RuntimeError("cuGraphGetNodes")
+    kernels = 0
+    for node in nodes:
+        if cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) != 0:
+            raise RuntimeError("cuGraphNodeGetType")
+        kernels += kind.value == 0
+    return kernels
+
+
 def _time(torch, dist, stream, fn, warmup, steps):
     with torch.cuda.stream(stream):
         for _ in range(warmup):
@@ -154,6 +176,12 @@ def run_prefill(args, torch, dist, rank, world, local_rank):
     kv.set_launch_overlap(0 if args.no_overlap else 1)   # every kernel of the chunk waits for its predecessor itself
     ms = _time(torch, dist, stream, step, args.warmup, args.steps)
     kv.set_launch_overlap(0)
+
+    def layer():
+        kv.launch_kv_store_quant(views[0], k_new[0], v_new[0], w, T, P, rope_mode=kv.RopeMode.SECTIONED64, theta=1.0e6)
+        kv.launch_suffix_attention_quant(views[0], q[0], gate[0], out[0], ws, T, P, query_heads=hq, scale=D ** -0.5, prepared_rows=P if ahead else 0)
+
+    per_layer = _kernels(torch, layer) + (1 if ahead else 0)   # store, pre-pass (or two), attention, and its merge where the KV range is split
     check = None
     if rank == 0 and not args.no_check:
         ko = _oracle()
@@ -172,7 +200,7 @@ def run_prefill(args, torch, dist, rank, world, local_rank):
                                    f"kv heads split over {world} GPU(s); kernel {args.prefill_kernel}", "l2": "L2 flushed implicitly: 16 layer caches of 19 MB rotate"},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": tf_peak * world, "unit": "TFLOP/s", "frac": achieved / (tf_peak * world),
                          "traffic": None, "peak_kind": f"{kind} (bf16_tflops_sustained) x {world} GPUs"},
-            "check": check, "gpu_launches": args.steps * LAYERS * (2 if ws is None else (5 if ahead else 4)),
+            "check": check, "gpu_launches": args.steps * LAYERS * per_layer,
             "prefix_prepass": "beside the previous layers' attention (second stream, two workspaces)" if ahead else "inside the layer's own launch sequence"}
 
 
@@ -460,8 +488,9 @@ def run_append(args, torch, dist, rank, world, local_rank):
 
 def run_decode256(args, torch, dist, rank, world, local_rank):
     """Decode attention alone on the reference's own geometry: 24 query heads over 4 kv heads, head_dim 256, q8_0 K/V, one
-    session of `--context` positions per GPU, 16 attention layers (the hybrid model's count), no append.  Stage 1 on the
-    tcgen05 kernel for head_dim 256 plus the merge kernel; `--decode-kernel mma` runs the generic stage 1 instead."""
+    session of `--context` positions per GPU, 16 attention layers (the hybrid model's count), no append.  The tcgen05
+    kernel for head_dim 256 with its merge inside; contexts up to 10000 positions, and `--decode-kernel mma`, take the streaming
+    kernel for all modes."""
     from miinfer_b200 import kv
 
     L, HQ, HKV, D, LAYERS = args.context, 24, 4, 256, min(args.layers, 16)
@@ -501,7 +530,9 @@ def run_decode256(args, torch, dist, rank, world, local_rank):
     bytes_launch = L * HKV * (D + 2 * (D // 32)) * 2
     bw_peak, _, kind_peak = _peaks()
     achieved = bytes_launch * LAYERS / (ms * 1e-3) / 1e9
-    streaming = kind == 2 and args.decode_kernel != "mma"
+    wide = kind == 2 and args.decode_kernel != "mma" and L * HKV > 40000   # shorter sessions: the streaming kernel
+    per_layer = _kernels(torch, lambda: kv.launch_decode_attention_quant(views[0], q[0], query_heads=HQ, scale=D ** -0.5, cache_length=L, output=out[0],
+                                                                         workspace=ws))
     return {"metric": "q8_0_kv_decode_attention_gbs_head_dim_256", "value": achieved * world, "unit": "GB/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "int8 KV / fp32 accumulate", "data": "synthetic",
@@ -509,9 +540,9 @@ def run_decode256(args, torch, dist, rank, world, local_rank):
                        "l2": f"inputs larger than L2: {bytes_launch * LAYERS / 1e6:.0f} MB of KV per step"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": bw_peak, "unit": "GB/s", "frac": achieved / bw_peak, "traffic": None,
                          "peak_kind": f"{kind_peak} (hbm_gbs)",
-                         "kernel": "decode_tc5_wide_kernel + merge_kernel" if streaming else "decode_generic_kernel + merge_kernel",
-                         "us_per_launch_pair": ms * 1e3 / LAYERS, "algorithmic_bytes_per_launch": bytes_launch},
-            "check": check, "gpu_launches": args.steps * LAYERS * 2}
+                         "kernel": "decode_tc5_wide_kernel (merge fused in)" if wide else "decode_stream_kernel (merge fused in)",
+                         "us_per_launch": ms * 1e3 / LAYERS, "algorithmic_bytes_per_launch": bytes_launch},
+            "check": check, "gpu_launches": args.steps * LAYERS * per_layer}
 
 
 def run(args, torch, dist, rank, world, local_rank):
