@@ -53,7 +53,8 @@ struct AppendParams {
 constexpr int kAppendWarps = 2;
 constexpr int kUnitElems = 1024;       // 32 q8_0 blocks: one scale per lane
 template <bool IN_F16>
-constexpr int kAppendCtasPerSm = IN_F16 ? 10 : 8;   // 20 warps of 96 registers: a unit, the next one's raw input and the rotation (fp32 input: 16 of 128)
+constexpr int kAppendCtasPerSm = IN_F16 ? 10 : 8;   // 20 warps of 96 registers: a unit, the next one's raw input and the rotation (fp32 input: 16 of 128);
+                                                    // head_dim 256 with fp16 input spills 8 bytes of them
 
 // Two fp32 products in one instruction (each rounds like its scalar form; .ftz as the scalar intrinsics under this build).
 using Pair = unsigned long long;

@@ -1,7 +1,8 @@
-// Split-K GQA decode attention: entry points, the log-sum-exp merge kernel and
-// the generic stage-1 kernel that covers every cache mode (fp16 or int8 K/V,
-// block or row scales).  The specialised int8 streaming kernel lives in
-// decode_q8.cu and is preferred whenever it supports the geometry.
+// Split-K GQA decode attention: entry points, the choice of the kernel and its
+// splits, and the log-sum-exp merge kernel of launches that do not merge inside.
+// Stage 1 (with the merge and a decode step's append inside) is decode_tc5.cu and
+// decode_q8.cu for int8 at head_dim 128, decode_tc5_wide.cu for int8 at head_dim
+// 256, decode_stream.cu for every other mode and shape and for short sessions.
 //
 // Stage-1 arithmetic follows MIInfer's decode kernel
 // (gfx906/kernels/qwen3_primitives.hip:7371-7485) with the per-row scale
@@ -119,11 +120,12 @@ int launch_merge(const MergeParams& p, uint32_t groups, cudaStream_t stream) {
 
 // max_length x kv heads up to which a single session takes the mma.sync kernel.  Measured (decode step, q8_0, us): 8 kv heads of
 // 128 dims: 6.5 against 8.2 at 1500 positions, 8.3 / 8.5 at 3000, 8.8 / 8.7 at 4096, 9.6 / 9.1 at 6000; 4 kv heads of 256 dims: 7.9 /
-// 12.7 at 1500, 9.7 / 10.3 at 4096, 11.4 / 11.4 at 7777, 14.0 / 13.1 at 12000 (one scale per row: 12.8 / 12.6 there).
+// 12.7 at 1500, 9.7 / 10.3 at 4096, 11.4 / 11.4 at 7777, 14.0 / 13.1 at 12000 (one scale per row: 12.8 / 12.6 there).  The lines lie where
+// the two are level within the runs' spread; other head counts were not measured and go by the rows, which is what fills the device.
 constexpr uint64_t kStreamRows128 = 32768, kStreamRows256 = 40000;
 
-// Runs stage 1 (streaming kernel if available, else generic) into the workspace.
-// Workspace layout: [tagged partials of the streaming kernel (zero between launches)] [m] [l] [acc].
+// Runs stage 1 and, where the merge fits inside the launch, the merge.
+// Workspace layout: [tagged partials of the merge inside (zero between launches)] [m] [l] [acc].
 int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, void* workspace,
                       size_t workspace_bytes, uint32_t num_splits_arg, const MergeParams& merge, bool* merged,
                       cudaStream_t stream) {

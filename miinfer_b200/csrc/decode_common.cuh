@@ -80,11 +80,12 @@ struct DecodeParams {
     float* ws_m;                             // [sessions][num_splits][query_heads]
     float* ws_l;
     float* ws_acc;                           // [sessions][num_splits][query_heads][d]
-    // Fused merge (streaming kernel only): when `ws_tagged` is non-null the partials go out as tagged 8-byte words
-    // ([sessions][num_splits][query_heads][head_dim + 2]) and designated CTAs combine all splits and write `fuse`'s
+    // Fused merge: when `ws_tagged` is non-null the partials go out as tagged 8-byte words
+    // ([sessions][num_splits][query_heads][head_dim / 128][128 + 2]) and designated CTAs combine all splits and write `fuse`'s
     // outputs; the words must be zero on entry and are zero again on exit.
-    // Fused single-token append (streaming kernel, one session): the warp that owns the last tile quantises the new
-    // token's K/V row of its kv head and stores it at position end-1 before it loads that tile.
+    // Fused single-token append (one session): a warp of the CTA that owns the last tile quantises the new token's K/V row of
+    // its kv head and stores it at position end-1; the row is patched into the tile once that has landed (decode_q8.cu stores the
+    // row first and loads the tile afterwards).
     const void* new_key;                     // [kv_heads*d] of new_is_f16 ? fp16 : fp32, or null = no fused append
     const void* new_value;
     int new_is_f16;
@@ -146,7 +147,7 @@ __device__ __forceinline__ const b200kv_view& session_view(const DecodeParams& p
 int launch_merge(const MergeParams& p, uint32_t groups, cudaStream_t stream);
 
 // Stage 1 into `workspace` (fills p.num_splits and p.ws_*).  num_splits_arg: 0 =
-// choose; top bit set = use the generic kernel even where a fast one exists.
+// choose; B200KV_SPLITS_FORCE_GENERIC = the streaming kernel for all modes even where a specialised one exists.
 // `merge` describes where the combined result goes; *merged is set when the stage-1 kernel did the
 // combine itself (then no launch_merge is needed).
 int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, void* workspace,
@@ -169,13 +170,13 @@ int launch_decode_stream(const DecodeParams& p, const b200kv_view& geometry, uin
 int launch_decode_q8(const DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream);
 // The same launch on the tcgen05 kernel (decode_tc5.cu); B200KV_ERR_UNSUPPORTED where it does not apply.
 int launch_decode_tc5(const DecodeParams& p, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream);
-// head_dim 256 on tcgen05 (stage 1 only, plain partials, one session): decode_tc5_wide.cu
+// int8 K and V at head_dim 256 on tcgen05 (one session, merge and append inside): decode_tc5_wide.cu
 bool decode_tc5_wide_ok(const b200kv_view& view, uint32_t query_heads);
 uint32_t pick_splits_tc5_wide(const b200kv_view& view, uint32_t max_length);
 int launch_decode_tc5_wide(const DecodeParams& p, const b200kv_view& geometry, cudaStream_t stream);
 uint32_t pick_splits_q8(const b200kv_view& geometry, uint32_t query_heads, uint32_t sessions, uint32_t max_length);
 // TMA descriptors of a view's int8 K and V planes (rows of head_dim bytes, 128-byte swizzle).
-// B200KV_ERR_UNSUPPORTED when the view cannot take the streaming kernel (then the generic kernel is used).
+// B200KV_ERR_UNSUPPORTED when the view cannot take the kernels that need them (then decode_stream.cu is used).
 int encode_kv_maps(const b200kv_view& view, uint32_t tile_positions, CUtensorMap* kmap, CUtensorMap* vmap);
 bool q8_fast_path_ok(const b200kv_view& view, uint32_t query_heads);
 

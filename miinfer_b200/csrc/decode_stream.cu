@@ -12,7 +12,7 @@
 //  * Each warp walks its own tiles of 16 positions (warp w of W takes tiles w, w + W, ...): no barrier between warps until the
 //    end.  A tile is two UNITS, its K rows and its V rows, which the warp copies with cp.async into a private ring (about 24 KB;
 //    8 warps on an SM keep 130 KB or more in flight), 16-byte chunks XORed with the row number so that ldmatrix
-//    reads without bank conflicts.  Rows of any alignment above 16 bytes work, rows past the end are zero-filled.
+//    reads without bank conflicts (255 registers a thread at head_dim 256: q8_0 on both sides spills 8 bytes).  Rows of any alignment above 16 bytes work, rows past the end are zero-filled.
 //  * S = Q K^T and O = P V run on mma.sync m16n8k16 with fp32 accumulation.  M = 16 is 8 heads x 2 terms: rows 0-7 hold the
 //    high and rows 8-15 the low fp16 half of every query element (and of every weight), 22 bits in all, so the products are
 //    those of an fp32 kernel and the two halves of a score sit in one thread.  K and V are exact in fp16: fp16 planes as they

@@ -26,7 +26,8 @@
 //     At head_dim 128 a CTA takes TWO row tiles where there are enough of them (512 softmax threads; S and O of both fill
 //     TMEM, so Q is an A operand in shared memory): a single tile's loop waits for its softmax (about 1 us a pair of KV tiles against
 //     0.5 us of MMAs), two share every K and V tile and one's MMAs run under the other's softmax.  2048 fresh
-//     tokens, 32/8 heads: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA.
+//     tokens, 32/8 heads: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA (96 registers a
+//     thread, 20 bytes of them spilled).
 // Every mbarrier wait is bounded; a wait that runs out poisons the output rows with NaN, and the CTA still frees
 // its TMEM and exits.
 #include "decode_common.cuh"
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const __grid_constan
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<size_t>(p.total_rows) * VPR) return;
     const uint32_t gr = static_cast<uint32_t>(idx / VPR), c = static_cast<uint32_t>(idx % VPR) * 4;
-    // every load of the row's splits is issued before the first is used; an empty split's O was never written and counts for nothing
+    // every load of the row's splits is issued before the first is used; an empty split's O is zeros and counts for nothing
     float2 ml[MAX_SPLITS];
     float4 o[MAX_SPLITS];
 #pragma unroll
@@ -858,6 +859,7 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
 //   20 tokens over 16000 (4 units):   5 splits 77 us, 8: 66, 16: 58     37 over 3001 (8):  5: 38, 8: 35, 12: 34, 16: 34
 //   128 over 8192 (24):   5: 54, 6: 52, 8 (a second wave): 69           300 over 8192 (60): 1: 124, 2: 92, 4: 102
 //   512 over 8192 (96):   1: 127, 2: 158, 3 (what filling the last wave best asks for): 138
+// The estimate takes the best column of each but one: 6 for 37 over 3001, where partial_us, that of launches with more rows, is too high.
 static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t most, uint32_t head_dim) {
     const double tile_us = head_dim == 256 ? 0.73 : 0.52, wave_us = 8.0, merge_us = 3.0, partial_us = head_dim == 256 ? 0.11 : 0.055;
     uint32_t best = 1;

@@ -488,8 +488,8 @@ def set_launch_overlap(tail_positions: int) -> None:
 
 
 def decode_kernel_kind(view: View, query_heads: int) -> int:
-    """1: decode attention on this view runs a streaming int8 kernel (head_dim 128); 2: the tcgen05 stage 1 for head_dim 256;
-    0: the generic kernel."""
+    """1: decode attention on this view runs an int8 kernel for head_dim 128; 2: the tcgen05 kernel for head_dim 256; 0: the streaming
+    kernel for all modes (which also takes short single sessions of the other two, unless the caller gives a split count)."""
     return int(lib.b200kv_decode_kernel_kind(C.byref(view), query_heads))
 
 
