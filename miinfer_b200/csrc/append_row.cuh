@@ -20,17 +20,25 @@ __device__ __forceinline__ void row_rotation(Rotation<D>& r, int lane, uint32_t 
         for (int j = 0; j < D / 64; ++j) sincos_pinned(__fmul_rn(static_cast<float>(position), inv_freq[lane + 32 * j]), &r.sn[j], &r.cs[j]);
     } else if (rope_mode == B200KV_ROPE_SECTIONED64) {
         float angle = static_cast<float>(position);
-        for (int i = 0; i < lane; ++i) angle = __fmul_rn(angle, sectioned_step);
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) angle = i < lane ? __fmul_rn(angle, sectioned_step) : angle;   // as many products as the lane's number, no branch per product
         sincos_pinned(angle, &r.sn[0], &r.cs[0]);
     }
 }
 
+// A lane's norm weights, fetched ahead of the row's arithmetic (in the middle of it they were a trip to L2 of their own).
+template <int D>
+__device__ __forceinline__ void load_norm_weight(const float* k_norm_weight, int lane, float (&w)[D / 32]) {
+#pragma unroll
+    for (int j = 0; j < D / 32; ++j) w[j] = k_norm_weight != nullptr ? k_norm_weight[lane + 32 * j] : 1.0f;
+}
+
 // K side before quantization: optional RMSNorm * weight, then RoPE.
 template <int D>
-__device__ __forceinline__ void transform_k_row(float (&k)[D / 32], int lane, const float* k_norm_weight, float epsilon, int rope_mode,
+__device__ __forceinline__ void transform_k_row(float (&k)[D / 32], int lane, bool norm, const float (&w)[D / 32], float epsilon, int rope_mode,
                                                 const Rotation<D>& r) {
     constexpr int NJ = D / 32;
-    if (k_norm_weight != nullptr) {
+    if (norm) {
         // the reference's shared-memory tree (stride D/2 .. 1) as register adds + a shuffle-down tree over the same pairs
         float sq[NJ];
 #pragma unroll
@@ -45,7 +53,7 @@ __device__ __forceinline__ void transform_k_row(float (&k)[D / 32], int lane, co
         ss = __shfl_sync(0xffffffffu, ss, 0);
         const float rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, static_cast<float>(D)), epsilon)));
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) k[j] = __fmul_rn(__fmul_rn(k[j], rms), k_norm_weight[lane + 32 * j]);
+        for (int j = 0; j < NJ; ++j) k[j] = __fmul_rn(__fmul_rn(k[j], rms), w[j]);
     }
     if (rope_mode == B200KV_ROPE_NEOX_FULL) {
 #pragma unroll

@@ -240,10 +240,11 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     pdl_wait();
     // The new row of a fused append is fetched now, while the memory system is still quiet: once every warp's ring
     // is streaming, a dependent load waits behind tens of megabytes of queued tile traffic (microseconds).
-    float new_k[4], new_v[4];
+    float new_k[4], new_v[4], norm[4];
     if (owner) {
         tail::load_new_row<kD>(p.new_key, p.new_is_f16, kv_head, lane, new_k);
         tail::load_new_row<kD>(p.new_value, p.new_is_f16, kv_head, lane, new_v);
+        load_norm_weight<kD>(p.k_norm_weight, lane, norm);
     }
     {
         // the tile that holds the row of a fused append is loaded only after that row has been stored (below)
@@ -294,7 +295,7 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
         Rotation<kD> rot;
         row_rotation<kD>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);
         tail::RowScratch<kD>* no_copy = nullptr;
-        tail::store_new_key<kD>(p, view, new_k, rot, head_row0 + end - 1, lane, no_copy);
+        tail::store_new_key<kD>(p, view, new_k, norm, rot, head_row0 + end - 1, lane, no_copy);
         tail::store_new_value<kD>(view, new_v, head_row0 + end - 1, lane, no_copy);
         __threadfence();
         asm volatile("fence.proxy.async;" ::: "memory");

@@ -222,8 +222,11 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     Rotation<D> rot{};
     if (makes_key) row_rotation<D>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();
-    float new_x[D / 32];
-    if (makes_key || makes_value) tail::load_new_row<D>(makes_key ? p.new_key : p.new_value, p.new_is_f16, kv_head, lane, new_x);
+    float new_x[D / 32], norm[D / 32];
+    if (makes_key || makes_value) {
+        tail::load_new_row<D>(makes_key ? p.new_key : p.new_value, p.new_is_f16, kv_head, lane, new_x);
+        load_norm_weight<D>(p.k_norm_weight, lane, norm);
+    }
     while (next_unit < P::kUnits - 1) issue();
     if (p.new_key != nullptr) pdl_launch_dependents();   // an appending launch: see pdl_launch_dependents
 
@@ -277,7 +280,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     __syncthreads();
     const float qmul = qmul_s[lane >> 2];
     if (makes_key || makes_value) {
-        if (makes_key) tail::store_new_key<D>(p, view, new_x, rot, head_row0 + end - 1, lane, new_row);
+        if (makes_key) tail::store_new_key<D>(p, view, new_x, norm, rot, head_row0 + end - 1, lane, new_row);
         else tail::store_new_value<D>(view, new_x, head_row0 + end - 1, lane, new_row + 1);
         __threadfence_block();
         asm volatile("bar.arrive 3, 96;" ::: "memory");

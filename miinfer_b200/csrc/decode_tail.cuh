@@ -100,9 +100,9 @@ __device__ __forceinline__ void store_new_row(const float (&x)[D / 32], bool q8,
     }
 }
 template <int D, int BYTES>
-__device__ __forceinline__ void store_new_key(const DecodeParams& p, const b200kv_view& view, float (&k)[D / 32], const Rotation<D>& rot,
+__device__ __forceinline__ void store_new_key(const DecodeParams& p, const b200kv_view& view, float (&k)[D / 32], const float (&norm)[D / 32], const Rotation<D>& rot,
                                               uint64_t row_index, int lane, RowScratch<BYTES>* scratch) {
-    transform_k_row<D>(k, lane, p.k_norm_weight, p.epsilon, p.rope_mode, rot);
+    transform_k_row<D>(k, lane, p.k_norm_weight != nullptr, norm, p.epsilon, p.rope_mode, rot);
     store_new_row<D, BYTES>(k, (view.quant_mode & 1u) != 0, view.qblock == D, view.key_q8, view.key_f16, view.key_scales, row_index, lane, scratch);
 }
 template <int D, int BYTES>

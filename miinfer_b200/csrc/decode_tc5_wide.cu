@@ -244,10 +244,11 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     Rotation<kD> rot{};
     if (appends) row_rotation<kD>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();
-    float new_k[kD / 32], new_v[kD / 32];
+    float new_k[kD / 32], new_v[kD / 32], norm[kD / 32];
     if (appends) {
         tail::load_new_row<kD>(p.new_key, p.new_is_f16, kv_head, lane, new_k);
         tail::load_new_row<kD>(p.new_value, p.new_is_f16, kv_head, lane, new_v);
+        load_norm_weight<kD>(p.k_norm_weight, lane, norm);
     }
     // the rest of the first ring fill, by the thread that set the barriers up
     if (warp == kProducerWarp && lane == 0)
@@ -382,7 +383,7 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
     } else if (warp == kPvWarp) {
         // =============================== the fused append, then the issuer of O^T = V^T . P ===============================
         if (appends) {
-            tail::store_new_key<kD>(p, view, new_k, rot, head_row0 + end - 1, lane, new_row);
+            tail::store_new_key<kD>(p, view, new_k, norm, rot, head_row0 + end - 1, lane, new_row);
             tail::store_new_value<kD>(view, new_v, head_row0 + end - 1, lane, new_row + 1);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_row);
