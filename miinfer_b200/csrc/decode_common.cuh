@@ -139,6 +139,13 @@ __device__ __forceinline__ void resolve_range(const DecodeParams& p, uint32_t se
     *begin = p.range_begin < length ? p.range_begin : length;
 }
 
+// The first of `total` tiles that belongs to part `i` of `parts` (i <= parts <= kMaxSplitsPerSession): floor(total * i / parts), a product that
+// does not fit 32 bits, from 32-bit divisions.
+__device__ __forceinline__ uint32_t part_begin(uint32_t total, uint32_t i, uint32_t parts) {
+    const uint32_t q = total / parts, r = total - q * parts;
+    return q * i + r * i / parts;
+}
+
 __device__ __forceinline__ const b200kv_view& session_view(const DecodeParams& p, uint32_t session) {
     return p.views != nullptr ? p.views[session].view : p.view;
 }

@@ -27,6 +27,10 @@
 // 9.8 at 6001 (the kernel this one replaced and its merge kernel: 64), 24.6 at 32768 (5.5 TB/s), 82 at 131072 (6.5 TB/s: the copy
 // rate); q8_0 7.8 us at 1500, 22.0 at 32768 (254), 65 at 131072 -- there the conversions of int8 show, and the tcgen05 kernels
 // are faster.  24 sessions of 200 to 6000 positions in one launch, q8_0: 44 us (657).
+// A decode step's launch at a few thousand positions is a chain of latencies, instruction fetches above all (2.2 of the 7.5 cycles a warp
+// spends on an instruction at 7777 positions, one scale per row); hence partials emitted two dims at a time, the copies' code once for
+// both sides, 32-bit split bounds, and the merge's gate fetched early.  Step of 24 / 4 heads of 256, append and merge included, in a graph: q8_0 4000
+// positions 9.9 -> 9.0 us, one scale per row 7777 11.3 -> 10.6, fp16 6001 11.4 -> 10.75.
 #include "decode_tail.cuh"
 
 #include <climits>
@@ -152,8 +156,8 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         }
     }
     // this CTA's positions: whole tiles counted from `begin`
-    const uint64_t tiles = (end - begin + kTile - 1) / kTile;
-    const uint32_t t0 = static_cast<uint32_t>(tiles * split / num_splits), t1 = static_cast<uint32_t>(tiles * (split + 1) / num_splits);
+    const uint32_t tiles = (end - begin) / kTile + ((end - begin) % kTile != 0);
+    const uint32_t t0 = part_begin(tiles, split, num_splits), t1 = part_begin(tiles, split + 1, num_splits);
     const uint32_t pos0 = begin + t0 * kTile;
     const int my_tiles = static_cast<int>((t1 - t0 + WARPS - 1 - warp) / WARPS);   // tiles of this warp
 
@@ -209,7 +213,9 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         const int t = next_unit >> 1;
         if (t < my_tiles) {
             const uint32_t dst = ring + next_slot * P::kSlot;
-            if (next_unit & 1) copy_side(std::integral_constant<int, VF>{}, v_rows, v_scales, tile_pos(t), dst);
+            const bool v = next_unit & 1;
+            if constexpr (KF == VF) copy_side(std::integral_constant<int, KF>{}, v ? v_rows : k_rows, v ? v_scales : k_scales, tile_pos(t), dst);   // half the code
+            else if (v) copy_side(std::integral_constant<int, VF>{}, v_rows, v_scales, tile_pos(t), dst);
             else copy_side(std::integral_constant<int, KF>{}, k_rows, k_scales, tile_pos(t), dst);
         }
         cp_commit();                              // an empty group keeps the count
@@ -407,8 +413,11 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
                     }
                 }
             } else {
+                // Launches of few tiles a warp run through most code once or twice and wait for instructions more than for anything else: one
+                // session's score loop is rolled up.
+                constexpr int kRolled = HOLD || WARPS == 4 ? D / 16 : 2;
                 float hi[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
+#pragma unroll kRolled
                 for (int k0 = 0; k0 < D / 16; k0 += kChain<KF>) {
                     float acc[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
 #pragma unroll
@@ -610,13 +619,16 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         tot_s[2 * tid + 1] = L;
     }
     __syncthreads();
-    for (int idx = tid; idx < G * D; idx += P::kThreads) {
+    for (int idx = 2 * tid; idx < G * D; idx += 2 * P::kThreads) {
         const int h = idx / D, dim = idx % D;
-        float a = 0.0f;
+        float2 a = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w)
-            a = fmaf(reinterpret_cast<const float*>(smem + P::kOffRing + w * (P::kUnits * P::kSlot))[h * P::kOutStride + dim], ml_s[(w * 8 + h) * 2], a);
-        tail::emit_partial<SEG>(p, session, split, num_splits, kv_head * G + h, dim, a, tot_s[2 * h] * 0.6931471805599453f, tot_s[2 * h + 1]);
+        for (int w = 0; w < WARPS; ++w) {
+            const float2 x = *reinterpret_cast<const float2*>(smem + P::kOffRing + w * (P::kUnits * P::kSlot) + (h * P::kOutStride + dim) * 4);
+            const float f = ml_s[(w * 8 + h) * 2];
+            a.x = fmaf(x.x, f, a.x); a.y = fmaf(x.y, f, a.y);
+        }
+        tail::emit_partial2<SEG>(p, session, split, num_splits, kv_head * G + h, dim, a, tot_s[2 * h] * 0.6931471805599453f, tot_s[2 * h + 1]);
     }
     if (p.ws_tagged == nullptr) return;           // a separate merge kernel follows
     __syncthreads();

@@ -152,6 +152,24 @@ __device__ __forceinline__ void emit_partial(const DecodeParams& p, uint32_t ses
         if (dim == 0) { p.ws_m[slot_idx] = m_nat; p.ws_l[slot_idx] = lt; }
     }
 }
+// The same for dims `dim` and `dim + 1` of a launch whose threads hold pairs (dim even).
+__device__ __forceinline__ void st_tagged2(uint64_t* dst, float a, float b, uint32_t tag) {   // each 8-byte half is indivisible
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1,%2};" ::"l"(dst), "l"(tagged_word(a, tag)), "l"(tagged_word(b, tag)) : "memory");
+}
+template <int SEG>
+__device__ __forceinline__ void emit_partial2(const DecodeParams& p, uint32_t session, uint32_t split, uint32_t num_splits,
+                                              uint32_t head, int dim, float2 at, float m_nat, float lt) {
+    if (p.ws_tagged == nullptr || (num_splits == 1 && p.fuse.xchg.world <= 1)) {
+        emit_partial<SEG>(p, session, split, num_splits, head, dim, at.x, m_nat, lt);
+        emit_partial<SEG>(p, session, split, num_splits, head, dim + 1, at.y, m_nat, lt);
+        return;
+    }
+    const size_t slot_idx = (static_cast<size_t>(session) * p.num_splits + split) * p.query_heads + head;
+    const int seg = SEG == 1 ? 0 : dim / kSegDims, in_seg = SEG == 1 ? dim : dim % kSegDims;
+    uint64_t* dst = p.ws_tagged + (slot_idx * SEG + seg) * kSegWords;
+    st_tagged2(dst + in_seg, at.x, at.y, p.tag);
+    if (in_seg == 0) st_tagged2(dst + kSegDims, m_nat, lt, p.tag);
+}
 // True when emit_partial wrote final results or plain partials, i.e. no in-launch merge follows for this CTA's work.
 __device__ __forceinline__ bool merge_not_needed(const DecodeParams& p, uint32_t num_splits) {
     return p.ws_tagged == nullptr || (num_splits == 1 && p.fuse.xchg.world <= 1);
@@ -232,9 +250,13 @@ __device__ __forceinline__ void exchange_partials(const DecodeParams& p, uint32_
 // re-quantisation of the gated output the reference's stage 2 offers for the projection that follows
 // (.hip:2354-2383: blocks of 32, d = amax/127, q = roundf(x/d) clamped to +-127, s = d * sum(q), both fp16).
 template <int SEG>
+__device__ __forceinline__ size_t merged_index(const MergeParams& f, uint32_t session, uint32_t head, int seg, int pr) {
+    return ((static_cast<size_t>(session) * f.query_heads + head) * SEG + seg) * kSegDims + 2 * pr;
+}
+template <int SEG>
 __device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t session, uint32_t head, int seg, int pr, float2 tot, float gsum,
-                                             float m_merged) {
-    const size_t out_idx = ((static_cast<size_t>(session) * f.query_heads + head) * SEG + seg) * kSegDims + 2 * pr;
+                                             float m_merged, float2 gt) {
+    const size_t out_idx = merged_index<SEG>(f, session, head, seg, pr);
     if (f.out_m != nullptr) {   // sequence shard: one merged, unnormalised partial
         *reinterpret_cast<float2*>(f.out_acc + out_idx) = tot;
         if (pr == 0 && seg == 0) {
@@ -248,7 +270,6 @@ __device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t sess
     if (f.output != nullptr) *reinterpret_cast<float2*>(f.output + out_idx) = o;
     if (f.gated_output != nullptr || f.gated_output_q8 != nullptr) {
         if (f.gate != nullptr) {
-            const float2 gt = *reinterpret_cast<const float2*>(f.gate + out_idx);
             o.x *= 1.0f / (1.0f + __expf(-gt.x)); o.y *= 1.0f / (1.0f + __expf(-gt.y));
         }
         if (f.gated_output != nullptr) *reinterpret_cast<float2*>(f.gated_output + out_idx) = o;
@@ -304,6 +325,10 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
         const int seg = static_cast<int>(u0 % SEG);
         const size_t stride = static_cast<size_t>(p.query_heads) * SEG * kSegWords;   // words between consecutive splits
         uint64_t* base = p.ws_tagged + ((static_cast<size_t>(session) * p.num_splits * p.query_heads + head) * SEG + seg) * kSegWords;
+        // the gate is fetched ahead of the polls: behind them its trip to L2 was the last thing the launch waited for
+        float2 gate = make_float2(0.0f, 0.0f);
+        if (grp == 0 && p.fuse.gate != nullptr && p.fuse.out_m == nullptr)
+            gate = *reinterpret_cast<const float2*>(p.fuse.gate + merged_index<SEG>(p.fuse, session, head, seg, pr));
         bool lost = false;
         float2 tot = make_float2(0.0f, 0.0f);
         float Mg = -INFINITY, lg = 0.0f;
@@ -397,7 +422,7 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
             if constexpr (SEG == 1) {   // the cross-GPU exchange is the 128-dim kernels'
                 if (p.fuse.xchg.world > 1) exchange_partials(p, head, pr, m_merged, tot, gsum, lost);
             }
-            write_merged<SEG>(p.fuse, session, head, seg, pr, tot, gsum, m_merged);
+            write_merged<SEG>(p.fuse, session, head, seg, pr, tot, gsum, m_merged, gate);
         }
         asm volatile("bar.sync 2, %0;" ::"n"(THREADS) : "memory");   // the fold area is reused by the next head of this CTA
     }

@@ -194,9 +194,9 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
 
     // ---- this CTA's tiles (tiles are aligned to multiples of 128 positions of the cache) --------------------
     const uint32_t tile_begin = begin / kTileM, tile_end = (end + kTileM - 1) / kTileM;
-    const uint64_t total_tiles = end > begin ? tile_end - tile_begin : 0;
-    const uint32_t t0 = tile_begin + static_cast<uint32_t>(total_tiles * split / num_splits);
-    const uint32_t t1 = tile_begin + static_cast<uint32_t>(total_tiles * (split + 1) / num_splits);
+    const uint32_t total_tiles = end > begin ? tile_end - tile_begin : 0;
+    const uint32_t t0 = tile_begin + part_begin(total_tiles, split, num_splits);
+    const uint32_t t1 = tile_begin + part_begin(total_tiles, split + 1, num_splits);
     const int ntiles = static_cast<int>(t1 - t0);
     const bool fuse = tail::appends_row(p, begin, end);
     const bool owner = fuse && ntiles > 0 && t1 == tile_end;   // this CTA holds the tile of the appended token

@@ -158,9 +158,9 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
 
     // ---- this CTA's tiles (tiles are aligned to multiples of 128 positions of the cache) --------------------
     const uint32_t tile_begin = begin / kTileM, tile_end = (end + kTileM - 1) / kTileM;
-    const uint64_t total_tiles = end > begin ? tile_end - tile_begin : 0;
-    const uint32_t t0 = tile_begin + static_cast<uint32_t>(total_tiles * split / num_splits);
-    const uint32_t t1 = tile_begin + static_cast<uint32_t>(total_tiles * (split + 1) / num_splits);
+    const uint32_t total_tiles = end > begin ? tile_end - tile_begin : 0;
+    const uint32_t t0 = tile_begin + part_begin(total_tiles, split, num_splits);
+    const uint32_t t1 = tile_begin + part_begin(total_tiles, split + 1, num_splits);
     const int ntiles = static_cast<int>(t1 - t0);
     // With launch overlap the previous kernel may still be appending: rows at or above early_end wait for it.
     // The row that this launch appends does not count: the copy of it that comes with its tile is overwritten in shared memory.
