@@ -157,7 +157,16 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     }
     // this CTA's positions: whole tiles counted from `begin`
     const uint32_t tiles = (end - begin) / kTile + ((end - begin) % kTile != 0);
-    const uint32_t t0 = part_begin(tiles, split, num_splits), t1 = part_begin(tiles, split + 1, num_splits);
+    // One session's last splits hold a round of tiles (one per warp) less than the others: as many CTAs as the launch before has mergers find
+    // an SM only when those leave, 1 to 2 us behind the others, and the merge waits for the slowest.  From about two rounds per CTA on: below
+    // (and with a short kernel between two launches, which lets the mergers leave) the longer splits' extra round costs as much.  fp16 cache, us a
+    // layer: 24 / 4 heads of 256, 12000 positions 13.5 -> 12.5, 30000 24.1 -> 23.5; 32 / 8 heads of 128, 5000 9.1 -> 8.0, 10000 11.6 -> 10.5;
+    // without the line, 4000 positions of the first went from 9.0 to 9.7 and 6001 behind a query-side kernel from 12.2 to 12.5.
+    const uint32_t mergers = G * SEG, late = p.lengths == nullptr && num_splits > 2 * mergers ? mergers : 0u, padded = tiles + late * WARPS;
+    const bool uneven = late > 0 && padded >= (2 * WARPS + 2) * num_splits;
+    const uint32_t parted = uneven ? padded : tiles;
+    auto begin_of = [&](uint32_t i) { return part_begin(parted, i, num_splits) - (uneven && i + late > num_splits ? (i + late - num_splits) * WARPS : 0u); };
+    const uint32_t t0 = begin_of(split), t1 = begin_of(split + 1);
     const uint32_t pos0 = begin + t0 * kTile;
     const int my_tiles = static_cast<int>((t1 - t0 + WARPS - 1 - warp) / WARPS);   // tiles of this warp
 

@@ -112,6 +112,27 @@ def test_error_of_fp16_caches_is_that_of_fp32_sums(cuda, d, H, Hq, L, splits, bo
     assert rel <= bound, rel
 
 
+# One session's last splits get a round of tiles less from (2 x 8 + 2) x splits tiles (one session's mergers x 8 counted in) on: both sides of that
+# line, a ragged last tile, an explicit number of splits, the append in the last (shorter) split; fp16 caches, so fp32 sums
+@pytest.mark.parametrize("d,H,Hq,L,splits", [(128, 8, 32, 4656, 0), (128, 8, 32, 4657, 0), (128, 8, 32, 4700, 0), (256, 4, 24, 9104, 0), (256, 4, 24, 9105, 0),
+                                             (128, 8, 32, 2064, 9), (128, 8, 32, 2065, 9), (128, 8, 32, 2065, 8), (128, 1, 1, 40000, 0)])
+def test_shorter_last_splits(cuda, d, H, Hq, L, splits):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(L)
+    st = kv.AttentionLayerKvCacheStorage(L + 3, kv.KvCacheQuantMode.kFp16Fp16, kv_heads=H, head_dim=d, qblock=d)
+    k, v = (torch.randn(L, H * d, generator=g, device="cuda").half() for _ in range(2))
+    q, ws = torch.randn(Hq, d, generator=g, device="cuda").half(), kv.decode_workspace(Hq, d)
+    out, stepped = (torch.full((Hq, d), float("nan"), device="cuda") for _ in range(2))
+    kv.launch_kv_store_quant(st.view(), k[:-1], v[:-1], None, L - 1, 0, rope_mode=kv.RopeMode.NONE)
+    kv.launch_decode_step(st.view(), k[-1], v[-1], q, query_heads=Hq, scale=d ** -0.5, rope_mode=kv.RopeMode.NONE, output=stepped, workspace=ws,
+                          position=L - 1, num_splits=splits)
+    kv.launch_decode_attention_quant(st.view(), q, query_heads=Hq, scale=d ** -0.5, cache_length=L, output=out, workspace=ws, num_splits=splits)
+    K, V = (x.double().view(L, H, 1, d).expand(L, H, Hq // H, d).reshape(L, Hq, d) for x in (k, v))
+    ref = torch.einsum("hl,lhd->hd", (torch.einsum("hd,lhd->hl", q.double(), K) * d ** -0.5).softmax(-1), V)
+    for o in (stepped, out):
+        assert torch.isfinite(o).all() and ((o.double() - ref).norm() / ref.norm()).item() <= REL
+
+
 @pytest.mark.parametrize("poison", [float("nan"), 3.0])
 def test_separate_merge_reads_only_what_its_launch_wrote(cuda, poison):
     """More splits than fit on the device with their merge: the merge kernel follows, and reads all splits of all sessions.  What an
