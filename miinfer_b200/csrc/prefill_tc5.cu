@@ -13,8 +13,8 @@
 //         tensor copies (64x64 boxes, 128-byte swizzle: exactly the canonical shared-memory layout of the MMA
 //         operands; the two tiles of a pair lie in rows 0-63 and 64-127 of every slab, one B operand);
 //       - one thread issues S = Q.K^T for a pair of tiles at once (tcgen05.mma M128 x N128, K = d, Q read from
-//         TMEM: an MMA of this shape costs about the same at N = 64 and N = 128, so pairs halve the time the score
-//         MMAs hold the tensor pipe), another O += P.V per tile (M128 x N = d, K = 64; V consumed MN-major, as
+//         TMEM: issuing such an MMA takes this thread 50 to 100 clocks, the tensor pipe 32 at N = 64 and 64 at N = 128, so
+//         pairs keep the issue out of the pipe's way), another O += P.V per tile (M128 x N = d, K = 64; V consumed MN-major, as
 //         stored) into the O accumulator in TMEM; completion is tracked by tcgen05.commit on mbarriers;
 //       - two groups of 128 softmax threads, one thread per row in each, take the first and the second tile of
 //         every pair: tcgen05.ld the S row, scale/mask (causal length per row, .hip:6829), online softmax in base
@@ -332,8 +332,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     } else if (warp == kSWarp) {
         // =============================== S = Q.K^T issuer ===============================
         // One chain of D/16 MMAs per PAIR of tiles (N = 128: the first tile's scores land in S columns 0-63, the second
-        // one's in 64-127).  An MMA instruction of this shape costs about 90 clocks whatever its N up to 128, so a
-        // pair costs what a single tile would.
+        // one's in 64-127): half as many instructions to issue as tile by tile.
         if (lane == 0) {
             constexpr uint32_t idesc_pair = umma_idesc(kBM, 2 * kBN, 0, 0), idesc_one = umma_idesc(kBM, kBN, 0, 0);
             const bool have_q = mbar_wait(bar(Q_FULL), 0);
