@@ -175,6 +175,8 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     const bool tagged_fit = plain_offset >= slots * partial_floats(geometry.head_dim) * sizeof(uint64_t);
     p.num_splits = num_splits;
     p.fuse = merge;
+    // the merge inside a launch fetches the gate ahead of its polls: not where nothing gated is asked for, so that nothing need lie there
+    if (merge.gated_output == nullptr && merge.gated_output_q8 == nullptr) p.fuse.gate = nullptr;
     p.ws_m = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + plain_offset);
     p.ws_l = p.ws_m + slots;
     p.ws_acc = p.ws_l + slots;

@@ -246,13 +246,15 @@ __device__ __forceinline__ void exchange_partials(const DecodeParams& p, uint32_
         for (uint32_t w = 0; w < x.world; ++w) zero2(in + w * words_per_rank + kD);
 }
 
-// Normalise, gate and store the merged result of one head (64 threads, two dims each), with the optional Q8_1
-// re-quantisation of the gated output the reference's stage 2 offers for the projection that follows
-// (.hip:2354-2383: blocks of 32, d = amax/127, q = roundf(x/d) clamped to +-127, s = d * sum(q), both fp16).
+// Where a merged result's dims 2 pr and 2 pr + 1 of a segment lie in the gate and in the outputs.
 template <int SEG>
 __device__ __forceinline__ size_t merged_index(const MergeParams& f, uint32_t session, uint32_t head, int seg, int pr) {
     return ((static_cast<size_t>(session) * f.query_heads + head) * SEG + seg) * kSegDims + 2 * pr;
 }
+// Normalise, gate and store the merged result of one head (64 threads, two dims each), with the optional Q8_1
+// re-quantisation of the gated output the reference's stage 2 offers for the projection that follows
+// (.hip:2354-2383: blocks of 32, d = amax/127, q = roundf(x/d) clamped to +-127, s = d * sum(q), both fp16).
+// `gt`: the gate's two values, which the caller has read where f.gate is set and out_m is not; without a gate it is not looked at.
 template <int SEG>
 __device__ __forceinline__ void write_merged(const MergeParams& f, uint32_t session, uint32_t head, int seg, int pr, float2 tot, float gsum,
                                              float m_merged, float2 gt) {
@@ -325,7 +327,8 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
         const int seg = static_cast<int>(u0 % SEG);
         const size_t stride = static_cast<size_t>(p.query_heads) * SEG * kSegWords;   // words between consecutive splits
         uint64_t* base = p.ws_tagged + ((static_cast<size_t>(session) * p.num_splits * p.query_heads + head) * SEG + seg) * kSegWords;
-        // the gate is fetched ahead of the polls: behind them its trip to L2 was the last thing the launch waited for
+        // the gate (set only where something gated is asked for) is fetched ahead of the polls: behind them its trip to L2 was the last
+        // thing the launch waited for
         float2 gate = make_float2(0.0f, 0.0f);
         if (grp == 0 && p.fuse.gate != nullptr && p.fuse.out_m == nullptr)
             gate = *reinterpret_cast<const float2*>(p.fuse.gate + merged_index<SEG>(p.fuse, session, head, seg, pr));

@@ -94,19 +94,44 @@ def captured_node_types(call):
     return [kind.value for node in nodes if cu.cuGraphNodeGetType(node, C.byref(kind)) == 0]
 
 
+def _captured_kernel_nodes(call):
+    import ctypes as C
+
+    class KernelNode(C.Structure):   # CUDA_KERNEL_NODE_PARAMS_v2
+        _fields_ = [("func", C.c_void_p), ("dims", C.c_uint * 7), ("params", C.POINTER(C.c_void_p)), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+    graph, cu, nodes = _captured_nodes(call)
+    kernels = []
+    for node in nodes:
+        k = KernelNode()
+        assert cu.cuGraphKernelNodeGetParams_v2(node, C.byref(k)) == 0
+        kernels.append(k)
+    return graph, cu, kernels
+
+
 def captured_kernels(call):
     """Mangled names of the kernels that `call(stream)` captures; nothing runs."""
     import ctypes as C
 
-    class KernelNode(C.Structure):   # CUDA_KERNEL_NODE_PARAMS_v2
-        _fields_ = [("func", C.c_void_p), ("dims", C.c_uint * 7), ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
-
-    graph, cu, nodes = _captured_nodes(call)
+    graph, cu, kernels = _captured_kernel_nodes(call)
     names = []
-    for node in nodes:
-        k, name = KernelNode(), C.c_char_p()
-        assert cu.cuGraphKernelNodeGetParams_v2(node, C.byref(k)) == 0
+    for k in kernels:
+        name = C.c_char_p()
         rc = cu.cuFuncGetName(C.byref(name), C.c_void_p(k.func)) if k.func else cu.cuKernelGetName(C.byref(name), C.c_void_p(k.kern))
         assert rc == 0
         names.append(name.value.decode())
     return names
+
+
+def captured_parameter_blocks(call):
+    """The first parameter, as bytes, of every kernel that `call(stream)` captures; nothing runs."""
+    import ctypes as C
+
+    graph, cu, kernels = _captured_kernel_nodes(call)
+    blocks = []
+    for k in kernels:
+        offset, size = C.c_size_t(), C.c_size_t()
+        info, handle = (cu.cuFuncGetParamInfo, k.func) if k.func else (cu.cuKernelGetParamInfo, k.kern)
+        assert info(C.c_void_p(handle), C.c_size_t(0), C.byref(offset), C.byref(size)) == 0
+        blocks.append(C.string_at(k.params[0], size.value))
+    return blocks

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import kvoracle as ko
-from gpu_util import assert_planes_equal, to_dev, upload
+from gpu_util import assert_planes_equal, captured_parameter_blocks, to_dev, upload
 from miinfer_b200 import kv
 
 pytestmark = pytest.mark.gpu
@@ -300,3 +300,28 @@ def test_the_separate_merge_can_be_asked_for(cuda, d, H, Hq, qb, mode):
                 err = np.linalg.norm(got[i].cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref)
                 assert err <= 2e-4, (splits, n, err)
     assert bool((tagged == 171).all())
+
+
+@pytest.mark.parametrize("d,H,Hq,mode,splits,path", [(128, 8, 32, 0, 3, 0), (256, 4, 24, 0, 3, 0), (256, 4, 24, 3, 3, 0), (128, 8, 32, 3, 3, 0), (128, 8, 32, 3, 3, 1)])
+def test_a_launch_that_writes_nothing_gated_is_given_no_gate(cuda, d, H, Hq, mode, splits, path):
+    """What a launch does not get it cannot read: the gate's address is in the parameters of launches with a gated output and of no others (only captured)."""
+    L = 1504
+    st = kv.AttentionLayerKvCacheStorage(L, kv.KvCacheQuantMode(mode), kv_heads=H, head_dim=d, qblock=32 if mode else d)
+    q, k = torch.zeros(2, Hq, d, device="cuda", dtype=torch.float16), torch.zeros(1, H * d, device="cuda", dtype=torch.float16)
+    gate, out, ws = torch.zeros(2, Hq, d, device="cuda"), torch.zeros(2, Hq, d, device="cuda"), kv.decode_workspace(Hq, d, 2)
+    table, lengths, views = kv.view_table(2), torch.tensor([L, 300], dtype=torch.int32, device="cuda"), [st.view(), st.view()]
+    common = dict(query_heads=Hq, scale=d ** -0.5, gate=gate, workspace=ws, num_splits=splits)
+    kv.set_decode_kernel(path)
+    try:
+        kv.launch_decode_attention_batched(views, table, lengths, L, q, output=out, **common)   # fills the table
+        torch.cuda.synchronize()
+        calls = [lambda **o: kv.launch_decode_attention_quant(st.view(), q[0], cache_length=L, **common, **o),
+                 lambda **o: kv.launch_decode_step(st.view(), k, k, q[0], position=L - 1, **common, **o),
+                 lambda **o: kv.launch_decode_attention_batched(None, table, lengths, L, q, **common, **o)]
+        for call in calls:
+            for outputs, wanted in ((dict(output=out), False), (dict(gated_output=out), True)):
+                blocks = captured_parameter_blocks(lambda stream: call(**outputs))
+                assert len(blocks) == 1   # the merge is inside
+                assert (gate.data_ptr().to_bytes(8, "little") in blocks[0]) == wanted
+    finally:
+        kv.set_decode_kernel(0)
