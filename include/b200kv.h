@@ -159,8 +159,11 @@ B200KV_API int b200kv_device_check(int device);
  * Device-side state
  * (decode_state, lengths) is read early, so it must not be written by a kernel
  * that itself triggers dependents early; kernels of this library never do, and
- * an ordinary kernel between two launches acts as a full barrier.  0 turns the
- * overlap off again. */
+ * an ordinary kernel between two launches acts as a full barrier.  The splits
+ * of a single session's decode launch of several thousand positions may be cut
+ * differently with overlap on than with it off (the last ones shorter), so
+ * that outputs then agree to fp32 rounding and not to the bit; cache rows are the
+ * same bits.  0 turns the overlap off again. */
 B200KV_API int b200kv_set_launch_overlap(uint32_t tail_positions);
 
 /* Registers a 4-byte-aligned DEVICE word (on the current device; NULL = none, the default) into which every later

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "kv_common.cuh"
+#include "split_bounds.h"
 
 #include <cuda.h>  // CUtensorMap and its enums only; the encoder is fetched at run time, libcuda is not linked
 
@@ -95,6 +96,7 @@ struct DecodeParams {
     float sectioned_step;
     float inv_freq[128];                     // NeoX frequencies, head_dim / 2 of them
     uint32_t overlap_tail;                   // launch overlap: the last n positions of the range are read only after pdl_wait
+    uint32_t late_splits;                    // decode_stream.cu, one session: splits per kv head that start behind the mergers of the launch before
     uint32_t head_fastest;                   // tcgen05 kernel: grid is (kv heads, splits, sessions) instead of (splits, kv heads, sessions)
     uint64_t* ws_tagged;
     uint32_t tag;                            // tag of this launch's words in ws_tagged (never 0; differs from the previous launch's)
@@ -137,13 +139,6 @@ __device__ __forceinline__ void resolve_range(const DecodeParams& p, uint32_t se
     if (length > view.capacity) length = static_cast<uint32_t>(view.capacity);
     *end = length;
     *begin = p.range_begin < length ? p.range_begin : length;
-}
-
-// The first of `total` tiles that belongs to part `i` of `parts` (i <= parts <= kMaxSplitsPerSession): floor(total * i / parts), a product that
-// does not fit 32 bits, from 32-bit divisions.
-__device__ __forceinline__ uint32_t part_begin(uint32_t total, uint32_t i, uint32_t parts) {
-    const uint32_t q = total / parts, r = total - q * parts;
-    return q * i + r * i / parts;
 }
 
 __device__ __forceinline__ const b200kv_view& session_view(const DecodeParams& p, uint32_t session) {

@@ -157,16 +157,8 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     }
     // this CTA's positions: whole tiles counted from `begin`
     const uint32_t tiles = (end - begin) / kTile + ((end - begin) % kTile != 0);
-    // One session's last splits hold a round of tiles (one per warp) less than the others: as many CTAs as the launch before has mergers find
-    // an SM only when those leave, 1 to 2 us behind the others, and the merge waits for the slowest.  From about two rounds per CTA on: below
-    // (and with a short kernel between two launches, which lets the mergers leave) the longer splits' extra round costs as much.  fp16 cache, us a
-    // layer: 24 / 4 heads of 256, 12000 positions 13.5 -> 12.5, 30000 24.1 -> 23.5; 32 / 8 heads of 128, 5000 9.1 -> 8.0, 10000 11.6 -> 10.5;
-    // without the line, 4000 positions of the first went from 9.0 to 9.7 and 6001 behind a query-side kernel from 12.2 to 12.5.
-    const uint32_t mergers = G * SEG, late = p.lengths == nullptr && num_splits > 2 * mergers ? mergers : 0u, padded = tiles + late * WARPS;
-    const bool uneven = late > 0 && padded >= (2 * WARPS + 2) * num_splits;
-    const uint32_t parted = uneven ? padded : tiles;
-    auto begin_of = [&](uint32_t i) { return part_begin(parted, i, num_splits) - (uneven && i + late > num_splits ? (i + late - num_splits) * WARPS : 0u); };
-    const uint32_t t0 = begin_of(split), t1 = begin_of(split + 1);
+    const TileRange range = split_tiles<WARPS>(tiles, split, num_splits, p.late_splits);
+    const uint32_t t0 = range.begin, t1 = range.end;
     const uint32_t pos0 = begin + t0 * kTile;
     const int my_tiles = static_cast<int>((t1 - t0 + WARPS - 1 - warp) / WARPS);   // tiles of this warp
 
@@ -662,7 +654,7 @@ int launch_one(const DecodeParams& p, bool hold, dim3 grid, cudaStream_t s) {
 template <int D, int WARPS>
 int launch_mode(const DecodeParams& p, const b200kv_view& g, dim3 grid, cudaStream_t s) {
     const bool blocks = g.qblock == 32;
-    const bool hold = p.split_positions / kTile > static_cast<uint32_t>(kLongTiles * WARPS);   // positions a split may have, over its warps
+    const bool hold = p.split_positions / kTile > static_cast<uint32_t>(kLongTiles * WARPS);   // positions a split may have, over its warps (shorter last splits give no warp more tiles)
     switch (g.quant_mode) {
         case B200KV_F16_F16: return launch_one<D, F16, F16, WARPS>(p, hold, grid, s);
         case B200KV_Q8_F16: return blocks ? launch_one<D, BLOCK, F16, WARPS>(p, hold, grid, s) : launch_one<D, ROW, F16, WARPS>(p, hold, grid, s);
@@ -713,6 +705,14 @@ int launch_decode_stream(const DecodeParams& p_in, const b200kv_view& geometry, 
     if (p.split_positions < 128u) p.split_positions = 128u;
     const bool many = many_sessions(p);
     p.head_fastest = many ? 0u : 1u;
+    // One session under launch overlap: as many CTAs as the launch before has mergers find an SM only when those leave, 1 to 2 us behind the others, and
+    // the merge waits for the slowest; their splits hold a round of tiles less where that costs the others none (split_bounds.h).  Step, fp16 cache, us a
+    // layer, even -> shorter last splits, launches back to back: 32 / 8 heads of 128, 5000 positions 9.1 -> 8.15, 10000 11.6 -> 10.7, 30000 22.4 ->
+    // 22.05; 24 / 4 heads of 256, 10000 13.05 -> 11.6, 20000 18.25 -> 17.1, 30000 24.15 -> 23.25.  Nobody is late behind a kernel that does not let its
+    // dependents in early, which a launch cannot know: there the longer splits cost 0 to 1.8 % (10000: 15.55 -> 15.8 and 16.75 -> 16.95).  Without the
+    // rule's rounds (13000 positions of the second, 6600 of the first) they cost 3 to 5 % there and without overlap.
+    const uint32_t mergers = p.query_heads / geometry.kv_heads * (geometry.head_dim / 128u);
+    p.late_splits = many ? 0u : late_splits(p.overlap_tail > 0, p.ws_tagged != nullptr, geometry.kv_heads, p.num_splits, mergers, device_sms());
     const dim3 grid = many ? dim3(p.num_splits, geometry.kv_heads, p.sessions) : dim3(geometry.kv_heads, p.num_splits, 1);
     if (geometry.head_dim == 128) return many ? launch_mode<128, 4>(p, geometry, grid, stream) : launch_mode<128, 8>(p, geometry, grid, stream);
     return many ? launch_mode<256, 4>(p, geometry, grid, stream) : launch_mode<256, 8>(p, geometry, grid, stream);

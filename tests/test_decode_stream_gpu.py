@@ -112,8 +112,8 @@ def test_error_of_fp16_caches_is_that_of_fp32_sums(cuda, d, H, Hq, L, splits, bo
     assert rel <= bound, rel
 
 
-# One session's last splits get a round of tiles less from (2 x 8 + 2) x splits tiles (one session's mergers x 8 counted in) on: both sides of that
-# line, a ragged last tile, an explicit number of splits, the append in the last (shorter) split; fp16 caches, so fp32 sums
+# Either side of lengths at which the longest split goes into another round of tiles, a ragged last tile, an explicit number of splits, the append in the
+# last split; fp16 caches, so fp32 sums
 @pytest.mark.parametrize("d,H,Hq,L,splits", [(128, 8, 32, 4656, 0), (128, 8, 32, 4657, 0), (128, 8, 32, 4700, 0), (256, 4, 24, 9104, 0), (256, 4, 24, 9105, 0),
                                              (128, 8, 32, 2064, 9), (128, 8, 32, 2065, 9), (128, 8, 32, 2065, 8), (128, 1, 1, 40000, 0)])
 def test_shorter_last_splits(cuda, d, H, Hq, L, splits):
@@ -131,6 +131,57 @@ def test_shorter_last_splits(cuda, d, H, Hq, L, splits):
     ref = torch.einsum("hl,lhd->hd", (torch.einsum("hd,lhd->hl", q.double(), K) * d ** -0.5).softmax(-1), V)
     for o in (stepped, out):
         assert torch.isfinite(o).all() and ((o.double() - ref).norm() / ref.norm()).item() <= REL
+
+
+# steps from just below to just above the length from which, under launch overlap, one session's last splits are a round of tiles shorter
+# (csrc/split_bounds.h: three rounds of 8 x 16 positions per split, 18 and 37 splits)
+@pytest.mark.parametrize("d,H,Hq,qb,mode,line", [(128, 8, 32, 128, 0, 4608), (128, 8, 32, 32, 3, 4608), (128, 8, 32, 128, 1, 4608), (256, 4, 24, 256, 3, 9472),
+                                                 (256, 4, 24, 32, 2, 9472)])
+def test_overlapped_steps_whose_last_splits_are_shorter(cuda, d, H, Hq, qb, mode, line):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d + mode)
+    below, steps = 3, 8
+    L0 = line - below
+    k, v = (torch.randn(L0 + steps, H * d, generator=g, device="cuda").half() for _ in range(2))
+    q = torch.randn(steps, Hq, d, generator=g, device="cuda").half()
+    states = [kv.make_decode_state(L0 + i) for i in range(steps)]
+    results = []
+    try:
+        for overlap in (0, 1):
+            kv.set_launch_overlap(overlap)
+            st = kv.AttentionLayerKvCacheStorage(line + 500, kv.KvCacheQuantMode(mode), kv_heads=H, head_dim=d, qblock=qb)
+            ws, out = kv.decode_workspace(Hq, d), torch.full((steps, Hq, d), float("nan"), device="cuda")
+            m, l, acc = (torch.empty(*shape, device="cuda") for shape in ((Hq,), (Hq,), (Hq, d)))
+            kv.launch_kv_store_quant(st.view(), k[:L0], v[:L0], None, L0, 0, rope_mode=kv.RopeMode.NONE)
+            torch.cuda.synchronize()
+            for i in range(steps):   # back to back: copies of step i + 1 start while step i merges
+                kv.launch_decode_step(st.view(), k[L0 + i:L0 + i + 1], v[L0 + i:L0 + i + 1], q[i], query_heads=Hq, scale=d ** -0.5, rope_mode=kv.RopeMode.NONE,
+                                      output=out[i], workspace=ws, num_splits=kv.FORCE_GENERIC, decode_state=states[i])
+            kv.launch_decode_partials(st.view(), q[0], query_heads=Hq, scale=d ** -0.5, range_begin=2, range_end=line + 4, part_m=m, part_l=l, part_acc=acc,
+                                      workspace=ws, num_splits=kv.FORCE_GENERIC)
+            torch.cuda.synchronize()
+            results.append((out.double(), (acc / l[:, None]).double(), st.planes()))
+    finally:
+        kv.set_launch_overlap(0)
+    (out0, part0, planes0), (out1, part1, planes1) = results
+    assert all(torch.equal(a, b) for a, b in zip(planes0, planes1))
+    assert torch.equal(out0[:below], out1[:below]) and not torch.equal(out0[below:], out1[below:])   # even splits on both sides, then not
+    for a, b in ((out0, out1), (part0, part1)):
+        assert torch.isfinite(b).all() and ((a - b).norm() / a.norm()).item() <= REL
+    # the steps without overlap against float64 over the cache as it lies
+    K, V = (_plane(st, side, line + 1) for side in ("key", "value"))
+    s = torch.einsum("hgd,hld->hgl", q[below].double().view(H, Hq // H, d), K) * d ** -0.5
+    ref = torch.einsum("hgl,hld->hgd", s.softmax(-1), V).reshape(Hq, d)
+    assert ((out1[below] - ref).norm() / ref.norm()).item() <= REL
+
+
+def _plane(st, side, length):
+    """A side's first rows as the cache holds them, in float64: [kv heads][length][head_dim]."""
+    q8 = getattr(st, f"{side}_cache_q8")
+    if q8 is None:
+        return getattr(st, f"{side}_cache")[:, :length].double()
+    scales = getattr(st, f"{side}_scales")[:, :length].double()
+    return (q8[:, :length].double().unflatten(-1, (scales.shape[-1], -1)) * scales.unsqueeze(-1)).flatten(-2)
 
 
 @pytest.mark.parametrize("poison", [float("nan"), 3.0])
