@@ -111,3 +111,35 @@ def test_decode_state_advance_matches_the_reference_bookkeeping(cuda):
         assert np.array_equal(state_dev.cpu().numpy().view(np.uint32), state_host)
         assert np.array_equal(out_dev.cpu().numpy().view(np.uint32), out_host)
     assert state_host[1] == 108 and state_host[2] == 8 and state_host[3] == 1
+
+
+@pytest.mark.parametrize("d,Hq,H,rope", [(256, 24, 4, 2), (128, 32, 8, 1)])
+@pytest.mark.parametrize("tokens_on_device", [True, False])
+def test_query_side_behind_the_kernel_that_writes_its_input(cuda, d, Hq, H, rope, tokens_on_device):
+    """With launch overlap on, the kernel asks for the projection's lines before the kernel in front of it has written them: what it then uses has to
+    be what was written.  A decode launch writes the projection, the query side takes it apart, and its query goes into the next decode launch."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d)
+    L, steps = 700, 40
+    k, v = (torch.randn(L, H * d, generator=g, device="cuda").half() for _ in range(2))
+    q0 = torch.randn(Hq, d, generator=g, device="cuda")
+    st, ws, state = kv.AttentionLayerKvCacheStorage(L, kv.KvCacheQuantMode.kFp16Fp16, kv_heads=H, head_dim=d, qblock=d), kv.decode_workspace(Hq, d), kv.make_decode_state(123)
+    kv.launch_kv_store_quant(st.view(), k, v, None, L, 0, rope_mode=kv.RopeMode.NONE)
+    results = []
+    try:
+        for overlap in (0, 1):
+            kv.set_launch_overlap(overlap)
+            q, projection = q0.clone(), torch.zeros(Hq, d, device="cuda")   # one of half as many heads: [Hq / 2][q | gate]
+            gate, kept = torch.zeros(Hq // 2, d, device="cuda"), torch.zeros(steps, 2, Hq // 2, d, device="cuda")
+            torch.cuda.synchronize()
+            for i in range(steps):
+                kv.launch_decode_attention_quant(st.view(), q, query_heads=Hq, scale=d ** -0.5, cache_length=L - i, output=projection, workspace=ws)
+                where = dict(decode_state=state) if tokens_on_device else {}
+                kv.launch_q_split_norm_rope(projection, None, q[:Hq // 2], gate, 1, 123, heads=Hq // 2, head_dim=d, rope_mode=kv.RopeMode(rope), **where)
+                kv.launch_q_split_norm_rope(projection, None, kept[i, 0], kept[i, 1], 1, 123, heads=Hq // 2, head_dim=d, rope_mode=kv.RopeMode(rope), **where)
+            torch.cuda.synchronize()
+            results.append(kept)
+    finally:
+        kv.set_launch_overlap(0)
+    assert torch.isfinite(results[0]).all() and results[0].abs().max() > 0
+    assert torch.equal(*results)
