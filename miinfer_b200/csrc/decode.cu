@@ -118,10 +118,13 @@ int launch_merge(const MergeParams& p, uint32_t groups, cudaStream_t stream) {
     return B200KV_OK;
 }
 
-// max_length x kv heads up to which a single session takes the mma.sync kernel.  Measured (decode step, q8_0, us): 8 kv heads of
-// 128 dims: 6.5 against 8.2 at 1500 positions, 8.3 / 8.5 at 3000, 8.8 / 8.7 at 4096, 9.6 / 9.1 at 6000; 4 kv heads of 256 dims: 7.9 /
-// 12.7 at 1500, 9.7 / 10.3 at 4096, 11.4 / 11.4 at 7777, 14.0 / 13.1 at 12000 (one scale per row: 12.8 / 12.6 there).  The lines lie where
-// the two are level within the runs' spread; other head counts were not measured and go by the rows, which is what fills the device.
+// max_length x kv heads up to which a single session takes the mma.sync kernel.  Measured (decode steps back to back in a graph, us a layer, mma.sync /
+// tcgen05; in brackets without launch overlap): 8 kv heads of 128 dims, q8_0: 4096 positions 8.5 / 8.85 (10.2 / 10.8), 4500 9.05 / 8.9 (10.45 / 10.9),
+// 5000 8.3 / 8.75 (11.0 / 11.4), 6000 8.8 / 8.9 (11.25 / 11.7), 7000 9.7 / 9.0 (12.4 / 12.0).  4 kv heads of 256, q8_0: 5000 10.65 / 12.3 (12.7 / 13.15),
+// 8000 11.1 / 12.3 (14.2 / 13.8), 9728 12.05 / 13.0 (15.4 / 14.5), 12000 12.8 / 13.3 (16.5 / 15.3), 14000 14.45 / 14.1 (17.2 / 16.0); one scale
+// per row: 8000 10.8 / 11.6 (13.6 / 13.15), 12000 12.2 / 12.75 (15.8 / 14.7), 16000 14.2 / 14.25 (17.45 / 16.0).  So the lines lie inside the range in
+// which neither kernel is ahead in every mode: with overlap the two are level at about 6000 and 13000 to 16000 positions, without it
+// at about 6500 and 7500, and the slower one costs up to 6 %.  Other head counts were not measured and go by the rows, which is what fills the device.
 constexpr uint64_t kStreamRows128 = 32768, kStreamRows256 = 40000;
 
 // Runs stage 1 and, where the merge fits inside the launch, the merge.

@@ -12,7 +12,7 @@
 //  * Each warp walks its own tiles of 16 positions (warp w of W takes tiles w, w + W, ...): no barrier between warps until the
 //    end.  A tile is two UNITS, its K rows and its V rows, which the warp copies with cp.async into a private ring (about 24 KB;
 //    8 warps on an SM keep 130 KB or more in flight), 16-byte chunks XORed with the row number so that ldmatrix
-//    reads without bank conflicts (255 registers a thread at head_dim 256: q8_0 on both sides spills 8 bytes).  Rows of any alignment above 16 bytes work, rows past the end are zero-filled.
+//    reads without bank conflicts (242 to 255 registers a thread at head_dim 256, no spills).  Rows of any alignment above 16 bytes work, rows past the end are zero-filled.
 //  * S = Q K^T and O = P V run on mma.sync m16n8k16 with fp32 accumulation.  M = 16 is 8 heads x 2 terms: rows 0-7 hold the
 //    high and rows 8-15 the low fp16 half of every query element (and of every weight), 22 bits in all, so the products are
 //    those of an fp32 kernel and the two halves of a score sit in one thread.  K and V are exact in fp16: fp16 planes as they
@@ -23,14 +23,14 @@
 //  * Online softmax per warp in base 2 with a lazy reference: the accumulators are rescaled only when a head's maximum has
 //    grown by more than 2^4 since the last rescale.  P V runs on weights scaled by a power of two that keeps weight x value scale
 //    within fp16's normal range (chosen from the value scales seen; re-chosen, with a rescale, when larger ones appear).
-// Measured, 4 kv heads, d = 256, 24 query heads, one layer's attention with its merge: fp16 cache 7.2 us at 1500 positions,
-// 9.8 at 6001 (the kernel this one replaced and its merge kernel: 64), 24.6 at 32768 (5.5 TB/s), 82 at 131072 (6.5 TB/s: the copy
-// rate); q8_0 7.8 us at 1500, 22.0 at 32768 (254), 65 at 131072 -- there the conversions of int8 show, and the tcgen05 kernels
-// are faster.  24 sessions of 200 to 6000 positions in one launch, q8_0: 44 us (657).
-// A decode step's launch at a few thousand positions is a chain of latencies, instruction fetches above all (2.2 of the 7.5 cycles a warp
-// spends on an instruction at 7777 positions, one scale per row); hence partials emitted two dims at a time, the copies' code once for
-// both sides, 32-bit split bounds, and the merge's gate fetched early.  Step of 24 / 4 heads of 256, append and merge included, in a graph: q8_0 4000
-// positions 9.9 -> 9.0 us, one scale per row 7777 11.3 -> 10.6, fp16 6001 11.4 -> 10.75.
+// Measured, decode steps of 4 kv heads of 256 and 24 query heads back to back in a graph, append and merge inside, us a layer: fp16 cache 6.9 at
+// 1500 positions, 10.9 at 6001 (the kernel this one replaced and its merge kernel: 64), 26.1 at 32768 (5.1 TB/s), 90 at 131072 (6.0 TB/s); q8_0
+// 8.4 at 1500, 9.2 at 4000, 23.5 at 32768 (254), 77 at 131072 -- there the conversions of int8 show, and the tcgen05 kernels are faster.
+// 24 sessions of 200 to 6000 positions in one launch, q8_0: 44 us (657).
+// At a few thousand positions a launch is a chain of latencies.  Of the 7.0 cycles a warp spends on an instruction at 7777 positions, one scale per
+// row, 1.3 wait for the instruction itself, 1.2 for memory and 1.1 for the one before; hence partials emitted two dims at a time, the copies' code
+// once for both sides, 32-bit split bounds, and the merge's gate fetched early.  Together: q8_0 4000 positions 9.9 -> 9.0 us, one scale per row 7777
+// 11.3 -> 10.6, fp16 6001 11.4 -> 10.75.
 #include "decode_tail.cuh"
 
 #include <climits>
