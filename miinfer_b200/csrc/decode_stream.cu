@@ -23,9 +23,9 @@
 //  * Online softmax per warp in base 2 with a lazy reference: the accumulators are rescaled only when a head's maximum has
 //    grown by more than 2^4 since the last rescale.  P V runs on weights scaled by a power of two that keeps weight x value scale
 //    within fp16's normal range (chosen from the value scales seen; re-chosen, with a rescale, when larger ones appear).
-// Measured, decode steps of 4 kv heads of 256 and 24 query heads back to back in a graph, append and merge inside, us a layer: fp16 cache 6.9 at
+// Measured, decode steps of 4 kv heads of 256 and 24 query heads back to back in a graph, append and merge inside, us a layer: fp16 cache 7.0 at
 // 1500 positions, 10.9 at 6001 (the kernel this one replaced and its merge kernel: 64), 26.1 at 32768 (5.1 TB/s), 90 at 131072 (6.0 TB/s); q8_0
-// 8.4 at 1500, 9.2 at 4000, 23.5 at 32768 (254), 77 at 131072 -- there the conversions of int8 show, and the tcgen05 kernels are faster.
+// 7.7 at 1500, 9.1 at 4000, 23.5 at 32768 (254), 77 at 131072 -- there the conversions of int8 show, and the tcgen05 kernels are faster.
 // 24 sessions of 200 to 6000 positions in one launch, q8_0: 44 us (657).
 // At a few thousand positions a launch is a chain of latencies.  Of the 7.0 cycles a warp spends on an instruction at 7777 positions, one scale per
 // row, 1.3 wait for the instruction itself, 1.2 for memory and 1.1 for the one before; hence partials emitted two dims at a time, the copies' code
