@@ -168,7 +168,7 @@ def test_overlapped_steps_whose_last_splits_are_shorter(cuda, d, H, Hq, qb, mode
     assert torch.equal(out0[:below], out1[:below]) and not torch.equal(out0[below:], out1[below:])   # even splits on both sides, then not
     for a, b in ((out0, out1), (part0, part1)):
         assert torch.isfinite(b).all() and ((a - b).norm() / a.norm()).item() <= REL
-    # the steps without overlap against float64 over the cache as it lies
+    # a step above the line, with overlap, against float64 over the rows as the cache holds them
     K, V = (_plane(st, side, line + 1) for side in ("key", "value"))
     s = torch.einsum("hgd,hld->hgl", q[below].double().view(H, Hq // H, d), K) * d ** -0.5
     ref = torch.einsum("hgl,hld->hgd", s.softmax(-1), V).reshape(Hq, d)
