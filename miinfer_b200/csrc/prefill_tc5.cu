@@ -718,37 +718,49 @@ struct DequantParams {
     uint32_t row_end;    // the chunk (b200kv_prefill_prepare), possibly beside the previous layer's attention
 };
 
+// A thread converts kDequantUnits pieces of 8 elements, a block's threads side by side and all of a thread's loads in flight together: a warp
+// reads 256 contiguous bytes and writes 512.  Bound by the bytes to and from L2 (19 MB in, 36 MB out for 8704 positions of 4 kv heads of 256);
+// with one piece of 16 elements a thread, in four waves of blocks, a layer of 512 tokens over 8192 took 118.2 us in place of 114.8, one of 128
+// tokens (8 kv heads of 128) 43.0 in place of 41.0.
+constexpr int kDequantUnits = 8;
 template <int D>
-__global__ void __launch_bounds__(256) dequant_prefix_kernel(const __grid_constant__ DequantParams p) {
-    constexpr int CPR = D / 16;
+__global__ void __launch_bounds__(256, 4) dequant_prefix_kernel(const __grid_constant__ DequantParams p) {
+    constexpr uint32_t CPR = D / 8;
     pdl_launch_dependents();
     pdl_wait();   // the cache rows of this chunk come from the append kernel just before
     const uint32_t head = blockIdx.y, side = blockIdx.z;   // side 0 = K, 1 = V
     const uint32_t mode = p.view.quant_mode;
     const bool q8 = side == 0 ? (mode == B200KV_Q8_F16 || mode == B200KV_Q8_Q8) : (mode == B200KV_F16_Q8 || mode == B200KV_Q8_Q8);
-    const int8_t* q = side == 0 ? p.view.key_q8 : p.view.value_q8;
-    const __half* sc = static_cast<const __half*>(side == 0 ? p.view.key_scales : p.view.value_scales);
-    const __half* f16 = static_cast<const __half*>(side == 0 ? p.view.key_f16 : p.view.value_f16);
-    __half* out = (side == 0 ? p.k_out : p.v_out) + static_cast<size_t>(head) * p.scratch_rows * D;
     const uint32_t nblk = D / p.view.qblock;
     const uint64_t head_row0 = static_cast<uint64_t>(head) * p.view.capacity;
-    const size_t total = static_cast<size_t>(p.row_end) * CPR;   // rows past `rows` are zero-filled: the last tile reads them
-    for (size_t idx = static_cast<size_t>(p.row_begin) * CPR + static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-         idx += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint32_t pos = static_cast<uint32_t>(idx / CPR), c16 = static_cast<uint32_t>(idx % CPR);
-        uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-        if (pos >= p.rows) {
-            // padding row of the last tile: P is 0 there, but 0 * (stale NaN) would still poison O
-        } else if (q8) {
-            const uint64_t grow = head_row0 + pos;
-            const uint4 raw = *reinterpret_cast<const uint4*>(q + grow * D + c16 * 16);
-            dequant16(raw, sc[grow * nblk + (nblk == 1 ? 0 : c16 / 2)], &lo, &hi);
+    const int8_t* q = (side == 0 ? p.view.key_q8 : p.view.value_q8) + head_row0 * D;
+    const __half* sc = static_cast<const __half*>(side == 0 ? p.view.key_scales : p.view.value_scales) + head_row0 * nblk;
+    const __half* f16 = static_cast<const __half*>(side == 0 ? p.view.key_f16 : p.view.value_f16) + head_row0 * D;
+    __half* out = (side == 0 ? p.k_out : p.v_out) + static_cast<size_t>(head) * p.scratch_rows * D;
+    const uint32_t row0 = p.row_begin + blockIdx.x * (256 * kDequantUnits / CPR) + threadIdx.x / CPR, c = threadIdx.x % CPR;
+    uint4 v[kDequantUnits];   // int8: the first two words
+    __half scale[kDequantUnits];
+#pragma unroll
+    for (int i = 0; i < kDequantUnits; ++i) {
+        const uint32_t pos = row0 + i * (256 / CPR);
+        // padding rows of the last tile are zeroed: P is 0 there, but 0 * (stale NaN) would still poison O
+        v[i] = make_uint4(0, 0, 0, 0);
+        scale[i] = __ushort_as_half(0);
+        if (pos >= p.rows) continue;
+        const size_t at = static_cast<size_t>(pos) * D + c * 8;
+        if (q8) {
+            const uint2 raw = *reinterpret_cast<const uint2*>(q + at);
+            v[i].x = raw.x; v[i].y = raw.y;
+            scale[i] = sc[static_cast<size_t>(pos) * nblk + (nblk == 1 ? 0 : c / 4)];
         } else {
-            const uint4* src = reinterpret_cast<const uint4*>(f16 + (head_row0 + pos) * D + c16 * 16);
-            lo = src[0]; hi = src[1];
+            v[i] = *reinterpret_cast<const uint4*>(f16 + at);
         }
-        uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(pos) * D + c16 * 16);
-        dst[0] = lo; dst[1] = hi;
+    }
+#pragma unroll
+    for (int i = 0; i < kDequantUnits; ++i) {
+        const uint32_t pos = row0 + i * (256 / CPR);
+        if (pos >= p.row_end) break;
+        *reinterpret_cast<uint4*>(out + static_cast<size_t>(pos) * D + c * 8) = q8 ? dequant8(make_uint2(v[i].x, v[i].y), scale[i]) : v[i];
     }
 }
 
@@ -798,9 +810,8 @@ int launch_dequant(const b200kv_view& view, __half* k_scratch, __half* v_scratch
     dp.scratch_rows = scratch_rows;
     dp.row_begin = row_begin;
     dp.row_end = row_end;
-    const size_t units = static_cast<size_t>(row_end - row_begin) * (D / 16);
-    unsigned blocks = static_cast<unsigned>((units + 255) / 256);
-    if (blocks > 148u * 4u) blocks = 148u * 4u;
+    constexpr uint32_t rows_per_block = 256 * kDequantUnits / (D / 8);
+    const unsigned blocks = (row_end - row_begin + rows_per_block - 1) / rows_per_block;
     B200KV_CUDA_TRY(launch_kernel(dequant_prefix_kernel<D>, dim3(blocks, view.kv_heads, 2), dim3(256), 0, stream, true, dp));
     return B200KV_OK;
 }
