@@ -27,8 +27,8 @@
 //     At head_dim 128 a CTA takes TWO row tiles where there are enough of them (512 softmax threads; S, P and O of both fill
 //     TMEM, so Q is an A operand in shared memory): a single tile's loop waits for its softmax (about 1 us a pair of KV tiles against
 //     0.5 us of MMAs), two share every K and V tile and one's MMAs run under the other's softmax.  2048 fresh
-//     tokens, 32/8 heads: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA
-//     (96 registers a thread, a few bytes of them spilled).
+//     tokens, 32/8 heads: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA, 51 with Q ahead of the rings and
+//     P in TMEM (96 registers a thread, 12 bytes of them spilled).
 // Every mbarrier wait is bounded; a wait that runs out poisons the output rows with NaN, and the CTA still frees
 // its TMEM and exits.
 #include "decode_common.cuh"
@@ -172,6 +172,10 @@ __device__ __forceinline__ void umma_f16_a_tmem(uint32_t tmem_d, uint32_t tmem_a
     asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Brings [src, src + bytes) on its way to L2; both multiples of 16.
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // A wait of a whole warp, which stays together: all lanes go on or none.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 // One lane of a converged warp, always the same one.
@@ -229,6 +233,29 @@ struct Layout {
     [[maybe_unused]] static constexpr uint32_t kColP = 128;
     static constexpr uint32_t kColS = 0, kColQ = kPInTmem ? 192 : 128, kColO = 256;
     static_assert(RT == 1 ? kColQ + D / 2 <= kColO && kColO + D <= 512 : kColO + 2 * D <= 512, "TMEM columns");
+};
+
+// Elements in front of a row of [token][query_heads][D], for rows (tokens' heads of one kv head) four apart: one division, then additions.  (Two
+// divisions for each of a thread's eight rows were 1.3 us of a CTA's start and as much of its end.)
+template <int D>
+struct RowWalk {
+    size_t off, step, wrap;
+    uint32_t in_group, step_in_group, G;
+    __device__ __forceinline__ RowWalk(uint32_t row, uint32_t kv_head, uint32_t G_, uint32_t query_heads) {
+        G = G_;
+        asm volatile("" : "+r"(row));   // worked out anew where it is used: no registers for it in between
+        const uint32_t token = row / G, tokens = 4 / G;
+        in_group = row - token * G;
+        step_in_group = 4 - tokens * G;
+        off = (static_cast<size_t>(token) * query_heads + kv_head * G + in_group) * D;
+        step = (static_cast<size_t>(tokens) * query_heads + step_in_group) * D;
+        wrap = static_cast<size_t>(query_heads - G) * D;
+    }
+    __device__ __forceinline__ void next() {
+        off += step;
+        in_group += step_in_group;
+        if (in_group >= G) { in_group -= G; off += wrap; }
+    }
 };
 
 template <int D, int RT>
@@ -325,6 +352,9 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             const int row_base = static_cast<int>(kv_head * p.scratch_rows);
             for (int i = 0; 2 * i < ntiles; ++i) {
                 const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
+                // Q first: nothing can start without it, and 148 CTAs that fill their rings at once keep L2 busy for over 3 us.  The first pair of K
+                // tiles goes along with it, the other stages are asked for when it is in.
+                if (i == 1 && !mbar_wait(bar(Q_FULL), 0)) break;
                 if (!mbar_wait(bar(K_EMPTY + ps), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) break;
                 mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
                 for (int t = 0; t < n; ++t)
@@ -335,7 +365,14 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         }
     } else if (warp == kTmaVWarp) {
         // =============================== TMA producer, V tiles ===============================
-        if (lane == 0) {
+        const bool have_q = mbar_wait(bar(Q_FULL), 0);
+        // The gate on its way to L2 for the epilogue or the merge: the kv head's G rows of a token are contiguous, a lane takes a token.
+        if (p.gate != nullptr && split_u == 0) {
+            const uint32_t t_last = (min(row0 + L::kRows, total_rows) - 1) / G;
+            for (uint32_t t = row0 / G + lane; t <= t_last; t += 32)
+                prefetch_l2(p.gate + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D, G * D * 4);
+        }
+        if (have_q && lane == 0) {
             const int row_base = static_cast<int>(kv_head * p.scratch_rows);
             for (int j = 0; j < ntiles; ++j) {
                 const int st = j & 1;
@@ -451,8 +488,9 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         // Q: the CTA's rows as fp16 pairs in TMEM (row = lane, dims 2c and 2c+1 in column c), the A operand of every S MMA:
         // read from there it costs no shared-memory bandwidth.  Each of a row's two softmax threads stores half of the
         // row.  A warp reads its 32 rows four at a time, 128 (fp32: 256) contiguous bytes each, and turns them through
-        // its own 4 KB of the P tiles (a load per thread and row touched 32 lines an instruction); the first K
-        // and V tiles are on their way meanwhile.
+        // its own 4 KB of the P tiles (a load per thread and row touched 32 lines an instruction); the first pair of K
+        // tiles is on its way meanwhile.  From the dependency wait to the last row: 0.8 us (two row tiles of 128 dims; 3.8 behind full rings and with
+        // a division a row), 3.3 us (one of 256 from HBM; 4.5).
         uint8_t* const turn = smem + L::kOffP + warp * 4096;   // [32 rows][8 chunks of 16 B], chunk c of row r at c ^ (r & 7)
         const int turn_row = lane >> 3, turn_chunk = lane & 7;
         const int rt = RT == 1 ? 0 : warp >> 3;                // row tile
@@ -460,24 +498,33 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         {
             const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
             const int half = (warp >> 2) & 1;
-#pragma unroll 1
-            for (int c0 = 0; c0 < D / 4; c0 += 32) {   // 32 columns = 64 dims per store
-                uint4 v[8];
+            constexpr int kTurns = D / 128;            // 32 columns = 64 dims per store; all loads are in flight together
+            uint4 q[kTurns][8];
+            auto fetch = [&](auto f16) {
+                RowWalk<D> at(warp_row0 + turn_row, kv_head, G, p.query_heads);
+                at.off += half * (D / 2) + turn_chunk * 8;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t row = warp_row0 + 4 * i + turn_row;
-                    v[i] = make_uint4(0, 0, 0, 0);
-                    if (row < total_rows) {
-                        const size_t e = (static_cast<size_t>(row / G) * p.query_heads + kv_head * G + row % G) * D + half * (D / 2) + c0 * 2 + turn_chunk * 8;
-                        if (p.q_is_f16) {
-                            v[i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + e);
+                for (int i = 0; i < 8; ++i, at.next())
+#pragma unroll
+                    for (int k = 0; k < kTurns; ++k) {
+                        q[k][i] = make_uint4(0, 0, 0, 0);
+                        if (warp_row0 + 4 * i + turn_row >= total_rows) continue;
+                        if (f16()) {
+                            q[k][i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + at.off + k * 64);
                         } else {
-                            const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + e);
-                            const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + e + 4);
-                            v[i] = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
+                            const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + at.off + k * 64);
+                            const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + at.off + k * 64 + 4);
+                            q[k][i] = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
                         }
                     }
-                }
+            };
+            if constexpr (RT == 2) fetch([&] { return p.q_is_f16 != 0; });   // (a branch around both: 1 % slower with two row tiles, 2 to 6 % faster with one)
+            else if (p.q_is_f16) fetch([] { return true; });
+            else fetch([] { return false; });
+#pragma unroll
+            for (int k = 0; k < kTurns; ++k) {
+                const int c0 = 32 * k;
+                uint4 (&v)[8] = q[k];
                 if constexpr (!L::kQInTmem) {   // the swizzled A operand itself: slab `half * D/128 + c0/32` of the row tile
                     uint8_t* slab = smem + L::kOffQ + rt * L::kQBytes + (half * (D / 128) + c0 / 32) * (kBM * 128) + (warp & 3) * (32 * 128);
 #pragma unroll
@@ -567,10 +614,10 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
 #pragma unroll
                 for (int i = 0; i < kBN; ++i) s[i] = (pos0 + i < len) ? s[i] : -INFINITY;
             }
-            float mt = -INFINITY;
+            float m4[4] = {s[0], s[1], s[2], s[3]};   // four chains
 #pragma unroll
-            for (int i = 0; i < kBN; ++i) mt = fmaxf(mt, s[i]);
-            mt *= p.scale_log2;   // scale > 0: the maximum commutes with it
+            for (int i = 4; i < kBN; ++i) m4[i & 3] = fmaxf(m4[i & 3], s[i]);
+            const float mt = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;   // scale > 0: the maximum commutes with it
             // the reference as the previous tile (the other group's) left it; lazy rescale: keep it unless this tile's
             // maximum outgrew it by more than the threshold
             float m_prev = -INFINITY;
@@ -629,6 +676,15 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             mbar_arrive(bar(P_FULL + 2 * rt + st));
         }
         // ---- epilogue: O / sum, gate, store; each thread of a row's pair half of the columns ----
+        const bool partial = nsplit > 1, gated = !partial && p.gate != nullptr;
+        const size_t part_row0 = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0;
+        RowWalk<D> first(warp_row0 + turn_row, kv_head, G, p.query_heads);   // of the output (a split's partials: [row][D])
+        if (partial) {
+            first.off = (part_row0 + (warp_row0 - row0) + turn_row) * D;
+            first.step = 4 * D;
+            first.step_in_group = 0;
+        }
+        first.off += grp * (D / 2) + 4 * turn_chunk;
         if (!failed && nt > 0 && !mbar_wait(bar(O_DONE + rt), 0)) failed = true;
         tc_fence_after();
         {
@@ -646,28 +702,20 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             const int hsel = grp;
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
             const bool have_o = nt > 0 && !__any_sync(0xffffffffu, failed);
-            const bool partial = nsplit > 1;
-            const size_t part_row0 = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0;
             if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum
                 p.part_ml[part_row0 + rt * kBM + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
             // Rows leave 32 columns at a time through the same 4 KB per warp: read back four rows an instruction, 128
             // contiguous bytes each, so that the gate is fetched and the result stored in whole lines.
-            size_t out_off[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t row = warp_row0 + 4 * i + turn_row;
-                out_off[i] = partial ? (part_row0 + (row - row0)) * D : (static_cast<size_t>(row / G) * p.query_heads + kv_head * G + row % G) * D;
-            }
             float* const dst = partial ? p.part_o : p.out;
             const float factor = partial ? 1.0f : inv;
-            const bool gated = !partial && p.gate != nullptr;
 #pragma unroll 1
             for (int c0 = hsel * (D / 2); c0 < (hsel + 1) * (D / 2); c0 += 32) {
                 float4 g[8];
                 if (gated) {
+                    RowWalk<D> at = first;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (warp_row0 + 4 * i + turn_row < total_rows) g[i] = *reinterpret_cast<const float4*>(p.gate + out_off[i] + c0 + 4 * turn_chunk);
+                    for (int i = 0; i < 8; ++i, at.next())
+                        if (warp_row0 + 4 * i + turn_row < total_rows) g[i] = *reinterpret_cast<const float4*>(p.gate + at.off);
                 }
                 float o[32];
                 // tcgen05.ld is warp-collective: every lane takes part, rows past the launch only skip the store
@@ -686,17 +734,21 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 for (int c = 0; c < 8; ++c)
                     *reinterpret_cast<float4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
                 __syncwarp();
+                RowWalk<D> at = first;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int row = 4 * i + turn_row;
                     float4 v = *reinterpret_cast<const float4*>(turn + row * 128 + ((turn_chunk ^ (row & 7)) << 4));
-                    if (warp_row0 + row >= total_rows) continue;
-                    if (gated) {
-                        v.x *= 1.0f / (1.0f + __expf(-g[i].x)); v.y *= 1.0f / (1.0f + __expf(-g[i].y));
-                        v.z *= 1.0f / (1.0f + __expf(-g[i].z)); v.w *= 1.0f / (1.0f + __expf(-g[i].w));
+                    if (warp_row0 + row < total_rows) {
+                        if (gated) {
+                            v.x *= 1.0f / (1.0f + __expf(-g[i].x)); v.y *= 1.0f / (1.0f + __expf(-g[i].y));
+                            v.z *= 1.0f / (1.0f + __expf(-g[i].z)); v.w *= 1.0f / (1.0f + __expf(-g[i].w));
+                        }
+                        *reinterpret_cast<float4*>(dst + at.off) = v;
                     }
-                    *reinterpret_cast<float4*>(dst + out_off[i] + c0 + 4 * turn_chunk) = v;
+                    at.next();
                 }
+                first.off += 32;
                 __syncwarp();
             }
         }
