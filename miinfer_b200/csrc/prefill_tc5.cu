@@ -976,19 +976,23 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
 }
 
 // How many KV splits: the number with the least estimated time, for `units` row-tile CTAs of up to `tiles` KV tiles.  A wave of
-// 148 CTAs costs its tiles and about 8 us of set-up, Q, epilogue and launch; a split launch also its merge, 3 us and
-// the partials' way out and back.  Measured per layer, all kernels (head_dim 256 / 24 heads, q8_0):
-//   20 tokens over 16000 (4 units):   5 splits 77 us, 8: 66, 16: 58     37 over 3001 (8):  5: 38, 8: 35, 12: 34, 16: 34
-//   128 over 8192 (24):   5: 54, 6: 52, 8 (a second wave): 69           300 over 8192 (60): 1: 124, 2: 92, 4: 102
-//   512 over 8192 (96):   1: 127, 2: 158, 3 (what filling the last wave best asks for): 138
-// The estimate takes the best column of each but one: 6 for 37 over 3001, where partial_us, that of launches with more rows, is too high.
+// 148 CTAs costs its tiles and about 3 us; CTAs take the place of one another as they end, so a last wave that is not full costs less
+// than a whole one.  A split costs its partials' way out and back.  Measured per layer, all kernels (head_dim 256 / 24 heads and 128 / 32, q8_0):
+//   256:  20 tokens over 16000 (4 units):  8: 58, 12: 52, 16: 50         37 over 3001 (8):  6: 29.6, 8: 29.0, 10: 28.5, 16: 28.8
+//         128 over 8192 (24):  5: 50, 6: 48, 8: 65                       300 over 8192 (60):  1: 116, 2: 78, 3: 99
+//         512 over 8192 (96):  1: 117, 2: 139, 3: 110, 4: 142            512 over 2000 (96):  1: 54, 2: 65, 3: 60
+//   128:  37 over 3001 (16):  6: 21.1, 8: 20.2, 10: 28.8                 100 over 1000 (32):  1: 22.1, 3: 18.6, 4: 18.5
+//         200 over 2000 (56):  1: 34, 2: 29, 3: 36                       300 over 4000 (80):  1: 56, 2: 58, 3: 48, 4: 57
+//         400 over 16000 (104, two row tiles each):  1: 176, 2: 168, 3: 174, 4: 146
+// The estimate takes the best column of each.
 static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t most, uint32_t head_dim) {
-    const double tile_us = head_dim == 256 ? 0.73 : 0.52, wave_us = 8.0, merge_us = 3.0, partial_us = head_dim == 256 ? 0.11 : 0.055;
+    const double tile_us = head_dim == 256 ? 0.6 : 0.4, wave_us = 3.0, partial_us = head_dim == 256 ? 0.03 : 0.01;
     uint32_t best = 1;
     double best_us = 0.0;
     for (uint32_t s = 1; s <= kMaxKvSplits && s <= (most > 1 ? most : 1); ++s) {
-        const uint64_t ctas = static_cast<uint64_t>(units) * s, waves = (ctas + 147) / 148;
-        const double us = static_cast<double>(waves) * (tiles * tile_us / s + wave_us) + (s > 1 ? merge_us + partial_us * static_cast<double>(ctas) : 0.0);
+        const uint64_t ctas = static_cast<uint64_t>(units) * s, full = ctas / 148, rest = ctas % 148;
+        const double waves = static_cast<double>(full) + (rest == 0 ? 0.0 : full == 0 ? 1.0 : 0.6 + 0.4 * static_cast<double>(rest) / 148.0);
+        const double us = waves * (tiles * tile_us / s + wave_us) + (s > 1 ? partial_us * static_cast<double>(ctas) : 0.0);
         if (s == 1 || us < best_us) { best = s; best_us = us; }
     }
     return best;
