@@ -697,13 +697,14 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             if constexpr (RT == 1) asm volatile("bar.sync 2, 256;" ::: "memory");
             else asm volatile("bar.sync %0, 256;" ::"r"(2 + rt) : "memory");
             l_sum = sums[r] + sums[kBM + r];
-            if (l_sum != l_sum) failed = true;   // either thread of the row gave up
+            // The warp's O may be read.  A sum that is NaN, because the row's other thread gave up or because of the data, is its own row's affair.
+            const bool have_o = nt > 0 && !__any_sync(0xffffffffu, failed);
+            if (l_sum != l_sum) failed = true;
             const float m_ref = m_final;
             const int hsel = grp;
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
-            const bool have_o = nt > 0 && !__any_sync(0xffffffffu, failed);
-            if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum
-                p.part_ml[part_row0 + rt * kBM + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
+            if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum (and an empty one by its maximum, so a poisoned one has a finite one)
+                p.part_ml[part_row0 + rt * kBM + r] = failed ? make_float2(0.0f, __int_as_float(0x7fc00000)) : make_float2(m_ref, len == 0 ? 0.0f : l_sum);
             // Rows leave 32 columns at a time through the same 4 KB per warp: read back four rows an instruction, 128
             // contiguous bytes each, so that the gate is fetched and the result stored in whole lines.
             float* const dst = partial ? p.part_o : p.out;
