@@ -615,9 +615,10 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             tc_fence_before();
             mbar_arrive(bar(S_EMPTY + 2 * rt + st));   // this row of S is in registers
             const uint32_t pos0 = static_cast<uint32_t>(tile0 + j) * kBN;
-            // Raw scores stay unscaled; the softmax scale is folded into the exponent: p = 2^(s*c - m*c).  The loop's instructions count (beside 1024 or
-            // 2048 clocks of MMAs a pair of tiles an SM's schedulers issue some 1600 of them): products and sums go in pairs, maxima three values at a time.
-            // 32 / 8 heads of 128, 1024 tokens over 8192: 168.0 -> 163.7 us; 24 / 4 of 256, 512 over 8192: 111.6 -> 110.3.
+            // Raw scores stay unscaled; the softmax scale is folded into the exponent: p = 2^(s*c - m*c).  The loop's instructions count: products and
+            // sums go in pairs, maxima three values at a time.  32 / 8 heads of 128, 1024 tokens over 8192: 168.0 -> 163.7 us; 24 / 4 of 256, 512 over
+            // 8192: 111.6 -> 110.3.  (The compiler's schedule of this loop depends on what follows it: always measure 1024 over 8192 and 512 over 8192.
+            // With the maximum of a poisoned split replaced below, where it is stored, they took 179 and 113 us.)
             // Only the tiles that straddle this row's causal length need the mask.
             if (pos0 + kBN > len) {
 #pragma unroll
@@ -720,8 +721,8 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             const float m_ref = m_final;
             const int hsel = grp;
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
-            if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum (and an empty one by its maximum, so a poisoned one has a finite one)
-                p.part_ml[part_row0 + rt * kBM + r] = failed ? make_float2(0.0f, __int_as_float(0x7fc00000)) : make_float2(m_ref, len == 0 ? 0.0f : l_sum);
+            if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum
+                p.part_ml[part_row0 + rt * kBM + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
             // Rows leave 32 columns at a time through the same 4 KB per warp: read back four rows an instruction, 128
             // contiguous bytes each, so that the gate is fetched and the result stored in whole lines.
             float* const dst = partial ? p.part_o : p.out;
@@ -820,7 +821,7 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const __grid_constan
     float lsum = 0.0f;
 #pragma unroll
     for (uint32_t s = 0; s < MAX_SPLITS; ++s) {
-        if (ml[s].y <= 0.0f || ml[s].x == -INFINITY) continue;
+        if (ml[s].y <= 0.0f || (ml[s].x == -INFINITY && ml[s].y == ml[s].y)) continue;   // a sum that is NaN poisons its row
         const float w = exp2f(ml[s].x - M);
         acc.x = fmaf(o[s].x, w, acc.x); acc.y = fmaf(o[s].y, w, acc.y); acc.z = fmaf(o[s].z, w, acc.z); acc.w = fmaf(o[s].w, w, acc.w);
         lsum = fmaf(ml[s].y, w, lsum);
