@@ -63,7 +63,7 @@ struct Plan {
     static constexpr int kQBytes = D / 16 * 32 * 16;                                    // A fragments of Q: [k step][lane][16 bytes]
     static constexpr int kSlot = Unit<D, KF>::kBytes > Unit<D, VF>::kBytes ? Unit<D, KF>::kBytes : Unit<D, VF>::kBytes;
     using Scratch = tail::RowScratch<2 * D>;                                            // an appended row, one side
-    static constexpr int kMisc = WARPS * 8 * 8 + 8 * 4 + 8 * 8 + 2 * static_cast<int>(sizeof(Scratch));   // per-warp (m, l), qmul, merged (m, l), row
+    static constexpr int kMisc = WARPS * 8 * 8 + 8 * 4 + 2 * static_cast<int>(sizeof(Scratch));   // per-warp (m, l), qmul, row
     static constexpr int kRing = 26 * 1024;                                             // per warp
     static constexpr int kUnits = kRing / kSlot < 12 ? kRing / kSlot : 12;
     static constexpr int kOffRing = kQBytes;
@@ -181,8 +181,7 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
     const uint32_t ring = smem_u32(smem) + P::kOffRing + warp * (P::kUnits * P::kSlot);
     float* ml_s = reinterpret_cast<float*>(smem + P::kOffMisc);     // [WARPS][8] {m, l}
     float* qmul_s = ml_s + WARPS * 16;                              // [8]
-    float* tot_s = qmul_s + 8;                                      // [8] {m, l} over the CTA's warps
-    typename P::Scratch* new_row = reinterpret_cast<typename P::Scratch*>(tot_s + 16);   // K, V
+    typename P::Scratch* new_row = reinterpret_cast<typename P::Scratch*>(qmul_s + 8);   // K, V
 
     // ---- one unit (K or V rows of the warp's tile t) into ring slot `slot` -----------------------------------
     auto copy_side = [&](auto fmt_c, const uint8_t* rows, const uint8_t* scales, uint32_t pos, uint32_t dst) {
@@ -606,30 +605,26 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
         }
     }
     __syncthreads();
-    if (tid < 8) {   // merged (m, l) of head tid; each warp's share of it replaces its m
-        float M = -INFINITY, L = 0.0f;
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, ml_s[(w * 8 + tid) * 2]);
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
-            const float m = ml_s[(w * 8 + tid) * 2], f = m == -INFINITY ? 0.0f : exp2f(m - M);
-            L = fmaf(ml_s[(w * 8 + tid) * 2 + 1], f, L);
-            ml_s[(w * 8 + tid) * 2] = f;
-        }
-        tot_s[2 * tid] = M;
-        tot_s[2 * tid + 1] = L;
-    }
-    __syncthreads();
     for (int idx = 2 * tid; idx < G * D; idx += 2 * P::kThreads) {
         const int h = idx / D, dim = idx % D;
+        // The head's maximum and sum over the warps, by every thread for itself: one barrier and eight threads' chain less (us a layer: 32 / 8 heads of 128,
+        // q8_0 2000 positions 7.10 -> 6.97, fp16 5000 7.86 -> 7.70; 24 / 4 of 256, q8_0 4000 9.92 -> 9.79, one scale per row 7777 12.21 -> 12.09).
+        float2 ml[WARPS];
+        float M = -INFINITY, L = 0.0f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            ml[w] = *reinterpret_cast<const float2*>(ml_s + (w * 8 + h) * 2);
+            M = fmaxf(M, ml[w].x);
+        }
         float2 a = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) {
             const float2 x = *reinterpret_cast<const float2*>(smem + P::kOffRing + w * (P::kUnits * P::kSlot) + (h * P::kOutStride + dim) * 4);
-            const float f = ml_s[(w * 8 + h) * 2];
+            const float f = ml[w].x == -INFINITY ? 0.0f : exp2f(ml[w].x - M);
+            L = fmaf(ml[w].y, f, L);
             a.x = fmaf(x.x, f, a.x); a.y = fmaf(x.y, f, a.y);
         }
-        tail::emit_partial2<SEG>(p, session, split, num_splits, kv_head * G + h, dim, a, tot_s[2 * h] * 0.6931471805599453f, tot_s[2 * h + 1]);
+        tail::emit_partial2<SEG>(p, session, split, num_splits, kv_head * G + h, dim, a, M * 0.6931471805599453f, L);
     }
     if (p.ws_tagged == nullptr) return;           // a separate merge kernel follows
     __syncthreads();
