@@ -207,24 +207,24 @@ struct Layout {
     static constexpr int kTmaVWarp = kTmaWarp + 3;         // TMA producer of the V tiles (a K load never waits for a V stage)
     static constexpr int kThreads = kSoftmaxThreads + 128;
     static constexpr int kRows = RT * kBM;
-    static constexpr bool kQInTmem = RT == 1;              // two row tiles' S and O fill TMEM: their Q stays in shared memory
+    static constexpr bool kQInTmem = RT == 1;              // two row tiles' S, P and O fill TMEM: their Q stays in shared memory
     static constexpr int kSlabs = D / 64;                  // 128-byte (64 x fp16) slabs along d
     static constexpr int kTileBytes = kSlabs * kBN * 128;  // one K or V tile: [slab][row][128 B]
     static constexpr int kPairBytes = 2 * kTileBytes;      // two K tiles as one B operand: [slab][128 rows][128 B]
     static constexpr int kOffK = 0;
     static constexpr int kOffV = kOffK + kKPairs * kPairBytes;
-    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // [row tile][2][row][128 B] fp16 P tiles
+    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // [row tile][2][row][128 B] fp16 P tiles; Q and O are turned there (kPInTmem: only that)
     static constexpr int kPBytes = kBM * 128;
     static constexpr int kOffQ = kOffP + RT * 2 * kPBytes; // [row tile][slab][row][128 B]
     static constexpr int kQBytes = kSlabs * kBM * 128;
     static constexpr int kOffBar = kOffQ + (kQInTmem ? 0 : RT * kQBytes);
-    // mbarriers; the ones after V_EMPTY are per row tile, S_EMPTY and the P pairs per row tile and softmax group
     // head_dim 128: P as an A operand in TMEM, which takes its writes and reads out of shared memory, the bound of the tile loop (192 KB a tile of
     // two row tiles at 128 bytes a clock; 160 now), and S tile by tile.  32 / 8 heads, us a layer: 1024 tokens over 8192 184.6 -> 168.0, 300 over
     // 4000 63.0 -> 56.7, 128 over 8192 41.0 -> 39.2, 2048 fresh 61.7 -> 60.4.  At 256 S, Q and O leave no columns for P beside a pair
     // of S tiles; with single ones in their place a layer of 512 tokens over 8192 took 134 us, not 125.
     static constexpr bool kPInTmem = D == 128;
     static constexpr int kSBufs = RT == 1 ? 2 : 1;         // kPInTmem: S tiles of a row tile
+    // mbarriers; the ones after V_EMPTY are per row tile, S_EMPTY and the P pairs (kPInTmem: S_FULL too) per row tile and softmax group
     static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = S_FULL + (kPInTmem ? 2 * RT : 1), P_FULL = S_EMPTY + 2 * RT,
                          P_EMPTY = P_FULL + 2 * RT, O_DONE = P_EMPTY + 2 * RT, Q_FULL = O_DONE + RT, kNumBars = Q_FULL + 1;
     static constexpr int kOffSlot = kOffBar + (kNumBars * 8 + 15) / 16 * 16;
