@@ -22,13 +22,13 @@
 //         than 2^8; P <= 256 fits fp16; the row's reference maximum is handed from tile to tile through shared
 //         memory), write P as fp16 into one of two swizzled A-operand tiles, and at the end scale O by 1/sum,
 //         apply the sigmoid gate (.hip:6714-6723) and store.
-//     TMEM: S (pair) | Q | O = 128 + d/2 + d columns.  Shared memory: 2 x 2 K tiles + 2 V tiles + 2 P tiles.  At head_dim 128 S comes
-//     tile by tile and P lies in TMEM as well (Layout::kPInTmem).
-//     At head_dim 128 a CTA takes TWO row tiles where there are enough of them (512 softmax threads; S, P and O of both fill
+//     TMEM: S (pair) | Q | O = 128 + d/2 + d columns.  Shared memory: 2 x 2 K tiles + 2 V tiles + 2 P tiles.  A single row tile of
+//     head_dim 128 has S tile by tile and P in TMEM as well (Layout::kPInTmem).
+//     At head_dim 128 a CTA takes TWO row tiles where there are enough of them (512 softmax threads; S and O of both fill
 //     TMEM, so Q is an A operand in shared memory): a single tile's loop waits for its softmax (about 1 us a pair of KV tiles against
 //     0.5 us of MMAs), two share every K and V tile and one's MMAs run under the other's softmax.  2048 fresh
-//     tokens, 32/8 heads: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA, 51 with Q ahead of the rings and
-//     P in TMEM (96 registers a thread, 12 bytes of them spilled).
+//     tokens, 32/8 heads, when the choice was made: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA
+//     (96 registers a thread, 12 bytes of them spilled).
 // Every mbarrier wait is bounded; a wait that runs out poisons the output rows with NaN, and the CTA still frees
 // its TMEM and exits.
 #include "decode_common.cuh"
@@ -213,19 +213,20 @@ struct Layout {
     static constexpr int kPairBytes = 2 * kTileBytes;      // two K tiles as one B operand: [slab][128 rows][128 B]
     static constexpr int kOffK = 0;
     static constexpr int kOffV = kOffK + kKPairs * kPairBytes;
-    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // [row tile][2][row][128 B] fp16 P tiles; Q and O are turned there (kPInTmem: only that)
+    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // [row tile][2][row][128 B] fp16 P tiles; Q (kQInTmem) and O are turned there (kPInTmem: only that)
     static constexpr int kPBytes = kBM * 128;
     static constexpr int kOffQ = kOffP + RT * 2 * kPBytes; // [row tile][slab][row][128 B]
     static constexpr int kQBytes = kSlabs * kBM * 128;
     static constexpr int kOffBar = kOffQ + (kQInTmem ? 0 : RT * kQBytes);
-    // head_dim 128: P as an A operand in TMEM, which takes its writes and reads out of shared memory, the bound of the tile loop (192 KB a tile of
-    // two row tiles at 128 bytes a clock; 160 now), and S tile by tile.  32 / 8 heads, us a layer: 1024 tokens over 8192 184.6 -> 168.0, 300 over
-    // 4000 63.0 -> 56.7, 128 over 8192 41.0 -> 39.2, 2048 fresh 61.7 -> 60.4.  At 256 S, Q and O leave no columns for P beside a pair
-    // of S tiles; with single ones in their place a layer of 512 tokens over 8192 took 134 us, not 125.
-    static constexpr bool kPInTmem = D == 128;
-    static constexpr int kSBufs = RT == 1 ? 2 : 1;         // kPInTmem: S tiles of a row tile
+    // One row tile of head_dim 128: P as an A operand in TMEM, which takes its writes and reads out of shared memory, and S tile by tile in two
+    // buffers.  32 / 8 heads, us a layer: 1024 tokens over 8192 184.6 -> 168.0, 300 over 4000 63.0 -> 56.7, 128 over 8192 41.0 -> 39.2.
+    // At 256 S, Q and O leave no columns for P beside a pair of S tiles; with single ones in their place a layer of 512 tokens over 8192 took
+    // 134 us, not 125.  Two row tiles have columns for one S tile each beside P, and score MMAs of N = 64 then read Q from shared memory
+    // for every tile, not for every pair (96 KB of operands, not 64): 32 / 8 heads, a layer of 3000 over 8192 in a long run of
+    // them 545 us that way and 533 with S in pairs and P in shared memory, 1200 over 4000 156 and 150, 1400 over 2048 100.0 and 97.4, 2048 fresh 59.2 and 59.2.
+    static constexpr bool kPInTmem = D == 128 && RT == 1;
     // mbarriers; the ones after V_EMPTY are per row tile, S_EMPTY and the P pairs (kPInTmem: S_FULL too) per row tile and softmax group
-    static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = S_FULL + (kPInTmem ? 2 * RT : 1), P_FULL = S_EMPTY + 2 * RT,
+    static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = S_FULL + (kPInTmem ? 2 : RT), P_FULL = S_EMPTY + 2 * RT,
                          P_EMPTY = P_FULL + 2 * RT, O_DONE = P_EMPTY + 2 * RT, Q_FULL = O_DONE + RT, kNumBars = Q_FULL + 1;
     static constexpr int kOffSlot = kOffBar + (kNumBars * 8 + 15) / 16 * 16;
     static constexpr int kOffRef = kOffSlot + 16;                 // [rows] {reference maximum, sequence}: handed from tile to tile
@@ -236,10 +237,10 @@ struct Layout {
     static constexpr int kAlloc = kTotal;   // the dynamic shared memory is declared 1024-byte aligned; the kernel checks it
     static_assert(kAlloc <= 232448, "227 KB per CTA");
     static constexpr uint32_t kTmemCols = 512;
-    // S: RT x 2 x 64 (kPInTmem: RT x kSBufs x 64), P (kPInTmem): RT x 2 x 32 (fp16 pairs), Q (RT == 1): D/2 (fp16 pairs), O: RT x D
+    // S: RT x 2 x 64, P (kPInTmem): 2 x 32 (fp16 pairs), Q (RT == 1): D/2 (fp16 pairs), O: RT x D
     [[maybe_unused]] static constexpr uint32_t kColP = 128;
     static constexpr uint32_t kColS = 0, kColQ = kPInTmem ? 192 : 128, kColO = 256;
-    static_assert(RT == 1 ? kColQ + D / 2 <= kColO && kColO + D <= 512 : kColO + 2 * D <= 512, "TMEM columns");
+    static_assert(RT == 1 ? kColQ + D / 2 <= kColO && kColO + D <= 512 : 2 * 128 <= kColO && kColO + 2 * D <= 512, "TMEM columns");
 };
 
 // Elements in front of a row of [token][query_heads][D], for rows (tokens' heads of one kv head) four apart: one division, then additions.  (Two
@@ -392,33 +393,52 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         }
     } else if (warp == kSWarp) {
         // =============================== S = Q.K^T issuer ===============================
+        // The warp stays together and one lane issues (D == 128): loop counters and descriptors live in uniform registers, which an MMA takes them from
+        // (from a branch on the lane number an MMA cost 50 to 105 clocks to issue, against the 32 to 64 these run).
         if constexpr (L::kPInTmem) {
-            // The warp stays together and one lane issues: loop counters and descriptors live in uniform registers, which an MMA takes them from (from a
-            // branch on the lane number an MMA cost 50 to 105 clocks to issue, against the 32 to 48 these run).
             constexpr uint32_t idesc = umma_idesc(kBM, kBN, 0, 0);
-            const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024), q_desc = umma_desc(sbase + L::kOffQ, 16, 1024);
+            const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024);
             bool ok = mbar_wait_warp(bar(Q_FULL), 0);
             for (int j = 0; ok && j < ntiles; ++j) {
                 const int i = j >> 1, ps = i % kKPairs;
                 if ((j & 1) == 0 && !mbar_wait_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
-                const int before = j - L::kSBufs;   // the tile whose scores the softmax threads must have read
-                const uint64_t b = k_desc + ((ps * L::kPairBytes + (j & 1) * (kBN * 128)) >> 4);
+                ok = mbar_wait_warp(bar(S_EMPTY + (j & 1)), static_cast<uint32_t>(i & 1) ^ 1);   // the scores of tile j - 2 have been read
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t b = k_desc + ((ps * L::kPairBytes + (j & 1) * (kBN * 128)) >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < D / 16; ++kk)
+                        umma_f16_a_tmem(tmem_base + L::kColS + (j & 1) * kBN, tmem_base + L::kColQ + kk * 8,
+                                        b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4), idesc, kk > 0);
+                    umma_commit(bar(S_FULL + (j & 1)));
+                    if ((j & 1) == 1 || j + 1 == ntiles) umma_commit(bar(K_EMPTY + ps));
+                }
+                __syncwarp();
+            }
+        } else if constexpr (!L::kQInTmem) {
+            constexpr uint32_t idesc_pair = umma_idesc(kBM, 2 * kBN, 0, 0), idesc_one = umma_idesc(kBM, kBN, 0, 0);
+            const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024), q_desc = umma_desc(sbase + L::kOffQ, 16, 1024);
+            bool ok = mbar_wait_warp(bar(Q_FULL), 0);
+            for (int i = 0; ok && 2 * i < ntiles; ++i) {
+                const int ps = i % kKPairs;
+                const uint32_t ph = static_cast<uint32_t>(i & 1) ^ 1, idesc = ntiles - 2 * i >= 2 ? idesc_pair : idesc_one;
+                if (!mbar_wait_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
+                const uint64_t b = k_desc + ((ps * L::kPairBytes) >> 4);
 #pragma unroll
                 for (int rt = 0; rt < RT; ++rt) {
-                    if (RT > 1 && rt >= live_tiles) break;
-                    ok = before < 0 || mbar_wait_warp(bar(S_EMPTY + 2 * rt + (before & 1)), static_cast<uint32_t>((before >> 1) & 1));
+                    if (rt >= live_tiles) break;
+                    // both groups have read the previous pair's scores (only the last pair can be a single tile)
+                    ok = mbar_wait_warp(bar(S_EMPTY + 2 * rt), ph) && mbar_wait_warp(bar(S_EMPTY + 2 * rt + 1), ph);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint32_t d = tmem_base + L::kColS + (L::kSBufs == 2 ? (j & 1) * kBN : rt * kBN);
 #pragma unroll
-                        for (int kk = 0; kk < D / 16; ++kk) {
-                            const uint64_t bk = b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4);
-                            if constexpr (L::kQInTmem) umma_f16_a_tmem(d, tmem_base + L::kColQ + kk * 8, bk, idesc, kk > 0);
-                            else umma_f16(d, q_desc + ((rt * L::kQBytes + (kk >> 2) * (kBM * 128) + (kk & 3) * 32) >> 4), bk, idesc, kk > 0);
-                        }
-                        umma_commit(bar(S_FULL + 2 * rt + (j & 1)));
-                        if (rt + 1 == live_tiles && ((j & 1) == 1 || j + 1 == ntiles)) umma_commit(bar(K_EMPTY + ps));
+                        for (int kk = 0; kk < D / 16; ++kk)
+                            umma_f16(tmem_base + L::kColS + rt * 2 * kBN, q_desc + ((rt * L::kQBytes + (kk >> 2) * (kBM * 128) + (kk & 3) * 32) >> 4),
+                                     b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4), idesc, kk > 0);
+                        umma_commit(bar(S_FULL + rt));   // scores ready for both softmax groups
+                        if (rt + 1 == live_tiles) umma_commit(bar(K_EMPTY + ps));
                     }
                     __syncwarp();
                 }
@@ -445,9 +465,9 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         }
     } else if (warp == kPvWarp) {
         // =============================== O += P.V issuer ===============================
-        if constexpr (L::kPInTmem) {
+        if constexpr (D == 128) {
             constexpr uint32_t idesc_o = umma_idesc(kBM, D, 0, 1);
-            const uint64_t v_desc = umma_desc(sbase + L::kOffV, kBN * 128, 1024);
+            const uint64_t v_desc = umma_desc(sbase + L::kOffV, kBN * 128, 1024), p_desc = umma_desc(sbase + L::kOffP, 16, 1024);
             bool ok = true;
             for (int j = 0; ok && j < ntiles; ++j) {
                 const int st = j & 1;
@@ -462,8 +482,12 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                     tc_fence_after();
                     if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < kBN / 16; ++kk)
-                            umma_f16_a_tmem(tmem_base + L::kColO + rt * D, tmem_base + L::kColP + (2 * rt + st) * (kBN / 2) + kk * 8, b + ((kk * (16 * 128)) >> 4), idesc_o, (j > 0 || kk > 0));
+                        for (int kk = 0; kk < kBN / 16; ++kk) {
+                            const uint64_t bk = b + ((kk * (16 * 128)) >> 4);   // V: MN-major, 16 positions per step
+                            const uint32_t o = tmem_base + L::kColO + rt * D;
+                            if constexpr (L::kPInTmem) umma_f16_a_tmem(o, tmem_base + L::kColP + st * (kBN / 2) + kk * 8, bk, idesc_o, (j > 0 || kk > 0));
+                            else umma_f16(o, p_desc + (((2 * rt + st) * L::kPBytes + kk * 32) >> 4), bk, idesc_o, (j > 0 || kk > 0));   // P: K-major, one 128-byte slab
+                        }
                         umma_commit(bar(P_EMPTY + 2 * rt + st));   // P buffer free, O holds tiles 0..j
                         if (j == ntiles - 1) umma_commit(bar(O_DONE + rt));   // O complete: the epilogue's signal for both groups
                         if (rt + 1 == live_tiles) umma_commit(bar(V_EMPTY + st));
@@ -598,10 +622,10 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             }
         };
         const int st = grp;
-        const uint32_t s_col = L::kColS + (L::kPInTmem && L::kSBufs == 1 ? rt : grp) * kBN, o_col = L::kColO + rt * D;
+        const uint32_t s_col = L::kColS + (2 * rt + grp) * kBN, o_col = L::kColO + rt * D;
         for (int j = grp; j < nt; j += 2) {
             const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);   // parity of the tile's pair
-            if (!mbar_wait(bar(S_FULL + (L::kPInTmem ? 2 * rt + st : 0)), ph)) { failed = true; break; }
+            if (!mbar_wait(bar(S_FULL + (L::kPInTmem ? st : rt)), ph)) { failed = true; break; }
             tc_fence_after();
             float s[kBN];
             {
@@ -680,7 +704,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 }
             }
             if constexpr (L::kPInTmem) {
-                tmem_st32_bits(tmem_base + lane_addr + L::kColP + (2 * rt + st) * (kBN / 2), pk);
+                tmem_st32_bits(tmem_base + lane_addr + L::kColP + st * (kBN / 2), pk);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // and the rescale's stores, if any
             } else {
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // the rescale's stores, if any
