@@ -1024,18 +1024,25 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
     return static_cast<size_t>(splits) * kv_heads * rows_padded * (head_dim + 2) * sizeof(float);
 }
 
-// How many KV splits: the number with the least estimated time, for `units` row-tile CTAs of up to `tiles` KV tiles.  A wave of
-// 148 CTAs costs its tiles and about 3 us; CTAs take the place of one another as they end, so a last wave that is not full costs less
-// than a whole one.  A split costs its partials' way out and back.  Measured per layer, all kernels (head_dim 256 / 24 heads and 128 / 32, q8_0):
-//   256:  20 tokens over 16000 (4 units):  8: 58, 12: 52, 16: 50         37 over 3001 (8):  6: 29.6, 8: 29.0, 10: 28.5, 16: 28.8
-//         128 over 8192 (24):  5: 50, 6: 48, 8: 65                       300 over 8192 (60):  1: 116, 2: 78, 3: 99
-//         512 over 8192 (96):  1: 117, 2: 139, 3: 110, 4: 142            512 over 2000 (96):  1: 54, 2: 65, 3: 60
-//   128:  37 over 3001 (16):  6: 21.1, 8: 20.2, 10: 28.8                 100 over 1000 (32):  1: 22.1, 3: 18.6, 4: 18.5
-//         200 over 2000 (56):  1: 34, 2: 29, 3: 36                       300 over 4000 (80):  1: 56, 2: 58, 3: 48, 4: 57
-//         400 over 16000 (104, two row tiles each):  1: 176, 2: 168, 3: 174, 4: 146
-// The estimate takes the best column of each.
-static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t most, uint32_t head_dim) {
-    const double tile_us = head_dim == 256 ? 0.6 : 0.4, wave_us = 3.0, partial_us = head_dim == 256 ? 0.03 : 0.01;
+// How many KV splits: the number with the least estimated time, for `units` CTAs of one or two row tiles and up to `tiles` KV tiles.  A wave of
+// 148 CTAs costs its tiles and a few us; CTAs take the place of one another as they end, so a last wave that is not full costs less
+// than a whole one.  A split costs its partials' way out and back.  Measured for a layer with its store kernel, us in a short burst (and, where the power
+// limit makes it another, in a long run), q8_0, the estimate's choice marked *:
+//   24 heads of 256:  20 tokens over 16000 (4 units):  8: 55, 12: 49, *16: 48        37 over 3001 (8):  6: 26.3, 8: 26.1, 10: 23.9, *11: 23.9, 16: 24.4
+//                     64 over 8192 (12):  8: 37, *12: 35, 13: 49                     128 over 8192 (24):  5: 45, *6: 44, 7: 64
+//                     300 over 8192 (60):  1: 123, *2: 77, 3: 98                     512 over 2000 (96):  *1: 50, 2: 61, 3: 57
+//                     512 over 8192 (96):  1: 123 (125), 2: 134 (137), *3: 110 (127), 4: 129 (139)
+//   32 of 128:        37 over 3001 (16):  6: 21.1, 8: 20.4, *9: 19.2, 10: 26.6       100 over 1000 (32):  1: 22.0, 3: 18.5, *4: 18.4
+//                     200 over 2000 (56):  1: 34, *2: 28, 3: 35                      300 over 4000 (80):  1: 57, 2: 57, *3: 48, 4: 56
+//                     400 over 16000 (104):  1: 184 (179), 2: 163 (170), 3: 176 (177), *4: 142 (165)
+//   the same, two row tiles a CTA:  1200 over 4000 (152):  1: 150, *2: 148, 3: 150 (153)        1200 over 8192:  1: 280, 2: 243 (250), *3: 237 (248), 4: 242 (255)
+//                     1600 over 4000 (200):  *1: 169 (171), 2: 167 (178)             1500 over 20000 (192):  1: 673, 2: 550 (620), *3: 534 (607), 4: 635 (650)
+//                     3000 over 8192 (376):  *1: 493 (542), 2: 565 (594)             4096 over 8192 (512):  *1: 706 (756), 2: 713 (790)
+// Two row tiles a CTA have costs of their own: with the single tiles', 1600 over 4000 and 4096 over 8192 were cut in 2, 2048 over 32000 in 4 (1128, long
+// run 1269; whole, as now: 1112 and 1218).
+static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t most, uint32_t head_dim, uint32_t tiles_per_cta) {
+    const double tile_us = tiles_per_cta == 2 ? 1.0 : head_dim == 256 ? 0.6 : 0.4, wave_us = 3.0;
+    const double partial_us = tiles_per_cta == 2 ? 0.07 : head_dim == 256 ? 0.03 : 0.01;
     uint32_t best = 1;
     double best_us = 0.0;
     for (uint32_t s = 1; s <= kMaxKvSplits && s <= (most > 1 ? most : 1); ++s) {
@@ -1092,7 +1099,7 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
         // where the chunk's own triangle is longer than its prefix, eight of the prefix, which is all that its first rows see.
         const uint32_t tiles = static_cast<uint32_t>((rows + kBN - 1) / kBN), prefix_tiles = (base_position + kBN - 1) / kBN;
         const uint32_t most = prefill_state != nullptr ? 1 : base_position >= token_count ? tiles / 3 : prefix_tiles / 8;
-        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, most, view.head_dim);
+        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, most, view.head_dim, tiles_per_cta);
         const size_t scratch = prefill_tc5_workspace_bytes(static_cast<uint32_t>(rows), view.kv_heads, view.head_dim);
         while (want > 1 && workspace_bytes < scratch + 1024 + prefill_tc5_split_bytes(token_count, query_heads, view.kv_heads, view.head_dim, want)) --want;
         if (want > 1) {

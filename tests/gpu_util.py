@@ -123,6 +123,11 @@ def captured_kernels(call):
     return names
 
 
+def captured_grids(call):
+    """Grid sizes of the kernels that `call(stream)` captures; nothing runs."""
+    return [tuple(k.dims[:3]) for k in _captured_kernel_nodes(call)[2]]
+
+
 def captured_parameter_blocks(call):
     """The first parameter, as bytes, of every kernel that `call(stream)` captures; nothing runs."""
     import ctypes as C
