@@ -625,7 +625,9 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         const uint32_t s_col = L::kColS + (2 * rt + grp) * kBN, o_col = L::kColO + rt * D;
         for (int j = grp; j < nt; j += 2) {
             const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);   // parity of the tile's pair
-            if (!mbar_wait(bar(S_FULL + (L::kPInTmem ? st : rt)), ph)) { failed = true; break; }
+            // The loop holds warp-wide loads, stores and votes, so a warp leaves it as a whole: a lane whose wait runs out goes on, with values nobody
+            // will see, up to the one vote below.
+            bool lost = !mbar_wait(bar(S_FULL + (L::kPInTmem ? st : rt)), ph);
             tc_fence_after();
             float s[kBN];
             {
@@ -641,8 +643,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             const uint32_t pos0 = static_cast<uint32_t>(tile0 + j) * kBN;
             // Raw scores stay unscaled; the softmax scale is folded into the exponent: p = 2^(s*c - m*c).  The loop's instructions count: products and
             // sums go in pairs, maxima three values at a time.  32 / 8 heads of 128, 1024 tokens over 8192: 168.0 -> 163.7 us; 24 / 4 of 256, 512 over
-            // 8192: 111.6 -> 110.3.  (The compiler's schedule of this loop depends on what follows it: always measure 1024 over 8192 and 512 over 8192.
-            // With the maximum of a poisoned split replaced below, where it is stored, they took 179 and 113 us.)
+            // 8192: 111.6 -> 110.3.
             // Only the tiles that straddle this row's causal length need the mask.
             if (pos0 + kBN > len) {
 #pragma unroll
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             // the reference as the previous tile (the other group's) left it; lazy rescale: keep it unless this tile's
             // maximum outgrew it by more than the threshold
             float m_prev = -INFINITY;
-            if (j > 0 && !ref_after(static_cast<uint32_t>(j), &m_prev)) { failed = true; break; }
+            if (j > 0 && !ref_after(static_cast<uint32_t>(j), &m_prev)) lost = true;
             float alpha = 1.0f, m_new = m_prev;
             if (mt > m_prev + kRescaleThreshold || (m_prev == -INFINITY && mt > -INFINITY)) {
                 alpha = (m_prev == -INFINITY) ? 0.0f : ex2_approx(m_prev - mt);
@@ -668,6 +669,10 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             // published at once (the other group's thread of this row waits for it): no later work may be scheduled before it
             asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(smem_u32(const_cast<unsigned long long*>(ref))),
                          "l"((static_cast<unsigned long long>(static_cast<uint32_t>(j) + 1u) << 32) | __float_as_uint(m_new)) : "memory");
+            // What follows takes the reference out of a shuffle, which goes out behind the store.  Without it versions of this loop that differ in their
+            // exits alone took 166 or 182 us for 1024 over 8192 (32 / 8 heads of 128), the slow ones with five more polls of the reference a
+            // tile: the store came late.  No version without P in TMEM had that, and there the shuffle costs 1 to 2 %.
+            if constexpr (L::kPInTmem) m_new = __shfl_sync(0xffffffffu, m_new, lane);
             rebase(m_new);
             const float neg_ref = (m_new == -INFINITY) ? 0.0f : -m_new;
             Pair sum = 0;
@@ -687,12 +692,13 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 l_sum += halves.x + halves.y;
             }
             // this group's P buffer is free once the P.V of its previous tile has completed
-            if (!mbar_wait(bar(P_EMPTY + 2 * rt + st), ph ^ 1)) { failed = true; break; }
+            if (!mbar_wait(bar(P_EMPTY + 2 * rt + st), ph ^ 1)) lost = true;
             tc_fence_after();
-            if (__any_sync(0xffffffffu, alpha != 1.0f) && j > 0) {
+            if (__any_sync(0xffffffffu, alpha != 1.0f || lost) && (j > 0 || __any_sync(0xffffffffu, lost))) {
                 // rare: the reference moved.  O holds tiles 0..j-1 once the previous tile's P.V (the other group's) has
                 // completed; then this warp rescales its 32 rows of O in TMEM before its own P is released.
-                if (!mbar_wait(bar(P_EMPTY + 2 * rt + (st ^ 1)), static_cast<uint32_t>(((j - 1) >> 1) & 1))) { failed = true; break; }
+                if (j > 0 && !mbar_wait(bar(P_EMPTY + 2 * rt + (st ^ 1)), static_cast<uint32_t>(((j - 1) >> 1) & 1))) lost = true;
+                if (__any_sync(0xffffffffu, lost)) { failed = true; break; }
                 tc_fence_after();
 #pragma unroll 1
                 for (int c0 = 0; c0 < D; c0 += 32) {
