@@ -346,7 +346,7 @@ decode_q8_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__
     int stage = 0;
     uint32_t phase = 0;
     for (int i = 0; i < ntiles; ++i) {
-        if (!mbar_wait(bars + stage * 8, phase)) { failed = true; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(bars + stage * 8, phase))) { failed = true; break; }   // the whole warp: the loop holds MMAs and votes
         const uint32_t pos0 = (t0 + i) * kTile;
         const int lo = begin > pos0 ? static_cast<int>(begin - pos0) : 0;
         const int hi = end - pos0 < static_cast<uint32_t>(kTile) ? static_cast<int>(end - pos0) : kTile;

@@ -22,7 +22,7 @@ def bodies(text, head):
     return found
 
 
-@pytest.mark.parametrize("name,head", [("prefill_tc5.cu", "for (int j = grp; j < nt; j += 2) {")])
+@pytest.mark.parametrize("name,head", [("prefill_tc5.cu", "for (int j = grp; j < nt; j += 2) {"), ("decode_q8.cu", "for (int i = 0; i < ntiles; ++i) {")])
 def test_left_by_whole_warps(name, head):
     loops = bodies(re.sub(r"//[^\n]*", "", (CSRC / name).read_text()), head)
     assert len(loops) == 1 and re.search(r"_sync\(|tmem_ld|mma_", loops[0])
