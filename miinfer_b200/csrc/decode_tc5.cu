@@ -573,7 +573,7 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
         }
         if (TL && tid == 0) tl[5] = global_ns();
         // ---- the CTA's partial leaves at once: thread = dim holds all four heads ----
-        if (lane == 0 && failed) atomicOr(fail_flag, 1u);
+        if (failed) atomicOr(fail_flag, 1u);
         asm volatile("bar.sync 3, 128;" ::: "memory");
         float lt[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll

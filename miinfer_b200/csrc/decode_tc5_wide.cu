@@ -598,8 +598,8 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
         if (lane == 0) {
 #pragma unroll
             for (int h = 0; h < G; ++h) lsm[(grp * 4 + wq) * 8 + h] = l_run[h];
-            if (failed) atomicOr(fail_flag, 1u);
         }
+        if (failed) atomicOr(fail_flag, 1u);
         // ---- the odd tiles' group hands its state to the even tiles' group through its own P buffer (the P.V MMAs that read it
         //      have completed; the other buffer may still be feeding the even group's last P.V) ----
         float* hand = reinterpret_cast<float*>(smem + L::kOffP + L::kPBuf);   // [3 * G][128]: acc of half 0, acc of half 1, maxima

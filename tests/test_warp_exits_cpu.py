@@ -30,3 +30,19 @@ def test_left_by_whole_warps(name, head):
     assert exits
     for line in exits:
         assert re.search(r"if \(!?(__any_sync|__all_sync|mbar_wait_warp)\(", line), line.strip()
+
+
+@pytest.mark.parametrize("name", ["decode_tc5.cu", "decode_tc5_wide.cu"])
+def test_any_lane_poisons_its_partial(name):
+    """These loops are not left: waits behind one that ran out are passed by, and the CTA's partial becomes NaN, whichever lane it was."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    at = [m.start() for m in re.finditer(r"atomicOr\(fail_flag", text)]
+    assert len(at) == 1
+    opened = []
+    for i, c in enumerate(text[:at[0]]):
+        if c == "{":
+            opened.append(text[text.rfind("\n", 0, i) + 1:i])
+        elif c == "}":
+            opened.pop()
+    guards = [g for g in opened + [text[text.rfind("\n", 0, at[0]) + 1:at[0]]] if re.search(r"\b(lane|tid)\b", g)]
+    assert not guards, guards
