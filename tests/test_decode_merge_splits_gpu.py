@@ -25,12 +25,29 @@ def test_split_counts(cuda, splits, d, H, G, mode, rel):
     q, gate = torch.randn(Hq, d, generator=g, device="cuda"), torch.randn(Hq, d, generator=g, device="cuda")
     out, gated = torch.empty(Hq, d, device="cuda"), torch.empty(Hq, d, device="cuda")
     ws = kv.decode_workspace(Hq, d)
-    for _ in range(2):      # the second launch finds the words of the first one zeroed
+
+    def go():
         kv.launch_decode_attention_quant(st.view(), q, query_heads=Hq, scale=d ** -0.5, cache_length=L, output=out, gate=gate, gated_output=gated,
                                          workspace=ws, num_splits=splits)
-    torch.cuda.synchronize()
-    p = (torch.einsum("hgd,hld->hgl", q.double().view(H, G, d), k) * d ** -0.5).softmax(-1)
-    ref = torch.einsum("hgl,hld->hgd", p, v).flatten(0, 1)
-    assert ((out.double() - ref).norm() / ref.norm()).item() <= rel
-    ref = ref * gate.double().sigmoid()
-    assert ((gated.double() - ref).norm() / ref.norm()).item() <= rel
+
+    def check():
+        torch.cuda.synchronize()
+        p = (torch.einsum("hgd,hld->hgl", q.double().view(H, G, d), k) * d ** -0.5).softmax(-1)
+        ref = torch.einsum("hgl,hld->hgd", p, v).flatten(0, 1)
+        assert ((out.double() - ref).norm() / ref.norm()).item() <= rel
+        ref = ref * gate.double().sigmoid()
+        assert ((gated.double() - ref).norm() / ref.norm()).item() <= rel
+        assert ws.count_nonzero().item() == 0      # what a merge reads it zeroes
+
+    go()
+    check()
+    # replays of a captured launch share its tag: words that one left behind would pass for the next one's
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        go()
+    for _ in range(3):
+        q.copy_(torch.randn(Hq, d, generator=g, device="cuda"))
+        out.fill_(float("nan"))
+        gated.fill_(float("nan"))
+        graph.replay()
+        check()
