@@ -56,20 +56,17 @@ template <bool IN_F16>
 constexpr int kAppendCtasPerSm = IN_F16 ? 10 : 8;   // 20 warps of 96 registers: a unit, the next one's raw input and the rotation (fp32 input: 16 of 128);
                                                     // head_dim 256 with fp16 input spills 8 bytes of them
 
-// Two fp32 products in one instruction (each rounds like its scalar form; .ftz as the scalar intrinsics under this build).
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pack(float lo, float hi) { Pair r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ float2 unpack(Pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+// Two fp32 products in one instruction (.ftz as the scalar intrinsics under this build).
 __device__ __forceinline__ Pair mul2(Pair a, Pair b) { Pair r; asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 // Sums of products are taken one at a time: an f32x2 add behind an f32x2 multiply came out contracted (measured: single
 // fp16 results one unit off the oracle's), the scalar intrinsics never are.
 __device__ __forceinline__ Pair add_products(Pair t, Pair u) {
-    const float2 a = unpack(t), b = unpack(u);
-    return pack(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+    const float2 a = unpack_pair(t), b = unpack_pair(u);
+    return pack_pair(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
 }
 __device__ __forceinline__ Pair sub_products(Pair t, Pair u) {
-    const float2 a = unpack(t), b = unpack(u);
-    return pack(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
+    const float2 a = unpack_pair(t), b = unpack_pair(u);
+    return pack_pair(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
 }
 
 // Four consecutive input elements as they lie in memory, and as two pairs of floats.
@@ -96,26 +93,26 @@ template <bool IN_F16>
 __device__ __forceinline__ void widen(const Raw4<IN_F16>& r, Pair (&x)[2]) {
     if constexpr (IN_F16) {
         const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&r.v.y));
-        x[0] = pack(a.x, a.y); x[1] = pack(b.x, b.y);
+        x[0] = pack_pair(a.x, a.y); x[1] = pack_pair(b.x, b.y);
     } else {
-        x[0] = pack(r.v.x, r.v.y); x[1] = pack(r.v.z, r.v.w);
+        x[0] = pack_pair(r.v.x, r.v.y); x[1] = pack_pair(r.v.z, r.v.w);
     }
 }
 __device__ __forceinline__ float amax4(const Pair (&x)[2]) {
-    const float2 a = unpack(x[0]), b = unpack(x[1]);
+    const float2 a = unpack_pair(x[0]), b = unpack_pair(x[1]);
     return fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))), 0.0f);   // a NaN counts as 0, as in warp_amax
 }
 // round to nearest even, saturate to [-128, 127], NaN -> 0: quantize_s8 on four values, packed
 __device__ __forceinline__ uint32_t quantize4(const Pair (&x)[2], float inv) {
-    const Pair inv2 = pack(inv, inv);
-    const float2 a = unpack(mul2(x[0], inv2)), b = unpack(mul2(x[1], inv2));
+    const Pair inv2 = pack_pair(inv, inv);
+    const float2 a = unpack_pair(mul2(x[0], inv2)), b = unpack_pair(mul2(x[1], inv2));
     uint32_t w;
     asm("{ .reg .b32 t; cvt.pack.sat.s8.s32.b32 t, %4, %3, 0; cvt.pack.sat.s8.s32.b32 %0, %2, %1, t; }"
         : "=r"(w) : "r"(__float2int_rn(a.x)), "r"(__float2int_rn(a.y)), "r"(__float2int_rn(b.x)), "r"(__float2int_rn(b.y)));
     return w;
 }
 __device__ __forceinline__ uint2 half4(const Pair (&x)[2]) {
-    const float2 a = unpack(x[0]), b = unpack(x[1]);
+    const float2 a = unpack_pair(x[0]), b = unpack_pair(x[1]);
     const __half2 lo = __floats2half2_rn(a.x, a.y), hi = __floats2half2_rn(b.x, b.y);
     return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
@@ -198,10 +195,10 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
 #pragma unroll
             for (int i = 0; i < SC; ++i) sincos_pinned(__fmul_rn(static_cast<float>(position), freq[i]), &s[i], &c[i]);
             if constexpr (RPS == 1) {
-                sn[0] = pack(s[0], s[1]); sn[1] = pack(s[2], s[3]);
-                cs[0] = pack(c[0], c[1]); cs[1] = pack(c[2], c[3]);
+                sn[0] = pack_pair(s[0], s[1]); sn[1] = pack_pair(s[2], s[3]);
+                cs[0] = pack_pair(c[0], c[1]); cs[1] = pack_pair(c[2], c[3]);
             } else {
-                const Pair sm = pack(s[0], s[1]), cm = pack(c[0], c[1]);
+                const Pair sm = pack_pair(s[0], s[1]), cm = pack_pair(c[0], c[1]);
                 const Pair so = __shfl_xor_sync(0xffffffffu, sm, 16), co = __shfl_xor_sync(0xffffffffu, cm, 16);
                 sn[0] = sub ? so : sm; sn[1] = sub ? sm : so;
                 cs[0] = sub ? co : cm; cs[1] = sub ? cm : co;
@@ -213,8 +210,8 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int src = 4 * (lane & 7) + 2 * i;
-                sn[i] = pack(__shfl_sync(0xffffffffu, s, src), __shfl_sync(0xffffffffu, s, src + 1));
-                cs[i] = pack(__shfl_sync(0xffffffffu, c, src), __shfl_sync(0xffffffffu, c, src + 1));
+                sn[i] = pack_pair(__shfl_sync(0xffffffffu, s, src), __shfl_sync(0xffffffffu, s, src + 1));
+                cs[i] = pack_pair(__shfl_sync(0xffffffffu, c, src), __shfl_sync(0xffffffffu, c, src + 1));
             }
         }
     };
@@ -233,7 +230,7 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
                 for (int s = 0; s < 4; ++s) {
                     const bool up2 = lane & (LPR / 2), up1 = lane & (LPR / 4);
                     const Pair q01 = add_products(mul2(a[s][0], a[s][0]), mul2(b[s][0], b[s][0])), q23 = add_products(mul2(a[s][1], a[s][1]), mul2(b[s][1], b[s][1]));   // stride D/2
-                    const float2 t = unpack(add_products(up2 ? q23 : q01, __shfl_xor_sync(0xffffffffu, up2 ? q01 : q23, LPR / 2)));                                // stride D/4
+                    const float2 t = unpack_pair(add_products(up2 ? q23 : q01, __shfl_xor_sync(0xffffffffu, up2 ? q01 : q23, LPR / 2)));                                // stride D/4
                     float ss = __fadd_rn(up1 ? t.y : t.x, __shfl_xor_sync(0xffffffffu, up1 ? t.x : t.y, LPR / 4));                                        // stride D/8
 #pragma unroll
                     for (int o = LPR / 8; o > 0; o >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));                                        // down to stride 4
@@ -246,12 +243,12 @@ append_kernel(const __grid_constant__ AppendParams p, const bool vec) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float* src = p.k_norm_weight + (i >> 1) * (D / 2) + 4 * l + 2 * (i & 1);
-                    w[i] = pack(src[0], src[1]);
+                    w[i] = pack_pair(src[0], src[1]);
                 }
 #pragma unroll
                 for (int s = 0; s < 4; ++s) {
                     const float r = __shfl_sync(0xffffffffu, r_mine, (lane & ~3) | s);
-                    const Pair r2 = pack(r, r);
+                    const Pair r2 = pack_pair(r, r);
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         a[s][i] = mul2(mul2(a[s][i], r2), w[i]);

@@ -75,6 +75,11 @@ int snapshot_copy_layers(const b200kv_view* views, uint32_t layers, uint64_t tok
 
 // ---- device helpers ------------------------------------------------------------
 
+// Two fp32 values for the f32x2 instructions (each half rounds like its scalar form).
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pack_pair(float lo, float hi) { Pair r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 unpack_pair(Pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -176,10 +176,7 @@ __device__ __forceinline__ void umma_f16_a_tmem(uint32_t tmem_d, uint32_t tmem_a
 __device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
-// Two fp32 values in one instruction (each rounds like its scalar form), and the largest of three.
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pack_pair(float lo, float hi) { Pair r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ float2 unpack_pair(Pair v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+// Two fp32 values in one instruction, and the largest of three.
 __device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) { Pair r; asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ Pair add_pair(Pair a, Pair b) { Pair r; asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.ftz.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
