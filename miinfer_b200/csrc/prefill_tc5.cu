@@ -584,8 +584,8 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             mbar_arrive(bar(Q_FULL));
-            // P tiles are written by every warp of a group: nobody may write one while a neighbour still turns rows in it
-            asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
+            // Where Q is turned in the P tiles: a P tile is written by every warp of a group, and nobody may write one while a neighbour still turns rows in it
+            if constexpr (L::kQInTmem && !L::kPInTmem) asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
         }
         // =============================== softmax rows ===============================
         // Two groups of 128 threads, one thread per query row in each: warps 0-3 take the even tiles, warps 4-7 the odd
