@@ -387,8 +387,8 @@ __device__ __forceinline__ void fused_merge(const DecodeParams& p, uint32_t sess
                 tot.x = fmaf(fa[u], a, tot.x);
                 tot.y = fmaf(fb[u], a, tot.y);
             }
-            // consumed: accumulator words by the thread that read them; (m, l) words are read by all 64 threads of
-            // the group, so they are zeroed after the fold barrier below
+            // consumed: accumulator words by the thread that read them; (m, l) words are read by a lane of each of the
+            // group's two warps, so they are zeroed after the fold barrier below
 #pragma unroll
             for (int u = 0; u < kBatch; ++u)
                 if (sp0 + grp + kGroups * u < S) zero2(base + (sp0 + grp + kGroups * u) * stride + 2 * pr);

@@ -1006,7 +1006,7 @@ int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half*
         mp.total_rows = p.token_count * G;
         const size_t work = static_cast<size_t>(mp.total_rows) * (D / 4);
         // A thread's loads are laid out for the most splits of its kernel: 38, 64, 93 and 114 registers, i.e. six, four, two and two blocks an SM.  24 / 4 heads
-        // of 256, us a layer, for 4 and 16 alone -> these: 128 over 8192 (6 splits) 47.5 -> 44.7, 37 over 3001 (10) 26.5 -> 25.8.
+        // of 256, us a layer, for 4 and 16 alone -> these: 128 over 8192 (6 splits) 47.5 -> 44.7, 37 over 3001 (11) 26.5 -> 25.8.
         const auto merge = p.kv_splits <= 4   ? prefill_merge_kernel<D, 4>
                            : p.kv_splits <= 8  ? prefill_merge_kernel<D, 8>
                            : p.kv_splits <= 12 ? prefill_merge_kernel<D, 12>
