@@ -584,8 +584,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             mbar_arrive(bar(Q_FULL));
-            // Where Q is turned in the P tiles: a P tile is written by every warp of a group, and nobody may write one while a neighbour still turns rows in it
-            if constexpr (L::kQInTmem && !L::kPInTmem) asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
+            // no barrier: what a warp turns its rows in are its own rows of its group's P tile
         }
         // =============================== softmax rows ===============================
         // Two groups of 128 threads, one thread per query row in each: warps 0-3 take the even tiles, warps 4-7 the odd
@@ -669,9 +668,10 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             // published at once (the other group's thread of this row waits for it): no later work may be scheduled before it
             asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(smem_u32(const_cast<unsigned long long*>(ref))),
                          "l"((static_cast<unsigned long long>(static_cast<uint32_t>(j) + 1u) << 32) | __float_as_uint(m_new)) : "memory");
-            // What follows takes the reference out of a shuffle, which goes out behind the store.  Without it versions of this loop that differ in their
-            // exits alone took 166 or 182 us for 1024 over 8192 (32 / 8 heads of 128), the slow ones with five more polls of the reference a
-            // tile: the store came late.  No version without P in TMEM had that, and there the shuffle costs 1 to 2 %.
+            // One row tile of 128 comes at 166 or 182 us for 1024 over 8192 (32 / 8 heads) by small things around this loop, its exits or the text of the epilogue:
+            // in the slow builds a warp polls the other group's reference five times more a tile.  With this one's exits it is 182, and 167 with the
+            // reference of what follows out of a shuffle behind the store.  That holds for this text only: measure 1024 over 8192 after a change.
+            // Without P in TMEM the shuffle costs 1 to 2 %.
             if constexpr (L::kPInTmem) m_new = __shfl_sync(0xffffffffu, m_new, lane);
             rebase(m_new);
             const float neg_ref = (m_new == -INFINITY) ? 0.0f : -m_new;
