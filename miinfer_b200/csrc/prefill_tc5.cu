@@ -9,31 +9,28 @@
 //  2. The attention kernel gives each CTA 128 query ROWS of one kv head (a row is a (token, head-of-group)
 //     pair, so the G heads of a group share every K/V tile) and walks the causal range in tiles of 64 positions,
 //     two tiles at a time:
-//       - two threads feed the K ring (two stages of a PAIR of tiles each) and the V ring (two tiles) with TMA
+//       - the K ring (two stages of a PAIR of tiles each) and the V ring are fed with TMA
 //         tensor copies (64x64 boxes, 128-byte swizzle: exactly the canonical shared-memory layout of the MMA
 //         operands; the two tiles of a pair lie in rows 0-63 and 64-127 of every slab, one B operand);
-//       - one thread issues S = Q.K^T for a pair of tiles at once (tcgen05.mma M128 x N128, K = d, Q read from
-//         TMEM: issuing such an MMA takes this thread 50 to 100 clocks, the tensor pipe 32 at N = 64 and 64 at N = 128, so
-//         pairs keep the issue out of the pipe's way), another O += P.V per tile (M128 x N = d, K = 64; V consumed MN-major, as
-//         stored) into the O accumulator in TMEM; completion is tracked by tcgen05.commit on mbarriers;
-//       - two groups of 128 softmax threads, one thread per row in each, take the first and the second tile of
-//         every pair: tcgen05.ld the S row, scale/mask (causal length per row, .hip:6829), online softmax in base
-//         2 with LAZY rescaling (O and the running sums are only rescaled when a row's maximum grows by more
-//         than 2^8; P <= 256 fits fp16; the row's reference maximum is handed from tile to tile through shared
-//         memory), write P as fp16 into one of two swizzled A-operand tiles, and at the end scale O by 1/sum,
-//         apply the sigmoid gate (.hip:6714-6723) and store.
-//     TMEM: S (pair) | Q | O = 128 + d/2 + d columns.  Shared memory: 2 x 2 K tiles + 2 V tiles + 2 P tiles.  A single row tile of
-//     head_dim 128 has S tile by tile and P in TMEM as well (Layout::kPInTmem).
-//     At head_dim 128 a CTA takes TWO row tiles where there are enough of them (512 softmax threads; S and O of both fill
-//     TMEM, so Q is an A operand in shared memory): a single tile's loop waits for its softmax (about 1 us a pair of KV tiles against
-//     0.5 us of MMAs), two share every K and V tile and one's MMAs run under the other's softmax.  2048 fresh
-//     tokens, 32/8 heads, when the choice was made: 79 us as single tiles dispatched shortest first, 66 longest first, 56 with two per CTA
-//     (96 registers a thread, 12 bytes of them spilled).
+//       - one lane of a warp that stays together issues S = Q.K^T (tcgen05.mma M128, K = d, Q read from TMEM), another O += P.V per tile
+//         (M128 x N = d, K = 64; V consumed MN-major, as stored) into the O accumulator in TMEM; completion is tracked by
+//         tcgen05.commit on mbarriers;
+//       - groups of 128 softmax threads, one thread per row in each, take the tiles in turn: tcgen05.ld the S row, scale/mask (causal
+//         length per row, .hip:6829), online softmax in base 2 with LAZY rescaling (O and the running sums are only rescaled when a row's
+//         maximum grows by more than 2^8; P <= 256 fits fp16; the row's reference maximum is handed from tile to tile through shared
+//         memory), hand P over as fp16, and at the end scale O by 1/sum, apply the sigmoid gate (.hip:6714-6723) and store.
+//     head_dim 256: two groups; S for a pair of tiles at once (N = 128: issuing an MMA takes 50 clocks and more, the tensor pipe 32 at N = 64 and 64 at
+//     N = 128), P in shared memory.  TMEM: S (pair) | Q | O.
+//     head_dim 128: S tile by tile into four buffers of TMEM columns, P written over its own scores (the A operand of P.V comes from there), two warps that
+//     issue S.  One row tile a CTA has four groups and four tiles under way (a tile takes 790 clocks, 512 of them MMAs; the softmax threads' chain through
+//     it 3000).  A CTA takes TWO row tiles, two groups and buffers each, where there are enough of them: they share every K and V tile, and set-up, Q and output
+//     come once for both; their S and O fill TMEM, so Q is an A operand in shared memory.
 // Every mbarrier wait is bounded; a wait that runs out poisons the output rows with NaN, and the CTA still frees
 // its TMEM and exits.
 #include "decode_common.cuh"
 #include "dequant.cuh"
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -182,6 +179,17 @@ __device__ __forceinline__ Pair add_pair(Pair a, Pair b) { Pair r; asm("add.rn.f
 __device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.ftz.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 // A wait of a whole warp, which stays together: all lanes go on or none.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+// The same for two barriers, asked at once.
+__device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
+    bool ok = false;
+    for (uint32_t spin = 0; spin < kSpin && !ok; ++spin) {
+        uint32_t a, b;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(a) : "r"(bar_a), "r"(parity_a) : "memory");
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(b) : "r"(bar_b), "r"(parity_b) : "memory");
+        ok = (a & b) != 0;
+    }
+    return __all_sync(0xffffffffu, ok);
+}
 // One lane of a converged warp, always the same one.
 __device__ __forceinline__ bool elect_one() {
     uint32_t ok;
@@ -197,12 +205,14 @@ __device__ __forceinline__ float ex2_approx(float x) {
 template <int D, int RT>
 struct Layout {
     // warps: two softmax groups per row tile (one thread per query row: even tiles, odd tiles), then one warp per role
-    static constexpr int kSoftmaxThreads = RT * 256;
+    static constexpr int kGroups = D == 128 ? 4 / RT : 2;  // softmax groups of a row tile; tile j is group j % kGroups's
+    static constexpr int kSoftmaxThreads = RT * kGroups * 128;
     static constexpr int kTmaWarp = kSoftmaxThreads / 32;  // TMA producer of the K tiles
     static constexpr int kSWarp = kTmaWarp + 1;            // S = Q.K^T issuer / TMEM owner
-    static constexpr int kPvWarp = kTmaWarp + 2;           // O += P.V issuer
-    static constexpr int kTmaVWarp = kTmaWarp + 3;         // TMA producer of the V tiles (a K load never waits for a V stage)
-    static constexpr int kThreads = kSoftmaxThreads + 128;
+    static constexpr int kIssuers = D == 128 ? 2 : 1;      // warps that issue S (two row tiles: one each; one: even and odd tiles)
+    static constexpr int kPvWarp = kSWarp + kIssuers;      // O += P.V issuer
+    static constexpr int kTmaVWarp = kPvWarp + 1;         // D == 256: TMA producer of the V tiles (a K load never waits for a V stage)
+    static constexpr int kThreads = (kPvWarp + (D == 256 ? 2 : 1)) * 32;
     static constexpr int kRows = RT * kBM;
     static constexpr bool kQInTmem = RT == 1;              // two row tiles' S, P and O fill TMEM: their Q stays in shared memory
     static constexpr int kSlabs = D / 64;                  // 128-byte (64 x fp16) slabs along d
@@ -210,63 +220,65 @@ struct Layout {
     static constexpr int kPairBytes = 2 * kTileBytes;      // two K tiles as one B operand: [slab][128 rows][128 B]
     static constexpr int kOffK = 0;
     static constexpr int kOffV = kOffK + kKPairs * kPairBytes;
-    static constexpr int kOffP = kOffV + 2 * kTileBytes;   // [row tile][2][row][128 B] fp16 P tiles; Q (kQInTmem) and O are turned there (kPInTmem: only that)
+    static constexpr int kVTiles = D == 128 ? 5 : 2;       // V ring: with one producer for K and V, K must not wait for a V stage
+    static constexpr int kOffP = kOffV + kVTiles * kTileBytes;   // D == 256: [group][row][128 B] fp16 P tiles; 4 KB a warp in which Q (kQInTmem) and O are turned (two row tiles: over their Q)
     static constexpr int kPBytes = kBM * 128;
-    static constexpr int kOffQ = kOffP + RT * 2 * kPBytes; // [row tile][slab][row][128 B]
+    static constexpr int kOffQ = kOffP + (kQInTmem ? RT * kGroups * kPBytes : 0); // [row tile][slab][row][128 B]
     static constexpr int kQBytes = kSlabs * kBM * 128;
     static constexpr int kOffBar = kOffQ + (kQInTmem ? 0 : RT * kQBytes);
-    // One row tile of head_dim 128: P as an A operand in TMEM, which takes its writes and reads out of shared memory, and S tile by tile in two
-    // buffers.  32 / 8 heads, us a layer: 1024 tokens over 8192 184.6 -> 168.0, 300 over 4000 63.0 -> 56.7, 128 over 8192 41.0 -> 39.2.
+    // head_dim 128: P as an A operand in TMEM, in the first 32 columns of its own scores, which takes its writes and reads out of shared memory, and S tile
+    // by tile in as many buffers as there are groups.  32 / 8 heads, us a layer, against two groups (one row tile) and pairs of S tiles with P in shared
+    // memory (two): 461 over 8919 109 -> 97, 1024 over 8192 180 -> 169, 2048 fresh 58.7 -> 57.1.
     // At 256 S, Q and O leave no columns for P beside a pair of S tiles; with single ones in their place a layer of 512 tokens over 8192 took
-    // 134 us, not 125.  Two row tiles have columns for one S tile each beside P, and score MMAs of N = 64 then read Q from shared memory
-    // for every tile, not for every pair (96 KB of operands, not 64): 32 / 8 heads, a layer of 3000 over 8192 in a long run of
-    // them 545 us that way and 533 with S in pairs and P in shared memory, 1200 over 4000 156 and 150, 1400 over 2048 100.0 and 97.4, 2048 fresh 59.2 and 59.2.
-    static constexpr bool kPInTmem = D == 128 && RT == 1;
+    // 134 us, not 125.
+    static constexpr bool kPInTmem = D == 128;
     // mbarriers; the ones after V_EMPTY are per row tile, S_EMPTY and the P pairs (kPInTmem: S_FULL too) per row tile and softmax group
-    static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, S_FULL = 8, S_EMPTY = S_FULL + (kPInTmem ? 2 : RT), P_FULL = S_EMPTY + 2 * RT,
-                         P_EMPTY = P_FULL + 2 * RT, O_DONE = P_EMPTY + 2 * RT, Q_FULL = O_DONE + RT, kNumBars = Q_FULL + 1;
+    static constexpr int kBufs = RT * kGroups;
+    static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = V_FULL + kVTiles, S_FULL = V_EMPTY + kVTiles, S_EMPTY = S_FULL + (kPInTmem ? kBufs : RT),
+                         P_FULL = S_EMPTY + (kPInTmem ? 0 : kBufs), P_EMPTY = P_FULL + kBufs, O_DONE = P_EMPTY + kBufs, Q_FULL = O_DONE + RT, kNumBars = Q_FULL + 1;
     static constexpr int kOffSlot = kOffBar + (kNumBars * 8 + 15) / 16 * 16;
     static constexpr int kOffRef = kOffSlot + 16;                 // [rows] {reference maximum, sequence}: handed from tile to tile
     // [2 groups][128 rows] partial row sums of a row tile in its epilogue, where its own score MMAs are through: over the K
     // ring, or over the row tile's Q where the other row tile may still need K
-    static constexpr int kOffSum = kQInTmem ? kOffK : kOffQ, kSumStride = kQBytes;
-    static constexpr int kTotal = kOffRef + kRows * 8;
+    static constexpr int kSumStride = kGroups * kBM * 4;
+    static constexpr int kOffSum = kQInTmem ? kOffK : kOffRef + kRows * 8;
+    static constexpr int kTotal = kOffRef + kRows * 8 + (kQInTmem ? 0 : RT * kSumStride);
     static constexpr int kAlloc = kTotal;   // the dynamic shared memory is declared 1024-byte aligned; the kernel checks it
     static_assert(kAlloc <= 232448, "227 KB per CTA");
     static constexpr uint32_t kTmemCols = 512;
-    // S: RT x 2 x 64, P (kPInTmem): 2 x 32 (fp16 pairs), Q (RT == 1): D/2 (fp16 pairs), O: RT x D
-    [[maybe_unused]] static constexpr uint32_t kColP = 128;
-    static constexpr uint32_t kColS = 0, kColQ = kPInTmem ? 192 : 128, kColO = 256;
-    static_assert(RT == 1 ? kColQ + D / 2 <= kColO && kColO + D <= 512 : 2 * 128 <= kColO && kColO + 2 * D <= 512, "TMEM columns");
+    // S: RT x kGroups x 64, P (kPInTmem, fp16 pairs) in the first 32 of its S; Q (RT == 1): D/2 (fp16 pairs), O: RT x D
+    static constexpr uint32_t kColS = 0, kColQ = kPInTmem ? 384 : 128, kColO = 256;
+    static_assert(kColO + RT * D <= 512 && (RT == 2 || (kPInTmem ? kColO + D <= kColQ && kColQ + D / 2 <= 512 : kColQ + D / 2 <= kColO)), "TMEM columns");
 };
 
-// Elements in front of a row of [token][query_heads][D], for rows (tokens' heads of one kv head) four apart: one division, then additions.  (Two
-// divisions for each of a thread's eight rows were 1.3 us of a CTA's start and as much of its end.)
+// The eight rows a lane takes of a warp's 32 (every fourth from `row`; rows are tokens' heads of one kv head) in [token][query_heads][D]: elements from
+// the row of the warp's first token, which lie close enough for 32 bits.  One division, then additions.  (Two divisions for each row were 1.3 us
+// of a CTA's start and as much of its end, 64-bit offsets worked out along with the loads and stores 0.3 us of each 32 columns of output.)
 template <int D>
-struct RowWalk {
-    size_t off, step, wrap;
-    uint32_t in_group, step_in_group, G;
-    __device__ __forceinline__ RowWalk(uint32_t row, uint32_t kv_head, uint32_t G_, uint32_t query_heads) {
-        G = G_;
-        asm volatile("" : "+r"(row));   // worked out anew where it is used: no registers for it in between
-        const uint32_t token = row / G, tokens = 4 / G;
-        in_group = row - token * G;
-        step_in_group = 4 - tokens * G;
-        off = (static_cast<size_t>(token) * query_heads + kv_head * G + in_group) * D;
-        step = (static_cast<size_t>(tokens) * query_heads + step_in_group) * D;
-        wrap = static_cast<size_t>(query_heads - G) * D;
-    }
-    __device__ __forceinline__ void next() {
-        off += step;
-        in_group += step_in_group;
-        if (in_group >= G) { in_group -= G; off += wrap; }
+struct RowOffsets {
+    uint32_t rel[8];
+    int valid;   // rows that exist: the first `valid` of the eight
+    __device__ __forceinline__ RowOffsets(uint32_t warp_row0, uint32_t turn_row, uint32_t G, uint32_t query_heads, uint32_t total_rows) {
+        const uint32_t tokens = 4 / G, step_in_group = 4 - tokens * G;
+        uint32_t in_group = warp_row0 % G + turn_row, token = in_group / G;
+        in_group -= token * G;
+        uint32_t off = (token * query_heads + in_group) * D;
+        const uint32_t step = (tokens * query_heads + step_in_group) * D, wrap = (query_heads - G) * D;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            rel[i] = off;
+            off += step;
+            in_group += step_in_group;
+            if (in_group >= G) { in_group -= G; off += wrap; }
+        }
+        valid = warp_row0 + turn_row < total_rows ? static_cast<int>(min((total_rows - warp_row0 - turn_row + 3) / 4, 8u)) : 0;
     }
 };
 
 template <int D, int RT>
 __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel(const __grid_constant__ Tc5Params p) {
     using L = Layout<D, RT>;
-    constexpr int kThreads = L::kThreads, kSoftmaxThreads = L::kSoftmaxThreads;
+    constexpr int kThreads = L::kThreads;
     constexpr int kTmaWarp = L::kTmaWarp, kSWarp = L::kSWarp, kPvWarp = L::kPvWarp, kTmaVWarp = L::kTmaVWarp;
     constexpr int K_FULL = L::K_FULL, K_EMPTY = L::K_EMPTY, V_FULL = L::V_FULL, V_EMPTY = L::V_EMPTY, S_FULL = L::S_FULL, S_EMPTY = L::S_EMPTY,
                   P_FULL = L::P_FULL, P_EMPTY = L::P_EMPTY, O_DONE = L::O_DONE, Q_FULL = L::Q_FULL;
@@ -330,10 +342,16 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         return;
     }
 
+    const int live_tiles = min(RT, static_cast<int>((total_rows - row0 + kBM - 1) / kBM));   // row tiles that hold rows
     // ---- set-up: barriers, TMEM, Q tile -----------------------------------------------------------------
     if (tid == 0) {
-        for (int i = 0; i < L::kNumBars; ++i)
-            mbar_init(bar(i), i >= S_EMPTY && i < P_EMPTY ? kBM : i == Q_FULL ? kSoftmaxThreads : 1);   // S_EMPTY and P_FULL: a group's threads
+        for (int i = 0; i < L::kNumBars; ++i) {
+            uint32_t count = 1;
+            if (i >= S_EMPTY && i < P_EMPTY) count = kBM;   // S_EMPTY and P_FULL: a group's threads
+            else if (i == Q_FULL) count = RT * 256;
+            else if (i >= K_EMPTY && i < V_FULL) count = RT == 2 ? live_tiles : L::kIssuers;   // K: the warps that read it
+            mbar_init(bar(i), count);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < L::kRows * 2; i += kThreads) reinterpret_cast<uint32_t*>(smem + L::kOffRef)[i] = 0;
@@ -345,11 +363,57 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // The query rows on their way to L2 (a prefetch reads nothing yet: whatever still writes them, the loads behind the wait see), and where they lie.  With
+    // more than a wave of CTAs there is nothing to wait for.  (24 / 4 heads, 37 fp32 tokens over 3001: 24.3 -> 24.1 us a layer.)
+    if (warp == kTmaWarp && split_u == 0 && gridDim.x <= 148) {
+        const uint32_t elem = p.q_is_f16 ? 2 : 4, t_last = (min(row0 + L::kRows, total_rows) - 1) / G;
+        for (uint32_t t = row0 / G + lane; t <= t_last; t += 32)
+            prefetch_l2(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D * elem, G * D * elem);
+    }
+    const int turn_row = lane >> 3, turn_chunk = lane & 7;
+    const int rt = RT == 1 ? 0 : warp >> 3;                // row tile
+    const uint32_t tile_row0 = row0 + rt * kBM, warp_row0 = tile_row0 + (warp & 3) * 32;
+    const RowOffsets<D> rows(warp_row0, turn_row, G, p.query_heads, total_rows);
     pdl_wait();   // Q, the fp16 scratch and the device-side state come from preceding kernels
     bool failed = false;
-    const int live_tiles = min(RT, static_cast<int>((total_rows - row0 + kBM - 1) / kBM));   // row tiles that hold rows
 
-    if (warp == kTmaWarp) {
+    if (D == 128 && warp == kTmaWarp) {
+        // =============================== TMA producer, K and V tiles ===============================
+        const int row_base = static_cast<int>(kv_head * p.scratch_rows);
+        auto load_k = [&](int i) -> bool {   // a pair of tiles: tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab
+            const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
+            if (!mbar_wait(bar(K_EMPTY + ps), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) return false;
+            mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
+            for (int t = 0; t < n; ++t)
+                for (int s = 0; s < L::kSlabs; ++s)
+                    tma_load_2d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
+                                row_base + (tile0 + 2 * i + t) * kBN, bar(K_FULL + ps));
+            return true;
+        };
+        auto load_v = [&](int j) -> bool {
+            const int st = j % L::kVTiles;
+            if (!mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) return false;
+            mbar_expect_tx(bar(V_FULL + st), L::kTileBytes);
+            for (int s = 0; s < L::kSlabs; ++s)
+                tma_load_2d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, row_base + (tile0 + j) * kBN, bar(V_FULL + st));
+            return true;
+        };
+        bool ok = true;
+        if (lane == 0 && ntiles > 0) ok = load_k(0);
+        __syncwarp();
+        ok = mbar_wait(bar(Q_FULL), 0) && ok;
+        if (p.gate != nullptr && split_u == 0) {
+            const uint32_t t_last = (min(row0 + L::kRows, total_rows) - 1) / G;
+            for (uint32_t t = row0 / G + lane; t <= t_last; t += 32)
+                prefetch_l2(p.gate + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D, G * D * 4);
+        }
+        if (lane == 0) {
+            for (int j = 0; ok && j < ntiles; ++j) {
+                if ((j & 1) == 0 && j + 2 < ntiles) ok = load_k((j >> 1) + 1);
+                ok = ok && load_v(j);
+            }
+        }
+    } else if (warp == kTmaWarp) {
         // =============================== TMA producer, K tiles ===============================
         // A ring stage holds a PAIR of tiles, tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab, so that
         // one MMA instruction (N = 128) covers both.
@@ -368,7 +432,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                                     row_base + (tile0 + 2 * i + t) * kBN, bar(K_FULL + ps));
             }
         }
-    } else if (warp == kTmaVWarp) {
+    } else if (D == 256 && warp == kTmaVWarp) {
         // =============================== TMA producer, V tiles ===============================
         const bool have_q = mbar_wait(bar(Q_FULL), 0);
         // The gate on its way to L2 for the epilogue or the merge: the kv head's G rows of a token are contiguous, a lane takes a token.
@@ -380,135 +444,116 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         if (have_q && lane == 0) {
             const int row_base = static_cast<int>(kv_head * p.scratch_rows);
             for (int j = 0; j < ntiles; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);
-                if (!mbar_wait(bar(V_EMPTY + st), ph ^ 1)) break;
+                const int st = j % L::kVTiles;
+                if (!mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) break;
                 mbar_expect_tx(bar(V_FULL + st), L::kTileBytes);
                 for (int s = 0; s < L::kSlabs; ++s)
                     tma_load_2d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, row_base + (tile0 + j) * kBN, bar(V_FULL + st));
             }
         }
-    } else if (warp == kSWarp) {
+    } else if (warp >= kSWarp && warp < kPvWarp) {
         // =============================== S = Q.K^T issuer ===============================
         // The warp stays together and one lane issues (D == 128): loop counters and descriptors live in uniform registers, which an MMA takes them from
         // (from a branch on the lane number an MMA cost 50 to 105 clocks to issue, against the 32 to 64 these run).
         if constexpr (L::kPInTmem) {
             constexpr uint32_t idesc = umma_idesc(kBM, kBN, 0, 0);
+            const int rt = RT == 2 ? warp - kSWarp : 0, first = RT == 2 ? 0 : warp - kSWarp;
+            constexpr int kStep = RT == 2 ? 1 : L::kIssuers;
             const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024);
-            bool ok = mbar_wait_warp(bar(Q_FULL), 0);
-            for (int j = 0; ok && j < ntiles; ++j) {
-                const int i = j >> 1, ps = i % kKPairs;
-                if ((j & 1) == 0 && !mbar_wait_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
-                ok = mbar_wait_warp(bar(S_EMPTY + (j & 1)), static_cast<uint32_t>(i & 1) ^ 1);   // the scores of tile j - 2 have been read
+            [[maybe_unused]] const uint64_t q_desc = umma_desc(sbase + L::kOffQ + rt * L::kQBytes, 16, 1024);
+            bool ok = rt < live_tiles && mbar_wait_warp(bar(Q_FULL), 0);
+            for (int j = first; ok && j < ntiles; j += kStep) {
+                const int i = j >> 1, ps = i % kKPairs, buf = rt * L::kGroups + j % L::kGroups;
+                // the K pair is there, and the weights that lie in the buffer have been used
+                ok = mbar_wait2_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1), bar(P_EMPTY + buf), static_cast<uint32_t>((j / L::kGroups) & 1) ^ 1);
                 if (!ok) break;
                 tc_fence_after();
+                const uint64_t b = k_desc + ((ps * L::kPairBytes + (j & 1) * (kBN * 128)) >> 4);
+                const uint32_t d = tmem_base + L::kColS + buf * kBN;
                 if (elect_one()) {
-                    const uint64_t b = k_desc + ((ps * L::kPairBytes + (j & 1) * (kBN * 128)) >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk)
-                        umma_f16_a_tmem(tmem_base + L::kColS + (j & 1) * kBN, tmem_base + L::kColQ + kk * 8,
-                                        b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4), idesc, kk > 0);
-                    umma_commit(bar(S_FULL + (j & 1)));
-                    if ((j & 1) == 1 || j + 1 == ntiles) umma_commit(bar(K_EMPTY + ps));
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint64_t bk = b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4);
+                        if constexpr (L::kQInTmem) umma_f16_a_tmem(d, tmem_base + L::kColQ + kk * 8, bk, idesc, kk > 0);
+                        else umma_f16(d, q_desc + (((kk >> 2) * (kBM * 128) + (kk & 3) * 32) >> 4), bk, idesc, kk > 0);
+                    }
+                    umma_commit(bar(S_FULL + buf));
+                    if (RT == 1 || (j & 1) == 1 || j + 1 == ntiles) umma_commit(bar(K_EMPTY + ps));   // this warp is through with the pair
                 }
                 __syncwarp();
             }
-        } else if constexpr (!L::kQInTmem) {
-            constexpr uint32_t idesc_pair = umma_idesc(kBM, 2 * kBN, 0, 0), idesc_one = umma_idesc(kBM, kBN, 0, 0);
-            const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024), q_desc = umma_desc(sbase + L::kOffQ, 16, 1024);
-            bool ok = mbar_wait_warp(bar(Q_FULL), 0);
-            for (int i = 0; ok && 2 * i < ntiles; ++i) {
-                const int ps = i % kKPairs;
-                const uint32_t ph = static_cast<uint32_t>(i & 1) ^ 1, idesc = ntiles - 2 * i >= 2 ? idesc_pair : idesc_one;
-                if (!mbar_wait_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
-                const uint64_t b = k_desc + ((ps * L::kPairBytes) >> 4);
-#pragma unroll
-                for (int rt = 0; rt < RT; ++rt) {
-                    if (rt >= live_tiles) break;
-                    // both groups have read the previous pair's scores (only the last pair can be a single tile)
-                    ok = mbar_wait_warp(bar(S_EMPTY + 2 * rt), ph) && mbar_wait_warp(bar(S_EMPTY + 2 * rt + 1), ph);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int kk = 0; kk < D / 16; ++kk)
-                            umma_f16(tmem_base + L::kColS + rt * 2 * kBN, q_desc + ((rt * L::kQBytes + (kk >> 2) * (kBM * 128) + (kk & 3) * 32) >> 4),
-                                     b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4), idesc, kk > 0);
-                        umma_commit(bar(S_FULL + rt));   // scores ready for both softmax groups
-                        if (rt + 1 == live_tiles) umma_commit(bar(K_EMPTY + ps));
-                    }
-                    __syncwarp();
-                }
-            }
-        } else if (lane == 0) {
+        } else {
             // One chain of D/16 MMAs per PAIR of tiles (N = 128: the first tile's scores land in S columns 0-63, the second
             // one's in 64-127): half as many instructions to issue as tile by tile.
             constexpr uint32_t idesc_pair = umma_idesc(kBM, 2 * kBN, 0, 0), idesc_one = umma_idesc(kBM, kBN, 0, 0);
-            const bool have_q = mbar_wait(bar(Q_FULL), 0);
-            for (int i = 0; have_q && 2 * i < ntiles; ++i) {
+            const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024);
+            bool ok = mbar_wait_warp(bar(Q_FULL), 0);
+            for (int i = 0; ok && 2 * i < ntiles; ++i) {
                 const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
-                if (!mbar_wait(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1))) break;
+                const uint32_t ph = static_cast<uint32_t>(i & 1) ^ 1, idesc = n == 2 ? idesc_pair : idesc_one;
                 // both groups have read the previous pair's scores (only the last pair can be a single tile)
-                if (!mbar_wait(bar(S_EMPTY), static_cast<uint32_t>(i & 1) ^ 1) || !mbar_wait(bar(S_EMPTY + 1), static_cast<uint32_t>(i & 1) ^ 1)) break;
+                ok = mbar_wait2_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1), bar(S_EMPTY), ph) && mbar_wait_warp(bar(S_EMPTY + 1), ph);
+                if (!ok) break;
                 tc_fence_after();
+                const uint64_t b = k_desc + ((ps * L::kPairBytes) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t b = sbase + L::kOffK + ps * L::kPairBytes + (kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32;
-                    umma_f16_a_tmem(tmem_base + L::kColS, tmem_base + L::kColQ + kk * 8, umma_desc(b, 16, 1024), n == 2 ? idesc_pair : idesc_one, kk > 0);
+                    for (int kk = 0; kk < D / 16; ++kk)
+                        umma_f16_a_tmem(tmem_base + L::kColS, tmem_base + L::kColQ + kk * 8, b + (((kk >> 2) * (2 * kBN * 128) + (kk & 3) * 32) >> 4), idesc, kk > 0);
+                    umma_commit(bar(S_FULL));         // scores ready for both softmax groups
+                    umma_commit(bar(K_EMPTY + ps));   // K stage may be refilled
                 }
-                umma_commit(bar(S_FULL));         // scores ready for both softmax groups
-                umma_commit(bar(K_EMPTY + ps));   // K stage may be refilled
+                __syncwarp();
             }
         }
     } else if (warp == kPvWarp) {
         // =============================== O += P.V issuer ===============================
         if constexpr (D == 128) {
             constexpr uint32_t idesc_o = umma_idesc(kBM, D, 0, 1);
+            const uint64_t v_desc = umma_desc(sbase + L::kOffV, kBN * 128, 1024);
+            bool ok = true;
+            for (int j = 0; ok && j < ntiles; ++j) {
+                const int vs = j % L::kVTiles, st = j % L::kGroups;
+                const uint32_t ph = static_cast<uint32_t>((j / L::kGroups) & 1);
+                const uint64_t b = v_desc + ((vs * L::kTileBytes) >> 4);
+#pragma unroll
+                for (int rt = 0; rt < RT; ++rt) {
+                    if (RT > 1 && rt >= live_tiles) break;
+                    const int buf = rt * L::kGroups + st;
+                    ok = rt == 0 ? mbar_wait2_warp(bar(V_FULL + vs), static_cast<uint32_t>((j / L::kVTiles) & 1), bar(P_FULL + buf), ph) : mbar_wait_warp(bar(P_FULL + buf), ph);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < kBN / 16; ++kk)   // V: MN-major, 16 positions per step
+                            umma_f16_a_tmem(tmem_base + L::kColO + rt * D, tmem_base + L::kColS + buf * kBN + kk * 8, b + ((kk * (16 * 128)) >> 4), idesc_o, (j > 0 || kk > 0));
+                        umma_commit(bar(P_EMPTY + buf));   // the buffer is free for scores, O holds tiles 0..j
+                        if (j == ntiles - 1) umma_commit(bar(O_DONE + rt));   // O complete: the epilogue's signal for all groups
+                        if (rt + 1 == live_tiles) umma_commit(bar(V_EMPTY + vs));
+                    }
+                    __syncwarp();
+                }
+            }
+        } else {
+            constexpr uint32_t idesc_o = umma_idesc(kBM, D, 0, 1);
             const uint64_t v_desc = umma_desc(sbase + L::kOffV, kBN * 128, 1024), p_desc = umma_desc(sbase + L::kOffP, 16, 1024);
             bool ok = true;
             for (int j = 0; ok && j < ntiles; ++j) {
                 const int st = j & 1;
                 const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);
-                if (!mbar_wait_warp(bar(V_FULL + st), ph)) break;
-                const uint64_t b = v_desc + ((st * L::kTileBytes) >> 4);
-#pragma unroll
-                for (int rt = 0; rt < RT; ++rt) {
-                    if (RT > 1 && rt >= live_tiles) break;
-                    ok = mbar_wait_warp(bar(P_FULL + 2 * rt + st), ph);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int kk = 0; kk < kBN / 16; ++kk) {
-                            const uint64_t bk = b + ((kk * (16 * 128)) >> 4);   // V: MN-major, 16 positions per step
-                            const uint32_t o = tmem_base + L::kColO + rt * D;
-                            if constexpr (L::kPInTmem) umma_f16_a_tmem(o, tmem_base + L::kColP + st * (kBN / 2) + kk * 8, bk, idesc_o, (j > 0 || kk > 0));
-                            else umma_f16(o, p_desc + (((2 * rt + st) * L::kPBytes + kk * 32) >> 4), bk, idesc_o, (j > 0 || kk > 0));   // P: K-major, one 128-byte slab
-                        }
-                        umma_commit(bar(P_EMPTY + 2 * rt + st));   // P buffer free, O holds tiles 0..j
-                        if (j == ntiles - 1) umma_commit(bar(O_DONE + rt));   // O complete: the epilogue's signal for both groups
-                        if (rt + 1 == live_tiles) umma_commit(bar(V_EMPTY + st));
-                    }
-                    __syncwarp();
-                }
-            }
-        } else if (lane == 0) {
-            constexpr uint32_t idesc_o = umma_idesc(kBM, D, 0, 1);
-            for (int j = 0; j < ntiles; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);
-                if (!mbar_wait(bar(V_FULL + st), ph)) break;
-                if (!mbar_wait(bar(P_FULL + st), ph)) break;
+                ok = mbar_wait2_warp(bar(V_FULL + st), ph, bar(P_FULL + st), ph);
+                if (!ok) break;
                 tc_fence_after();
+                const uint64_t a = p_desc + ((st * L::kPBytes) >> 4), b = v_desc + ((st * L::kTileBytes) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < kBN / 16; ++kk) {
-                    const uint32_t b = sbase + L::kOffV + st * L::kTileBytes + kk * (16 * 128);      // V: MN-major, 16 positions per step
-                    const uint32_t a = sbase + L::kOffP + st * L::kPBytes + kk * 32;                // P: K-major, one 128-byte slab
-                    umma_f16(tmem_base + L::kColO, umma_desc(a, 16, 1024), umma_desc(b, kBN * 128, 1024), idesc_o, (j > 0 || kk > 0));
+                    for (int kk = 0; kk < kBN / 16; ++kk)
+                        umma_f16(tmem_base + L::kColO, a + ((kk * 32) >> 4), b + ((kk * (16 * 128)) >> 4), idesc_o, (j > 0 || kk > 0));
+                    umma_commit(bar(P_EMPTY + st));   // P buffer free, O holds tiles 0..j
+                    if (j == ntiles - 1) umma_commit(bar(O_DONE));   // O complete: the epilogue's signal for both groups
+                    umma_commit(bar(V_EMPTY + st));
                 }
-                umma_commit(bar(P_EMPTY + st));   // P buffer free, O holds tiles 0..j
-                if (j == ntiles - 1) umma_commit(bar(O_DONE));   // O complete: the epilogue's signal for both groups
-                umma_commit(bar(V_EMPTY + st));
+                __syncwarp();
             }
         }
     } else {
@@ -520,28 +565,24 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         // tiles is on its way meanwhile.  From the dependency wait to the last row: 0.8 us (two row tiles of 128 dims; 3.8 behind full rings and with
         // a division a row), 3.3 us (one of 256 from HBM; 4.5).
         uint8_t* const turn = smem + L::kOffP + warp * 4096;   // [32 rows][8 chunks of 16 B], chunk c of row r at c ^ (r & 7)
-        const int turn_row = lane >> 3, turn_chunk = lane & 7;
-        const int rt = RT == 1 ? 0 : warp >> 3;                // row tile
-        const uint32_t tile_row0 = row0 + rt * kBM, warp_row0 = tile_row0 + (warp & 3) * 32;
-        {
+        if (L::kSoftmaxThreads == RT * 256 || warp < 8) {
             const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
             const int half = (warp >> 2) & 1;
             constexpr int kTurns = D / 128;            // 32 columns = 64 dims per store; all loads are in flight together
             uint4 q[kTurns][8];
             auto fetch = [&](auto f16) {
-                RowWalk<D> at(warp_row0 + turn_row, kv_head, G, p.query_heads);
-                at.off += half * (D / 2) + turn_chunk * 8;
+                const size_t base0 = (static_cast<size_t>(warp_row0 / G) * p.query_heads + kv_head * G) * D + half * (D / 2) + turn_chunk * 8;
 #pragma unroll
-                for (int i = 0; i < 8; ++i, at.next())
+                for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int k = 0; k < kTurns; ++k) {
                         q[k][i] = make_uint4(0, 0, 0, 0);
-                        if (warp_row0 + 4 * i + turn_row >= total_rows) continue;
+                        if (i >= rows.valid) continue;
                         if (f16()) {
-                            q[k][i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + at.off + k * 64);
+                            q[k][i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + base0 + rows.rel[i] + k * 64);
                         } else {
-                            const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + at.off + k * 64);
-                            const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p.q) + at.off + k * 64 + 4);
+                            const float* src = static_cast<const float*>(p.q) + base0 + rows.rel[i] + k * 64;
+                            const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
                             q[k][i] = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
                         }
                     }
@@ -560,22 +601,22 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                         const int row = 4 * i + turn_row;
                         *reinterpret_cast<uint4*>(slab + row * 128 + ((turn_chunk ^ (row & 7)) << 4)) = v[i];
                     }
-                    continue;
-                }
+                } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int row = 4 * i + turn_row;
-                    *reinterpret_cast<uint4*>(turn + row * 128 + ((turn_chunk ^ (row & 7)) << 4)) = v[i];
-                }
-                __syncwarp();
-                uint32_t w[32];
+                    for (int i = 0; i < 8; ++i) {
+                        const int row = 4 * i + turn_row;
+                        *reinterpret_cast<uint4*>(turn + row * 128 + ((turn_chunk ^ (row & 7)) << 4)) = v[i];
+                    }
+                    __syncwarp();
+                    uint32_t w[32];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 q4 = *reinterpret_cast<const uint4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4));
-                    w[4 * c] = q4.x; w[4 * c + 1] = q4.y; w[4 * c + 2] = q4.z; w[4 * c + 3] = q4.w;
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 q4 = *reinterpret_cast<const uint4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4));
+                        w[4 * c] = q4.x; w[4 * c + 1] = q4.y; w[4 * c + 2] = q4.z; w[4 * c + 3] = q4.w;
+                    }
+                    __syncwarp();
+                    tmem_st32_bits(tmem_base + lane_base + L::kColQ + half * (D / 4) + c0, w);
                 }
-                __syncwarp();
-                tmem_st32_bits(tmem_base + lane_base + L::kColQ + half * (D / 4) + c0, w);
             }
             if constexpr (L::kQInTmem) {
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -587,15 +628,14 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             // no barrier: what a warp turns its rows in are its own rows of its group's P tile
         }
         // =============================== softmax rows ===============================
-        // Two groups of 128 threads, one thread per query row in each: warps 0-3 take the even tiles, warps 4-7 the odd
-        // ones (a warp reaches the 32 TMEM lanes of its number modulo 4), so two tiles are in flight: while one group
-        // works through its exponentials the other one's S arrives and its P.V runs.  A row's reference maximum is handed
+        // Groups of 128 threads, one thread per query row in each, take the tiles in turn (a warp reaches the 32 TMEM lanes of its number modulo
+        // 4), so as many tiles are in flight: while one group works through its exponentials the others' S arrive and their P.V run.  A row's reference maximum is handed
         // from tile to tile through an 8-byte {value, sequence} word in shared memory; each thread keeps the partial row
         // sum of its own tiles, relative to the reference it last saw.
-        const int r = tid & (kBM - 1), grp = (tid >> 7) & 1;   // row of this thread in its row tile == its TMEM lane; tile parity
+        const int r = tid & (kBM - 1), grp = (tid >> 7) % L::kGroups;   // row of this thread in its row tile == its TMEM lane; its tiles
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t gr = tile_row0 + r;
-        const int nt = RT == 1 || rt < live_tiles ? ntiles : 0;
+        const int walked = RT == 1 || rt < live_tiles ? ntiles : 0;
         uint32_t len = 0;
         if (gr < total_rows) {
             const uint32_t token = gr / G;
@@ -620,13 +660,15 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 m_known = m_new;
             }
         };
-        const int st = grp;
-        const uint32_t s_col = L::kColS + (2 * rt + grp) * kBN, o_col = L::kColO + rt * D;
+        const int buf = rt * L::kGroups + grp;
+        const uint32_t s_col = L::kColS + buf * kBN, o_col = L::kColO + rt * D;
+        const int nt = L::kGroups == 4 ? (walked + grp + 1) / 2 : walked;
         for (int j = grp; j < nt; j += 2) {
-            const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);   // parity of the tile's pair
+            const int t = L::kGroups == 4 ? 2 * j - grp : j;   // the tile: every second, or with four groups every fourth from the group's first
+            const uint32_t ph = static_cast<uint32_t>((t / L::kGroups) & 1);   // parity of the group's tile
             // The loop holds warp-wide loads, stores and votes, so a warp leaves it as a whole: a lane whose wait runs out goes on, with values nobody
             // will see, up to the one vote below.
-            bool lost = !mbar_wait(bar(S_FULL + (L::kPInTmem ? st : rt)), ph);
+            bool lost = !mbar_wait(bar(S_FULL + (L::kPInTmem ? buf : rt)), ph);
             tc_fence_after();
             float s[kBN];
             {
@@ -637,9 +679,11 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
 #pragma unroll
                 for (int i = 0; i < 32; ++i) { s[i] = __uint_as_float(lo[i]); s[32 + i] = __uint_as_float(hi[i]); }
             }
-            tc_fence_before();
-            mbar_arrive(bar(S_EMPTY + 2 * rt + st));   // this row of S is in registers
-            const uint32_t pos0 = static_cast<uint32_t>(tile0 + j) * kBN;
+            if constexpr (!L::kPInTmem) {
+                tc_fence_before();
+                mbar_arrive(bar(S_EMPTY + buf));   // this row of S is in registers
+            }
+            const uint32_t pos0 = static_cast<uint32_t>(tile0 + t) * kBN;
             // Raw scores stay unscaled; the softmax scale is folded into the exponent: p = 2^(s*c - m*c).  The loop's instructions count: products and
             // sums go in pairs, maxima three values at a time.  32 / 8 heads of 128, 1024 tokens over 8192: 168.0 -> 163.7 us; 24 / 4 of 256, 512 over
             // 8192: 111.6 -> 110.3.
@@ -659,7 +703,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             // the reference as the previous tile (the other group's) left it; lazy rescale: keep it unless this tile's
             // maximum outgrew it by more than the threshold
             float m_prev = -INFINITY;
-            if (j > 0 && !ref_after(static_cast<uint32_t>(j), &m_prev)) lost = true;
+            if (t > 0 && !ref_after(static_cast<uint32_t>(t), &m_prev)) lost = true;
             float alpha = 1.0f, m_new = m_prev;
             if (mt > m_prev + kRescaleThreshold || (m_prev == -INFINITY && mt > -INFINITY)) {
                 alpha = (m_prev == -INFINITY) ? 0.0f : ex2_approx(m_prev - mt);
@@ -667,12 +711,15 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             }
             // published at once (the other group's thread of this row waits for it): no later work may be scheduled before it
             asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(smem_u32(const_cast<unsigned long long*>(ref))),
-                         "l"((static_cast<unsigned long long>(static_cast<uint32_t>(j) + 1u) << 32) | __float_as_uint(m_new)) : "memory");
-            // One row tile of 128 comes at 166 or 182 us for 1024 over 8192 (32 / 8 heads) by small things around this loop, its exits or the text of the epilogue:
-            // in the slow builds a warp polls the other group's reference five times more a tile.  With this one's exits it is 182, and 167 with the
-            // reference of what follows out of a shuffle behind the store.  That holds for this text only: measure 1024 over 8192 after a change.
-            // Without P in TMEM the shuffle costs 1 to 2 %.
-            if constexpr (L::kPInTmem) m_new = __shfl_sync(0xffffffffu, m_new, lane);
+                         "l"((static_cast<unsigned long long>(static_cast<uint32_t>(t) + 1u) << 32) | __float_as_uint(m_new)) : "memory");
+            // At 128 it is read back as well: what follows depends on the value read, so no exponential can be scheduled ahead of the store.  (Without that the store
+            // came behind all of them, by the compiler's choice and by small changes around it: a tile of one row tile took 1050 clocks, not 820.)  At 256, whose
+            // two groups wait less for each other, the value out of a shuffle behind the store does better: us a layer back to back, as it comes / read back / shuffled,
+            // 512 over 8192 127.1 / 126.2 / 125.0, 300 over 8192 83.3 / 86.6 / 81.5, 37 over 3001 24.1 / 24.5 / 24.1.
+            if constexpr (D == 128)
+                asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(m_new) : "r"(smem_u32(const_cast<unsigned long long*>(ref))) : "memory");
+            else
+                m_new = __shfl_sync(0xffffffffu, m_new, lane);
             rebase(m_new);
             const float neg_ref = (m_new == -INFINITY) ? 0.0f : -m_new;
             Pair sum = 0;
@@ -692,12 +739,14 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 l_sum += halves.x + halves.y;
             }
             // this group's P buffer is free once the P.V of its previous tile has completed
-            if (!mbar_wait(bar(P_EMPTY + 2 * rt + st), ph ^ 1)) lost = true;
-            tc_fence_after();
-            if (__any_sync(0xffffffffu, alpha != 1.0f || lost) && (j > 0 || __any_sync(0xffffffffu, lost))) {
-                // rare: the reference moved.  O holds tiles 0..j-1 once the previous tile's P.V (the other group's) has
+            if constexpr (!L::kPInTmem) {
+                if (!mbar_wait(bar(P_EMPTY + buf), ph ^ 1)) lost = true;
+                tc_fence_after();
+            }
+            if (__any_sync(0xffffffffu, alpha != 1.0f || lost) && (t > 0 || __any_sync(0xffffffffu, lost))) {
+                // rare: the reference moved.  O holds tiles 0..t-1 once the previous tile's P.V (the other group's) has
                 // completed; then this warp rescales its 32 rows of O in TMEM before its own P is released.
-                if (j > 0 && !mbar_wait(bar(P_EMPTY + 2 * rt + (st ^ 1)), static_cast<uint32_t>(((j - 1) >> 1) & 1))) lost = true;
+                if (t > 0 && !mbar_wait(bar(P_EMPTY + rt * L::kGroups + (t - 1) % L::kGroups), static_cast<uint32_t>(((t - 1) / L::kGroups) & 1))) lost = true;
                 if (__any_sync(0xffffffffu, lost)) { failed = true; break; }
                 tc_fence_after();
 #pragma unroll 1
@@ -710,94 +759,107 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 }
             }
             if constexpr (L::kPInTmem) {
-                tmem_st32_bits(tmem_base + lane_addr + L::kColP + st * (kBN / 2), pk);
+                tmem_st32_bits(tmem_base + lane_addr + s_col, pk);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // and the rescale's stores, if any
             } else {
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");   // the rescale's stores, if any
-                uint8_t* prow = smem + L::kOffP + (2 * rt + st) * L::kPBytes + r * 128;
+                uint8_t* prow = smem + L::kOffP + buf * L::kPBytes + r * 128;
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
                     *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             tc_fence_before();
-            mbar_arrive(bar(P_FULL + 2 * rt + st));
+            mbar_arrive(bar(P_FULL + buf));
         }
         // ---- epilogue: O / sum, gate, store; each thread of a row's pair half of the columns ----
         const bool partial = nsplit > 1, gated = !partial && p.gate != nullptr;
         const size_t part_row0 = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0;
-        RowWalk<D> first(warp_row0 + turn_row, kv_head, G, p.query_heads);   // of the output (a split's partials: [row][D])
-        if (partial) {
-            first.off = (part_row0 + (warp_row0 - row0) + turn_row) * D;
-            first.step = 4 * D;
-            first.step_in_group = 0;
+        constexpr int kCols = D / L::kGroups;
+        const int col0 = grp * kCols;
+        const RowOffsets<D> rows(warp_row0, turn_row, G, p.query_heads, total_rows);   // worked out anew: no registers for it in between
+        const size_t out0 = (static_cast<size_t>(warp_row0 / G) * p.query_heads + kv_head * G) * D + col0 + 4 * turn_chunk;
+        float4 g[8];
+        auto fetch_gate = [&](int i, int c0) {
+            if (i < rows.valid) g[i] = *reinterpret_cast<const float4*>(p.gate + out0 + rows.rel[i] + c0);
+        };
+        // D == 256: ahead of the last P.V, the next columns' behind the use of these (at 128 there are no registers for that)
+        if (D == 256 && gated) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) fetch_gate(i, 0);
         }
-        first.off += grp * (D / 2) + 4 * turn_chunk;
-        if (!failed && nt > 0 && !mbar_wait(bar(O_DONE + rt), 0)) failed = true;
+        if (!failed && walked > 0 && !mbar_wait(bar(O_DONE + rt), 0)) failed = true;
         tc_fence_after();
         {
             float m_final = -INFINITY;
-            if (!failed && nt > 0 && !ref_after(static_cast<uint32_t>(nt), &m_final)) failed = true;
+            if (!failed && walked > 0 && !ref_after(static_cast<uint32_t>(walked), &m_final)) failed = true;
             rebase(m_final);
             float* sums = reinterpret_cast<float*>(smem + L::kOffSum + rt * L::kSumStride);
             sums[grp * kBM + r] = failed ? __int_as_float(0x7fc00000) : l_sum;
             // the row tile's threads (a branch over two constant barriers duplicates what follows: 4 % slower with two row tiles)
-            if constexpr (RT == 1) asm volatile("bar.sync 2, 256;" ::: "memory");
+            if constexpr (RT == 1) asm volatile("bar.sync 2, %0;" ::"n"(L::kSoftmaxThreads) : "memory");
             else asm volatile("bar.sync %0, 256;" ::"r"(2 + rt) : "memory");
             l_sum = sums[r] + sums[kBM + r];
+            if constexpr (L::kGroups == 4) l_sum += sums[2 * kBM + r] + sums[3 * kBM + r];
             // The warp's O may be read.  A sum that is NaN, because the row's other thread gave up or because of the data, is its own row's affair.
-            const bool have_o = nt > 0 && !__any_sync(0xffffffffu, failed);
+            const bool have_o = walked > 0 && !__any_sync(0xffffffffu, failed);
             if (l_sum != l_sum) failed = true;
             const float m_ref = m_final;
-            const int hsel = grp;
             const float inv = l_sum > 0.0f ? 1.0f / l_sum : 0.0f;
-            if (partial && gr < total_rows && hsel == 0)   // a poisoned or empty partial is recognised by its sum
+            if (partial && gr < total_rows && grp == 0)   // a poisoned or empty partial is recognised by its sum
                 p.part_ml[part_row0 + rt * kBM + r] = make_float2(m_ref, failed ? __int_as_float(0x7fc00000) : (len == 0 ? 0.0f : l_sum));
             // Rows leave 32 columns at a time through the same 4 KB per warp: read back four rows an instruction, 128
             // contiguous bytes each, so that the gate is fetched and the result stored in whole lines.
-            float* const dst = partial ? p.part_o : p.out;
-            const float factor = partial ? 1.0f : inv;
+            float* const dst = partial ? p.part_o + (part_row0 + (warp_row0 - row0) + turn_row) * D + col0 + 4 * turn_chunk : p.out + out0;
+            const bool zero = len == 0 && !partial;
+            const float factor = failed ? __int_as_float(0x7fc00000) : partial ? 1.0f : inv;
 #pragma unroll 1
-            for (int c0 = hsel * (D / 2); c0 < (hsel + 1) * (D / 2); c0 += 32) {
-                float4 g[8];
+            for (int c0 = 0; c0 < kCols; c0 += 32) {
+                [[maybe_unused]] float4 gs[8];
                 if (gated) {
-                    RowWalk<D> at = first;
+                    if constexpr (D == 256) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i, at.next())
-                        if (warp_row0 + 4 * i + turn_row < total_rows) g[i] = *reinterpret_cast<const float4*>(p.gate + at.off);
+                        for (int i = 0; i < 8; ++i) {
+                            gs[i].x = 1.0f / (1.0f + __expf(-g[i].x)); gs[i].y = 1.0f / (1.0f + __expf(-g[i].y));
+                            gs[i].z = 1.0f / (1.0f + __expf(-g[i].z)); gs[i].w = 1.0f / (1.0f + __expf(-g[i].w));
+                        }
+                    }
+                    if (D == 128 || c0 + 32 < kCols) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) fetch_gate(i, D == 128 ? c0 : c0 + 32);
+                    }
                 }
                 float o[32];
                 // tcgen05.ld is warp-collective: every lane takes part, rows past the launch only skip the store
                 if (have_o) {
-                    tmem_ld32(tmem_base + lane_addr + o_col + c0, o);
+                    tmem_ld32(tmem_base + lane_addr + o_col + col0 + c0, o);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) o[i] = 0.0f;
                 }
+                if (zero && !failed) {   // no position visible: zeros whatever lies there
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    o[i] = (len == 0 && !partial) ? 0.0f : o[i] * factor;
-                    if (failed) o[i] = __int_as_float(0x7fc00000);
+                    for (int i = 0; i < 32; ++i) o[i] = 0.0f;
                 }
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
-                    *reinterpret_cast<float4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+                    *reinterpret_cast<float4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+                        make_float4(o[4 * c] * factor, o[4 * c + 1] * factor, o[4 * c + 2] * factor, o[4 * c + 3] * factor);
                 __syncwarp();
-                RowWalk<D> at = first;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int row = 4 * i + turn_row;
                     float4 v = *reinterpret_cast<const float4*>(turn + row * 128 + ((turn_chunk ^ (row & 7)) << 4));
-                    if (warp_row0 + row < total_rows) {
-                        if (gated) {
+                    if (gated) {
+                        if constexpr (D == 256) {
+                            v.x *= gs[i].x; v.y *= gs[i].y; v.z *= gs[i].z; v.w *= gs[i].w;
+                        } else {
                             v.x *= 1.0f / (1.0f + __expf(-g[i].x)); v.y *= 1.0f / (1.0f + __expf(-g[i].y));
                             v.z *= 1.0f / (1.0f + __expf(-g[i].z)); v.w *= 1.0f / (1.0f + __expf(-g[i].w));
                         }
-                        *reinterpret_cast<float4*>(dst + at.off) = v;
                     }
-                    at.next();
+                    if (i < rows.valid) *reinterpret_cast<float4*>(dst + (partial ? static_cast<uint32_t>(4 * i * D) : rows.rel[i]) + c0) = v;
                 }
-                first.off += 32;
                 __syncwarp();
             }
         }
@@ -1030,31 +1092,32 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
     return static_cast<size_t>(splits) * kv_heads * rows_padded * (head_dim + 2) * sizeof(float);
 }
 
-// How many KV splits: the number with the least estimated time, for `units` CTAs of one or two row tiles and up to `tiles` KV tiles.  A wave of
-// 148 CTAs costs its tiles and a few us; CTAs take the place of one another as they end, so a last wave that is not full costs less
-// than a whole one.  A split costs its partials' way out and back.  Measured for a layer with its store kernel, us in a short burst (and, where the power
-// limit makes it another, in a long run), q8_0, the estimate's choice marked *:
-//   24 heads of 256:  20 tokens over 16000 (4 units):  8: 55, 12: 49, *16: 48        37 over 3001 (8):  6: 26.3, 8: 26.1, 10: 23.9, *11: 23.9, 16: 24.4
-//                     64 over 8192 (12):  8: 37, *12: 35, 13: 49                     128 over 8192 (24):  5: 45, *6: 44, 7: 64
-//                     300 over 8192 (60):  1: 123, *2: 77, 3: 98                     512 over 2000 (96):  *1: 50, 2: 61, 3: 57
-//                     512 over 8192 (96):  1: 123 (125), 2: 134 (137), *3: 110 (127), 4: 129 (139)
-//   32 of 128:        37 over 3001 (16):  6: 21.1, 8: 20.4, *9: 19.2, 10: 26.6       100 over 1000 (32):  1: 22.0, 3: 18.5, *4: 18.4
-//                     200 over 2000 (56):  1: 34, *2: 28, 3: 35                      300 over 4000 (80):  1: 57, 2: 57, *3: 48, 4: 56
-//                     400 over 16000 (104):  1: 184 (179), 2: 163 (170), 3: 176 (177), *4: 142 (165)
-//   the same, two row tiles a CTA:  1200 over 4000 (152):  1: 150, *2: 148, 3: 150 (153)        1200 over 8192:  1: 280, 2: 243 (250), *3: 237 (248), 4: 242 (255)
+// How many KV splits: the number with the least estimated time, for `units` CTAs of one or two row tiles, up to `tiles` KV tiles and `average` of them.  A wave
+// of 148 CTAs costs its tiles and a few us; CTAs take the place of one another as they end, so a last wave that is not full may cost less than a whole
+// one, and from the second wave on the length that counts may lie between the longest causal range and the average; a split costs its partials' way out
+// and back, and the merge.  The constants of single row tiles are fitted to 66 (head_dim 128) and 93 (256) chunks of 16 to 2048 tokens over 0 to 32000 at 32 / 8 and 24 / 4
+// heads, every number of splits timed: the choice is 0.4 and 0.3 % above the best on average, 6.5 and 5 % at most (1.5 and 0.6, 12 and 15 % with the constants before).  us a layer with the store kernel, in a short
+// burst (and, where the power limit makes it another, in a long run), q8_0, the choice marked *:
+//   32 heads of 128:  37 over 3000 (16 units):  1: 37.3, 4: 21.5, 6: 20.6, *9: 20.0, 10: 26.7       128 over 8192 (32):  1: 74, 2: 50, *4: 37.2, 5: 52
+//                     300 over 300 (80):  *1: 18.7, 2: 26.7       300 over 8192:  1: 84, 2: 87, *3: 69.6, 4: 81       461 over 8192 (120):  *1: 87, 2: 94, 3: 103
+//   24 of 256:        20 over 16000 (4):  8: 55, 12: 49, *16: 48                     37 over 3000 (8):  1: 50, 4: 25.6, 8: 23.6, *10: 22.5, 11: 22.7, 16: 22.5
+//                     128 over 8192 (24):  1: 101, 4: 46.7, *6: 43.6, 7: 60          300 over 8192 (60):  1: 111, *2: 78, 3: 98
+//                     300 over 300 (60):  1: 30.5, *2: 26.4, 3: 32.8           1024 over 16000 (192):  1: 427, *2: 370 (434), 3: 399 (430)
+//                     461 over 8192 (88):  1: 126, 2: 128, *3: 105, 4: 132           512 over 8192 (96):  1: 123 (125), 2: 134 (137), *3: 110 (125), 4: 129 (139)
+// Two row tiles a CTA have costs of their own, as measured when their weights still went through shared memory:
+//                     1200 over 4000 (152):  1: 150, *2: 148, 3: 150 (153)        1200 over 8192:  1: 280, 2: 243 (250), *3: 237 (248), 4: 242 (255)
 //                     1600 over 4000 (200):  *1: 169 (171), 2: 167 (178)             1500 over 20000 (192):  1: 673, 2: 550 (620), *3: 534 (607), 4: 635 (650)
 //                     3000 over 8192 (376):  *1: 493 (542), 2: 565 (594)             4096 over 8192 (512):  *1: 706 (756), 2: 713 (790)
-// Two row tiles a CTA have costs of their own: with the single tiles', 1600 over 4000 and 4096 over 8192 were cut in 2, 2048 over 32000 in 4 (1128, long
-// run 1269; whole, as now: 1112 and 1218).
-static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, uint32_t most, uint32_t head_dim, uint32_t tiles_per_cta) {
-    const double tile_us = tiles_per_cta == 2 ? 1.0 : head_dim == 256 ? 0.6 : 0.4, wave_us = 3.0;
-    const double partial_us = tiles_per_cta == 2 ? 0.07 : head_dim == 256 ? 0.03 : 0.01;
+static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, double average, uint32_t most, uint32_t head_dim, uint32_t tiles_per_cta) {
+    struct Costs { double tile_us, wave_us, last_wave, longest, merge_us, partial_us; };
+    const Costs c = tiles_per_cta == 2 ? Costs{1.0, 3.0, 0.6, 1.0, 0.0, 0.07} : head_dim == 256 ? Costs{0.62, 12.4, 0.5, 0.42, 0.0, 0.024} : Costs{0.43, 1.95, 1.0, 0.07, 1.3, 0.017};
     uint32_t best = 1;
     double best_us = 0.0;
     for (uint32_t s = 1; s <= kMaxKvSplits && s <= (most > 1 ? most : 1); ++s) {
         const uint64_t ctas = static_cast<uint64_t>(units) * s, full = ctas / 148, rest = ctas % 148;
-        const double waves = static_cast<double>(full) + (rest == 0 ? 0.0 : full == 0 ? 1.0 : 0.6 + 0.4 * static_cast<double>(rest) / 148.0);
-        const double us = waves * (tiles * tile_us / s + wave_us) + (s > 1 ? partial_us * static_cast<double>(ctas) : 0.0);
+        const double waves = static_cast<double>(full) + (rest == 0 ? 0.0 : full == 0 ? 1.0 : c.last_wave + (1.0 - c.last_wave) * static_cast<double>(rest) / 148.0);
+        const double walked = ctas <= 148 ? tiles : c.longest * tiles + (1.0 - c.longest) * average;
+        const double us = waves * (walked * c.tile_us / s + c.wave_us) + (s > 1 ? c.merge_us + c.partial_us * static_cast<double>(ctas) : 0.0);
         if (s == 1 || us < best_us) { best = s; best_us = us; }
     }
     return best;
@@ -1092,20 +1155,20 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     p.capacity = view.capacity;
     p.scratch_rows = scratch_rows;
     p.scale_log2 = scale * 1.4426950408889634f;
-    // head_dim 128: two row tiles per CTA where that still leaves every SM a CTA.  Both take the same K and V tiles, and one tile's
-    // MMAs run under the other one's softmax.  Fewer rows spread better as single tiles.
+    // head_dim 128: two row tiles per CTA where that still leaves every SM a CTA.  Both take the same K and V tiles, and set-up, Q and output come once for both.
+    // Fewer rows spread better as single tiles.
     const uint32_t row_tiles_128 = static_cast<uint32_t>((static_cast<uint64_t>(token_count) * (query_heads / view.kv_heads) + kBM - 1) / kBM);
     const uint32_t tiles_per_cta = view.head_dim == 128 && (row_tiles_128 + 1) / 2 * static_cast<uint64_t>(view.kv_heads) >= 148 ? 2u : 1u;
     // KV split when the row tiles alone leave SMs idle and the caller's workspace has room for the partials
     p.kv_splits = 1;
     {
-        const uint32_t G = query_heads / view.kv_heads;
-        const uint32_t row_tiles = (token_count * G + tiles_per_cta * kBM - 1) / (tiles_per_cta * kBM);
+        const uint32_t row_tiles = (row_tiles_128 + tiles_per_cta - 1) / tiles_per_cta;
         // A device-side state leaves the range unknown here (no split).  Every split walks a few tiles: three of the longest range, or,
         // where the chunk's own triangle is longer than its prefix, eight of the prefix, which is all that its first rows see.
         const uint32_t tiles = static_cast<uint32_t>((rows + kBN - 1) / kBN), prefix_tiles = (base_position + kBN - 1) / kBN;
         const uint32_t most = prefill_state != nullptr ? 1 : base_position >= token_count ? tiles / 3 : prefix_tiles / 8;
-        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, most, view.head_dim, tiles_per_cta);
+        const double average = std::min<double>(tiles, (base_position + 0.5 * token_count) / kBN);
+        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, average, most, view.head_dim, tiles_per_cta);
         const size_t scratch = prefill_tc5_workspace_bytes(static_cast<uint32_t>(rows), view.kv_heads, view.head_dim);
         while (want > 1 && workspace_bytes < scratch + 1024 + prefill_tc5_split_bytes(token_count, query_heads, view.kv_heads, view.head_dim, want)) --want;
         if (want > 1) {
