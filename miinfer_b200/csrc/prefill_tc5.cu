@@ -46,7 +46,7 @@ constexpr float kRescaleThreshold = 8.0f;        // log2 units
 constexpr uint32_t kMaxKvSplits = 16;
 
 struct Tc5Params {
-    CUtensorMap kmap, vmap;      // fp16 [kv_heads * rows][d], box 64 x 64, 128-byte swizzle
+    CUtensorMap kmap, vmap;      // fp16 [kv_heads][rows][d], box 1 x 64 x 64, 128-byte swizzle; zeros past the rows
     const void* q;               // [token][query_heads][D]
     int q_is_f16;
     const float* gate;
@@ -80,9 +80,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
 
 // Shared-memory matrix descriptor (sm_100 format): start address, leading/stride byte offsets (all >> 4),
@@ -379,15 +379,14 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
 
     if (D == 128 && warp == kTmaWarp) {
         // =============================== TMA producer, K and V tiles ===============================
-        const int row_base = static_cast<int>(kv_head * p.scratch_rows);
         auto load_k = [&](int i) -> bool {   // a pair of tiles: tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab
             const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
             if (!mbar_wait(bar(K_EMPTY + ps), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) return false;
             mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
             for (int t = 0; t < n; ++t)
                 for (int s = 0; s < L::kSlabs; ++s)
-                    tma_load_2d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
-                                row_base + (tile0 + 2 * i + t) * kBN, bar(K_FULL + ps));
+                    tma_load_3d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
+                                (tile0 + 2 * i + t) * kBN, kv_head, bar(K_FULL + ps));
             return true;
         };
         auto load_v = [&](int j) -> bool {
@@ -395,7 +394,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             if (!mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) return false;
             mbar_expect_tx(bar(V_FULL + st), L::kTileBytes);
             for (int s = 0; s < L::kSlabs; ++s)
-                tma_load_2d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, row_base + (tile0 + j) * kBN, bar(V_FULL + st));
+                tma_load_3d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, (tile0 + j) * kBN, kv_head, bar(V_FULL + st));
             return true;
         };
         bool ok = true;
@@ -418,7 +417,6 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         // A ring stage holds a PAIR of tiles, tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab, so that
         // one MMA instruction (N = 128) covers both.
         if (lane == 0) {
-            const int row_base = static_cast<int>(kv_head * p.scratch_rows);
             for (int i = 0; 2 * i < ntiles; ++i) {
                 const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
                 // Q first: nothing can start without it, and 148 CTAs that fill their rings at once keep L2 busy for over 3 us.  The first pair of K
@@ -428,8 +426,8 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
                 for (int t = 0; t < n; ++t)
                     for (int s = 0; s < L::kSlabs; ++s)
-                        tma_load_2d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
-                                    row_base + (tile0 + 2 * i + t) * kBN, bar(K_FULL + ps));
+                        tma_load_3d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
+                                    (tile0 + 2 * i + t) * kBN, kv_head, bar(K_FULL + ps));
             }
         }
     } else if (D == 256 && warp == kTmaVWarp) {
@@ -442,13 +440,12 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 prefetch_l2(p.gate + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D, G * D * 4);
         }
         if (have_q && lane == 0) {
-            const int row_base = static_cast<int>(kv_head * p.scratch_rows);
             for (int j = 0; j < ntiles; ++j) {
                 const int st = j % L::kVTiles;
                 if (!mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) break;
                 mbar_expect_tx(bar(V_FULL + st), L::kTileBytes);
                 for (int s = 0; s < L::kSlabs; ++s)
-                    tma_load_2d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, row_base + (tile0 + j) * kBN, bar(V_FULL + st));
+                    tma_load_3d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, (tile0 + j) * kBN, kv_head, bar(V_FULL + st));
             }
         }
     } else if (warp >= kSWarp && warp < kPvWarp) {
@@ -714,12 +711,10 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                          "l"((static_cast<unsigned long long>(static_cast<uint32_t>(t) + 1u) << 32) | __float_as_uint(m_new)) : "memory");
             // At 128 it is read back as well: what follows depends on the value read, so no exponential can be scheduled ahead of the store.  (Without that the store
             // came behind all of them, by the compiler's choice and by small changes around it: a tile of one row tile took 1050 clocks, not 820.)  At 256, whose
-            // two groups wait less for each other, the value out of a shuffle behind the store does better: us a layer back to back, as it comes / read back / shuffled,
-            // 512 over 8192 127.1 / 126.2 / 125.0, 300 over 8192 83.3 / 86.6 / 81.5, 37 over 3001 24.1 / 24.5 / 24.1.
+            // two groups wait less for each other, it costs up to 5 % (300 over 8192, 24 / 4 heads), and a shuffle behind the store, which did better in one text of this
+            // kernel, 2 % in this one: 512 over 8192 125.8 us a layer back to back as it is, 129.5 with it.
             if constexpr (D == 128)
                 asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(m_new) : "r"(smem_u32(const_cast<unsigned long long*>(ref))) : "memory");
-            else
-                m_new = __shfl_sync(0xffffffffu, m_new, lane);
             rebase(m_new);
             const float neg_ref = (m_new == -INFINITY) ? 0.0f : -m_new;
             Pair sum = 0;
@@ -940,6 +935,7 @@ struct DequantParams {
     uint32_t scratch_rows;
     uint32_t row_begin;  // this launch converts positions [row_begin, row_end): the rows below were converted ahead of
     uint32_t row_end;    // the chunk (b200kv_prefill_prepare), possibly beside the previous layer's attention
+    uint32_t side0;      // first side the launch converts
 };
 
 // A thread converts kDequantUnits pieces of 8 elements, a block's threads side by side and all of a thread's loads in flight together: a warp
@@ -952,7 +948,7 @@ __global__ void __launch_bounds__(256, 4) dequant_prefix_kernel(const __grid_con
     constexpr uint32_t CPR = D / 8;
     pdl_launch_dependents();
     pdl_wait();   // the cache rows of this chunk come from the append kernel just before
-    const uint32_t head = blockIdx.y, side = blockIdx.z;   // side 0 = K, 1 = V
+    const uint32_t head = blockIdx.y, side = p.side0 + blockIdx.z;   // side 0 = K, 1 = V
     const uint32_t mode = p.view.quant_mode;
     const bool q8 = side == 0 ? (mode == B200KV_Q8_F16 || mode == B200KV_Q8_Q8) : (mode == B200KV_F16_Q8 || mode == B200KV_Q8_Q8);
     const uint32_t nblk = D / p.view.qblock;
@@ -1005,28 +1001,37 @@ EncodeFn tc5_encoder() {
     return fn;
 }
 
-bool encode_f16_plane(CUtensorMap* map, void* base, uint32_t d, uint64_t rows) {
+// Planes [kv_heads][plane_rows][d] of which `rows` rows a head are read.
+bool encode_f16_plane(CUtensorMap* map, const void* base, uint32_t d, uint64_t rows, uint64_t plane_rows, uint32_t kv_heads) {
     EncodeFn fn = tc5_encoder();
     if (fn == nullptr) return false;
-    const TensorMapKey key{base, rows, d * 2u, 128u, static_cast<uint32_t>(kBN), 2u};   // kind 2: fp16, 128-byte swizzle
-    if (tensor_map_lookup(key, map)) return true;
-    const cuuint64_t dims[2] = {d, rows};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(d) * 2};
-    const cuuint32_t box[2] = {64, kBN};
-    const cuuint32_t elem[2] = {1, 1};
-    if (fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    tensor_map_remember(key, *map);
-    return true;
+    const cuuint64_t dims[3] = {d, rows, kv_heads};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(d) * 2, plane_rows * d * 2};
+    const cuuint32_t box[3] = {64, kBN, 1};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The pre-pass over positions [row_begin, row_end) of every kv head, K and V.
+// An fp16 side of the cache is read where it lies; only int8 sides go through the scratch.  (The map ends at the visible rows, so the last tile's other rows
+// come as zeros, as in the scratch.)  24 / 4 heads of 256, us a layer: 67 over 4826 30.8 -> 24.0.  Where the caller has converted rows ahead
+// (b200kv_prefill_prepare) the copy is completed and used, and a chunk that sees no more than one tile goes through the scratch as well: what a call
+// leaves there is relied on in these two cases.
+struct Sides { bool k, v; };   // sides that go through the scratch
+Sides scratch_sides(const b200kv_view& view, uint64_t rows, uint32_t prepared_rows) {
+    const auto direct = [&](bool q8, const void* plane) {
+        return !q8 && prepared_rows == 0 && rows > kBN && (reinterpret_cast<uintptr_t>(plane) & 15) == 0 && view.capacity * view.head_dim * 2 < (1ull << 40);
+    };
+    return {!direct(is_k_q8(view.quant_mode), view.key_f16), !direct(is_v_q8(view.quant_mode), view.value_f16)};
+}
+
+// The pre-pass over positions [row_begin, row_end) of every kv head, of one or both sides.
 template <int D>
 int launch_dequant(const b200kv_view& view, __half* k_scratch, __half* v_scratch, uint32_t rows, uint32_t scratch_rows,
-                   uint32_t row_begin, uint32_t row_end, cudaStream_t stream) {
-    if (row_begin >= row_end) return B200KV_OK;
+                   uint32_t row_begin, uint32_t row_end, Sides sides, cudaStream_t stream) {
+    if (row_begin >= row_end || (!sides.k && !sides.v)) return B200KV_OK;
     DequantParams dp{};
+    dp.side0 = sides.k ? 0 : 1;
     dp.view = view;
     dp.k_out = k_scratch;
     dp.v_out = v_scratch;
@@ -1036,7 +1041,7 @@ int launch_dequant(const b200kv_view& view, __half* k_scratch, __half* v_scratch
     dp.row_end = row_end;
     constexpr uint32_t rows_per_block = 256 * kDequantUnits / (D / 8);
     const unsigned blocks = (row_end - row_begin + rows_per_block - 1) / rows_per_block;
-    B200KV_CUDA_TRY(launch_kernel(dequant_prefix_kernel<D>, dim3(blocks, view.kv_heads, 2), dim3(256), 0, stream, true, dp));
+    B200KV_CUDA_TRY(launch_kernel(dequant_prefix_kernel<D>, dim3(blocks, view.kv_heads, sides.k && sides.v ? 2 : 1), dim3(256), 0, stream, true, dp));
     return B200KV_OK;
 }
 
@@ -1049,7 +1054,7 @@ int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half*
     if (attr_err != cudaSuccess) { set_last_cuda_error(attr_err, "cudaFuncSetAttribute(prefill_tc5)"); return B200KV_ERR_CUDA; }
     if (rows > 0) {
         const int rc = launch_dequant<D>(view, k_scratch, v_scratch, rows, p.scratch_rows, prepared_rows < rows ? prepared_rows : rows,
-                                         p.scratch_rows, stream);
+                                         p.scratch_rows, scratch_sides(view, rows, prepared_rows), stream);
         if (rc != B200KV_OK) return rc;
     }
     const uint32_t G = p.query_heads / p.kv_heads;
@@ -1140,9 +1145,12 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     __half* k_scratch = reinterpret_cast<__half*>(ws);
     __half* v_scratch = k_scratch + static_cast<size_t>(view.kv_heads) * scratch_rows * view.head_dim;
     Tc5Params p{};
-    if (!encode_f16_plane(&p.kmap, k_scratch, view.head_dim, static_cast<uint64_t>(view.kv_heads) * scratch_rows) ||
-        !encode_f16_plane(&p.vmap, v_scratch, view.head_dim, static_cast<uint64_t>(view.kv_heads) * scratch_rows))
-        return B200KV_ERR_UNSUPPORTED;
+    const Sides sides = scratch_sides(view, rows, prepared_rows);
+    const auto encode = [&](CUtensorMap* map, bool scratch, const __half* copy, const void* plane) {
+        return scratch ? encode_f16_plane(map, copy, view.head_dim, scratch_rows, scratch_rows, view.kv_heads)
+                       : encode_f16_plane(map, plane, view.head_dim, rows, view.capacity, view.kv_heads);
+    };
+    if (!encode(&p.kmap, sides.k, k_scratch, view.key_f16) || !encode(&p.vmap, sides.v, v_scratch, view.value_f16)) return B200KV_ERR_UNSUPPORTED;
     p.q = q;
     p.q_is_f16 = q_is_f16;
     p.gate = gate;
@@ -1197,8 +1205,8 @@ int launch_prefill_tc5_prepare(const b200kv_view& view, uint32_t prepared_rows, 
     uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(workspace) + 1023) & ~static_cast<uintptr_t>(1023));
     __half* k_scratch = reinterpret_cast<__half*>(ws);
     __half* v_scratch = k_scratch + static_cast<size_t>(view.kv_heads) * scratch_rows * view.head_dim;
-    return view.head_dim == 128 ? launch_dequant<128>(view, k_scratch, v_scratch, prepared_rows, scratch_rows, 0, prepared_rows, stream)
-                                : launch_dequant<256>(view, k_scratch, v_scratch, prepared_rows, scratch_rows, 0, prepared_rows, stream);
+    return view.head_dim == 128 ? launch_dequant<128>(view, k_scratch, v_scratch, prepared_rows, scratch_rows, 0, prepared_rows, Sides{true, true}, stream)
+                                : launch_dequant<256>(view, k_scratch, v_scratch, prepared_rows, scratch_rows, 0, prepared_rows, Sides{true, true}, stream);
 }
 
 }  // namespace b200kv
