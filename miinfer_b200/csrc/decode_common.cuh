@@ -128,6 +128,17 @@ uint32_t* current_status_word();
 // Which streaming kernel serves int8 caches: 0 = the tcgen05 kernel where it applies, 1 = the warp-level mma kernel.
 int streaming_kernel_choice();
 
+// Brings [src, src + bytes) on its way to L2, whatever still writes it: a load behind the dependency wait sees that.  One warp, a line a lane and step.
+__device__ __forceinline__ void prefetch_lines(const void* src, uint32_t bytes, int lane) {
+    for (uint32_t at = lane * 128; at < bytes; at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(src) + at));
+}
+// One lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(ok));
+    return ok != 0;
+}
+
 // The scanned range [begin, end) of one session, resolved on the device the way
 // the reference resolves its DeviceDecodeState (position + 1 entries,
 // gfx906/kernels/qwen3_primitives.hip:7394-7395).

@@ -225,6 +225,8 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
 
     // old rows do not depend on the preceding kernels: their copies start before the wait for those
     while (next_unit < P::kUnits - 1 && (next_unit >> 1) < my_tiles && min(tile_pos(next_unit >> 1) + kTile, copy_end) <= early_end) issue();
+    if (split == 0 && warp == WARPS - 1)
+        prefetch_lines(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(session) * p.query_heads + kv_head * G) * D * (p.q_is_f16 ? 2 : 4), G * D * (p.q_is_f16 ? 2 : 4), lane);
     Rotation<D> rot{};
     if (makes_key) row_rotation<D>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();

@@ -100,6 +100,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (mbar_try(bar, parity)) return true;
     return false;
 }
+// Bounded wait of a whole warp for two phases, asked for together: all lanes go on or none.
+__device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
+    bool ok = false;
+    for (uint32_t spin = 0; spin < kSpin && !ok; ++spin) {
+        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
+        ok = a && b;
+    }
+    return __all_sync(0xffffffffu, ok);
+}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -262,6 +271,8 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     const bool appends = warp == kAppendWarp && owner;
+    if (split == 0 && warp == kPvWarp)
+        prefetch_lines(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(session) * p.query_heads + kv_head * G) * kD * (Q_F16 ? 2 : 4), G * kD * (Q_F16 ? 2 : 4), lane);
     Rotation<kD> rot{};
     if (appends) row_rotation<kD>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();
@@ -368,39 +379,41 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
         }
     } else if (warp == kMmaWarp) {
         // =============================== issuer of S^T = K . Q^T ===============================
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = umma_idesc_i8(kTileM, 16, 1, 1, 0);   // K (signed) x Q planes (signed), both K-major
-            for (int i = 0; i < ntiles; ++i) {
-                const int stage = i % kStages, buf = i & 1;
-                if (!mbar_wait(bar_s_empty(buf), static_cast<uint32_t>(((i >> 1) & 1) ^ 1))) { failed = true; break; }   // S buffer read out (tile i - 2)
-                if (!mbar_wait(bar_full(stage), static_cast<uint32_t>((i / kStages) & 1))) { failed = true; break; }     // tile landed
-                tc_fence_after();
-                const uint32_t kt = sbase + L::kOffK + stage * L::kKTile;
+        // The warp stays together and one lane issues: descriptors lie in uniform registers, which an MMA takes them from.
+        constexpr uint32_t idesc_s = umma_idesc_i8(kTileM, 16, 1, 1, 0);   // K (signed) x Q planes (signed), both K-major
+        const uint64_t k_desc = umma_desc(sbase + L::kOffK, 16, 1024, 2), q_desc = umma_desc(sbase + L::kOffQ, 16, 1024, 2);
+        for (int i = 0; i < ntiles; ++i) {
+            const int stage = i % kStages, buf = i & 1;
+            // S buffer read out (tile i - 2), tile landed
+            if (!mbar_wait_both(bar_s_empty(buf), static_cast<uint32_t>(((i >> 1) & 1) ^ 1), bar_full(stage), static_cast<uint32_t>((i / kStages) & 1))) { failed = true; break; }
+            tc_fence_after();
+            const uint64_t kt = k_desc + ((stage * L::kKTile) >> 4);
+            if (elect_one()) {
 #pragma unroll
                 for (int b = 0; b < 4; ++b)   // one q8_0 block of 32 dims per MMA, each into its own 16 columns
-                    umma_i8(tmem_base + kColS + buf * 64 + b * 16, umma_desc(kt + 32 * b, 16, 1024, 2),
-                            umma_desc(sbase + L::kOffQ + 32 * b, 16, 1024, 2), idesc_s, 0);
+                    umma_i8(tmem_base + kColS + buf * 64 + b * 16, kt + ((32 * b) >> 4), q_desc + ((32 * b) >> 4), idesc_s, 0);
                 umma_commit(bar_s_full(buf));
             }
+            __syncwarp();
         }
     } else if (warp == kPvWarp) {
         // =============================== issuer of O^T = V^T . P ===============================
-        if (lane == 0) {
-            constexpr uint32_t idesc_o = umma_idesc_i8(kD, 32, 1, 0, 1, 1);    // V^T (signed, MN-major) x P planes (unsigned, MN-major)
-            for (int i = 0; i < ntiles; ++i) {
-                const int stage = i % kStages, buf = i & 1;
-                if (!mbar_wait(bar_p_full(buf), static_cast<uint32_t>((i >> 1) & 1))) { failed = true; break; }
-                if (!mbar_wait(bar_full(stage), static_cast<uint32_t>((i / kStages) & 1))) { failed = true; break; }   // long complete: the V tile's landing, observed by this thread
-                tc_fence_after();
-                const uint32_t vt = sbase + L::kOffV + stage * L::kKTile;
-                const uint32_t pt = sbase + L::kOffP + buf * (kTileM * 32);
+        constexpr uint32_t idesc_o = umma_idesc_i8(kD, 32, 1, 0, 1, 1);    // V^T (signed, MN-major) x P planes (unsigned, MN-major)
+        const uint64_t v_desc = umma_desc(sbase + L::kOffV, kTileM * kD, 1024, 2), p_desc = umma_desc(sbase + L::kOffP, 32, 256, 6);
+        for (int i = 0; i < ntiles; ++i) {
+            const int stage = i % kStages, buf = i & 1;
+            // the weights, and (long complete) the V tile's landing, observed by these threads
+            if (!mbar_wait_both(bar_p_full(buf), static_cast<uint32_t>((i >> 1) & 1), bar_full(stage), static_cast<uint32_t>((i / kStages) & 1))) { failed = true; break; }
+            tc_fence_after();
+            const uint64_t vt = v_desc + ((stage * L::kKTile) >> 4), pt = p_desc + ((buf * (kTileM * 32)) >> 4);
+            if (elect_one()) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)   // 32 positions per MMA
-                    umma_i8(tmem_base + kColO + buf * 32, umma_desc(vt + j * (32 * kD), kTileM * kD, 1024, 2),
-                            umma_desc(pt + j * (32 * 32), 32, 256, 6), idesc_o, j > 0);
+                    umma_i8(tmem_base + kColO + buf * 32, vt + ((j * (32 * kD)) >> 4), pt + ((j * (32 * 32)) >> 4), idesc_o, j > 0);
                 umma_commit(bar_p_empty(buf));      // P buffer free, the tile's sums complete
                 umma_commit(bar_empty(stage));      // ring stage may be refilled
             }
+            __syncwarp();
         }
     }
 

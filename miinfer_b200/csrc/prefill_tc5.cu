@@ -190,12 +190,6 @@ __device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar_a, uint32_t parity_
     }
     return __all_sync(0xffffffffu, ok);
 }
-// One lane of a converged warp, always the same one.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(ok));
-    return ok != 0;
-}
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
