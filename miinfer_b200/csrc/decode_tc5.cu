@@ -16,7 +16,10 @@
 //    scales can be applied to exact int32 sums: 128 threads (one per position = TMEM lane) read their 32 sums with
 //    tcgen05.ld and finish the scores in fp32.
 //  * Online softmax in base 2: the tile maximum per head is found with redux.sync inside each warp and one exchange
-//    through shared memory between the four warps; the running maximum is uniform across the CTA.
+//    through shared memory between the four warps; the running maximum is uniform across the CTA.  A tile's time is this chain's, so its
+//    instructions count: weights relative to the tile come from an exponential of their own, not a quotient, they are rounded to whole numbers by adding 2^23,
+//    the rescale at a new maximum is branched around, maxima are reduced as floats, and the two barriers a tile waits for are asked at once.  With MMAs issued by an
+//    elected lane, us: 36 layers at 32768 positions 597 -> 566 -> 562 (issue, then the softmax), 16 at 16000 190 -> 184 -> 174, 80 sessions x 4 layers 796 -> 774 -> 726.
 //  * O^T += V^T . P: the V tile as it lies is the A operand again, this time MN-major (M = 128 dims, K = positions),
 //    and P is written by the 128 threads as unsigned 16-bit fixed point in two uint8 planes, pre-multiplied by the
 //    value scale of each block: P[position][(block, plane, head)] = 32 B-operand columns, MN-major too (rows of 32
@@ -33,7 +36,6 @@
 //    finish in the normal way (all later waits are skipped, barriers are still attended, TMEM is freed).
 #include "decode_tail.cuh"
 
-#include <climits>
 #include <cstring>
 
 namespace b200kv {
@@ -109,6 +111,14 @@ __device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a
     }
     return __all_sync(0xffffffffu, ok);
 }
+// The same of single lanes.
+__device__ __forceinline__ bool mbar_wait_both_lane(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
+    for (uint32_t spin = 0; spin < kSpin; ++spin) {
+        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
+        if (a && b) return true;
+    }
+    return false;
+}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -160,9 +170,8 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Order-preserving map of fp32 to int32 (for redux.sync.max) and back.
-__device__ __forceinline__ int ordered(float f) { const int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); }
-__device__ __forceinline__ float unordered(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+// Largest value of a warp; a NaN counts for nothing (its head's sum is NaN).
+__device__ __forceinline__ float warp_max_redux(float f) { float r; asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f)); return r; }
 
 // NBLK scales per row (4 = q8_0 blocks of 32, 1 = one per row); up to 4 query heads per kv head.
 template <int NBLK, bool Q_F16>
@@ -448,8 +457,8 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
 
         for (int i = 0; i < ntiles; ++i) {
             const int stage = i % kStages, buf = i & 1;
-            wait(bar_full(stage), static_cast<uint32_t>((i / kStages) & 1));      // the scale tiles of this stage (async-proxy writes)
-            wait(bar_s_full(buf), static_cast<uint32_t>((i >> 1) & 1));
+            // the scale tiles of this stage (async-proxy writes), and the scores
+            if (!failed && !mbar_wait_both_lane(bar_full(stage), static_cast<uint32_t>((i / kStages) & 1), bar_s_full(buf), static_cast<uint32_t>((i >> 1) & 1))) failed = true;
             if (TL && i == 0 && tid == 0) tl[3] = global_ns();
             tc_fence_after();
             int sv[4][8];   // per block: hi sums of heads 0-3, lo sums of heads 0-3
@@ -493,15 +502,15 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
             }
             // ---- tile maxima (scores per head, value scales per block): redux inside the warp, one exchange across the four ----
             {
-                int mx[4];
+                float mx[4];
                 uint32_t vmx[NBLK];
 #pragma unroll
-                for (int h = 0; h < 4; ++h) mx[h] = __reduce_max_sync(0xffffffffu, ordered(s[h]));
+                for (int h = 0; h < 4; ++h) mx[h] = warp_max_redux(s[h]);
 #pragma unroll
                 for (int b = 0; b < NBLK; ++b) vmx[b] = __reduce_max_sync(0xffffffffu, valid ? vs_bits[b] : 0u);   // positive fp16 order like integers
                 if (lane == 0) {
                     int* dst = xch + (buf * 4 + warp) * 8;
-                    *reinterpret_cast<int4*>(dst) = make_int4(mx[0], mx[1], mx[2], mx[3]);
+                    *reinterpret_cast<float4*>(dst) = make_float4(mx[0], mx[1], mx[2], mx[3]);
                     if constexpr (NBLK == 4) *reinterpret_cast<uint4*>(dst + 4) = make_uint4(vmx[0], vmx[1], vmx[2], vmx[3]);
                     else dst[4] = static_cast<int>(vmx[0]);
                 }
@@ -509,13 +518,13 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
             asm volatile("bar.sync 3, 128;" ::: "memory");
             float m_tile[4], vs_max[4];
             {
-                int mx[4] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN};
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                 uint32_t vmx[4] = {0, 0, 0, 0};
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
                     const int* src = xch + (buf * 4 + w) * 8;
-                    const int4 a = *reinterpret_cast<const int4*>(src);
-                    mx[0] = max(mx[0], a.x); mx[1] = max(mx[1], a.y); mx[2] = max(mx[2], a.z); mx[3] = max(mx[3], a.w);
+                    const float4 a = *reinterpret_cast<const float4*>(src);
+                    mx[0] = fmaxf(mx[0], a.x); mx[1] = fmaxf(mx[1], a.y); mx[2] = fmaxf(mx[2], a.z); mx[3] = fmaxf(mx[3], a.w);
                     if constexpr (NBLK == 4) {
                         const uint4 b = *reinterpret_cast<const uint4*>(src + 4);
                         vmx[0] = max(vmx[0], b.x); vmx[1] = max(vmx[1], b.y); vmx[2] = max(vmx[2], b.z); vmx[3] = max(vmx[3], b.w);
@@ -524,23 +533,29 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
                     }
                 }
 #pragma unroll
-                for (int h = 0; h < 4; ++h) m_tile[h] = unordered(mx[h]);
+                for (int h = 0; h < 4; ++h) m_tile[h] = mx[h];
 #pragma unroll
                 for (int b = 0; b < 4; ++b) vs_max[b] = __half2float(__ushort_as_half(static_cast<uint16_t>(vmx[NBLK == 4 ? b : 0])));
             }
             // ---- online softmax: new running maximum, weights, and the tile's fixed-point scales ----
             float wn[4], nscale[4];   // weights normalised to the tile maximum (<= 1); fixed-point scale of this tile (own block)
             const float vs_own = warp == 0 ? vs_max[0] : warp == 1 ? vs_max[1] : warp == 2 ? vs_max[2] : vs_max[3];
+            // (the maxima are the CTA's, so the branch is taken by all threads or none; after the first tiles it rarely is)
+            if (m_tile[0] > m_run[0] || m_tile[1] > m_run[1] || m_tile[2] > m_run[2] || m_tile[3] > m_run[3]) {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const float m_new = fmaxf(m_run[h], m_tile[h]);
+                    const float alpha = (m_run[h] == -INFINITY) ? 0.0f : exp2f(m_run[h] - m_new);
+                    acc[h] *= alpha; l_run[h] *= alpha; pend_a[h] *= alpha; pend_b[h] *= alpha;
+                    m_run[h] = m_new;
+                }
+            }
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                const float m_new = fmaxf(m_run[h], m_tile[h]);
-                const float alpha = (m_run[h] == -INFINITY) ? 0.0f : exp2f(m_run[h] - m_new);
-                acc[h] *= alpha; l_run[h] *= alpha; pend_a[h] *= alpha; pend_b[h] *= alpha;
-                m_run[h] = m_new;
-                const float w = (s[h] == -INFINITY) ? 0.0f : exp2f(s[h] - m_new);
+                const float w = (s[h] == -INFINITY) ? 0.0f : exp2f(s[h] - m_run[h]);
                 l_run[h] += w;
-                const float wmax = (m_tile[h] == -INFINITY) ? 0.0f : exp2f(m_tile[h] - m_new);
-                wn[h] = wmax > 0.0f ? __fdividef(w, wmax) : 0.0f;
+                const float wmax = (m_tile[h] == -INFINITY) ? 0.0f : exp2f(m_tile[h] - m_run[h]);
+                wn[h] = (s[h] == -INFINITY || !(wmax > 0.0f)) ? 0.0f : exp2f(s[h] - m_tile[h]);
                 nscale[h] = wmax * vs_own * (1.0f / kPMax);
             }
             // [block]: w * value_scale as 16-bit fixed point, then the planes: hi bytes of heads 0-3, lo bytes of heads 0-3
@@ -548,10 +563,12 @@ decode_tc5_kernel(const __grid_constant__ DecodeParams p, const __grid_constant_
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 const float wv = (valid && vs_max[b] > 0.0f) ? vs[b] * __fdividef(kPMax, vs_max[b]) : 0.0f;
+                // products of at most 65535 (and an ulp or two): beside 2^23 they come rounded to whole numbers in the low 16 bits.  (A NaN weight comes as 65535; its
+                // head's sum is NaN.)
                 uint32_t pq[4];
 #pragma unroll
-                for (int h = 0; h < 4; ++h) pq[h] = min(__float2uint_rn(wn[h] * wv), 65535u);
-                const uint32_t p01 = pq[0] | (pq[1] << 16), p23 = pq[2] | (pq[3] << 16);
+                for (int h = 0; h < 4; ++h) pq[h] = __float_as_uint(__fmaf_rn(wn[h], wv, 8388608.0f));
+                const uint32_t p01 = __byte_perm(pq[0], pq[1], 0x5410), p23 = __byte_perm(pq[2], pq[3], 0x5410);
                 p_hi[b] = __byte_perm(p01, p23, 0x7531);
                 p_lo[b] = __byte_perm(p01, p23, 0x6420);
             }

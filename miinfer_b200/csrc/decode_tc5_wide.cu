@@ -15,13 +15,14 @@
 //  * with one CTA on an SM nothing else hides a tile's chain S MMA -> softmax -> P -> P.V MMA -> fold, so two groups of 128
 //    softmax threads take the even and the odd tiles (S, P and O are double-buffered: a buffer per group), each with its own
 //    running maxima, sums and accumulators, which are merged once at the end;
+//  * the softmax's instructions as there, 48 weights a thread and tile.  24 / 4 heads, 16 layers, us, with MMAs issued by an elected lane and then the softmax: 32000
+//    positions 370 -> 339 -> 316, 16000 (a scale per row) 266 -> 243 -> 221, 100000 747 -> 699 -> 668;
 //  * the merge of the splits and the single-token append of a decode step run inside the launch, as there (decode_tail.cuh);
 //    the append is the P.V issuer warp's first job, which has nothing to do before the first tile's weights are there.
 //    (As launches of their own the merge cost 1.7 us at 32768 positions -- 21.1 against 19.4 us -- and the append 4 to 5 more.)
 //  * Every wait is bounded, as there.
 #include "decode_tail.cuh"
 
-#include <climits>
 #include <cstring>
 #include <mutex>
 
@@ -93,6 +94,14 @@ __device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a
     }
     return __all_sync(0xffffffffu, ok);
 }
+// The same of single lanes.
+__device__ __forceinline__ bool mbar_wait_both_lane(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
+    for (uint32_t spin = 0; spin < kSpin; ++spin) {
+        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
+        if (a && b) return true;
+    }
+    return false;
+}
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -135,9 +144,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&r)[16]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Order-preserving map of fp32 to int32 (for redux.sync.max) and back.
-__device__ __forceinline__ int ordered(float f) { const int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); }
-__device__ __forceinline__ float unordered(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+// Largest value of a warp; a NaN counts for nothing (its head's sum is NaN).
+__device__ __forceinline__ float warp_max_redux(float f) { float r; asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f)); return r; }
 
 // The appended row's 256 bytes into row r of a K or V tile (two 128-byte-wide halves, 128-byte swizzle); lanes 0-15.
 __device__ __forceinline__ void patch_row(uint8_t* tile, const uint8_t* row, uint32_t r, int lane) {
@@ -474,8 +482,8 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
             // other tile, the ring has three stages, so a group would skip phases of a stage; it therefore also waits for the
             // tile in between (the other group's), which has normally landed long before.
             if (i > 0) wait(bar_v_full((i - 1) % kVStages), static_cast<uint32_t>(((i - 1) / kVStages) & 1));
-            wait(bar_v_full(stage), static_cast<uint32_t>((i / kVStages) & 1));   // the scale tiles of this stage (async-proxy writes)
-            wait(bar_s_full(buf), static_cast<uint32_t>((i >> 1) & 1));
+            // the scale tiles of this stage (async-proxy writes), and the scores
+            if (!failed && !mbar_wait_both_lane(bar_v_full(stage), static_cast<uint32_t>((i / kVStages) & 1), bar_s_full(buf), static_cast<uint32_t>((i >> 1) & 1))) failed = true;
             tc_fence_after();
 
             const uint32_t pos = (t0 + i) * kTileM + ltid;
@@ -521,37 +529,46 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
             // ---- tile maxima (scores per head, value scales per block): redux inside the warp, one exchange across the group's four ----
             const int par = (i >> 1) & 1;   // the exchange area is double-buffered by the parity of the group's tile count
             {
-                int* dst = xch + ((grp * 2 + par) * 4 + wq) * 16;
+                float mx[8];
+                uint32_t vmx[8];
 #pragma unroll
-                for (int h = 0; h < G; ++h) {
-                    const int mx = __reduce_max_sync(0xffffffffu, ordered(s[h]));
-                    if (lane == 0) dst[h] = mx;
-                }
+                for (int h = 0; h < 8; ++h) mx[h] = h < G ? warp_max_redux(s[h < G ? h : 0]) : -INFINITY;
 #pragma unroll
-                for (int b = 0; b < (NBLK == 8 ? 8 : 1); ++b) {
-                    const uint32_t vmx = __reduce_max_sync(0xffffffffu, valid ? vs_bits[b] : 0u);   // positive fp16 order like integers
-                    if (lane == 0) dst[8 + b] = static_cast<int>(vmx);
+                for (int b = 0; b < 8; ++b) vmx[b] = b < NBLK ? __reduce_max_sync(0xffffffffu, valid ? vs_bits[b] : 0u) : 0u;   // positive fp16 order like integers
+                if (lane == 0) {
+                    float* dst = reinterpret_cast<float*>(xch + ((grp * 2 + par) * 4 + wq) * 16);
+                    *reinterpret_cast<float4*>(dst) = make_float4(mx[0], mx[1], mx[2], mx[3]);
+                    if constexpr (G > 4) *reinterpret_cast<float4*>(dst + 4) = make_float4(mx[4], mx[5], mx[6], mx[7]);
+                    *reinterpret_cast<uint4*>(dst + 8) = make_uint4(vmx[0], vmx[1], vmx[2], vmx[3]);
+                    if constexpr (NBLK == 8) *reinterpret_cast<uint4*>(dst + 12) = make_uint4(vmx[4], vmx[5], vmx[6], vmx[7]);
                 }
             }
             group_sync();
             float m_tile[G], vs_max[8];
             {
-                int mx[G];
                 uint32_t vmx[8];
 #pragma unroll
-                for (int h = 0; h < G; ++h) mx[h] = INT_MIN;
+                for (int h = 0; h < G; ++h) m_tile[h] = -INFINITY;
 #pragma unroll
                 for (int b = 0; b < 8; ++b) vmx[b] = 0;
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
-                    const int* src = xch + ((grp * 2 + par) * 4 + w) * 16;
+                    const float* src = reinterpret_cast<const float*>(xch + ((grp * 2 + par) * 4 + w) * 16);
 #pragma unroll
-                    for (int h = 0; h < G; ++h) mx[h] = max(mx[h], src[h]);
+                    for (int q = 0; q < (G + 3) / 4; ++q) {
+                        const float4 a = *reinterpret_cast<const float4*>(src + 4 * q);
+                        const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-                    for (int b = 0; b < (NBLK == 8 ? 8 : 1); ++b) vmx[b] = max(vmx[b], static_cast<uint32_t>(src[8 + b]));
+                        for (int h = 0; h < 4; ++h)
+                            if (4 * q + h < G) m_tile[4 * q + h < G ? 4 * q + h : 0] = fmaxf(m_tile[4 * q + h < G ? 4 * q + h : 0], av[h]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < (NBLK == 8 ? 2 : 1); ++q) {
+                        const uint4 b = *reinterpret_cast<const uint4*>(src + 8 + 4 * q);
+                        vmx[4 * q] = max(vmx[4 * q], b.x); vmx[4 * q + 1] = max(vmx[4 * q + 1], b.y);
+                        vmx[4 * q + 2] = max(vmx[4 * q + 2], b.z); vmx[4 * q + 3] = max(vmx[4 * q + 3], b.w);
+                    }
                 }
-#pragma unroll
-                for (int h = 0; h < G; ++h) m_tile[h] = unordered(mx[h]);
 #pragma unroll
                 for (int b = 0; b < 8; ++b) vs_max[b] = __half2float(__ushort_as_half(static_cast<uint16_t>(vmx[NBLK == 8 ? b : 0])));
             }
@@ -561,17 +578,26 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf)
                 vs_own[hf] = wq == 0 ? vs_max[4 * hf] : wq == 1 ? vs_max[4 * hf + 1] : wq == 2 ? vs_max[4 * hf + 2] : vs_max[4 * hf + 3];
+            // (the maxima are the group's, so the branch is taken by all its threads or none; after the first tiles it rarely is)
+            bool grew = false;
+#pragma unroll
+            for (int h = 0; h < G; ++h) grew = grew || m_tile[h] > m_run[h];
+            if (grew) {
+#pragma unroll
+                for (int h = 0; h < G; ++h) {
+                    const float m_new = fmaxf(m_run[h], m_tile[h]);
+                    const float alpha = (m_run[h] == -INFINITY) ? 0.0f : exp2f(m_run[h] - m_new);
+                    acc[0][h] *= alpha; acc[1][h] *= alpha; l_run[h] *= alpha;
+                    pend[0][h] *= alpha; pend[1][h] *= alpha;
+                    m_run[h] = m_new;
+                }
+            }
 #pragma unroll
             for (int h = 0; h < G; ++h) {
-                const float m_new = fmaxf(m_run[h], m_tile[h]);
-                const float alpha = (m_run[h] == -INFINITY) ? 0.0f : exp2f(m_run[h] - m_new);
-                acc[0][h] *= alpha; acc[1][h] *= alpha; l_run[h] *= alpha;
-                pend[0][h] *= alpha; pend[1][h] *= alpha;
-                m_run[h] = m_new;
-                const float w = (s[h] == -INFINITY) ? 0.0f : exp2f(s[h] - m_new);
+                const float w = (s[h] == -INFINITY) ? 0.0f : exp2f(s[h] - m_run[h]);
                 l_run[h] += w;
-                const float wmax = (m_tile[h] == -INFINITY) ? 0.0f : exp2f(m_tile[h] - m_new);
-                wn[h] = wmax > 0.0f ? __fdividef(w, wmax) : 0.0f;
+                const float wmax = (m_tile[h] == -INFINITY) ? 0.0f : exp2f(m_tile[h] - m_run[h]);
+                wn[h] = (s[h] == -INFINITY || !(wmax > 0.0f)) ? 0.0f : exp2f(s[h] - m_tile[h]);
                 nscale[0][h] = wmax * vs_own[0] * (1.0f / kPMax);
                 nscale[1][h] = wmax * vs_own[1] * (1.0f / kPMax);
             }
@@ -587,10 +613,13 @@ decode_tc5_wide_kernel(const __grid_constant__ DecodeParams p, const __grid_cons
 #pragma unroll
             for (int b = 0; b < 8; ++b) {
                 const float wv = (valid && vs_max[b] > 0.0f) ? vs[b] * __fdividef(kPMax, vs_max[b]) : 0.0f;
+                // products of at most 65535 (and an ulp or two): beside 2^23 they come rounded to whole numbers in the low 16 bits.  (A NaN weight comes as 65535; its
+                // head's sum is NaN.)
                 uint32_t pq[8];
 #pragma unroll
-                for (int h = 0; h < 8; ++h) pq[h] = h < G ? min(__float2uint_rn(wn[h < G ? h : 0] * wv), 65535u) : 0u;
-                const uint32_t p01 = pq[0] | (pq[1] << 16), p23 = pq[2] | (pq[3] << 16), p45 = pq[4] | (pq[5] << 16), p67 = pq[6] | (pq[7] << 16);
+                for (int h = 0; h < 8; ++h) pq[h] = h < G ? __float_as_uint(__fmaf_rn(wn[h < G ? h : 0], wv, 8388608.0f)) : 0u;
+                const uint32_t p01 = __byte_perm(pq[0], pq[1], 0x5410), p23 = __byte_perm(pq[2], pq[3], 0x5410), p45 = __byte_perm(pq[4], pq[5], 0x5410),
+                               p67 = __byte_perm(pq[6], pq[7], 0x5410);
                 const uint32_t hi_a = __byte_perm(p01, p23, 0x7531), hi_b = __byte_perm(p45, p67, 0x7531);
                 const uint32_t lo_a = __byte_perm(p01, p23, 0x6420), lo_b = __byte_perm(p45, p67, 0x6420);
                 // half b >> 2, span (b >> 1) & 1, chunk b & 1
