@@ -337,8 +337,57 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     }
 
     const int live_tiles = min(RT, static_cast<int>((total_rows - row0 + kBM - 1) / kBM));   // row tiles that hold rows
-    // ---- set-up: barriers, TMEM, Q tile -----------------------------------------------------------------
-    if (tid == 0) {
+    // ---- set-up: barriers, TMEM, Q ---------------------------------------------------------------------------
+    // At head_dim 128 nothing of this waits for the rest: a CTA that takes another's place has its Q on its way into registers and its first K tiles into their
+    // ring before its barriers are everybody's, and the CTA before has called its Q to L2.  (Set-up, then the loads: 1.5 us of every CTA but the first
+    // wave's, which set up ahead of the dependency wait.  32 / 8 heads, us a layer: 1024 over 8192 175.5 -> 171, 37 over 3000 20.35 -> 19.7, 225 fresh 13.5 -> 13.0.  At 256 the same text
+    // comes out of the compiler with a slower tile loop, 512 over 8192 125.7 -> 130.7.)
+    constexpr bool kEarlyQ = D == 128;
+    const int turn_row = lane >> 3, turn_chunk = lane & 7;
+    const int rt = RT == 1 ? 0 : warp >> 3;                // row tile
+    const uint32_t tile_row0 = row0 + rt * kBM, warp_row0 = tile_row0 + (warp & 3) * 32;
+    // A pair of K tiles into its ring stage, tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab (D == 256: one MMA instruction of N = 128 covers
+    // both).
+    auto issue_k = [&](int i) {
+        const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
+        mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
+        for (int t = 0; t < n; ++t)
+            for (int s = 0; s < L::kSlabs; ++s)
+                tma_load_3d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
+                            (tile0 + 2 * i + t) * kBN, kv_head, bar(K_FULL + ps));
+    };
+    // The query rows from r0 on of kv head `head` on their way to L2 (a prefetch reads nothing yet: whatever still writes them, the loads behind the wait
+    // see).  A warp.
+    auto prefetch_q = [&](uint32_t r0, uint32_t head) {
+        const uint32_t elem = p.q_is_f16 ? 2 : 4, t_last = (min(r0 + L::kRows, total_rows) - 1) / G;
+        for (uint32_t t = r0 / G + lane; t <= t_last; t += 32)
+            prefetch_l2(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(t) * p.query_heads + head * G) * D * elem, G * D * elem);
+    };
+    constexpr int kTurns = D / 128;            // 32 columns = 64 dims per store; all loads are in flight together
+    constexpr int kQWarps = RT * 8;            // two threads of a row each take half of it
+    auto fetch_q = [&](const RowOffsets<D>& rows, uint4 (&q)[kTurns][8]) {
+        auto fetch = [&](auto f16) {
+            const size_t base0 = (static_cast<size_t>(warp_row0 / G) * p.query_heads + kv_head * G) * D + ((warp >> 2) & 1) * (D / 2) + turn_chunk * 8;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int k = 0; k < kTurns; ++k) {
+                    q[k][i] = make_uint4(0, 0, 0, 0);
+                    if (i >= rows.valid) continue;
+                    if (f16()) {
+                        q[k][i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + base0 + rows.rel[i] + k * 64);
+                    } else {
+                        const float* src = static_cast<const float*>(p.q) + base0 + rows.rel[i] + k * 64;
+                        const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+                        q[k][i] = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
+                    }
+                }
+        };
+        if constexpr (RT == 2) fetch([&] { return p.q_is_f16 != 0; });   // (a branch around both: 1 % slower with two row tiles, 2 to 6 % faster with one)
+        else if (p.q_is_f16) fetch([] { return true; });
+        else fetch([] { return false; });
+    };
+    if (kEarlyQ ? warp == kTmaWarp && lane == 0 : tid == 0) {
         for (int i = 0; i < L::kNumBars; ++i) {
             uint32_t count = 1;
             if (i >= S_EMPTY && i < P_EMPTY) count = kBM;   // S_EMPTY and P_FULL: a group's threads
@@ -353,34 +402,39 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    [[maybe_unused]] uint4 early_q[kTurns][8];
+    // one wave of CTAs: Q ahead of the wait (24 / 4 heads, 37 fp32 tokens over 3001: 24.3 -> 24.1 us a layer)
+    if (kEarlyQ && warp == kTmaWarp && split_u == 0 && gridDim.x <= 148) prefetch_q(row0, kv_head);
+    if constexpr (kEarlyQ) {
+        if (warp < kQWarps) {
+            const RowOffsets<D> rows(warp_row0, turn_row, G, p.query_heads, total_rows);
+            pdl_wait();   // Q, the fp16 scratch and the device-side state come from preceding kernels
+            fetch_q(rows, early_q);
+        } else {
+            pdl_wait();
+            if (warp == kTmaWarp && lane == 0 && ntiles > 0) issue_k(0);
+        }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // The query rows on their way to L2 (a prefetch reads nothing yet: whatever still writes them, the loads behind the wait see), and where they lie.  With
-    // more than a wave of CTAs there is nothing to wait for.  (24 / 4 heads, 37 fp32 tokens over 3001: 24.3 -> 24.1 us a layer.)
-    if (warp == kTmaWarp && split_u == 0 && gridDim.x <= 148) {
-        const uint32_t elem = p.q_is_f16 ? 2 : 4, t_last = (min(row0 + L::kRows, total_rows) - 1) / G;
-        for (uint32_t t = row0 / G + lane; t <= t_last; t += 32)
-            prefetch_l2(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D * elem, G * D * elem);
-    }
-    const int turn_row = lane >> 3, turn_chunk = lane & 7;
-    const int rt = RT == 1 ? 0 : warp >> 3;                // row tile
-    const uint32_t tile_row0 = row0 + rt * kBM, warp_row0 = tile_row0 + (warp & 3) * 32;
-    const RowOffsets<D> rows(warp_row0, turn_row, G, p.query_heads, total_rows);
-    pdl_wait();   // Q, the fp16 scratch and the device-side state come from preceding kernels
+    if (!kEarlyQ && warp == kTmaWarp && split_u == 0 && gridDim.x <= 148) prefetch_q(row0, kv_head);
+    [[maybe_unused]] const RowOffsets<D> late_rows(warp_row0, turn_row, G, p.query_heads, total_rows);
+    if constexpr (!kEarlyQ) pdl_wait();
     bool failed = false;
+    // The query rows of the CTA that takes this one's place, as far as the order of dispatch tells.  A warp.
+    auto next_q = [&] {
+        const uint32_t next = blockIdx.x + 148;
+        if (next < gridDim.x && next % p.kv_splits == 0)
+            prefetch_q(((total_rows + L::kRows - 1) / L::kRows - 1 - next / p.kv_splits / p.kv_heads) * L::kRows, next / p.kv_splits % p.kv_heads);
+    };
 
     if (D == 128 && warp == kTmaWarp) {
         // =============================== TMA producer, K and V tiles ===============================
-        auto load_k = [&](int i) -> bool {   // a pair of tiles: tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab
-            const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
-            if (!mbar_wait(bar(K_EMPTY + ps), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) return false;
-            mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
-            for (int t = 0; t < n; ++t)
-                for (int s = 0; s < L::kSlabs; ++s)
-                    tma_load_3d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
-                                (tile0 + 2 * i + t) * kBN, kv_head, bar(K_FULL + ps));
+        auto load_k = [&](int i) -> bool {
+            if (!mbar_wait(bar(K_EMPTY + i % kKPairs), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) return false;
+            issue_k(i);
             return true;
         };
         auto load_v = [&](int j) -> bool {
@@ -391,10 +445,8 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 tma_load_3d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, (tile0 + j) * kBN, kv_head, bar(V_FULL + st));
             return true;
         };
-        bool ok = true;
-        if (lane == 0 && ntiles > 0) ok = load_k(0);
-        __syncwarp();
-        ok = mbar_wait(bar(Q_FULL), 0) && ok;
+        bool ok = mbar_wait(bar(Q_FULL), 0);
+        next_q();
         if (p.gate != nullptr && split_u == 0) {
             const uint32_t t_last = (min(row0 + L::kRows, total_rows) - 1) / G;
             for (uint32_t t = row0 / G + lane; t <= t_last; t += 32)
@@ -408,22 +460,14 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         }
     } else if (warp == kTmaWarp) {
         // =============================== TMA producer, K tiles ===============================
-        // A ring stage holds a PAIR of tiles, tile 2i in rows 0-63 and tile 2i+1 in rows 64-127 of every slab, so that
-        // one MMA instruction (N = 128) covers both.
-        if (lane == 0) {
+        // Q first: nothing can start without it, and 148 CTAs that fill their rings at once keep L2 busy for over 3 us.  The first pair of K
+        // tiles goes along with it, the other stages are asked for when it is in.
+        if (lane == 0)
             for (int i = 0; 2 * i < ntiles; ++i) {
-                const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
-                // Q first: nothing can start without it, and 148 CTAs that fill their rings at once keep L2 busy for over 3 us.  The first pair of K
-                // tiles goes along with it, the other stages are asked for when it is in.
                 if (i == 1 && !mbar_wait(bar(Q_FULL), 0)) break;
-                if (!mbar_wait(bar(K_EMPTY + ps), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) break;
-                mbar_expect_tx(bar(K_FULL + ps), n * L::kTileBytes);
-                for (int t = 0; t < n; ++t)
-                    for (int s = 0; s < L::kSlabs; ++s)
-                        tma_load_3d(sbase + L::kOffK + ps * L::kPairBytes + s * (2 * kBN * 128) + t * (kBN * 128), &p.kmap, s * 64,
-                                    (tile0 + 2 * i + t) * kBN, kv_head, bar(K_FULL + ps));
+                if (!mbar_wait(bar(K_EMPTY + i % kKPairs), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) break;
+                issue_k(i);
             }
-        }
     } else if (D == 256 && warp == kTmaVWarp) {
         // =============================== TMA producer, V tiles ===============================
         const bool have_q = mbar_wait(bar(Q_FULL), 0);
@@ -556,31 +600,18 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         // tiles is on its way meanwhile.  From the dependency wait to the last row: 0.8 us (two row tiles of 128 dims; 3.8 behind full rings and with
         // a division a row), 3.3 us (one of 256 from HBM; 4.5).
         uint8_t* const turn = smem + L::kOffP + warp * 4096;   // [32 rows][8 chunks of 16 B], chunk c of row r at c ^ (r & 7)
-        if (L::kSoftmaxThreads == RT * 256 || warp < 8) {
+        if (warp < kQWarps) {
+            uint4 q[kTurns][8];
+            if constexpr (kEarlyQ) {
+#pragma unroll
+                for (int k = 0; k < kTurns; ++k)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) q[k][i] = early_q[k][i];
+            } else {
+                fetch_q(late_rows, q);
+            }
             const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
             const int half = (warp >> 2) & 1;
-            constexpr int kTurns = D / 128;            // 32 columns = 64 dims per store; all loads are in flight together
-            uint4 q[kTurns][8];
-            auto fetch = [&](auto f16) {
-                const size_t base0 = (static_cast<size_t>(warp_row0 / G) * p.query_heads + kv_head * G) * D + half * (D / 2) + turn_chunk * 8;
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int k = 0; k < kTurns; ++k) {
-                        q[k][i] = make_uint4(0, 0, 0, 0);
-                        if (i >= rows.valid) continue;
-                        if (f16()) {
-                            q[k][i] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(p.q) + base0 + rows.rel[i] + k * 64);
-                        } else {
-                            const float* src = static_cast<const float*>(p.q) + base0 + rows.rel[i] + k * 64;
-                            const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
-                            q[k][i] = make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
-                        }
-                    }
-            };
-            if constexpr (RT == 2) fetch([&] { return p.q_is_f16 != 0; });   // (a branch around both: 1 % slower with two row tiles, 2 to 6 % faster with one)
-            else if (p.q_is_f16) fetch([] { return true; });
-            else fetch([] { return false; });
 #pragma unroll
             for (int k = 0; k < kTurns; ++k) {
                 const int c0 = 32 * k;
