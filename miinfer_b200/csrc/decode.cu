@@ -159,7 +159,9 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     }
     const bool chosen = num_splits == 0;
     if (chosen) {
-        uint32_t fast = use_fast ? pick_splits_q8(geometry, p.query_heads, p.sessions, max_length) : 0;
+        uint32_t fast = !use_fast ? 0
+                      : !many && streaming_kernel_choice() != 1 ? pick_splits_tc5(geometry, p.query_heads, max_length)
+                                                                : pick_splits_q8(geometry, p.query_heads, p.sessions, max_length);
         if (fast == 0) use_fast = false;
         num_splits = use_fast ? fast
                    : use_wide ? pick_splits_tc5_wide(geometry, max_length)

@@ -187,6 +187,7 @@ int launch_decode_tc5(const DecodeParams& p, const b200kv_view& geometry, uint32
 bool decode_tc5_wide_ok(const b200kv_view& view, uint32_t query_heads);
 uint32_t pick_splits_tc5_wide(const b200kv_view& view, uint32_t max_length);
 int launch_decode_tc5_wide(const DecodeParams& p, const b200kv_view& geometry, cudaStream_t stream);
+uint32_t pick_splits_tc5(const b200kv_view& view, uint32_t query_heads, uint32_t max_length);
 uint32_t pick_splits_q8(const b200kv_view& geometry, uint32_t query_heads, uint32_t sessions, uint32_t max_length);
 // TMA descriptors of a view's int8 K and V planes (rows of head_dim bytes, 128-byte swizzle).
 // B200KV_ERR_UNSUPPORTED when the view cannot take the kernels that need them (then decode_stream.cu is used).

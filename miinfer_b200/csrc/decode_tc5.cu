@@ -36,6 +36,7 @@
 //    finish in the normal way (all later waits are skipped, barriers are still attended, TMEM is freed).
 #include "decode_tail.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 namespace b200kv {
@@ -651,6 +652,20 @@ int launch_one(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap
 }
 
 }  // namespace
+
+// Splits of one session, up to two CTAs per SM: two tiles each as long as every CTA finds a place at once, then the count with the least estimated time.  With launch
+// overlap the mergers of the launch before (one CTA a query head) hold places that long, and the last splits' CTAs start up to 2 us behind the others; a tile of a full
+// wave costs less than that, and every split is one more partial to merge.  36 or 37 splits at any length -> these, 32 / 8 heads, q8_0, 16 layers, us, with overlap
+// (without): 9000 positions 145 -> 132 (189 -> 189), 10000 163 -> 137 (198 -> 198), 12000 161 -> 142 (205 -> 201), 16000 174 -> 157 (221 -> 215), 20000 190 -> 182
+// (244 -> 236).  Below that the estimate is 1 to 2 % behind halves (5000: 122 / 124).  No more CTAs than places: 64 / 16 heads took 19 splits, two waves (12000: 296 -> 205).
+uint32_t pick_splits_tc5(const b200kv_view& view, uint32_t query_heads, uint32_t max_length) {
+    if (!q8_fast_path_ok(view, query_heads)) return 0;
+    const uint32_t kv = view.kv_heads, tiles = (max_length + kTileM - 1) / kTileM, halves = std::max(1u, static_cast<uint32_t>((max_length + 15ull) / (2 * kTileM)));
+    const uint32_t most = std::min(std::max(1u, 296u / kv), max_splits_per_session(1));
+    const uint32_t on_time = query_heads < 296u ? (296u - query_heads) / kv : 0;
+    if (halves <= on_time) return std::min(halves, most);
+    return cheapest_splits(tiles, std::min(most, halves), on_time, SplitCosts{450, 900, 45, 0, 150, 5});
+}
 
 int launch_decode_tc5(const DecodeParams& p_in, const b200kv_view& geometry, uint32_t max_length, cudaStream_t stream) {
     if (!q8_fast_path_ok(geometry, p_in.query_heads)) return B200KV_ERR_UNSUPPORTED;

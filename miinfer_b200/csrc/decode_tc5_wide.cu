@@ -23,6 +23,7 @@
 //  * Every wait is bounded, as there.
 #include "decode_tail.cuh"
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -756,14 +757,15 @@ bool decode_tc5_wide_ok(const b200kv_view& view, uint32_t query_heads) {
     return wide_encoder() != nullptr;
 }
 
-// One CTA per SM; every CTA should see at least two tiles.
+// At most one CTA per SM (19 splits of 8 heads are two waves: 48 / 8 heads, 10000 positions, 16 layers 436 -> 248 us); a full wave from five tiles a split on, where no
+// number was ahead by more than runs differ.  Below that the least estimated time: every split is a partial to merge, and a wave of more than 140 CTAs leaves the next
+// launch no SM to start on.  24 / 4 heads, q8_0, 16 layers, 37 splits -> these, us with launch overlap (without): 10200 positions 214 -> 199 (257 -> 241), 12000 216 -> 208
+// (260 -> 261), 16000 239 -> 232 (278 -> 276), 20000 257 -> 250 (292 -> 287).
 uint32_t pick_splits_tc5_wide(const b200kv_view& view, uint32_t max_length) {
-    uint32_t s = (148u + view.kv_heads / 2) / view.kv_heads;
+    const uint32_t most = std::min(std::max(1u, 148u / view.kv_heads), max_splits_per_session(1));
     const uint32_t tiles = (max_length + kTileM - 1) / kTileM;
-    if (s > tiles / 2) s = tiles / 2;
-    const uint32_t cap = max_splits_per_session(1);
-    if (s > cap) s = cap;
-    return s ? s : 1;
+    if (tiles >= 5 * most) return most;
+    return cheapest_splits(tiles, most, 140u / view.kv_heads, SplitCosts{850, 850, 70, 500, 0, ~0u});
 }
 
 // A single-session launch (p.num_splits and the workspace pointers set by the caller); B200KV_ERR_UNSUPPORTED when the

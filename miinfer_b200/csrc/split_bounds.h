@@ -18,6 +18,29 @@ B200KV_HD uint32_t part_begin(uint32_t total, uint32_t i, uint32_t parts) {
     return q * i + r * i / parts;
 }
 
+// Splits of one session for a pipelined kernel whose CTAs walk whole tiles, by the least estimated time (nanoseconds, fitted by the kernels that call this): the
+// longest split's tiles, the first three of which may cost less (they are on their way before the launch may begin), every split's partial on its way
+// through the merge, and splits past `on_time`, whose CTAs find a place only when the launch before has left its own.  Looked at are the fewest splits for every
+// longest part from the shortest possible to eight tiles more.  Parts of `fill` tiles or more share the memory's bandwidth: then as many of one length as there are places.
+struct SplitCosts { uint32_t early_tile, tile, split, late, per_late, fill; };
+B200KV_HD uint32_t cheapest_splits(uint32_t tiles, uint32_t most, uint32_t on_time, SplitCosts c) {
+    if (tiles == 0 || most <= 1) return 1;
+    const uint32_t shortest = (tiles + most - 1) / most;
+    uint32_t best = 1, best_longest = tiles;
+    uint64_t least = ~0ull;
+    for (uint32_t longest = shortest; longest <= tiles && longest <= shortest + 8; ++longest) {
+        const uint32_t splits = (tiles + longest - 1) / longest, early = longest < 3 ? longest : 3;
+        const uint64_t cost = static_cast<uint64_t>(early) * c.early_tile + static_cast<uint64_t>(longest - early) * c.tile + static_cast<uint64_t>(splits) * c.split +
+                              (splits > on_time ? c.late + static_cast<uint64_t>(splits - on_time) * c.per_late : 0);
+        if (cost < least) { least = cost; best = splits; best_longest = longest; }
+    }
+    if (best_longest >= c.fill && best_longest > 1) {
+        const uint32_t same = (tiles - 1) / (best_longest - 1), room = best <= on_time && on_time < most ? on_time : most;   // the most parts of that length
+        best = same < room ? same : room;
+    }
+    return best;
+}
+
 // Splits per kv head whose CTAs find an SM only when the mergers of the launch before leave theirs, one CTA per SM.  Only under launch overlap, behind a
 // launch of the same shape that merges inside (`mergers` units per kv head) and where both together are more than the device holds; never half of
 // the splits or more.
