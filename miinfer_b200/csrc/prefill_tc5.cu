@@ -5,7 +5,8 @@
 //
 //  1. A streaming pre-pass dequantises the positions the chunk can see, [0, kv_end), once per launch into an
 //     fp16 scratch in the caller's workspace (K and V planes, [kv_head][row][d]); with int8 -> fp16 exact up to
-//     the one rounding of q * scale.  The scratch (35.6 MB at 8704 x 4 x 256) stays in the 126 MB L2.
+//     the one rounding of q * scale.  The scratch (35.6 MB at 8704 x 4 x 256) stays in the 126 MB L2.  fp16 sides of the cache
+//     are read where they lie.
 //  2. The attention kernel gives each CTA 128 query ROWS of one kv head (a row is a (token, head-of-group)
 //     pair, so the G heads of a group share every K/V tile) and walks the causal range in tiles of 64 positions,
 //     two tiles at a time:
