@@ -225,8 +225,13 @@ __global__ void __launch_bounds__(WARPS * 32, 8 / WARPS) decode_stream_kernel(co
 
     // old rows do not depend on the preceding kernels: their copies start before the wait for those
     while (next_unit < P::kUnits - 1 && (next_unit >> 1) < my_tiles && min(tile_pos(next_unit >> 1) + kTile, copy_end) <= early_end) issue();
-    if (split == 0 && warp == WARPS - 1)
-        prefetch_lines(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(session) * p.query_heads + kv_head * G) * D * (p.q_is_f16 ? 2 : 4), G * D * (p.q_is_f16 ? 2 : 4), lane);
+    // The queries on their way to L2.  Not for one session over an int8 cache, whose launch is the shortest chain up to the wait.  Without -> with, us: fp16, one session, 32 / 8 heads
+    // of 128, 36 layers at 1081 positions 187.5 -> 184.5, 24 / 4 of 256, 16 at 2500 140.5 -> 139.2; many, int8, 24 / 4 of 256, 8 layers, 4 sessions of 2000 152.1 -> 149.3, 17 of 1389
+    // 146.0 -> 143.1; one session, q8_0, 32 / 8 of 128, 36 layers at 640 203.8 -> 206.7, 782 208.1 -> 209.6.
+    if constexpr (WARPS == 4 || (KF == F16 && VF == F16)) {
+        const uint32_t row = D * (p.q_is_f16 ? 2 : 4);
+        if (split == 0 && warp == WARPS - 1) prefetch_lines(static_cast<const uint8_t*>(p.q) + (static_cast<size_t>(session) * p.query_heads + kv_head * G) * row, G * row, lane);
+    }
     Rotation<D> rot{};
     if (makes_key) row_rotation<D>(rot, lane, end - 1, p.rope_mode, p.inv_freq, p.sectioned_step);   // needs the position only
     pdl_wait();
