@@ -231,7 +231,7 @@ struct Layout {
     // mbarriers; the ones after V_EMPTY are per row tile, S_EMPTY and the P pairs (kPInTmem: S_FULL too) per row tile and softmax group
     static constexpr int kBufs = RT * kGroups;
     static constexpr int K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = V_FULL + kVTiles, S_FULL = V_EMPTY + kVTiles, S_EMPTY = S_FULL + (kPInTmem ? kBufs : RT),
-                         P_FULL = S_EMPTY + (kPInTmem ? 0 : kBufs), P_EMPTY = P_FULL + kBufs, O_DONE = P_EMPTY + kBufs, Q_FULL = O_DONE + RT, kNumBars = Q_FULL + 1;
+                         P_FULL = S_EMPTY + (kPInTmem ? 0 : kBufs), P_EMPTY = P_FULL + kBufs, O_DONE = P_EMPTY + kBufs, Q_FULL = O_DONE + RT, V_TAIL = Q_FULL + 1, kNumBars = V_TAIL + 1;
     static constexpr int kOffSlot = kOffBar + (kNumBars * 8 + 15) / 16 * 16;
     static constexpr int kOffRef = kOffSlot + 16;                 // [rows] {reference maximum, sequence}: handed from tile to tile
     // [2 groups][128 rows] partial row sums of a row tile in its epilogue, where its own score MMAs are through: over the K
@@ -271,13 +271,14 @@ struct RowOffsets {
     }
 };
 
-template <int D, int RT>
+// STATE: the position comes from a device-side state (one row tile a CTA).
+template <int D, int RT, bool STATE>
 __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel(const __grid_constant__ Tc5Params p) {
     using L = Layout<D, RT>;
     constexpr int kThreads = L::kThreads;
     constexpr int kTmaWarp = L::kTmaWarp, kSWarp = L::kSWarp, kPvWarp = L::kPvWarp, kTmaVWarp = L::kTmaVWarp;
     constexpr int K_FULL = L::K_FULL, K_EMPTY = L::K_EMPTY, V_FULL = L::V_FULL, V_EMPTY = L::V_EMPTY, S_FULL = L::S_FULL, S_EMPTY = L::S_EMPTY,
-                  P_FULL = L::P_FULL, P_EMPTY = L::P_EMPTY, O_DONE = L::O_DONE, Q_FULL = L::Q_FULL;
+                  P_FULL = L::P_FULL, P_EMPTY = L::P_EMPTY, O_DONE = L::O_DONE, Q_FULL = L::Q_FULL, V_TAIL = L::V_TAIL;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw;
     const uint32_t sbase = smem_u32(smem);
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     const uint32_t kv_head = tile_head % p.kv_heads;
     const uint32_t G = p.query_heads / p.kv_heads;
     uint32_t base = p.base_position, count = p.token_count;
-    if (p.prefill_state != nullptr) {
+    if constexpr (STATE) {
         pdl_wait();   // the state may be the preceding kernel's output
         base = p.prefill_state->base_position;
         count = min(count, p.prefill_state->token_count);
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
         else fetch([] { return false; });
     };
     if (kEarlyQ ? warp == kTmaWarp && lane == 0 : tid == 0) {
-        for (int i = 0; i < L::kNumBars; ++i) {
+        for (int i = 0; i < (STATE ? L::kNumBars : L::V_TAIL); ++i) {
             uint32_t count = 1;
             if (i >= S_EMPTY && i < P_EMPTY) count = kBM;   // S_EMPTY and P_FULL: a group's threads
             else if (i == Q_FULL) count = RT * 256;
@@ -432,19 +433,38 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             prefetch_q(((total_rows + L::kRows - 1) / L::kRows - 1 - next / p.kv_splits / p.kv_heads) * L::kRows, next / p.kv_splits % p.kv_heads);
     };
 
+    auto copy_v = [&](int j, int full) {
+        mbar_expect_tx(bar(full), L::kTileBytes);
+        for (int s = 0; s < L::kSlabs; ++s)
+            tma_load_3d(sbase + L::kOffV + j % L::kVTiles * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, (tile0 + j) * kBN, kv_head, bar(full));
+    };
+    auto load_v = [&](int j) -> bool {
+        if (!mbar_wait(bar(V_EMPTY + j % L::kVTiles), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) return false;
+        copy_v(j, V_FULL + j % L::kVTiles);
+        return true;
+    };
+    // With a device-side state the maps end at the capacity and not at the visible rows: the last tile's rows from kv_end on bring whatever lies in the cache, and a weight of zero times NaN
+    // is NaN.  The warp that feeds the V ring clears them before it hands the tile over (the swizzle stays within a row).  A kernel of its own has it: the text alone
+    // cost the others up to 0.9 % (2048 fresh, 32 / 8 heads of 128).
+    [[maybe_unused]] const int whole_tiles = STATE && kv_end % kBN != 0 ? ntiles - 1 : ntiles;   // tiles handed over as they land
+    [[maybe_unused]] auto load_last_v = [&](bool ok) {   // a warp; `ok`: lane 0 has handed over the others
+        const int j = ntiles - 1, st = j % L::kVTiles;
+        if (lane == 0 && ok && mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) copy_v(j, V_TAIL);
+        __syncwarp();
+        if (!mbar_wait_warp(bar(V_TAIL), 0)) return;
+        for (int s = 0; s < L::kSlabs; ++s)
+            for (uint32_t at = kv_end % kBN * 128 + lane * 16; at < kBN * 128; at += 32 * 16)
+                *reinterpret_cast<uint4*>(smem + L::kOffV + st * L::kTileBytes + s * (kBN * 128) + at) = make_uint4(0, 0, 0, 0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(V_FULL + st));
+    };
+
     if (D == 128 && warp == kTmaWarp) {
         // =============================== TMA producer, K and V tiles ===============================
         auto load_k = [&](int i) -> bool {
             if (!mbar_wait(bar(K_EMPTY + i % kKPairs), static_cast<uint32_t>((i / kKPairs) & 1) ^ 1)) return false;
             issue_k(i);
-            return true;
-        };
-        auto load_v = [&](int j) -> bool {
-            const int st = j % L::kVTiles;
-            if (!mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) return false;
-            mbar_expect_tx(bar(V_FULL + st), L::kTileBytes);
-            for (int s = 0; s < L::kSlabs; ++s)
-                tma_load_3d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, (tile0 + j) * kBN, kv_head, bar(V_FULL + st));
             return true;
         };
         bool ok = mbar_wait(bar(Q_FULL), 0);
@@ -455,11 +475,13 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 prefetch_l2(p.gate + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D, G * D * 4);
         }
         if (lane == 0) {
-            for (int j = 0; ok && j < ntiles; ++j) {
+            for (int j = 0; ok && j < whole_tiles; ++j) {
                 if ((j & 1) == 0 && j + 2 < ntiles) ok = load_k((j >> 1) + 1);
                 ok = ok && load_v(j);
             }
         }
+        if constexpr (STATE)
+            if (whole_tiles < ntiles) load_last_v(ok);
     } else if (warp == kTmaWarp) {
         // =============================== TMA producer, K tiles ===============================
         // Q first: nothing can start without it, and 148 CTAs that fill their rings at once keep L2 busy for over 3 us.  The first pair of K
@@ -479,15 +501,11 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             for (uint32_t t = row0 / G + lane; t <= t_last; t += 32)
                 prefetch_l2(p.gate + (static_cast<size_t>(t) * p.query_heads + kv_head * G) * D, G * D * 4);
         }
-        if (have_q && lane == 0) {
-            for (int j = 0; j < ntiles; ++j) {
-                const int st = j % L::kVTiles;
-                if (!mbar_wait(bar(V_EMPTY + st), static_cast<uint32_t>((j / L::kVTiles) & 1) ^ 1)) break;
-                mbar_expect_tx(bar(V_FULL + st), L::kTileBytes);
-                for (int s = 0; s < L::kSlabs; ++s)
-                    tma_load_3d(sbase + L::kOffV + st * L::kTileBytes + s * (kBN * 128), &p.vmap, s * 64, (tile0 + j) * kBN, kv_head, bar(V_FULL + st));
-            }
-        }
+        bool ok = have_q;
+        if (lane == 0)
+            for (int j = 0; ok && j < whole_tiles; ++j) ok = load_v(j);
+        if constexpr (STATE)
+            if (whole_tiles < ntiles) load_last_v(ok);
     } else if (warp >= kSWarp && warp < kPvWarp) {
         // =============================== S = Q.K^T issuer ===============================
         // The warp stays together and one lane issues (D == 128): loop counters and descriptors live in uniform registers, which an MMA takes them from
@@ -1043,8 +1061,9 @@ bool encode_f16_plane(CUtensorMap* map, const void* base, uint32_t d, uint64_t r
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// An fp16 side of the cache is read where it lies; only int8 sides go through the scratch.  (The map ends at the visible rows, so the last tile's other rows
-// come as zeros, as in the scratch.)  24 / 4 heads of 256, us a layer: 67 over 4826 30.8 -> 24.0.  Where the caller has converted rows ahead
+// An fp16 side of the cache is read where it lies; only int8 sides go through the scratch.  (The map ends at the rows the launch may see, so the last tile's
+// other rows come as zeros, as in the scratch; with a device-side state that is the capacity, and the kernel clears what lies past the visible rows.)  24 / 4 heads of
+// 256, us a layer: 67 over 4826 30.8 -> 24.0.  Where the caller has converted rows ahead
 // (b200kv_prefill_prepare) the copy is completed and used, and a chunk that sees no more than one tile goes through the scratch as well: what a call
 // leaves there is relied on in these two cases.
 struct Sides { bool k, v; };   // sides that go through the scratch
@@ -1075,12 +1094,12 @@ int launch_dequant(const b200kv_view& view, __half* k_scratch, __half* v_scratch
     return B200KV_OK;
 }
 
-template <int D, int RT>
+template <int D, int RT, bool STATE>
 int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half* v_scratch, uint32_t rows, uint32_t prepared_rows,
                cudaStream_t stream) {
     using L = Layout<D, RT>;
     static std::atomic<uint64_t> done{0};   // one per kernel instantiation: devices that have opted in
-    const cudaError_t attr_err = opt_in_dynamic_smem(reinterpret_cast<const void*>(prefill_tc5_kernel<D, RT>), L::kAlloc, done);
+    const cudaError_t attr_err = opt_in_dynamic_smem(reinterpret_cast<const void*>(prefill_tc5_kernel<D, RT, STATE>), L::kAlloc, done);
     if (attr_err != cudaSuccess) { set_last_cuda_error(attr_err, "cudaFuncSetAttribute(prefill_tc5)"); return B200KV_ERR_CUDA; }
     if (rows > 0) {
         const int rc = launch_dequant<D>(view, k_scratch, v_scratch, rows, p.scratch_rows, prepared_rows < rows ? prepared_rows : rows,
@@ -1089,7 +1108,7 @@ int launch_tc5(const b200kv_view& view, Tc5Params& p, __half* k_scratch, __half*
     }
     const uint32_t G = p.query_heads / p.kv_heads;
     const uint32_t row_tiles = (p.token_count * G + L::kRows - 1) / L::kRows;
-    B200KV_CUDA_TRY(launch_kernel(prefill_tc5_kernel<D, RT>, dim3(row_tiles * p.kv_heads * p.kv_splits), dim3(L::kThreads), L::kAlloc, stream, true, p));
+    B200KV_CUDA_TRY(launch_kernel(prefill_tc5_kernel<D, RT, STATE>, dim3(row_tiles * p.kv_heads * p.kv_splits), dim3(L::kThreads), L::kAlloc, stream, true, p));
     if (p.kv_splits > 1) {
         PrefillMergeParams mp{};
         mp.part_o = p.part_o;
@@ -1194,9 +1213,9 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     p.scratch_rows = scratch_rows;
     p.scale_log2 = scale * 1.4426950408889634f;
     // head_dim 128: two row tiles per CTA where that still leaves every SM a CTA.  Both take the same K and V tiles, and set-up, Q and output come once for both.
-    // Fewer rows spread better as single tiles.
+    // Fewer rows spread better as single tiles.  (With a device-side state single tiles always: their kernel is the one that clears stale rows.)
     const uint32_t row_tiles_128 = static_cast<uint32_t>((static_cast<uint64_t>(token_count) * (query_heads / view.kv_heads) + kBM - 1) / kBM);
-    const uint32_t tiles_per_cta = view.head_dim == 128 && (row_tiles_128 + 1) / 2 * static_cast<uint64_t>(view.kv_heads) >= 148 ? 2u : 1u;
+    const uint32_t tiles_per_cta = view.head_dim == 128 && prefill_state == nullptr && (row_tiles_128 + 1) / 2 * static_cast<uint64_t>(view.kv_heads) >= 148 ? 2u : 1u;
     // KV split when the row tiles alone leave SMs idle and the caller's workspace has room for the partials
     p.kv_splits = 1;
     {
@@ -1218,7 +1237,10 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
             p.part_ml = reinterpret_cast<float2*>(p.part_o + static_cast<size_t>(want) * view.kv_heads * p.rows_padded * view.head_dim);
         }
     }
-    const auto launch = view.head_dim == 256 ? launch_tc5<256, 1> : tiles_per_cta == 2 ? launch_tc5<128, 2> : launch_tc5<128, 1>;
+    const auto launch = prefill_state != nullptr ? (view.head_dim == 256 ? launch_tc5<256, 1, true> : launch_tc5<128, 1, true>)
+                        : view.head_dim == 256   ? launch_tc5<256, 1, false>
+                        : tiles_per_cta == 2     ? launch_tc5<128, 2, false>
+                                                 : launch_tc5<128, 1, false>;
     return launch(view, p, k_scratch, v_scratch, static_cast<uint32_t>(rows), prepared_rows, stream);
 }
 
