@@ -754,11 +754,12 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             // published at once (the thread of the row's next tile waits for it): no later work may be scheduled before it
             asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(smem_u32(const_cast<unsigned long long*>(ref))),
                          "l"(reference_word(__float_as_uint(m_new), static_cast<uint32_t>(t) + 1u)) : "memory");
-            // At 128 it is read back as well: what follows depends on the number found beside it, so no exponential can be scheduled ahead of the store.  (Without that the store
-            // came behind all of them, by the compiler's choice and by small changes around it: a tile of one row tile took 1050 clocks, not 820.)  The value stays the
-            // thread's own whatever is found.  At 256, whose two groups wait less for each other, it costs up to 5 % (300 over 8192, 24 / 4 heads), and a shuffle behind
-            // the store, which did better in one text of this kernel, 2 % in this one: 512 over 8192 125.8 us a layer back to back as it is, 129.5 with it.
-            if constexpr (D == 128) {
+            // With four groups it is read back as well: what follows depends on the number found beside it, so no exponential can be scheduled ahead of the store.  (Without
+            // that the store came behind all of them, by the compiler's choice and by small changes around it: a tile took 1050 clocks, not 820.)  The value stays the thread's own
+            // whatever is found.  Two groups wait less for each other.  Two row tiles of 128, us: 2048 fresh x 8 layers 464.8 with it, 460.5 as it is, 1200 over 4000 1130 and
+            // 1117, 4096 over 8192 x 2 1500 and 1469.  At 256 it costs up to 5 % (300 over 8192, 24 / 4 heads), and a shuffle behind the store, which did better in one text of
+            // this kernel, 2 % in this one: 512 over 8192 125.8 us a layer back to back as it is, 129.5 with it.
+            if constexpr (L::kGroups == 4) {
                 uint32_t seq_found;
                 asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(seq_found) : "r"(smem_u32(const_cast<unsigned long long*>(ref)) + 4) : "memory");
                 m_new = __uint_as_float(own_reference(seq_found, __float_as_uint(m_new)));
