@@ -660,9 +660,9 @@ int launch_one(const DecodeParams& p, const CUtensorMap& kmap, const CUtensorMap
 // (244 -> 236).  Below that the estimate is 1 to 2 % behind halves (5000: 122 / 124).  No more CTAs than places: 64 / 16 heads took 19 splits, two waves (12000: 296 -> 205).
 uint32_t pick_splits_tc5(const b200kv_view& view, uint32_t query_heads, uint32_t max_length) {
     if (!q8_fast_path_ok(view, query_heads)) return 0;
-    const uint32_t kv = view.kv_heads, tiles = (max_length + kTileM - 1) / kTileM, halves = std::max(1u, static_cast<uint32_t>((max_length + 15ull) / (2 * kTileM)));
-    const uint32_t most = std::min(std::max(1u, 296u / kv), max_splits_per_session(1));
-    const uint32_t on_time = query_heads < 296u ? (296u - query_heads) / kv : 0;
+    const uint32_t kv = view.kv_heads, slots = 2 * device_sms(), tiles = (max_length + kTileM - 1) / kTileM, halves = std::max(1u, static_cast<uint32_t>((max_length + 15ull) / (2 * kTileM)));
+    const uint32_t most = std::min(std::max(1u, slots / kv), max_splits_per_session(1));
+    const uint32_t on_time = query_heads < slots ? (slots - query_heads) / kv : 0;
     if (halves <= on_time) return std::min(halves, most);
     return cheapest_splits(tiles, std::min(most, halves), on_time, SplitCosts{450, 900, 45, 0, 150, 5});
 }

@@ -758,14 +758,14 @@ bool decode_tc5_wide_ok(const b200kv_view& view, uint32_t query_heads) {
 }
 
 // At most one CTA per SM (19 splits of 8 heads are two waves: 48 / 8 heads, 10000 positions, 16 layers 436 -> 248 us); a full wave from five tiles a split on, where no
-// number was ahead by more than runs differ.  Below that the least estimated time: every split is a partial to merge, and a wave of more than 140 CTAs leaves the next
-// launch no SM to start on.  24 / 4 heads, q8_0, 16 layers, 37 splits -> these, us with launch overlap (without): 10200 positions 214 -> 199 (257 -> 241), 12000 216 -> 208
+// number was ahead by more than runs differ.  Below that the least estimated time: every split is a partial to merge, and a wave that leaves fewer than eight SMs free leaves the next
+// launch none to start on.  24 / 4 heads, q8_0, 16 layers, 37 splits -> these, us with launch overlap (without): 10200 positions 214 -> 199 (257 -> 241), 12000 216 -> 208
 // (260 -> 261), 16000 239 -> 232 (278 -> 276), 20000 257 -> 250 (292 -> 287).
 uint32_t pick_splits_tc5_wide(const b200kv_view& view, uint32_t max_length) {
-    const uint32_t most = std::min(std::max(1u, 148u / view.kv_heads), max_splits_per_session(1));
+    const uint32_t sms = device_sms(), most = std::min(std::max(1u, sms / view.kv_heads), max_splits_per_session(1));
     const uint32_t tiles = (max_length + kTileM - 1) / kTileM;
     if (tiles >= 5 * most) return most;
-    return cheapest_splits(tiles, most, 140u / view.kv_heads, SplitCosts{850, 850, 70, 500, 0, ~0u});
+    return cheapest_splits(tiles, most, (sms > 8 ? sms - 8 : 0) / view.kv_heads, SplitCosts{850, 850, 70, 500, 0, ~0u});
 }
 
 // A single-session launch (p.num_splits and the workspace pointers set by the caller); B200KV_ERR_UNSUPPORTED when the

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     };
     // With a device-side state the maps end at the capacity and not at the visible rows: the last tile's rows from kv_end on bring whatever lies in the cache, and a weight of zero times NaN
     // is NaN.  The warp that feeds the V ring clears them before it hands the tile over (the swizzle stays within a row).  A kernel of its own has it: the text alone
-    // cost the others up to 0.9 % (2048 fresh, 32 / 8 heads of 128).
+    // cost the others 0.6 % (37 over 3000, 32 / 8 heads of 128).
     [[maybe_unused]] const int whole_tiles = STATE && kv_end % kBN != 0 ? ntiles - 1 : ntiles;   // tiles handed over as they land
     [[maybe_unused]] auto load_last_v = [&](bool ok) {   // a warp; `ok`: lane 0 has handed over the others
         const int j = ntiles - 1, st = j % L::kVTiles;
