@@ -138,6 +138,8 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(ok));
     return ok != 0;
 }
+// Largest value of a warp; a NaN counts for nothing (its head's sum is NaN).
+__device__ __forceinline__ float warp_max_redux(float f) { float r; asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f)); return r; }
 
 // The scanned range [begin, end) of one session, resolved on the device the way
 // the reference resolves its DeviceDecodeState (position + 1 entries,

@@ -35,6 +35,7 @@
 //  * Every wait is bounded.  A wait that runs out sets a status bit, poisons the partial with NaN and lets the CTA
 //    finish in the normal way (all later waits are skipped, barriers are still attended, TMEM is freed).
 #include "decode_tail.cuh"
+#include "mbarrier_wait.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -54,7 +55,6 @@ constexpr int kStages = 3;
 constexpr int kThreads = 256;
 constexpr int kConsumers = 128;
 constexpr int kProducerWarp = 4, kMmaWarp = 5, kPvWarp = 6, kAppendWarp = 7;
-constexpr uint32_t kSpin = 1u << 20;
 constexpr uint32_t kTmemCols = 256;
 constexpr uint32_t kColS = 0;          // two S buffers of 4 blocks x 16 columns
 constexpr uint32_t kColO = 128;        // two O buffers of 32 columns: (block, plane, head)
@@ -90,35 +90,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm vo
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: false if the phase did not complete within the spin limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t spin = 0; spin < kSpin; ++spin)
-        if (mbar_try(bar, parity)) return true;
-    return false;
-}
-// Bounded wait of a whole warp for two phases, asked for together: all lanes go on or none.
-__device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
-    bool ok = false;
-    for (uint32_t spin = 0; spin < kSpin && !ok; ++spin) {
-        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
-        ok = a && b;
-    }
-    return __all_sync(0xffffffffu, ok);
-}
-// The same of single lanes.
-__device__ __forceinline__ bool mbar_wait_both_lane(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
-    for (uint32_t spin = 0; spin < kSpin; ++spin) {
-        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
-        if (a && b) return true;
-    }
-    return false;
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -170,9 +141,6 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Largest value of a warp; a NaN counts for nothing (its head's sum is NaN).
-__device__ __forceinline__ float warp_max_redux(float f) { float r; asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f)); return r; }
 
 // NBLK scales per row (4 = q8_0 blocks of 32, 1 = one per row); up to 4 query heads per kv head.
 template <int NBLK, bool Q_F16>

@@ -22,6 +22,7 @@
 //    (As launches of their own the merge cost 1.7 us at 32768 positions -- 21.1 against 19.4 us -- and the append 4 to 5 more.)
 //  * Every wait is bounded, as there.
 #include "decode_tail.cuh"
+#include "mbarrier_wait.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -38,7 +39,6 @@ constexpr int kVStages = 3;            // V tiles (and both scale tiles): held u
 constexpr int kThreads = 384;
 constexpr int kConsumers = 128;        // softmax threads per group; warps 0-3 take the even tiles, warps 4-7 the odd ones
 constexpr int kProducerWarp = 8, kMmaWarp = 9, kPvWarp = 10, kVProducerWarp = 11;
-constexpr uint32_t kSpin = 1u << 20;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColS = 0;          // two S buffers of 8 blocks x 16 columns
 constexpr uint32_t kColO = 256;        // two O buffers of 2 halves x 64 columns: (block of the half, plane, head)
@@ -73,35 +73,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm vo
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: false if the phase did not complete within the spin limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t spin = 0; spin < kSpin; ++spin)
-        if (mbar_try(bar, parity)) return true;
-    return false;
-}
-// Bounded wait of a whole warp for two phases, asked for together: all lanes go on or none.
-__device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
-    bool ok = false;
-    for (uint32_t spin = 0; spin < kSpin && !ok; ++spin) {
-        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
-        ok = a && b;
-    }
-    return __all_sync(0xffffffffu, ok);
-}
-// The same of single lanes.
-__device__ __forceinline__ bool mbar_wait_both_lane(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
-    for (uint32_t spin = 0; spin < kSpin; ++spin) {
-        const bool a = mbar_try(bar_a, parity_a), b = mbar_try(bar_b, parity_b);
-        if (a && b) return true;
-    }
-    return false;
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -144,9 +115,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&r)[16]) {
                  : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Largest value of a warp; a NaN counts for nothing (its head's sum is NaN).
-__device__ __forceinline__ float warp_max_redux(float f) { float r; asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(f)); return r; }
 
 // The appended row's 256 bytes into row r of a K or V tile (two 128-byte-wide halves, 128-byte swizzle); lanes 0-15.
 __device__ __forceinline__ void patch_row(uint8_t* tile, const uint8_t* row, uint32_t r, int lane) {

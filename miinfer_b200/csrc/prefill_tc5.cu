@@ -30,6 +30,7 @@
 // its TMEM and exits.
 #include "decode_common.cuh"
 #include "dequant.cuh"
+#include "mbarrier_wait.cuh"
 #include "reference_word.h"
 
 #include <algorithm>
@@ -43,7 +44,6 @@ namespace {
 constexpr int kBM = 128;          // query rows per row tile; a CTA takes one or two (RT)
 constexpr int kBN = 64;           // positions per KV tile
 constexpr int kKPairs = 2;                         // K ring: stages of two tiles each (one S MMA covers a pair)
-constexpr uint32_t kSpin = 1u << 20;
 constexpr float kRescaleThreshold = 8.0f;        // log2 units
 constexpr uint32_t kMaxKvSplits = 16;
 
@@ -72,15 +72,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm vo
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t spin = 0; spin < kSpin; ++spin) {
-        uint32_t ok;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    return false;
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -181,17 +172,6 @@ __device__ __forceinline__ Pair add_pair(Pair a, Pair b) { Pair r; asm("add.rn.f
 __device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.ftz.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 // A wait of a whole warp, which stays together: all lanes go on or none.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
-// The same for two barriers, asked at once.
-__device__ __forceinline__ bool mbar_wait2_warp(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
-    bool ok = false;
-    for (uint32_t spin = 0; spin < kSpin && !ok; ++spin) {
-        uint32_t a, b;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(a) : "r"(bar_a), "r"(parity_a) : "memory");
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(b) : "r"(bar_b), "r"(parity_b) : "memory");
-        ok = (a & b) != 0;
-    }
-    return __all_sync(0xffffffffu, ok);
-}
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -520,7 +500,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             for (int j = first; ok && j < ntiles; j += kStep) {
                 const int i = j >> 1, ps = i % kKPairs, buf = rt * L::kGroups + j % L::kGroups;
                 // the K pair is there, and the weights that lie in the buffer have been used
-                ok = mbar_wait2_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1), bar(P_EMPTY + buf), static_cast<uint32_t>((j / L::kGroups) & 1) ^ 1);
+                ok = mbar_wait_both(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1), bar(P_EMPTY + buf), static_cast<uint32_t>((j / L::kGroups) & 1) ^ 1);
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t b = k_desc + ((ps * L::kPairBytes + (j & 1) * (kBN * 128)) >> 4);
@@ -547,7 +527,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 const int ps = i % kKPairs, n = min(2, ntiles - 2 * i);
                 const uint32_t ph = static_cast<uint32_t>(i & 1) ^ 1, idesc = n == 2 ? idesc_pair : idesc_one;
                 // both groups have read the previous pair's scores (only the last pair can be a single tile)
-                ok = mbar_wait2_warp(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1), bar(S_EMPTY), ph) && mbar_wait_warp(bar(S_EMPTY + 1), ph);
+                ok = mbar_wait_both(bar(K_FULL + ps), static_cast<uint32_t>((i / kKPairs) & 1), bar(S_EMPTY), ph) && mbar_wait_warp(bar(S_EMPTY + 1), ph);
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t b = k_desc + ((ps * L::kPairBytes) >> 4);
@@ -575,7 +555,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 for (int rt = 0; rt < RT; ++rt) {
                     if (RT > 1 && rt >= live_tiles) break;
                     const int buf = rt * L::kGroups + st;
-                    ok = rt == 0 ? mbar_wait2_warp(bar(V_FULL + vs), static_cast<uint32_t>((j / L::kVTiles) & 1), bar(P_FULL + buf), ph) : mbar_wait_warp(bar(P_FULL + buf), ph);
+                    ok = rt == 0 ? mbar_wait_both(bar(V_FULL + vs), static_cast<uint32_t>((j / L::kVTiles) & 1), bar(P_FULL + buf), ph) : mbar_wait_warp(bar(P_FULL + buf), ph);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
@@ -596,7 +576,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             for (int j = 0; ok && j < ntiles; ++j) {
                 const int st = j & 1;
                 const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);
-                ok = mbar_wait2_warp(bar(V_FULL + st), ph, bar(P_FULL + st), ph);
+                ok = mbar_wait_both(bar(V_FULL + st), ph, bar(P_FULL + st), ph);
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t a = p_desc + ((st * L::kPBytes) >> 4), b = v_desc + ((st * L::kTileBytes) >> 4);
