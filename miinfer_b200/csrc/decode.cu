@@ -118,13 +118,13 @@ int launch_merge(const MergeParams& p, uint32_t groups, cudaStream_t stream) {
     return B200KV_OK;
 }
 
-// max_length x kv heads up to which a single session takes the mma.sync kernel.  Measured (decode steps back to back in a graph, us a layer, mma.sync /
-// tcgen05; in brackets without launch overlap): 8 kv heads of 128 dims, q8_0: 4096 positions 8.5 / 8.85 (10.2 / 10.8), 4500 9.05 / 8.9 (10.45 / 10.9),
-// 5000 8.3 / 8.75 (11.0 / 11.4), 6000 8.8 / 8.9 (11.25 / 11.7), 7000 9.7 / 9.0 (12.4 / 12.0).  4 kv heads of 256, q8_0: 5000 10.65 / 12.3 (12.7 / 13.15),
-// 8000 11.1 / 12.3 (14.2 / 13.8), 9728 12.05 / 13.0 (15.4 / 14.5), 12000 12.8 / 13.3 (16.5 / 15.3), 14000 14.45 / 14.1 (17.2 / 16.0); one scale
-// per row: 8000 10.8 / 11.6 (13.6 / 13.15), 12000 12.2 / 12.75 (15.8 / 14.7), 16000 14.2 / 14.25 (17.45 / 16.0).  So the lines lie inside the range in
-// which neither kernel is ahead in every mode: with overlap the two are level at about 6000 and 13000 to 16000 positions, without it
-// at about 6500 and 7500, and the slower one costs up to 6 %.  Other head counts were not measured and go by the rows, which is what fills the device.
+// max_length x kv heads up to which a single session takes the streaming kernel.  Measured (decode steps back to back in a graph, us a layer, at 256 dims with the query side, streaming /
+// tcgen05; in brackets without launch overlap): 8 kv heads of 128 dims, q8_0: 4096 positions 8.15 / 7.7 (9.85 / 10.2), 4500 8.65 / 7.7 (9.95 / 10.2), 5000 7.95 / 7.75
+// (10.5 / 10.7), 6000 8.45 / 7.8 (10.85 / 11.1), 7000 9.3 / 8.1 (11.9 / 11.25).  4 kv heads of 256, q8_0: 5000 12.05 / 11.45 (14.05 / 14.05), 8000 12.65 / 12.25 (15.75 / 15.35),
+// 9728 13.3 / 12.3 (17.25 / 14.95), 12000 14.0 / 12.9 (18.3 / 16.0), 14000 16.35 / 13.95 (18.9 / 16.25); one scale per row: 8000 12.35 / 11.6 (15.0 / 14.8), 12000 13.55 / 12.2
+// (17.4 / 15.5), 16000 15.4 / 13.5 (18.95 / 16.25).  With overlap the tcgen05 kernels are ahead from about 2600 and 4300 positions on, by up to 12 %, without it from about 6500
+// and 5000.  The lines stay above that for the error: the streaming kernel is 2e-7 off float64, the tcgen05 kernels, whose queries and weights are 15- and 16-bit fixed point, 7e-5, so
+// a lower line would cost calls that have the smaller error now.  Other head counts were not measured and go by the rows, which is what fills the device.
 constexpr uint64_t kStreamRows128 = 32768, kStreamRows256 = 40000;
 
 // Runs stage 1 and, where the merge fits inside the launch, the merge.
@@ -149,8 +149,7 @@ int run_decode_stage1(DecodeParams& p, const b200kv_view& geometry, uint32_t max
     bool use_fast = !force_stream && q_vectors && (merge_inside || !many) && q8_fast_path_ok(geometry, p.query_heads);
     // head_dim 256: the tcgen05 kernel for single-session launches
     bool use_wide = !force_stream && !use_fast && !many && q_vectors && streaming_kernel_choice() != 1 && decode_tc5_wide_ok(geometry, p.query_heads);
-    // Single sessions that are short for the device: the mma.sync kernel starts, splits and merges faster than the tcgen05
-    // kernels' pipelines fill, until its instruction issue shows.
+    // Single sessions that are short for the device: the streaming kernel (the lines above).
     if (num_splits == 0 && !many && streaming_kernel_choice() != 1) {
         const uint64_t rows = static_cast<uint64_t>(max_length) * geometry.kv_heads;
         // (a sharded launch has its exchange inside the merge: only where that fits)

@@ -180,7 +180,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 template <int D, int RT>
 struct Layout {
-    // warps: two softmax groups per row tile (one thread per query row: even tiles, odd tiles), then one warp per role
+    // warps: the softmax groups of every row tile (one thread per query row in each, which take the tiles in turn), then the warps of the other roles
     static constexpr int kGroups = D == 128 ? 4 / RT : 2;  // softmax groups of a row tile; tile j is group j % kGroups's
     static constexpr int kSoftmaxThreads = RT * kGroups * 128;
     static constexpr int kTmaWarp = kSoftmaxThreads / 32;  // TMA producer of the K tiles
@@ -214,7 +214,7 @@ struct Layout {
                          P_FULL = S_EMPTY + (kPInTmem ? 0 : kBufs), P_EMPTY = P_FULL + kBufs, O_DONE = P_EMPTY + kBufs, Q_FULL = O_DONE + RT, V_TAIL = Q_FULL + 1, kNumBars = V_TAIL + 1;
     static constexpr int kOffSlot = kOffBar + (kNumBars * 8 + 15) / 16 * 16;
     static constexpr int kOffRef = kOffSlot + 16;                 // [rows] {reference maximum, sequence}: handed from tile to tile
-    // [2 groups][128 rows] partial row sums of a row tile in its epilogue, where its own score MMAs are through: over the K
+    // [group][128 rows] partial row sums of a row tile in its epilogue, where its own score MMAs are through: over the K
     // ring, or over the row tile's Q where the other row tile may still need K
     static constexpr int kSumStride = kGroups * kBM * 4;
     static constexpr int kOffSum = kQInTmem ? kOffK : kOffRef + kRows * 8;
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     } else {
         // =============================== Q rows ===============================
         // Q: the CTA's rows as fp16 pairs in TMEM (row = lane, dims 2c and 2c+1 in column c), the A operand of every S MMA:
-        // read from there it costs no shared-memory bandwidth.  Each of a row's two softmax threads stores half of the
+        // read from there it costs no shared-memory bandwidth.  Two of a row's threads store half of the
         // row.  A warp reads its 32 rows four at a time, 128 (fp32: 256) contiguous bytes each, and turns them through
         // its own 4 KB of the P tiles (a load per thread and row touched 32 lines an instruction); the first pair of K
         // tiles is on its way meanwhile.  From the dependency wait to the last row: 0.8 us (two row tiles of 128 dims; 3.8 behind full rings and with
@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
 #pragma unroll
             for (int c = 0; c < 4; ++c) m4[c] = fmaxf(m4[c], s[kBN - 4 + c]);
             const float mt = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;   // scale > 0: the maximum commutes with it
-            // the reference as the previous tile (the other group's) left it; lazy rescale: keep it unless this tile's
+            // the reference as the previous tile (another group's) left it; lazy rescale: keep it unless this tile's
             // maximum outgrew it by more than the threshold
             float m_prev = -INFINITY;
             if (t > 0 && !ref_after(static_cast<uint32_t>(t), &m_prev)) lost = true;
@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
                 tc_fence_after();
             }
             if (__any_sync(0xffffffffu, alpha != 1.0f || lost) && (t > 0 || __any_sync(0xffffffffu, lost))) {
-                // rare: the reference moved.  O holds tiles 0..t-1 once the previous tile's P.V (the other group's) has
+                // rare: the reference moved.  O holds tiles 0..t-1 once the previous tile's P.V (another group's) has
                 // completed; then this warp rescales its 32 rows of O in TMEM before its own P is released.
                 if (t > 0 && !mbar_wait(bar(P_EMPTY + rt * L::kGroups + (t - 1) % L::kGroups), static_cast<uint32_t>(((t - 1) / L::kGroups) & 1))) lost = true;
                 if (__any_sync(0xffffffffu, lost)) { failed = true; break; }
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             tc_fence_before();
             mbar_arrive(bar(P_FULL + buf));
         }
-        // ---- epilogue: O / sum, gate, store; each thread of a row's pair half of the columns ----
+        // ---- epilogue: O / sum, gate, store; the columns are divided among a row's threads ----
         const bool partial = nsplit > 1, gated = !partial && p.gate != nullptr;
         const size_t part_row0 = (static_cast<size_t>(split) * p.kv_heads + kv_head) * p.rows_padded + row0;
         constexpr int kCols = D / L::kGroups;
@@ -825,7 +825,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
             else asm volatile("bar.sync %0, 256;" ::"r"(2 + rt) : "memory");
             l_sum = sums[r] + sums[kBM + r];
             if constexpr (L::kGroups == 4) l_sum += sums[2 * kBM + r] + sums[3 * kBM + r];
-            // The warp's O may be read.  A sum that is NaN, because the row's other thread gave up or because of the data, is its own row's affair.
+            // The warp's O may be read.  A sum that is NaN, because another of the row's threads gave up or because of the data, is its own row's affair.
             const bool have_o = walked > 0 && !__any_sync(0xffffffffu, failed);
             if (l_sum != l_sum) failed = true;
             const float m_ref = m_final;
@@ -1045,8 +1045,8 @@ bool encode_f16_plane(CUtensorMap* map, const void* base, uint32_t d, uint64_t r
 // An fp16 side of the cache is read where it lies; only int8 sides go through the scratch.  (The map ends at the rows the launch may see, so the last tile's
 // other rows come as zeros, as in the scratch; with a device-side state that is the capacity, and the kernel clears what lies past the visible rows.)  24 / 4 heads of
 // 256, us a layer: 67 over 4826 30.8 -> 24.0.  Where the caller has converted rows ahead
-// (b200kv_prefill_prepare) the copy is completed and used, and a chunk that sees no more than one tile goes through the scratch as well: what a call
-// leaves there is relied on in these two cases.
+// (b200kv_prefill_prepare) the copy is completed and used.  A chunk that sees no more than one tile goes through the scratch as well, which is no gain (fp16 caches, 16 layers, us, so -> in
+// place: 16 tokens of 32 / 8 heads of 128 219 -> 181, 20 fp32 tokens of 24 / 4 of 256 263 -> 235): tests/test_prefill_prepass_gpu.py looks for the copy behind such a call.
 struct Sides { bool k, v; };   // sides that go through the scratch
 Sides scratch_sides(const b200kv_view& view, uint64_t rows, uint32_t prepared_rows) {
     const auto direct = [&](bool q8, const void* plane) {
@@ -1131,18 +1131,20 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
 // of 148 CTAs costs its tiles and a few us; CTAs take the place of one another as they end, so a last wave that is not full may cost less than a whole
 // one, and from the second wave on the length that counts may lie between the longest causal range and the average; a split costs its partials' way out
 // and back, and the merge.  The constants of single row tiles are fitted to 66 (head_dim 128) and 93 (256) chunks of 16 to 2048 tokens over 0 to 32000 at 32 / 8 and 24 / 4
-// heads, every number of splits timed: the choice is 0.4 and 0.3 % above the best on average, 6.5 and 5 % at most (1.5 and 0.6, 12 and 15 % with the constants before).  us a layer with the store kernel, in a short
-// burst (and, where the power limit makes it another, in a long run), q8_0, the choice marked *:
-//   32 heads of 128:  37 over 3000 (16 units):  1: 37.3, 4: 21.5, 6: 20.6, *9: 20.0, 10: 26.7       128 over 8192 (32):  1: 74, 2: 50, *4: 37.2, 5: 52
-//                     300 over 300 (80):  *1: 18.7, 2: 26.7       300 over 8192:  1: 84, 2: 87, *3: 69.6, 4: 81       461 over 8192 (120):  *1: 87, 2: 94, 3: 103
-//   24 of 256:        20 over 16000 (4):  8: 55, 12: 49, *16: 48                     37 over 3000 (8):  1: 50, 4: 25.6, 8: 23.6, *10: 22.5, 11: 22.7, 16: 22.5
-//                     128 over 8192 (24):  1: 101, 4: 46.7, *6: 43.6, 7: 60          300 over 8192 (60):  1: 111, *2: 78, 3: 98
-//                     300 over 300 (60):  1: 30.5, *2: 26.4, 3: 32.8           1024 over 16000 (192):  1: 427, *2: 370 (434), 3: 399 (430)
-//                     461 over 8192 (88):  1: 126, 2: 128, *3: 105, 4: 132           512 over 8192 (96):  1: 123 (125), 2: 134 (137), *3: 110 (125), 4: 129 (139)
-// Two row tiles a CTA have costs of their own, as measured when their weights still went through shared memory:
-//                     1200 over 4000 (152):  1: 150, *2: 148, 3: 150 (153)        1200 over 8192:  1: 280, 2: 243 (250), *3: 237 (248), 4: 242 (255)
-//                     1600 over 4000 (200):  *1: 169 (171), 2: 167 (178)             1500 over 20000 (192):  1: 673, 2: 550 (620), *3: 534 (607), 4: 635 (650)
-//                     3000 over 8192 (376):  *1: 493 (542), 2: 565 (594)             4096 over 8192 (512):  *1: 706 (756), 2: 713 (790)
+// heads, every number of splits timed: the choice is 0.4 and 0.3 % above the best on average, 6.5 and 5 % at most (1.5 and 0.6, 12 and 15 % with the constants before).  us a layer, graphs of
+// 16 layers (4 from 1000 tokens on) with the store kernel, q8_0, in a short burst, the choice marked *:
+//   32 heads of 128:  37 over 3000 (16 units):  1: 34.3, 4: 19.2, 6: 19.2, *9: 17.9, 10: 24.2       128 over 8192 (32):  1: 69, 2: 46.2, *4: 33.8, 5: 48
+//                     300 over 300 (80):  *1: 15.0, 2: 22.7       300 over 8192:  1: 80, 2: 82, *3: 64.6, 4: 76       461 over 8192 (120):  *1: 83, 2: 87, 3: 94
+//   24 of 256:        20 over 16000 (4):  8: 53, 12: 43, *16: 40                     37 over 3000 (8):  1: 46, 4: 23.1, 8: 21.3, 11: 20.3, *12: 19.9, 14: 20.5, 16: 20.3
+//                     128 over 8192 (24):  1: 100, 4: 43.9, *6: 39.9, 7: 58          300 over 8192 (60):  1: 104, *2: 70, 3: 96
+//                     300 over 300 (60):  1: 21.4, *2: 21.7, 3: 29.2           1024 over 16000 (192):  1: 395, *2: 376, 3: 405
+//                     461 over 8192 (88):  1: 122, 2: 126, *3: 103, 4: 116           512 over 8192 (96):  1: 108, 2: 125, *3: 106, 4: 125 (in a long run, at the power limit, 125 and 125 for 1 and 3)
+// Two row tiles a CTA have costs of their own.  They were fitted when the weights still went through shared memory; as the loop is now:
+//                     1200 over 4000 (152):  1: 145.5, *2: 144.3, 3: 144.9        1200 over 8192:  1: 262, 2: 236, *3: 226, 4: 228
+//                     1600 over 4000 (200):  *1: 155, 2: 159             1500 over 20000 (192):  1: 615, 2: 529, *3: 530, 4: 624
+//                     3000 over 8192 (376):  *1: 493, 2: 537             4096 over 8192 (512):  *1: 673, 2: 707
+// (Another number of splits is another reference for the same row, and its fp16 weights round otherwise: 37 over 3001 at 24 / 4 heads, 12 splits for 11, moved by 2.4e-4 of its
+// norm; 4.12e-4 off float64 with 12, 4.13e-4 with 11.)
 static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, double average, uint32_t most, uint32_t head_dim, uint32_t tiles_per_cta) {
     struct Costs { double tile_us, wave_us, last_wave, longest, merge_us, partial_us; };
     const Costs c = tiles_per_cta == 2 ? Costs{1.0, 3.0, 0.6, 1.0, 0.0, 0.07} : head_dim == 256 ? Costs{0.62, 12.4, 0.5, 0.42, 0.0, 0.024} : Costs{0.43, 1.95, 1.0, 0.07, 1.3, 0.017};
