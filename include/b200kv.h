@@ -440,7 +440,7 @@ B200KV_API size_t b200kv_prefill_workspace_bytes(uint32_t token_count, uint32_t 
 /* Workspace that enables the tcgen05 kernel: room for the fp16 copy of the `rows` cache positions the chunk can see
  * (rows = base_position + token_count; the whole capacity when a device-side prefill_state is used).  35.6 MB for
  * 8704 rows x 4 kv heads x d=256.  The scratch is rewritten by every call; calls that overlap on the GPU need
- * separate workspaces.  Cache rows below `rows` must hold finite values (freshly created caches are zero). */
+ * separate workspaces.  The cache rows that the chunk's tokens see must hold finite values; rows past them may hold anything. */
 B200KV_API size_t b200kv_prefill_scratch_bytes(uint64_t rows, uint32_t kv_heads, uint32_t head_dim);
 /* Optional extra room behind that scratch (workspace_bytes >= scratch + this): when a chunk has too few query rows
  * to give every SM a row tile (37 tokens x 6 heads per kv head = 8 tiles on 148 SMs), the tcgen05 kernel may also
@@ -451,7 +451,8 @@ B200KV_API size_t b200kv_prefill_split_bytes(uint32_t token_count, uint32_t quer
 /* Replaces launch_qwen35_splitk_suffix_attention_quant
  * (qwen3_gpu_primitives.hpp:670-692; kernels .hip:6788-7119 and 6637-6725).
  * q, gate, gated_output: [token][query_heads][head_dim] (q of q_dtype, the
- * others fp32; gate may be NULL).  Query token t attends cache positions
+ * others fp32; gate may be NULL).  q is 16-byte aligned, the others 8-byte aligned, or 16-byte for the tcgen05 kernel.
+ * Query token t attends cache positions
  * [0, base_position + t + 1): the chunk must already have been appended.  A
  * non-NULL prefill_state overrides base_position/token_count on the device
  * (.hip:6810-6814).  Tokens whose causal length exceeds the capacity get a

@@ -70,10 +70,15 @@ int b200kv_prefill_attn_prepared(const b200kv_view* view, const void* q, int q_d
     if (q_dtype != B200KV_F16 && q_dtype != B200KV_F32) return B200KV_ERR_INVALID;
     if (query_heads == 0 || query_heads % view->kv_heads != 0 || !std::isfinite(scale)) return B200KV_ERR_INVALID;
     if (static_cast<uint64_t>(token_count) * (query_heads / view->kv_heads) > 0x7fffffffull) return B200KV_ERR_UNSUPPORTED;
+    // queries are fetched 16 bytes at a time, gate and output go four floats at a time in the tcgen05 kernel and two in the other
+    const auto aligned = [](const void* ptr, size_t bytes) { return reinterpret_cast<uintptr_t>(ptr) % bytes == 0; };   // null counts as aligned
+    if (!aligned(q, 16) || !aligned(gate, 8) || !aligned(gated_output, 8)) return B200KV_ERR_INVALID;
     if ((rc = ensure_device()) != B200KV_OK) return rc;
     // tcgen05 path when the caller provides the fp16 scratch; otherwise the register-resident mma.sync kernel
-    rc = launch_prefill_tc5(*view, q, q_dtype == B200KV_F16, gate, gated_output, token_count, base_position, prefill_state, query_heads,
-                            scale, workspace, workspace_bytes, prepared_rows, static_cast<cudaStream_t>(stream));
+    rc = B200KV_ERR_UNSUPPORTED;
+    if (aligned(gate, 16) && aligned(gated_output, 16))
+        rc = launch_prefill_tc5(*view, q, q_dtype == B200KV_F16, gate, gated_output, token_count, base_position, prefill_state, query_heads,
+                                scale, workspace, workspace_bytes, prepared_rows, static_cast<cudaStream_t>(stream));
     if (rc != B200KV_ERR_UNSUPPORTED) return rc;
     return launch_prefill_mma(*view, q, q_dtype == B200KV_F16, gate, gated_output, token_count, base_position, prefill_state,
                               query_heads, scale, static_cast<cudaStream_t>(stream));
