@@ -62,6 +62,7 @@ struct Tc5Params {
     // KV split: split z walks tiles [ntiles*z/S, ntiles*(z+1)/S) of its rows and leaves an unnormalised partial
     // (O, reference maximum, sum) for prefill_merge_kernel.  kv_splits == 1: the kernel writes the output itself.
     uint32_t kv_splits;
+    uint32_t sms;                // of the device: CTAs of a wave
     uint32_t rows_padded;        // query rows per kv head, rounded up to the row tile
     float* part_o;               // [split][kv_head][rows_padded][D]
     float2* part_ml;             // [split][kv_head][rows_padded] {maximum in log2 units, sum}
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     }
     [[maybe_unused]] uint4 early_q[kTurns][8];
     // one wave of CTAs: Q ahead of the wait (24 / 4 heads, 37 fp32 tokens over 3001: 24.3 -> 24.1 us a layer)
-    if (kEarlyQ && warp == kTmaWarp && split_u == 0 && gridDim.x <= 148) prefetch_q(row0, kv_head);
+    if (kEarlyQ && warp == kTmaWarp && split_u == 0 && gridDim.x <= p.sms) prefetch_q(row0, kv_head);
     if constexpr (kEarlyQ) {
         if (warp < kQWarps) {
             const RowOffsets<D> rows(warp_row0, turn_row, G, p.query_heads, total_rows);
@@ -402,13 +403,13 @@ __global__ void __launch_bounds__(Layout<D, RT>::kThreads, 1) prefill_tc5_kernel
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (!kEarlyQ && warp == kTmaWarp && split_u == 0 && gridDim.x <= 148) prefetch_q(row0, kv_head);
+    if (!kEarlyQ && warp == kTmaWarp && split_u == 0 && gridDim.x <= p.sms) prefetch_q(row0, kv_head);
     [[maybe_unused]] const RowOffsets<D> late_rows(warp_row0, turn_row, G, p.query_heads, total_rows);
     if constexpr (!kEarlyQ) pdl_wait();
     bool failed = false;
     // The query rows of the CTA that takes this one's place, as far as the order of dispatch tells.  A warp.
     auto next_q = [&] {
-        const uint32_t next = blockIdx.x + 148;
+        const uint32_t next = blockIdx.x + p.sms;
         if (next < gridDim.x && next % p.kv_splits == 0)
             prefetch_q(((total_rows + L::kRows - 1) / L::kRows - 1 - next / p.kv_splits / p.kv_heads) * L::kRows, next / p.kv_splits % p.kv_heads);
     };
@@ -1145,15 +1146,15 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
 //                     3000 over 8192 (376):  *1: 493, 2: 537             4096 over 8192 (512):  *1: 673, 2: 707
 // (Another number of splits is another reference for the same row, and its fp16 weights round otherwise: 37 over 3001 at 24 / 4 heads, 12 splits for 11, moved by 2.4e-4 of its
 // norm; 4.12e-4 off float64 with 12, 4.13e-4 with 11.)
-static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, double average, uint32_t most, uint32_t head_dim, uint32_t tiles_per_cta) {
+static uint32_t pick_kv_splits(uint32_t units, uint32_t tiles, double average, uint32_t most, uint32_t head_dim, uint32_t tiles_per_cta, uint32_t sms) {
     struct Costs { double tile_us, wave_us, last_wave, longest, merge_us, partial_us; };
     const Costs c = tiles_per_cta == 2 ? Costs{1.0, 3.0, 0.6, 1.0, 0.0, 0.07} : head_dim == 256 ? Costs{0.62, 12.4, 0.5, 0.42, 0.0, 0.024} : Costs{0.43, 1.95, 1.0, 0.07, 1.3, 0.017};
     uint32_t best = 1;
     double best_us = 0.0;
     for (uint32_t s = 1; s <= kMaxKvSplits && s <= (most > 1 ? most : 1); ++s) {
-        const uint64_t ctas = static_cast<uint64_t>(units) * s, full = ctas / 148, rest = ctas % 148;
-        const double waves = static_cast<double>(full) + (rest == 0 ? 0.0 : full == 0 ? 1.0 : c.last_wave + (1.0 - c.last_wave) * static_cast<double>(rest) / 148.0);
-        const double walked = ctas <= 148 ? tiles : c.longest * tiles + (1.0 - c.longest) * average;
+        const uint64_t ctas = static_cast<uint64_t>(units) * s, full = ctas / sms, rest = ctas % sms;
+        const double waves = static_cast<double>(full) + (rest == 0 ? 0.0 : full == 0 ? 1.0 : c.last_wave + (1.0 - c.last_wave) * static_cast<double>(rest) / sms);
+        const double walked = ctas <= sms ? tiles : c.longest * tiles + (1.0 - c.longest) * average;
         const double us = waves * (walked * c.tile_us / s + c.wave_us) + (s > 1 ? c.merge_us + c.partial_us * static_cast<double>(ctas) : 0.0);
         if (s == 1 || us < best_us) { best = s; best_us = us; }
     }
@@ -1195,10 +1196,11 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
     p.capacity = view.capacity;
     p.scratch_rows = scratch_rows;
     p.scale_log2 = scale * 1.4426950408889634f;
+    p.sms = device_sms();
     // head_dim 128: two row tiles per CTA where that still leaves every SM a CTA.  Both take the same K and V tiles, and set-up, Q and output come once for both.
     // Fewer rows spread better as single tiles.  (With a device-side state single tiles always: their kernel is the one that clears stale rows.)
     const uint32_t row_tiles_128 = static_cast<uint32_t>((static_cast<uint64_t>(token_count) * (query_heads / view.kv_heads) + kBM - 1) / kBM);
-    const uint32_t tiles_per_cta = view.head_dim == 128 && prefill_state == nullptr && (row_tiles_128 + 1) / 2 * static_cast<uint64_t>(view.kv_heads) >= 148 ? 2u : 1u;
+    const uint32_t tiles_per_cta = view.head_dim == 128 && prefill_state == nullptr && (row_tiles_128 + 1) / 2 * static_cast<uint64_t>(view.kv_heads) >= p.sms ? 2u : 1u;
     // KV split when the row tiles alone leave SMs idle and the caller's workspace has room for the partials
     p.kv_splits = 1;
     {
@@ -1208,7 +1210,7 @@ int launch_prefill_tc5(const b200kv_view& view, const void* q, int q_is_f16, con
         const uint32_t tiles = static_cast<uint32_t>((rows + kBN - 1) / kBN), prefix_tiles = (base_position + kBN - 1) / kBN;
         const uint32_t most = prefill_state != nullptr ? 1 : base_position >= token_count ? tiles / 3 : prefix_tiles / 8;
         const double average = std::min<double>(tiles, (base_position + 0.5 * token_count) / kBN);
-        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, average, most, view.head_dim, tiles_per_cta);
+        uint32_t want = pick_kv_splits(row_tiles * view.kv_heads, tiles, average, most, view.head_dim, tiles_per_cta, p.sms);
         const size_t scratch = prefill_tc5_workspace_bytes(static_cast<uint32_t>(rows), view.kv_heads, view.head_dim);
         while (want > 1 && workspace_bytes < scratch + 1024 + prefill_tc5_split_bytes(token_count, query_heads, view.kv_heads, view.head_dim, want)) --want;
         if (want > 1) {
