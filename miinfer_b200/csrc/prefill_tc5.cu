@@ -1129,7 +1129,7 @@ size_t prefill_tc5_split_bytes(uint32_t token_count, uint32_t query_heads, uint3
 }
 
 // How many KV splits: the number with the least estimated time, for `units` CTAs of one or two row tiles, up to `tiles` KV tiles and `average` of them.  A wave
-// of 148 CTAs costs its tiles and a few us; CTAs take the place of one another as they end, so a last wave that is not full may cost less than a whole
+// of a CTA an SM (148 where the costs were fitted) costs its tiles and a few us; CTAs take the place of one another as they end, so a last wave that is not full may cost less than a whole
 // one, and from the second wave on the length that counts may lie between the longest causal range and the average; a split costs its partials' way out
 // and back, and the merge.  The constants of single row tiles are fitted to 66 (head_dim 128) and 93 (256) chunks of 16 to 2048 tokens over 0 to 32000 at 32 / 8 and 24 / 4
 // heads, every number of splits timed: the choice is 0.4 and 0.3 % above the best on average, 6.5 and 5 % at most (1.5 and 0.6, 12 and 15 % with the constants before).  us a layer, graphs of

@@ -4,7 +4,7 @@ decode (one 131072-token session over the ranks).  bench.py dispatches here for 
 and calls `extras` to attach them as sub-records to its default line.  Every workload function can be run with
 `dist=None, world=1` inside a multi-rank job (rank 0 does that to measure a workload's own 1-GPU time), and every
 one ends with a comparison of one layer's output against the CPU oracle evaluated on the cache planes as they lie on
-the device (`check`): test infrastructure used as the checker, outside every timed region."""
+the device (`check`): test infrastructure, outside every timed region."""
 from __future__ import annotations
 
 import json

@@ -1,7 +1,7 @@
 /*
  * kv_oracle.c -- CPU restatement of MIInfer's quantized KV-cache hot path.
  *
- * TEST INFRASTRUCTURE ONLY.  This file is the checker the CUDA path is compared
+ * TEST INFRASTRUCTURE ONLY.  This file is the oracle the CUDA path is compared
  * with and the timed CPU baseline; nothing in the shipped library links, loads
  * or calls it.  Plain C (gcc, -O2 -ffp-contract=off -pthread).  Every function
  * names the reference file:line whose arithmetic it follows (paths are relative
